@@ -74,7 +74,22 @@ __device__ __forceinline__ void mse_candidate(int i, float grid, float mn, float
 __device__ __noinline__ void fit_group(const float* __restrict__ src, int n, int maxq, int sym,
                                        int mse_steps, float grid, float norm, float* scale, float* zero) {
   float mn = 0.f, mx = 0.f;
-  for (int t = 0; t < n; ++t) { const float v = src[t]; mn = fminf(mn, v); mx = fmaxf(mx, v); }
+  int t0 = 0;
+  // eight columns at a time in flight (the extrema do not depend on the order); the values of a
+  // group lie in the shared tile or in the matrix, 16-byte aligned in the usual shapes
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+    float mn4[4] = {0.f, 0.f, 0.f, 0.f}, mx4[4] = {0.f, 0.f, 0.f, 0.f};
+    for (; t0 + 8 <= n; t0 += 8) {
+      const float4 a = *reinterpret_cast<const float4*>(src + t0), b = *reinterpret_cast<const float4*>(src + t0 + 4);
+      mn4[0] = fminf(mn4[0], fminf(a.x, b.x)); mx4[0] = fmaxf(mx4[0], fmaxf(a.x, b.x));
+      mn4[1] = fminf(mn4[1], fminf(a.y, b.y)); mx4[1] = fmaxf(mx4[1], fmaxf(a.y, b.y));
+      mn4[2] = fminf(mn4[2], fminf(a.z, b.z)); mx4[2] = fmaxf(mx4[2], fmaxf(a.z, b.z));
+      mn4[3] = fminf(mn4[3], fminf(a.w, b.w)); mx4[3] = fmaxf(mx4[3], fmaxf(a.w, b.w));
+    }
+    mn = fminf(fminf(mn4[0], mn4[1]), fminf(mn4[2], mn4[3]));
+    mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+  }
+  for (int t = t0; t < n; ++t) { const float v = src[t]; mn = fminf(mn, v); mx = fmaxf(mx, v); }
   float s, z;
   params_from_range(mn, mx, maxq, sym, s, z);
   if (mse_steps > 0) {
@@ -111,6 +126,79 @@ __device__ __forceinline__ void apply_window(float4& t, const float* __restrict_
   }
 }
 
+// w[j] -= e * u[j] for the columns behind column i of the window (product and difference rounded)
+__device__ __forceinline__ void propagate(float (&w)[SUB], int i, float e, const float* __restrict__ urow) {
+  const float4* up = reinterpret_cast<const float4*>(urow);
+#pragma unroll
+  for (int j4 = (i + 1) / 4; j4 < SUB / 4; ++j4) {
+    const float4 u = up[j4];
+    if (4 * j4 + 0 > i) w[4 * j4 + 0] = __fsub_rn(w[4 * j4 + 0], __fmul_rn(e, u.x));
+    if (4 * j4 + 1 > i) w[4 * j4 + 1] = __fsub_rn(w[4 * j4 + 1], __fmul_rn(e, u.y));
+    if (4 * j4 + 2 > i) w[4 * j4 + 2] = __fsub_rn(w[4 * j4 + 2], __fmul_rn(e, u.z));
+    if (4 * j4 + 3 > i) w[4 * j4 + 3] = __fsub_rn(w[4 * j4 + 3], __fmul_rn(e, u.w));
+  }
+}
+
+// ---- the column step without divisions ------------------------------------------------------
+// What bounds a block of columns is the chain from one column of a row to the next: quotient,
+// rounding, quotient, update.  With two IEEE divisions and rintf it was about 440 cycles; the same
+// values come out of about 15 dependent additions and multiplications:
+//
+//  * rint(x / scale) from t = x * (1 / scale).  t and the rounded quotient both lie within
+//    3 * 2^-24 |t| of the true one, so they round to the same integer unless a half-integer is that
+//    near to t.  Such a column (and any non-finite t) makes the caller repeat the window with
+//    divisions.  Rounding to the nearest integer is the addition and subtraction of 1.5 * 2^23.
+//  * clamp(rint + zero, 0, maxq) - zero = clamp(rint, -zero, maxq - zero): all are integers below 2^24.
+//  * (x - dq) / u from the rounded reciprocal y of u: q1 = q0 + (r - q0 u) y is within one ulp of the
+//    quotient, and then q1 + (r - q1 u) y is the correctly rounded quotient (P. Markstein, Computation
+//    of elementary functions on the IBM RISC System/6000 processor, 1990, theorem 8.3), provided
+//    nothing over- or underflows: operands outside 2^-60 .. 2^60 also go the exact way.
+constexpr float SAFE_LO = 0x1p-60f, SAFE_HI = 0x1p60f;
+
+__device__ __forceinline__ float safe_reciprocal(float u) {
+  // NaN where the division-free step must not be used: it poisons the error, which is checked
+  return (u >= SAFE_LO && u <= SAFE_HI) ? __frcp_rn(u) : __int_as_float(0x7fffffff);
+}
+
+// One window of SUB columns of one row; false if it has to be repeated with divisions (w is not
+// changed in shared memory; codes and errors already stored are overwritten by the repetition).
+template <int NROWS>
+__device__ __forceinline__ bool fast_window(const float* __restrict__ wcols, const float* __restrict__ ublk,
+                                            const float* __restrict__ rdiag, float scale, float zero, float maxqf,
+                                            unsigned short* code_out, long long ldc, float* err_out, long long lde,
+                                            float (&er)[SUB]) {
+  constexpr float RINT = 12582912.f;   // 1.5 * 2^23
+  float w[SUB];
+#pragma unroll
+  for (int v = 0; v < SUB / 4; ++v) {
+    const float4 t = *reinterpret_cast<const float4*>(wcols + 4 * v);
+    w[4 * v] = t.x; w[4 * v + 1] = t.y; w[4 * v + 2] = t.z; w[4 * v + 3] = t.w;
+  }
+  const float rs = safe_reciprocal(scale);
+  const float lo = __fsub_rn(0.f, zero), hi = __fsub_rn(maxqf, zero);
+  bool bad = !(fabsf(zero) < 65536.f);
+#pragma unroll
+  for (int i = 0; i < SUB; ++i) {
+    const float x = w[i];
+    const float t = __fmul_rn(x, rs);
+    const float n = __fsub_rn(__fadd_rn(t, RINT), RINT);
+    bad |= !(__fmaf_rn(fabsf(t), 0x1p-21f, fabsf(__fsub_rn(t, n))) < 0.5f);
+    const float level = fminf(fmaxf(n, lo), hi);
+    const float r = __fsub_rn(x, __fmul_rn(scale, level));
+    bad |= (__float_as_uint(r) * 2u - 1u) < (__float_as_uint(SAFE_LO) * 2u - 1u);   // tiny and not zero
+    const float u = ublk[i * BLK + i], y = rdiag[i];
+    const float q0 = __fmul_rn(r, y);
+    const float q1 = __fmaf_rn(__fmaf_rn(-q0, u, r), y, q0);
+    const float e = __fmaf_rn(__fmaf_rn(-q1, u, r), y, q1);
+    bad |= !(fabsf(r) < SAFE_HI) || !(fabsf(e) < 0x1p120f);
+    er[i] = e;
+    code_out[i * ldc] = (unsigned short)__fadd_rn(level, zero);
+    err_out[i * lde] = e;
+    propagate(w, i, e, ublk + i * BLK);
+  }
+  return !bad;
+}
+
 // ALIGNED: every group starts on a multiple of SUB columns (per-channel, or a group size that is
 // a multiple of SUB), so the fit can only fall on the first column of a register window and the
 // other fifteen unrolled column steps carry no test and no call site for it.
@@ -121,7 +209,8 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
   constexpr bool HELPERS = WARPS <= 2;
   float* Us = sm;               // [BLK][BLK], upper triangle of the diagonal block of U
   float* Ws = sm + BLK * BLK;   // [NROWS][WS], block-entry values of the rows' columns
-  float* Es = Ws + NROWS * WS;  // [2][SUB][NROWS] errors of the last two windows (helpers only)
+  float* rdiag = Ws + NROWS * WS;   // [BLK] reciprocals of U's diagonal
+  float* Es = rdiag + BLK;          // [2][SUB][NROWS] errors of the last two windows (helpers only)
   const int tid = threadIdx.x;
   const int row0 = blockIdx.x * NROWS;
   const int count = a.count, i1 = a.i1;
@@ -158,6 +247,10 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
       Ws[r * WS + c] = (row0 + r < a.out && c < count) ? a.Wf[(long long)(row0 + r) * a.ldw + i1 + c] : 0.f;
     }
   }
+  if (ALIGNED) {
+    __syncthreads();
+    if (tid < BLK) rdiag[tid] = safe_reciprocal(Us[tid * BLK + tid]);
+  }
   __syncthreads();
 
   const int row = row0 + tid;
@@ -185,46 +278,51 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
   const int hrow = (tid - NROWS) % NROWS, gsel = (tid - NROWS) / NROWS;
   const bool helper = helped && tid >= NROWS && gsel < NSEL;
 
+  // parameters of the group that starts at column i1 + ci of the row
+  auto open_group = [&](int ci) {
+    const int col = i1 + ci, n = min(gs, a.d - col);
+    // the shared tile is still pristine only at the very first column of the block
+    fit_group((ci == 0 && n <= count) ? wrow : grow + col, n, a.maxq, a.sym, a.mse_steps, a.mse_grid,
+              a.mse_norm, &scale, &zero);
+    const long long g = col / gs;
+    a.scales[g * a.out + row] = scale;
+    a.zeros[g * a.out + row] = zero;
+  };
+
   for (int cb = 0; cb < count; cb += SUB) {
     float* es_buf = Es + ((cb / SUB) & 1) * SUB * NROWS;
     if (owner) {
-      float w[SUB], er[SUB];
-#pragma unroll
-      for (int v = 0; v < SUB / 4; ++v) {
-        const float4 t = *reinterpret_cast<const float4*>(wrow + cb + 4 * v);
-        w[4 * v] = t.x; w[4 * v + 1] = t.y; w[4 * v + 2] = t.z; w[4 * v + 3] = t.w;
+      float er[SUB];
+      bool exact = !ALIGNED || cb + SUB > count;
+      if (ALIGNED) {
+        if (gs != -1 && (i1 + cb) % gs == 0) open_group(cb);
+        if (!exact)
+          exact = !fast_window<NROWS>(wrow + cb, Us + cb * BLK + cb, rdiag + cb, scale, zero, maxqf,
+                                      code_out + (long long)cb * a.out, a.out, err_out + (long long)cb * a.lde,
+                                      a.lde, er);
       }
+      if (exact) {
+        float w[SUB];
 #pragma unroll
-      for (int i = 0; i < SUB; ++i) {
-        const int ci = cb + i;
-        er[i] = 0.f;
-        if (ci < count) {
-          const int col = i1 + ci;
-          if ((!ALIGNED || i == 0) && gs != -1 && col % gs == 0) {
-            const int n = min(gs, a.d - col);
-            // the shared tile is still pristine only at the very first column of the block
-            fit_group((ci == 0 && n <= count) ? wrow : grow + col, n, a.maxq, a.sym, a.mse_steps,
-                      a.mse_grid, a.mse_norm, &scale, &zero);
-            const int g = col / gs;
-            a.scales[(long long)g * a.out + row] = scale;
-            a.zeros[(long long)g * a.out + row] = zero;
-          }
-          const float x = w[i];
-          float q = __fadd_rn(rintf(__fdiv_rn(x, scale)), zero);
-          q = fminf(fmaxf(q, 0.f), maxqf);
-          const float dq = __fmul_rn(scale, __fsub_rn(q, zero));
-          const float e = __fdiv_rn(__fsub_rn(x, dq), Us[ci * BLK + ci]);
-          er[i] = e;
-          code_out[(long long)ci * a.out] = (unsigned short)q;
-          err_out[(long long)ci * a.lde] = e;
-          const float4* up = reinterpret_cast<const float4*>(Us + ci * BLK + cb);
+        for (int v = 0; v < SUB / 4; ++v) {
+          const float4 t = *reinterpret_cast<const float4*>(wrow + cb + 4 * v);
+          w[4 * v] = t.x; w[4 * v + 1] = t.y; w[4 * v + 2] = t.z; w[4 * v + 3] = t.w;
+        }
 #pragma unroll
-          for (int j4 = (i + 1) / 4; j4 < SUB / 4; ++j4) {
-            const float4 u = up[j4];
-            if (4 * j4 + 0 > i) w[4 * j4 + 0] = __fsub_rn(w[4 * j4 + 0], __fmul_rn(e, u.x));
-            if (4 * j4 + 1 > i) w[4 * j4 + 1] = __fsub_rn(w[4 * j4 + 1], __fmul_rn(e, u.y));
-            if (4 * j4 + 2 > i) w[4 * j4 + 2] = __fsub_rn(w[4 * j4 + 2], __fmul_rn(e, u.z));
-            if (4 * j4 + 3 > i) w[4 * j4 + 3] = __fsub_rn(w[4 * j4 + 3], __fmul_rn(e, u.w));
+        for (int i = 0; i < SUB; ++i) {
+          const int ci = cb + i;
+          er[i] = 0.f;
+          if (ci < count) {
+            if (!ALIGNED && gs != -1 && (i1 + ci) % gs == 0) open_group(ci);
+            const float x = w[i];
+            float q = __fadd_rn(rintf(__fdiv_rn(x, scale)), zero);
+            q = fminf(fmaxf(q, 0.f), maxqf);
+            const float dq = __fmul_rn(scale, __fsub_rn(q, zero));
+            const float e = __fdiv_rn(__fsub_rn(x, dq), Us[ci * BLK + ci]);
+            er[i] = e;
+            code_out[(long long)ci * a.out] = (unsigned short)q;
+            err_out[(long long)ci * a.lde] = e;
+            propagate(w, i, e, Us + ci * BLK + cb);
           }
         }
       }
@@ -474,7 +572,7 @@ __global__ void unpermute_outputs_kernel(const unsigned short* __restrict__ code
 template <int WARPS, bool ALIGNED>
 int launch_block_t(const ColArgs& a, cudaStream_t stream) {
   // tiles, plus the error windows the helper threads read (only CTAs with few rows have helpers)
-  const int smem = (BLK * BLK + WARPS * 32 * WS + (WARPS <= 2 ? 2 * SUB * WARPS * 32 : 0)) * (int)sizeof(float);
+  const int smem = (BLK * BLK + WARPS * 32 * WS + BLK + (WARPS <= 2 ? 2 * SUB * WARPS * 32 : 0)) * (int)sizeof(float);
   OC_OPT_IN_SMEM((gptq_block_kernel<WARPS, ALIGNED>), smem);
   gptq_block_kernel<WARPS, ALIGNED><<<dim3(oc_div_up(a.out, WARPS * 32), a.batch), LOADERS, smem, stream>>>(a);
   OC_CHECK_LAUNCH();
