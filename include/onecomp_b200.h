@@ -241,6 +241,14 @@ int oc_dequantize_packed(const int* qweight, const int* qzeros, const void* scal
                          const int* g_idx, int out, int d, int bits, void* w16, long long ldw,
                          void* stream);
 
+/* y[tokens, out] = x[tokens, d] * W^T (+ bias): fp16 in and out, fp32 sums, W decoded from the packed
+ * layout on the fly (the values of oc_dequantize_packed).  1..16 tokens, rows of x contiguous; d a multiple
+ * of 8; qweight, x and g_idx 16-byte aligned.  g_idx (entries below `groups`) NULL = one group; bias16 may be NULL.
+ * (reference: GPTQLinear.forward, onecomp/quantizer/gptq/gptq_layer.py:576-628) */
+int oc_packed_linear(const int* qweight, const int* qzeros, const void* scales16, const int* g_idx,
+                     int out, int d, int groups, int bits, const void* x16, int tokens, const void* bias16,
+                     void* y16, int sm_count, void* stream);
+
 /* fp32 GEMM engine: C = beta*C + alpha*opA(A)*opB(B); transX = 1 means the operand is
  * stored transposed ([K,M] / [N,K]); flags: see OC_GEMM_* in csrc/common.cuh (0 = dense). */
 int oc_gemm_f32(const float* A, long long lda, const float* B, long long ldb, float* C,

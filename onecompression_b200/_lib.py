@@ -42,6 +42,7 @@ SIGNATURES = {
     "oc_pack_qzeros": (_I, [_P, _I, _I, _I, _I, _P, _P]),
     "oc_unpack_qzeros": (_I, [_P, _I, _I, _I, _I, _P, _P]),
     "oc_dequantize_packed": (_I, [_P, _P, _P, _P, _I, _I, _I, _P, _L, _P]),
+    "oc_packed_linear": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _P, _I, _P, _P, _I, _P]),
     "oc_gemm_f32": (_I, [_P, _L, _P, _L, _P, _L, _I, _I, _I, _F, _F, _I, _I, _I, _P]),
     "oc_set_gemm_engine": (_I, [_I]),
     "oc_set_gemm_tile_shape": (_I, [_I]),
@@ -98,4 +99,4 @@ def ptr(t):
 def stream_handle():
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())

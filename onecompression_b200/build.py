@@ -29,6 +29,7 @@ SOURCES = {
     "moment_tc2.cu": [],
     "moment_noalloc.cu": [],
     "pack.cu": [],
+    "packed_linear.cu": [],
     "qep.cu": [],
     "rtn.cu": ["-fmad=false"],
     "rmsnorm.cu": [],

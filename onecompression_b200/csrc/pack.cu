@@ -76,41 +76,77 @@ __global__ void unpack_axis_kernel(const int* __restrict__ in, long long in_stri
 }
 
 // W^[r][c] = fp16( float(scale16[g][r]) * (q - zero) ), g = g_idx[c]; zero = (stored + 1) & mask
-__global__ void dequant_packed_kernel(const int* __restrict__ qweight, const int* __restrict__ qzeros,
-                                      const __half* __restrict__ scales, const int* __restrict__ g_idx,
-                                      int out, int d, int bits, long long ldz,
-                                      __half* __restrict__ w, long long ldw) {
-  __shared__ float t[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const unsigned mask = (1u << bits) - 1u;
-  for (int k = ty; k < 32; k += 8) {
-    const int c = c0 + k, r = r0 + tx;
-    if (c < d && r < out) {
-      unsigned q, z;
-      const int g = g_idx ? g_idx[c] : 0;
-      if (bits == 3) {
-        unsigned wq[3], wz[3];
-        for (int s = 0; s < 3; ++s) {
-          wq[s] = (unsigned)qweight[(long long)((c / 32) * 3 + s) * out + r];
-          wz[s] = (unsigned)qzeros[(long long)g * ldz + (r / 32) * 3 + s];
+//
+// Bound by HBM: bits / 8 bytes in and two out per weight.  A CTA makes 64 rows x 128 columns: a thread
+// decodes 32 columns of one row (neighbouring lanes hold neighbouring rows, so the packed words,
+// scales and zero points load coalesced; each word is read once, and scale and zero only where the
+// group changes from one column to the next), and the tile leaves through shared memory in
+// 256-byte row segments.  14336 x 4096, 4 bits: 306 us with one word, scale and zero load per weight,
+// 56 us now (2.6 TB/s; the caller's launch and L2 flush included).
+constexpr int DQ_ROWS = 64, DQ_COLS = 128, DQ_PITCH = DQ_COLS + 8;   // pitch: 16-byte accesses without conflicts
+template <int BITS>
+__global__ void __launch_bounds__(256) dequant_packed_kernel(const int* __restrict__ qweight,
+                                                             const int* __restrict__ qzeros,
+                                                             const __half* __restrict__ scales,
+                                                             const int* __restrict__ g_idx, int out, int d,
+                                                             long long ldz, __half* __restrict__ w, long long ldw) {
+  constexpr unsigned MASK = (1u << BITS) - 1u;
+  __shared__ __align__(16) __half tile[DQ_ROWS * DQ_PITCH];
+  const int tid = threadIdx.x, lr = tid % DQ_ROWS, lc = tid / DQ_ROWS * 32;
+  const int r = blockIdx.y * DQ_ROWS + lr, c0 = blockIdx.x * DQ_COLS + lc;
+  if (r < out && c0 < d) {
+    unsigned v[BITS];
+    const long long w0 = (long long)c0 / 32 * BITS;
+    const int words = min(BITS, (int)((long long)(d - c0) * BITS / 32));   // d is a multiple of the pack factor
+#pragma unroll
+    for (int j = 0; j < BITS; ++j) v[j] = j < words ? (unsigned)qweight[(w0 + j) * out + r] : 0u;
+    int group = -1;
+    float s = 0.f, z = 0.f;
+#pragma unroll
+    for (int k8 = 0; k8 < 4; ++k8) {
+      __align__(16) __half h[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = k8 * 8 + i, c = c0 + k, bit = k * BITS, wi = bit >> 5, off = bit & 31;
+        if (c < d) {
+          const int g = g_idx ? g_idx[c] : 0;
+          if (g != group) {
+            group = g;
+            s = __half2float(scales[(long long)g * out + r]);
+            unsigned zq;
+            if (BITS == 3) {
+              const int zb = 3 * (r & 31), zw = zb >> 5, zo = zb & 31;
+              const int* zr = qzeros + (long long)g * ldz + (r / 32) * 3;
+              zq = (unsigned)zr[zw] >> zo;
+              if (zo + 3 > 32) zq |= (unsigned)zr[zw + 1] << (32 - zo);
+            } else {
+              constexpr int F = 32 / (BITS == 3 ? 4 : BITS);
+              zq = (unsigned)qzeros[(long long)g * ldz + r / F] >> ((r % F) * BITS);
+            }
+            z = (float)(((zq & MASK) + 1u) & MASK);
+          }
+          unsigned q = v[wi] >> off;
+          if (off + BITS > 32) q |= v[wi + 1 < BITS ? wi + 1 : wi] << (32 - off);
+          h[i] = __float2half_rn(s * ((float)(q & MASK) - z));
+        } else {
+          h[i] = __ushort_as_half(0);
         }
-        q = unpack3(wq, c % 32);
-        z = unpack3(wz, r % 32);
-      } else {
-        const int f = 32 / bits;
-        q = ((unsigned)qweight[(long long)(c / f) * out + r] >> ((c % f) * bits)) & mask;
-        z = ((unsigned)qzeros[(long long)g * ldz + r / f] >> ((r % f) * bits)) & mask;
       }
-      z = (z + 1u) & mask;
-      const float s = __half2float(scales[(long long)g * out + r]);
-      t[k][tx] = s * ((float)q - (float)z);
+      *reinterpret_cast<uint4*>(tile + lr * DQ_PITCH + lc + k8 * 8) = *reinterpret_cast<const uint4*>(h);
     }
   }
   __syncthreads();
-  for (int k = ty; k < 32; k += 8) {
-    const int r = r0 + k, c = c0 + tx;
-    if (c < d && r < out) w[(long long)r * ldw + c] = __float2half_rn(t[tx][k]);
+  const bool vec = (ldw % 8 == 0) && ((reinterpret_cast<uintptr_t>(w) & 15) == 0);
+#pragma unroll
+  for (int it = 0; it < DQ_ROWS * DQ_COLS / 8 / 256; ++it) {
+    const int e = it * 256 + tid, row = e / (DQ_COLS / 8), c8 = e % (DQ_COLS / 8) * 8;
+    const int rr = blockIdx.y * DQ_ROWS + row, c = blockIdx.x * DQ_COLS + c8;
+    if (rr >= out || c >= d) continue;
+    const __half* src = tile + row * DQ_PITCH + c8;
+    __half* dst = w + (long long)rr * ldw + c;
+    if (vec && c + 8 <= d) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+    else
+      for (int i = 0; i < 8 && c + i < d; ++i) dst[i] = src[i];
   }
 }
 
@@ -176,8 +212,17 @@ extern "C" int oc_dequantize_packed(const int* qweight, const int* qzeros, const
   OC_REQUIRE(qweight && qzeros && scales16 && w16 && out > 0 && d > 0 && ldw >= d, "dequantize_packed: bad arguments");
   OC_REQUIRE(d % f == 0 && out % f == 0, "dequantize_packed: shape not divisible by the pack factor");
   const long long ldz = (bits == 3) ? out / 32 * 3 : out / f;
-  dequant_packed_kernel<<<dim3(oc_div_up(d, 32), oc_div_up(out, 32)), dim3(32, 8), 0, (cudaStream_t)stream>>>(
-      qweight, qzeros, (const __half*)scales16, g_idx, out, d, bits, ldz, (__half*)w16, ldw);
+  OC_REQUIRE(oc_div_up(out, DQ_ROWS) <= 65535, "dequantize_packed: too many rows");
+  const dim3 grid(oc_div_up(d, DQ_COLS), oc_div_up(out, DQ_ROWS));
+  cudaStream_t s = (cudaStream_t)stream;
+  const __half* sc = (const __half*)scales16;
+  __half* w = (__half*)w16;
+  switch (bits) {
+    case 2: dequant_packed_kernel<2><<<grid, 256, 0, s>>>(qweight, qzeros, sc, g_idx, out, d, ldz, w, ldw); break;
+    case 3: dequant_packed_kernel<3><<<grid, 256, 0, s>>>(qweight, qzeros, sc, g_idx, out, d, ldz, w, ldw); break;
+    case 4: dequant_packed_kernel<4><<<grid, 256, 0, s>>>(qweight, qzeros, sc, g_idx, out, d, ldz, w, ldw); break;
+    default: dequant_packed_kernel<8><<<grid, 256, 0, s>>>(qweight, qzeros, sc, g_idx, out, d, ldz, w, ldw);
+  }
   OC_CHECK_LAUNCH();
   return OC_OK;
 }

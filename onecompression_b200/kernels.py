@@ -25,7 +25,7 @@ _sm_count_cache: dict[int, int] = {}
 
 
 def sm_count(device) -> int:
-    idx = torch.device(device).index
+    idx = device if isinstance(device, int) else torch.device(device).index
     if idx is None:
         idx = torch.cuda.current_device()
     if idx not in _sm_count_cache:
@@ -567,6 +567,48 @@ def dequantize_packed(qweight, qzeros, scales, g_idx, wbits: int, shape) -> torc
         call("oc_dequantize_packed", ptr(qweight), ptr(qzeros), ptr(scales), ptr(g_idx), out, d,
              wbits, ptr(w), d, stream_handle())
     return w
+
+
+# Up to this many tokens the packed weight is decoded inside the product.
+PACKED_LINEAR_TOKENS = 16
+
+
+def packed_linear(x: torch.Tensor, qweight, qzeros, scales, g_idx, bias, wbits: int, out: int, d: int):
+    """x Wᵀ (+ bias) for at most ``PACKED_LINEAR_TOKENS`` tokens, W [out, d] decoded from the packed
+    layout inside the product.  None when the kernel does not take these tensors as they are (type,
+    layout, alignment, token count): dequantize and multiply then."""
+    # (a decode step makes hundreds of these calls, each a few microseconds on the GPU: the checks are
+    # written for little host time)
+    if x.dtype != torch.float16 or not x.is_cuda or x.dim() == 0 or x.shape[-1] != d or not x.is_contiguous():
+        return None
+    tokens = x.numel() // d
+    dev = x.get_device()
+    groups = scales.shape[0]
+    f = 32 if wbits == 3 else 32 // wbits
+    if (tokens < 1 or tokens > PACKED_LINEAR_TOKENS or d % 8 or d > 65536 or groups >= 65535 or d % f or out % f
+            or qweight.dtype != torch.int32 or qzeros.dtype != torch.int32 or g_idx.dtype != torch.int32
+            or scales.dtype != torch.float16
+            or qweight.get_device() != dev or qzeros.get_device() != dev or scales.get_device() != dev
+            or g_idx.get_device() != dev
+            or qweight.shape != (d * wbits // 32, out) or qzeros.shape != (groups, out * wbits // 32)
+            or scales.shape != (groups, out) or g_idx.shape != (d,)
+            or not (qweight.is_contiguous() and qzeros.is_contiguous() and scales.is_contiguous()
+                    and g_idx.is_contiguous())):
+        return None
+    px, pq, pg, ps = x.data_ptr(), qweight.data_ptr(), g_idx.data_ptr(), scales.data_ptr()
+    if (px | pq | pg) & 15 or ps & 7:
+        return None
+    if bias is not None and (bias.dtype != torch.float16 or bias.get_device() != dev or bias.shape != (out,)
+                             or not bias.is_contiguous()):
+        return None
+    y = x.new_empty((*x.shape[:-1], out))
+    args = (pq, qzeros.data_ptr(), ps, pg, out, d, groups, wbits, px, tokens, ptr(bias), y.data_ptr(), sm_count(dev))
+    if dev == torch.cuda.current_device():
+        call("oc_packed_linear", *args, stream_handle())
+    else:
+        with torch.cuda.device(dev):
+            call("oc_packed_linear", *args, stream_handle())
+    return y
 
 
 def rmsnorm_f16(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:

@@ -10,6 +10,7 @@ from __future__ import annotations
 from typing import Optional, Tuple, Union
 
 import torch
+from torch.autograd import forward_ad
 
 from ... import kernels
 
@@ -80,7 +81,8 @@ class GPTQLinear(torch.nn.Module):
     ``qzeros`` int32 (G, out·bits/32) holding (zero − 1) & mask, ``scales`` fp16 (G, out),
     ``g_idx`` int32 (in,), optional ``bias`` fp16.  Bit widths without a packed layout keep
     ``qweight`` (out, in) and ``qzeros`` (G, out) as plain integers.  ``forward`` dequantizes on
-    the GPU (one kernel for the packed layout) and applies the linear map.
+    the GPU (one kernel for the packed layout) and applies the linear map; for a few tokens both are
+    one kernel.
     """
 
     def __init__(self, in_features, out_features, wbits, groupsize, actorder, quantized_weight, scale,
@@ -147,7 +149,24 @@ class GPTQLinear(torch.nn.Module):
         w = self.scales[g, :].T.float() * (self.qweight.float() - zeros[g, :].T.float())
         return w.to(torch.float16)
 
+    def _decoded_in_product(self, x):
+        """The layer as one kernel, for a plain call on a few tokens; None otherwise.  Whatever watches
+        or transforms the operators of the forward pass (autograd, autocast, function transforms,
+        tracing, dispatch modes) keeps the dequantized weight and ``linear``."""
+        if (not self._weight_is_packed or type(x) is not torch.Tensor
+                or (x.requires_grad and torch.is_grad_enabled()) or forward_ad._current_level >= 0
+                or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling()
+                or torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack()
+                or torch._C._functorch.peek_interpreter_stack() is not None):
+            return None
+        b = self._buffers
+        return kernels.packed_linear(x, b["qweight"], b["qzeros"], b["scales"], b["g_idx"], b.get("bias"),
+                                     self.wbits, self.out_features, self.in_features)
+
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        y = self._decoded_in_product(x)
+        if y is not None:
+            return y
         w = self.dequantized_weight().to(x.dtype)
         b = self.bias.to(x.dtype) if self.bias is not None else None
         return torch.nn.functional.linear(x, w, b)

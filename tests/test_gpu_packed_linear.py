@@ -1,0 +1,69 @@
+"""The packed layer: decoding kernel and the product that decodes on the fly."""
+
+import pytest
+import torch
+from torch.autograd import forward_ad
+
+pytestmark = pytest.mark.gpu
+
+
+def layer(out, d, bits, gs, act, bias, seed=0):
+    from onecompression_b200.quantizer.gptq.gptq_layer import GPTQLinear
+
+    g = torch.Generator().manual_seed(seed)
+    groups = 1 if gs == -1 else (d + gs - 1) // gs
+    codes = torch.randint(0, 2 ** bits, (out, d), generator=g, dtype=torch.int32)
+    scale = (0.5 + torch.rand(groups, out, generator=g)).half() * 0.01
+    zero = torch.randint(1, 2 ** bits, (groups, out), generator=g, dtype=torch.int32)
+    perm = torch.randperm(d, generator=g) if act else None
+    b = torch.randn(out, generator=g).half() if bias else None
+    m = GPTQLinear(d, out, bits, gs, act, codes, scale, zero, perm=perm, bias=b)
+    order = perm if act else torch.arange(d)
+    grp = torch.empty(d, dtype=torch.long)
+    grp[order] = torch.arange(d) // (d if gs == -1 else gs)
+    w = (scale.float()[grp].t() * (codes.float() - zero.float()[grp].t())).half()
+    return m, w
+
+
+# out: less than a tile of rows, a tile and a rest; d: one unit, less than a share per warp, a rest of 32
+@pytest.mark.parametrize("bits,out,d", [(4, 8, 8), (4, 72, 1048), (4, 136, 4096), (2, 48, 2064), (2, 16, 16),
+                                        (3, 32, 32), (3, 96, 1056), (8, 4, 8), (8, 100, 520), (8, 68, 1028)])
+@pytest.mark.parametrize("gs,act", [(-1, False), (32, False), (128, True), (24, False), (8, True)])
+def test_packed_linear(bits, out, d, gs, act):
+    from onecompression_b200 import kernels as K
+
+    for bias in (False, True):
+        m, w = layer(out, d, bits, gs, act, bias)
+        assert torch.equal(m.dequantized_weight().cpu(), w)
+        for tokens in (1, 7, 8, 9, 16, 17):
+            x = torch.randn(tokens, d, generator=torch.Generator().manual_seed(tokens)).half()
+            want = x.double() @ w.double().t() + (m.bias.double().cpu() if bias else 0)
+            taken = m._decoded_in_product(x.cuda()) is not None
+            assert taken == (tokens <= K.PACKED_LINEAR_TOKENS and d % 8 == 0)
+            got = m(x.cuda()).cpu().double()
+            # fp32 sums of d products (d * 2^-24 of the sum of magnitudes) and one rounding to fp16
+            bound = d * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + 2.0 ** -11 * want.abs() + 2.0 ** -25
+            assert ((got - want).abs() <= bound).all()
+
+
+def test_packed_linear_keeps_the_general_path():
+    """Gradients, function transforms, autocast and unaligned or strided inputs go the way they went."""
+    m, w = layer(64, 256, 4, 64, False, False)
+    x = torch.randn(4, 256, device="cuda").half()
+    assert m._decoded_in_product(x) is not None
+    y = m(x)
+    xg = x.clone().requires_grad_()
+    m(xg).sum().backward()
+    assert torch.allclose(xg.grad.float(), w.cuda().float().sum(0).expand(4, -1), rtol=1e-2, atol=1e-2)
+    assert torch.allclose(torch.func.vmap(m)(x.unsqueeze(1)).squeeze(1), y, rtol=1e-2, atol=1e-2)
+    with forward_ad.dual_level():
+        tangent = forward_ad.unpack_dual(m(forward_ad.make_dual(x, x))).tangent
+    assert torch.allclose(tangent, y, rtol=1e-2, atol=1e-2)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert m(x).dtype == torch.bfloat16
+    wide = torch.zeros(4, 264, device="cuda").half()
+    for view in (wide[:, 4:260], wide[:, :256]):
+        view.copy_(x)
+        assert m._decoded_in_product(view) is None
+        assert torch.allclose(m(view), y, rtol=1e-2, atol=1e-2)
+    assert m(x[:0]).shape == (0, 64)
