@@ -385,12 +385,19 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
 // ---- preparation: fp16 -> fp32, act-order gather, dead columns, per-channel parameters ----
 // Wf[r][j] = dead[perm[j]] ? 0 : float(W[r][perm[j]]).  Per-channel scale / zero are fitted on
 // the whole original row before dead columns are zeroed (reference :690-695).
-__global__ void gptq_prepare_kernel(const void* __restrict__ W, int bf16, long long ldw_in, int out, int d,
-                                    const int* __restrict__ perm, const unsigned char* __restrict__ dead,
-                                    float* __restrict__ Wf, long long ldw, int per_channel, int maxq,
-                                    int sym, int mse_steps, float mse_grid, float mse_norm,
-                                    float* __restrict__ scales, float* __restrict__ zeros,
-                                    long long s_win, long long s_wf, long long s_par) {
+//
+// One CTA per row, bound by HBM (2 bytes in, 4 out per weight).  The row is read in order, eight
+// weights a thread, and with act-order passes through shared memory (`staged`: d floats), where the
+// permutation is a gather on chip instead of one 2-byte global access per weight.  28672 x 4096:
+// 313 us one weight per access, 106 us now; 4096 x 14336 with act-order 204, 107 us.
+__global__ void __launch_bounds__(256)
+gptq_prepare_kernel(const void* __restrict__ W, int bf16, long long ldw_in, int out, int d,
+                    const int* __restrict__ perm, const unsigned char* __restrict__ dead,
+                    float* __restrict__ Wf, long long ldw, int per_channel, int maxq,
+                    int sym, int mse_steps, float mse_grid, float mse_norm,
+                    float* __restrict__ scales, float* __restrict__ zeros,
+                    long long s_win, long long s_wf, long long s_par, int vec, int staged) {
+  extern __shared__ __align__(16) float row_s[];
   const int row = blockIdx.x;
   {
     const long long b = blockIdx.y;      // problem of a batch
@@ -402,11 +409,53 @@ __global__ void gptq_prepare_kernel(const void* __restrict__ W, int bf16, long l
   const long long src0 = (long long)row * ldw_in;
   float* dst = Wf + (long long)row * ldw;
   float mn = 0.f, mx = 0.f;
-  for (int j = threadIdx.x; j < d; j += blockDim.x) {
-    const int pj = perm ? perm[j] : j;
-    const float v = oc_ld16(W, src0 + pj, bf16);
-    mn = fminf(mn, v); mx = fmaxf(mx, v);
-    dst[j] = (dead && dead[pj]) ? 0.f : v;
+  if (perm && !staged) {
+    for (int j = threadIdx.x; j < d; j += blockDim.x) {
+      const int pj = perm[j];
+      const float v = oc_ld16(W, src0 + pj, bf16);
+      mn = fminf(mn, v); mx = fmaxf(mx, v);
+      dst[j] = (dead && dead[pj]) ? 0.f : v;
+    }
+  } else {
+    float* to = perm ? row_s : dst;
+    if (vec) {          // d, ldw_in multiples of 8, 16-byte aligned rows (dead: 8-byte)
+      for (int j = threadIdx.x * 8; j < d; j += blockDim.x * 8) {
+        const uint4 p = *reinterpret_cast<const uint4*>(static_cast<const char*>(W) + (src0 + j) * 2);
+        const uint2 dd = dead ? *reinterpret_cast<const uint2*>(dead + j) : make_uint2(0u, 0u);
+        const unsigned h[4] = {p.x, p.y, p.z, p.w}, dw[2] = {dd.x, dd.y};
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = bf16 ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&h[k]))
+                                : __half22float2(*reinterpret_cast<const __half2*>(&h[k]));
+          v[2 * k] = f.x; v[2 * k + 1] = f.y;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          mn = fminf(mn, v[k]); mx = fmaxf(mx, v[k]);
+          if ((dw[k >> 2] >> (8 * (k & 3))) & 0xffu) v[k] = 0.f;
+        }
+        *reinterpret_cast<float4*>(to + j) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4*>(to + j + 4) = make_float4(v[4], v[5], v[6], v[7]);
+      }
+    } else {
+      for (int j = threadIdx.x; j < d; j += blockDim.x) {
+        const float v = oc_ld16(W, src0 + j, bf16);
+        mn = fminf(mn, v); mx = fmaxf(mx, v);
+        to[j] = (dead && dead[j]) ? 0.f : v;
+      }
+    }
+    if (perm) {
+      __syncthreads();
+      if (vec && (reinterpret_cast<uintptr_t>(perm) & 15) == 0) {
+        for (int j = threadIdx.x * 4; j < d; j += blockDim.x * 4) {
+          const int4 q = *reinterpret_cast<const int4*>(perm + j);
+          *reinterpret_cast<float4*>(dst + j) = make_float4(row_s[q.x], row_s[q.y], row_s[q.z], row_s[q.w]);
+        }
+      } else {
+        for (int j = threadIdx.x; j < d; j += blockDim.x) dst[j] = row_s[perm[j]];
+      }
+    }
   }
   if (!per_channel) return;
   __shared__ float smn[32], smx[32], bc[4];
@@ -463,38 +512,6 @@ __device__ __forceinline__ void pack3(const unsigned (&v)[32], unsigned (&w)[3])
   }
 }
 
-// qweight[pr][r]: codes of original columns pr*f .. pr*f+f-1 (3 bit: 32 columns -> 3 words)
-__global__ void pack_qweight_kernel(const unsigned short* __restrict__ codesT, int out, int d,
-                                    const int* __restrict__ invperm, int bits,
-                                    int* __restrict__ qweight, long long ldq) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= out) return;
-  const unsigned mask = (1u << bits) - 1u;
-  if (bits == 3) {
-    const int c0 = blockIdx.y * 32;
-    unsigned v[32], w[3];
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      const int c = c0 + k;
-      const int j = invperm ? invperm[c] : c;
-      v[k] = codesT[(long long)j * out + r] & mask;
-    }
-    pack3(v, w);
-#pragma unroll
-    for (int t = 0; t < 3; ++t) qweight[(long long)(blockIdx.y * 3 + t) * ldq + r] = (int)w[t];
-  } else {
-    const int f = 32 / bits;
-    const int c0 = blockIdx.y * f;
-    unsigned word = 0u;
-    for (int k = 0; k < f; ++k) {
-      const int c = c0 + k;
-      const int j = invperm ? invperm[c] : c;
-      word |= ((unsigned)codesT[(long long)j * out + r] & mask) << (k * bits);
-    }
-    qweight[(long long)blockIdx.y * ldq + r] = (int)word;
-  }
-}
-
 // qzeros[g][w]: (zero - 1) & mask of rows w*f .. w*f+f-1 (3 bit: 32 rows -> 3 words)
 __global__ void pack_qzeros_kernel(const float* __restrict__ zeros, int out, int G, int bits,
                                    int* __restrict__ qzeros, long long ldz) {
@@ -532,41 +549,162 @@ __global__ void cast_params_kernel(const float* __restrict__ scales, const float
   if (zeros_i32) zeros_i32[(long long)g * lds + r] = (int)zeros[(long long)g * out + r];
 }
 
-// Original-order outputs through a 32x32 transpose: integer codes [out][d] and the fp16
+// Original-order outputs in one pass over the codes: packed words, integer codes [out][d] and the
 // dequantised weight  fp16( float(fp16(scale)) * (q - zero) )  (reference :153-168).
-__global__ void unpermute_outputs_kernel(const unsigned short* __restrict__ codesT, int out, int d,
-                                         const int* __restrict__ invperm, int gs,
-                                         const float* __restrict__ scales, const float* __restrict__ zeros,
-                                         int* __restrict__ codes, long long ldc,
-                                         void* __restrict__ what, long long ldwh, int bf16) {
-  __shared__ unsigned short tq[32][33];
-  __shared__ float tv[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  for (int k = ty; k < 32; k += 8) {
-    const int c = c0 + k, r = r0 + tx;
-    if (c < d && r < out) {
-      const int j = invperm ? invperm[c] : c;
-      const int g = (gs == -1) ? 0 : j / gs;
-      const unsigned short q = codesT[(long long)j * out + r];
-      tq[k][tx] = q;
-      const float s = __half2float(__float2half_rn(scales[(long long)g * out + r]));
-      tv[k][tx] = __fmul_rn(s, __fsub_rn((float)q, zeros[(long long)g * out + r]));
-    }
+//
+// Bound by HBM: 2 bytes of code in, bits / 8 + 2 out per weight.  A CTA takes 64 rows x 128 columns of
+// the original order, a warp 32 of the columns, a lane two neighbouring rows: a lane sees whole packed
+// words of its rows, reads the codes coalesced along the rows, and reads scale and zero point only
+// where the group changes.  The row-major outputs leave through shared memory, a row segment of 128
+// bytes a warp.  Packing and dequantising read the codes separately before: 28672 x 4096, 4 bits:
+// 151 + 387 us, 215 us now; 4096 x 4096, 3 bits: 11 + 55, 34 us.
+constexpr int FIN_ROWS = 64, FIN_COLS = 128;
+// Two neighbouring columns of a row share a 4-byte word of the tile.  Writers of a warp hold every other
+// row: 65 words apart, shifted by one in the second half, all 32 fall into different banks.
+constexpr int FIN_PITCH = FIN_COLS / 2 + 1, FIN_TILE = FIN_ROWS * FIN_PITCH + 1;
+__device__ __forceinline__ int fin_at(int row, int col) { return row * FIN_PITCH + (row >> 5) + (col >> 1); }
+struct FinishArgs {
+  const unsigned short* codesT; int out, d; const int* invperm; int gs;
+  const float* scales; const float* zeros;
+  int* qweight; long long ldq; int* codes; long long ldc; void* what; long long ldwh; int bf16;
+  long long s_codes, s_par, s_qw, s_out, s_what;   // strides between the problems of a batch
+};
+template <int BITS>   // 0: nothing is packed
+__global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
+  extern __shared__ unsigned fin_s[];        // one tile per row-major output
+  unsigned* tw = fin_s;
+  unsigned* tq = fin_s + (a.what ? FIN_TILE : 0);
+  {
+    const long long b = blockIdx.z;
+    a.codesT += b * a.s_codes; a.scales += b * a.s_par; a.zeros += b * a.s_par;
+    if (a.invperm) a.invperm += b * a.d;
+    if (a.qweight) a.qweight += b * a.s_qw;
+    if (a.codes) a.codes += b * a.s_out;
+    if (a.what) a.what = static_cast<char*>(a.what) + b * a.s_what * 2;
   }
-  __syncthreads();
-  for (int k = ty; k < 32; k += 8) {
-    const int r = r0 + k, c = c0 + tx;
-    if (c < d && r < out) {
-      if (codes) codes[(long long)r * ldc + c] = (int)tq[tx][k];
-      if (what) {
-        // the reference rounds to fp16 first and casts to the module's dtype afterwards
-        const __half h = __float2half_rn(tv[tx][k]);
-        if (bf16) static_cast<__nv_bfloat16*>(what)[(long long)r * ldwh + c] = __float2bfloat16_rn(__half2float(h));
-        else static_cast<__half*>(what)[(long long)r * ldwh + c] = h;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int r0 = blockIdx.y * FIN_ROWS, cb = blockIdx.x * FIN_COLS, c0 = cb + warp * 32;
+  const int r = r0 + 2 * lane;
+  const bool pair = (a.out & 1) == 0;          // two rows in one 4-byte access
+  if (c0 < a.d) {               // (the same for all lanes: they shuffle)
+    const bool one = r < a.out, two = r + 1 < a.out;
+    constexpr unsigned MASK = BITS ? (1u << BITS) - 1u : 0u;
+    unsigned word0[BITS ? BITS : 1], word1[BITS ? BITS : 1];   // the 32 columns' packed words of both rows
+#pragma unroll
+    for (int t = 0; t < (BITS ? BITS : 1); ++t) word0[t] = word1[t] = 0u;
+    // source column and group of column c0 + lane, handed round below
+    const int cl = c0 + lane;
+    const int jl = cl < a.d ? (a.invperm ? a.invperm[cl] : cl) : -1;
+    const int gl = (a.gs == -1 || jl < 0) ? 0 : jl / a.gs;
+    int group = -1;
+    float2 sc = make_float2(0.f, 0.f), zr = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int k8 = 0; k8 < 32; k8 += 8) {
+      unsigned q2[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int j = __shfl_sync(0xffffffffu, jl, k8 + i);
+        q2[i] = 0u;
+        if (j >= 0 && one) {
+          const unsigned short* p = a.codesT + (long long)j * a.out + r;
+          if (pair) q2[i] = *reinterpret_cast<const unsigned*>(p);
+          else q2[i] = (unsigned)p[0] | (two ? (unsigned)p[1] << 16 : 0u);
+        }
+      }
+      unsigned short ua[2], ub[2];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = k8 + i;
+        const unsigned qa = q2[i] & 0xffffu, qb = q2[i] >> 16;
+        if (BITS) {
+          const int bit = k * BITS, wi = bit >> 5, off = bit & 31;
+          word0[wi] |= (qa & MASK) << off;
+          word1[wi] |= (qb & MASK) << off;
+          if (off + BITS > 32) {
+            word0[wi + 1 < BITS ? wi + 1 : wi] |= (qa & MASK) >> (32 - off);
+            word1[wi + 1 < BITS ? wi + 1 : wi] |= (qb & MASK) >> (32 - off);
+          }
+        }
+        if (a.what) {
+          const int g = __shfl_sync(0xffffffffu, gl, k);
+          if (g != group) {
+            group = g;
+            const float* sp = a.scales + (long long)g * a.out + r;
+            const float* zp = a.zeros + (long long)g * a.out + r;
+            if (one) { sc.x = __half2float(__float2half_rn(sp[0])); zr.x = zp[0]; }
+            if (two) { sc.y = __half2float(__float2half_rn(sp[1])); zr.y = zp[1]; }
+          }
+          // the reference rounds to fp16 first and casts to the module's dtype afterwards
+          const __half ha = __float2half_rn(__fmul_rn(sc.x, __fsub_rn((float)qa, zr.x)));
+          const __half hb = __float2half_rn(__fmul_rn(sc.y, __fsub_rn((float)qb, zr.y)));
+          if (a.bf16) {
+            ua[k & 1] = __bfloat16_as_ushort(__float2bfloat16_rn(__half2float(ha)));
+            ub[k & 1] = __bfloat16_as_ushort(__float2bfloat16_rn(__half2float(hb)));
+          } else { ua[k & 1] = __half_as_ushort(ha); ub[k & 1] = __half_as_ushort(hb); }
+          if (k & 1) {
+            tw[fin_at(2 * lane, warp * 32 + k)] = (unsigned)ua[0] | ((unsigned)ua[1] << 16);
+            tw[fin_at(2 * lane + 1, warp * 32 + k)] = (unsigned)ub[0] | ((unsigned)ub[1] << 16);
+          }
+        }
+        if (a.codes && (k & 1)) {
+          tq[fin_at(2 * lane, warp * 32 + k)] = (q2[i - 1 >= 0 ? i - 1 : 0] & 0xffffu) | (qa << 16);
+          tq[fin_at(2 * lane + 1, warp * 32 + k)] = (q2[i - 1 >= 0 ? i - 1 : 0] >> 16) | (qb << 16);
+        }
+      }
+    }
+    if (BITS && a.qweight && one) {
+      const long long w0 = (long long)c0 / 32 * BITS;
+      const int words = min(BITS, (int)((long long)(a.d - c0) * BITS / 32));   // d is a multiple of the pack factor
+#pragma unroll
+      for (int t = 0; t < BITS; ++t) {
+        if (t >= words) continue;
+        int* p = a.qweight + (w0 + t) * a.ldq + r;
+        p[0] = (int)word0[t];
+        if (two) p[1] = (int)word1[t];
       }
     }
   }
+  if (!a.what && !a.codes) return;
+  __syncthreads();
+  const bool vec = ((a.ldwh | a.d) & 1) == 0 && (reinterpret_cast<uintptr_t>(a.what) & 3) == 0;
+  for (int row = warp; row < FIN_ROWS; row += 4) {
+    const int rr = r0 + row;
+    if (rr >= a.out) break;
+#pragma unroll
+    for (int h = 0; h < FIN_COLS / 64; ++h) {
+      const int k = h * 64 + 2 * lane, c = cb + k;
+      if (c >= a.d) continue;
+      if (a.what) {
+        unsigned short* w = static_cast<unsigned short*>(a.what) + (long long)rr * a.ldwh + c;
+        const unsigned v = tw[fin_at(row, k)];
+        if (vec) *reinterpret_cast<unsigned*>(w) = v;
+        else {
+          w[0] = (unsigned short)(v & 0xffffu);
+          if (c + 1 < a.d) w[1] = (unsigned short)(v >> 16);
+        }
+      }
+      if (a.codes) {
+        int* p = a.codes + (long long)rr * a.ldc + c;
+        const unsigned v = tq[fin_at(row, k)];
+        p[0] = (int)(v & 0xffffu);
+        if (c + 1 < a.d) p[1] = (int)(v >> 16);
+      }
+    }
+  }
+}
+
+int launch_finish(const FinishArgs& a, int bits, int batch, cudaStream_t stream) {
+  const dim3 grid(oc_div_up(a.d, FIN_COLS), oc_div_up(a.out, FIN_ROWS), batch);
+  const int smem = ((a.what ? 1 : 0) + (a.codes ? 1 : 0)) * FIN_TILE * 4;
+  switch (bits) {
+    case 2: finish_kernel<2><<<grid, 128, smem, stream>>>(a); break;
+    case 3: finish_kernel<3><<<grid, 128, smem, stream>>>(a); break;
+    case 4: finish_kernel<4><<<grid, 128, smem, stream>>>(a); break;
+    case 8: finish_kernel<8><<<grid, 128, smem, stream>>>(a); break;
+    default: finish_kernel<0><<<grid, 128, smem, stream>>>(a);
+  }
+  OC_CHECK_LAUNCH();
+  return OC_OK;
 }
 
 template <int WARPS, bool ALIGNED>
@@ -588,6 +726,8 @@ int launch_block(const ColArgs& a, cudaStream_t stream) {
 }
 
 long long round4(long long x) { return (x + 3) / 4 * 4; }
+
+constexpr int PREPARE_STAGED_D = 49152;   // widest row that the act-order gather keeps in shared memory
 
 }  // namespace
 
@@ -651,9 +791,13 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
 
   OC_REQUIRE(!mse || (q_grid >= 1 && q_norm > 0.f), "gptq_quantize: mse needs q_grid >= 1 and q_norm > 0");
   const int mse_steps = mse ? (int)(0.8 * q_grid) : 0;   // maxshrink = 0.8 as in the reference
-  gptq_prepare_kernel<<<dim3(out, batch), 256, 0, stream>>>(W, bf16, ldw_in, out, d, perm, dead, Wf, ldw,
-                                                            groupsize == -1 ? 1 : 0, maxq, sym, mse_steps,
-                                                            (float)q_grid, q_norm, scales, zeros, sWin, nWf, nPar);
+  const bool vec = d % 8 == 0 && ldw_in % 8 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
+                   (reinterpret_cast<uintptr_t>(dead) & 7) == 0;
+  const bool staged = perm && d <= PREPARE_STAGED_D;
+  if (staged) OC_OPT_IN_SMEM(gptq_prepare_kernel, PREPARE_STAGED_D * 4);
+  gptq_prepare_kernel<<<dim3(out, batch), 256, staged ? d * 4 : 0, stream>>>(
+      W, bf16, ldw_in, out, d, perm, dead, Wf, ldw, groupsize == -1 ? 1 : 0, maxq, sym, mse_steps,
+      (float)q_grid, q_norm, scales, zeros, sWin, nWf, nPar, vec, staged);
   OC_CHECK_LAUNCH();
 
   if (sm_count <= 0) sm_count = 148;
@@ -703,17 +847,15 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   const int f = (wbits == 3) ? 32 : ((wbits == 2 || wbits == 4 || wbits == 8) ? 32 / wbits : 1);
   const long long ldz = (wbits == 3) ? ld_out / 32 * 3 : ld_out / f;
   const long long prow = (wbits == 3) ? d / 32 * 3 : d / f;     // rows of one problem's packed weight
+  if (qweight || codes || what) {
+    FinishArgs f_args{codesT, out, d, invperm, groupsize, scales, zeros, qweight, ld_out, codes, d, what, ldwh, bf16,
+                      nCodes, nPar, prow * ld_out, (long long)out * d, (long long)out * ldwh};
+    const int rc = launch_finish(f_args, qweight ? wbits : 0, batch, stream);
+    if (rc) return rc;
+  }
   for (int b = 0; b < batch; ++b) {
-    const unsigned short* cT = codesT + b * nCodes;
     const float* sc = scales + b * nPar;
     const float* zr = zeros + b * nPar;
-    const int* ip = invperm ? invperm + (long long)b * d : nullptr;
-    if (qweight) {
-      const int prow_k = (wbits == 3) ? d / 32 : d / (32 / wbits);
-      pack_qweight_kernel<<<dim3(oc_div_up(out, tb), prow_k), tb, 0, stream>>>(cT, out, d, ip, wbits,
-                                                                               qweight + b * prow * ld_out, ld_out);
-      OC_CHECK_LAUNCH();
-    }
     if (qzeros) {
       pack_qzeros_kernel<<<dim3(oc_div_up(out / f, tb), G), tb, 0, stream>>>(zr, out, G, wbits,
                                                                              qzeros + b * G * ldz, ldz);
@@ -723,12 +865,6 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
       cast_params_kernel<<<dim3(oc_div_up(out, tb), G), tb, 0, stream>>>(
           sc, zr, out, G, scales16 ? scales16 + b * G * ld_out : nullptr, ld_out,
           scales32 ? scales32 + b * G * ld_out : nullptr, zeros_i32 ? zeros_i32 + b * G * ld_out : nullptr);
-      OC_CHECK_LAUNCH();
-    }
-    if (codes || what) {
-      void* wh = what ? (void*)((char*)what + (long long)b * out * ldwh * 2) : nullptr;
-      unpermute_outputs_kernel<<<dim3(oc_div_up(d, 32), oc_div_up(out, 32)), dim3(32, 8), 0, stream>>>(
-          cT, out, d, ip, groupsize, sc, zr, codes ? codes + (long long)b * out * d : nullptr, d, wh, ldwh, bf16);
       OC_CHECK_LAUNCH();
     }
   }
