@@ -151,193 +151,212 @@ __global__ void __launch_bounds__(256) reverse_upper_kernel(const float* __restr
   }
 }
 
+// Two fp32 FMAs in one instruction, each rounded like fmaf: d = a * b + c.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+
 // ---- one diagonal block: Cholesky of a (<=128)^2 block on one SM ----------------------------
-// A block (nb x nb, lower part read) -> L written back over the lower part, L^T over the upper.
-// A non-positive or non-finite pivot records (global index + 1) in *status (first one wins)
-// and continues with pivot 1 so that every later kernel still terminates.
+// A block (nb x nb, lower part read) -> L written back over the lower part, L^T over the upper
+// (nothing reads the upper part of a diagonal block of A as matrix data; the panel solve loads L^T
+// from there).  A non-positive or non-finite pivot records (global index + 1) in *status (first one
+// wins); what is computed behind it means nothing, and no kernel of the chain waits for a value.
 //
-// 16 x 16 threads, each holding an 8 x 8 sub-block in registers.  The eight columns of a
-// micro-panel are finished inside the one warp that holds that block column (the diagonal 8 x 8
-// block on one lane, its factor shuffled to the others), published to shared memory, and every
-// thread to the right applies them as eight rank-1 updates to its registers: one barrier per
-// eight columns.
-constexpr int POTRF_SMEM = (NB * (NB + 4) + 2 * 8 * (NB + 4)) * (int)sizeof(float);
-__global__ void __launch_bounds__(256) potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb,
+// A serial chain on one SM, 16 micro-panels of eight columns.  Two threads hold a row, in registers,
+// each every other group of four columns.  Per micro-panel the eight pivot rows publish their
+// 8 x 8 block; every thread factors it for itself (36 values, no further exchange) and solves its row
+// against it; the eight new columns go to shared memory, and every thread updates the rest of its
+// row, two columns per FMA instruction (fma.f32x2).  The register file moves eight columns to the left in
+// the update itself, so one loop body serves all micro-panels.  The operations on an entry are those of a
+// column-by-column elimination, in its order.
+// With 8 x 8 register blocks per thread, a single lane factoring the pivot block and half of the
+// lanes idle above the diagonal this took 31.5 us; now 25 us (per micro-panel 0.5 us of pivot chain, 0.6 us of
+// update, which shared-memory broadcasts bound: an entry of L loaded serves one row per lane).
+constexpr int LP = NB + 4;     // pitch of the published columns
+__global__ void __launch_bounds__(256, 1) potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb,
                                                           int* __restrict__ status, long long sW) {
   A += (long long)blockIdx.x * sW;
   status += blockIdx.x;
-  extern __shared__ __align__(16) float sm[];
-  // The block travels between global memory and the register blocks through shared memory, so
-  // that global accesses are whole rows.  Row r of the block sits at staging row (r % 8) * 16 + r / 8:
-  // the sixteen threads of a block column then read sixteen consecutive staging rows at once.
-  float (*St)[NB + 4] = reinterpret_cast<float (*)[NB + 4]>(sm);
-  // L of the current 8-column micro-panel, column-major [8][128], double buffered
-  float (*Lp)[8][NB + 4] = reinterpret_cast<float (*)[8][NB + 4]>(sm + NB * (NB + 4));
-  // block column tx of the 16 x 16 grid of 8 x 8 register blocks lives in one half-warp
-  const int tid = threadIdx.x, tx = tid >> 4, ty = tid & 15;
-  const int r0 = ty * 8, c0 = tx * 8;
+  __shared__ __align__(16) float Lp[8 * LP + 16];   // the micro-panel's columns, [8][row]
+  __shared__ __align__(16) float Pv[8][8];     // its pivot block
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = lane >> 4, r = warp * 16 + (lane & 15);    // this thread: row r, columns 8q + 4h .. 8q + 4h + 3
   float* Ab = A + (long long)k0 * lda + k0;
+  float* Ar = Ab + (long long)r * lda;
 
-  if (nb == NB) {
+  f32x2 a[32];                                 // a[2q], a[2q + 1]: group q of the remaining columns
 #pragma unroll
-    for (int it = 0; it < NB * NB / 4 / 256; ++it) {
-      const int e = it * 256 + tid, r = e / (NB / 4), c4 = e % (NB / 4);
-      *reinterpret_cast<float4*>(&St[(r & 7) * 16 + (r >> 3)][4 * c4]) =
-          *reinterpret_cast<const float4*>(Ab + (long long)r * lda + 4 * c4);
+  for (int q = 0; q < 16; ++q) {
+    const int c = 8 * q + 4 * h;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c <= r) {
+      if (nb == NB) v = *reinterpret_cast<const float4*>(Ar + c);
+      else if (r < nb) {
+        v.x = Ar[c];                           // c <= r < nb
+        if (c + 1 < nb) v.y = Ar[c + 1];
+        if (c + 2 < nb) v.z = Ar[c + 2];
+        if (c + 3 < nb) v.w = Ar[c + 3];
+      } else if (r - c < 4) {                  // rows behind the block: identity
+        v.x = r == c ? 1.f : 0.f; v.y = r == c + 1 ? 1.f : 0.f; v.z = r == c + 2 ? 1.f : 0.f; v.w = r == c + 3 ? 1.f : 0.f;
+      }
     }
-  } else {
-    for (int e = tid; e < NB * NB; e += 256) {
-      const int r = e / NB, c = e % NB;
-      St[(r & 7) * 16 + (r >> 3)][c] = (r < nb && c < nb) ? Ab[(long long)r * lda + c] : 0.f;
-    }
+    a[2 * q] = pack2(v.x, v.y);
+    a[2 * q + 1] = pack2(v.z, v.w);
+  }
+  if (r < 8) {
+    const float2 lo = unpack2(a[0]), hi = unpack2(a[1]);
+    *reinterpret_cast<float4*>(&Pv[r][4 * h]) = make_float4(lo.x, lo.y, hi.x, hi.y);
   }
   __syncthreads();
-  float a[8][8];
-#pragma unroll
-  for (int ii = 0; ii < 8; ++ii) {
-    const float4 lo = *reinterpret_cast<const float4*>(&St[ii * 16 + ty][c0]);
-    const float4 hi = *reinterpret_cast<const float4*>(&St[ii * 16 + ty][c0 + 4]);
-    const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc) {
-      const int r = r0 + ii, c = c0 + cc;
-      a[ii][cc] = (r < nb && c <= r) ? v[cc] : ((r == c) ? 1.f : 0.f);
-    }
-  }
 
+#pragma unroll 1
   for (int jb = 0; jb < NB / 8; ++jb) {
-    const int buf = jb & 1;
-    if ((tid >> 5) == (jb >> 1)) {
-      // ---- the micro-panel's eight columns, inside the one warp that holds them ----
-      // The lane with the diagonal 8 x 8 block factors it alone in registers; the factor's 28
-      // sub-diagonal entries and 8 reciprocal pivots go round by shuffles, and every other lane of
-      // the block column solves X L^T = B for its own 8 x 8 block by forward substitution: eight
-      // independent rows per lane, the same operations in the same order as a column-by-column
-      // elimination across the lanes, without its eight broadcast-scale-update rounds.
-      const int pl = ((jb & 1) << 4) + jb;          // lane that owns the diagonal 8 x 8 block
-      const bool mine = (tx == jb) && (ty > jb);
-      const bool is_pivot = (tx == jb) && (ty == jb);
-      float l[8][8], dinv[8];
+    const int j0 = 8 * jb;
+    float y[8];
+    const bool live = warp * 16 + 15 >= j0;    // the same for the whole warp
+    if (live) {
+      float l[8][8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        dinv[i] = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) l[i][j] = 0.f;
-      }
-      if (is_pivot) {
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          float p = a[jj][jj];
-          if (!(p > 0.f) || !isfinite(p)) {
-            atomicCAS(status, 0, k0 + jb * 8 + jj + 1);
-            p = 1.f;
-          }
-          // one approximate reciprocal square root, refined once, instead of an IEEE square
-          // root followed by IEEE divisions
-          float inv = rsqrtf(p);
-          inv = inv * fmaf(-0.5f * p * inv, inv, 1.5f);
-          dinv[jj] = inv;
-          a[jj][jj] = p * inv;
-#pragma unroll
-          for (int ii = jj + 1; ii < 8; ++ii) a[ii][jj] *= inv;
-#pragma unroll
-          for (int cc = jj + 1; cc < 8; ++cc)
-#pragma unroll
-            for (int ii = cc; ii < 8; ++ii) a[ii][cc] = fmaf(-a[ii][jj], a[cc][jj], a[ii][cc]);
+        const float4 lo = *reinterpret_cast<const float4*>(&Pv[i][0]);
+        l[i][0] = lo.x; l[i][1] = lo.y; l[i][2] = lo.z; l[i][3] = lo.w;
+        if (i >= 4) {
+          const float4 hi = *reinterpret_cast<const float4*>(&Pv[i][4]);
+          l[i][4] = hi.x; l[i][5] = hi.y; l[i][6] = hi.z; l[i][7] = hi.w;
         }
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < i; ++j) l[i][j] = a[i][j];
       }
+      {
+        const float2 m0 = unpack2(a[0]), m1 = unpack2(a[1]);
+        const float mine[4] = {m0.x, m0.y, m1.x, m1.y};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        dinv[i] = __shfl_sync(0xffffffffu, dinv[i], pl);
-#pragma unroll
-        for (int j = 0; j < i; ++j) l[i][j] = __shfl_sync(0xffffffffu, l[i][j], pl);
+        for (int i = 0; i < 4; ++i) {
+          const float other = __shfl_xor_sync(0xffffffffu, mine[i], 16);
+          y[i] = h ? other : mine[i];
+          y[4 + i] = h ? mine[i] : other;
+        }
       }
-      if (mine) {
+      int bad = 8;                             // first column with an unusable pivot
 #pragma unroll
-        for (int ii = 0; ii < 8; ++ii)
+      for (int jj = 0; jj < 8; ++jj) {
+        // (selections, not branches: the eight columns are one stretch of code, whose instructions
+        // fill the waits of the chain from pivot to pivot)
+        const float p = l[jj][jj];
+        const bool ok = p > 0.f && p < __int_as_float(0x7f800000);
+        bad = !ok && bad == 8 ? jj : bad;
+        // one approximate reciprocal square root, refined once, instead of an IEEE square
+        // root followed by IEEE divisions
+        float inv = rsqrtf(p);
+        inv = inv * fmaf(-0.5f * p * inv, inv, 1.5f);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float acc = a[ii][j];
+        for (int ii = jj + 1; ii < 8; ++ii) l[ii][jj] *= inv;
 #pragma unroll
-            for (int k = 0; k < j; ++k) acc = fmaf(-a[ii][k], l[j][k], acc);
-            a[ii][j] = acc * dinv[j];
+        for (int cc = jj + 1; cc < 8; ++cc)
+#pragma unroll
+          for (int ii = cc; ii < 8; ++ii) l[ii][cc] = fmaf(-l[ii][jj], l[cc][jj], l[ii][cc]);
+        // this row's entry of column jj, then its part in the columns behind
+        y[jj] *= inv;
+        if (r == j0 + jj) y[jj] = p * inv;
+#pragma unroll
+        for (int cc = jj + 1; cc < 8; ++cc) y[cc] = fmaf(-y[jj], l[cc][jj], y[cc]);
+      }
+      if (bad < 8 && r == j0 && h == 0) atomicCAS(status, 0, k0 + j0 + bad + 1);
+      const float4 m = h ? make_float4(y[4], y[5], y[6], y[7]) : make_float4(y[0], y[1], y[2], y[3]);
+      const float mv[4] = {m.x, m.y, m.z, m.w};
+      const int c = j0 + 4 * h;                // columns c .. c + 3 are this thread's to store
+      if (r >= j0 + 8) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) Lp[(4 * h + i) * LP + r] = mv[i];
+        if (nb == NB) *reinterpret_cast<float4*>(Ar + c) = m;
+        else if (r < nb) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) Ar[c + i] = mv[i];       // c + i < r < nb
+        }
+        if (r < nb) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) Ab[(long long)(c + i) * lda + r] = mv[i];
+        }
+      } else if (r >= j0 && r < nb) {          // pivot rows: up to the diagonal
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (c + i <= r) {
+            Ar[c + i] = mv[i];
+            Ab[(long long)(c + i) * lda + r] = mv[i];
           }
-      }
-      if (mine || is_pivot) {
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj)
-#pragma unroll
-          for (int ii = 0; ii < 8; ++ii) Lp[buf][jj][r0 + ii] = a[ii][jj];
       }
     }
     __syncthreads();
-    // ---- rank-8 update of everything to the right, one column of the panel at a time, in
-    // the order of eight successive rank-1 updates ----
-    if (tx > jb && ty >= tx) {
+    if (live) {
+      f32x2 ny[8];
 #pragma unroll
-      for (int jj = 0; jj < 8; ++jj) {
-        const float4 r_lo = *reinterpret_cast<const float4*>(&Lp[buf][jj][r0]);
-        const float4 r_hi = *reinterpret_cast<const float4*>(&Lp[buf][jj][r0 + 4]);
-        const float4 c_lo = *reinterpret_cast<const float4*>(&Lp[buf][jj][c0]);
-        const float4 c_hi = *reinterpret_cast<const float4*>(&Lp[buf][jj][c0 + 4]);
-        const float rc[8] = {r_lo.x, r_lo.y, r_lo.z, r_lo.w, r_hi.x, r_hi.y, r_hi.z, r_hi.w};
-        const float cv[8] = {c_lo.x, c_lo.y, c_lo.z, c_lo.w, c_hi.x, c_hi.y, c_hi.z, c_hi.w};
-        // (the entries above the diagonal of a diagonal block are updated too: nothing reads them)
+      for (int j = 0; j < 8; ++j) ny[j] = pack2(-y[j], -y[j]);
+      const float* lp = Lp + j0 + 8 + 4 * h;
 #pragma unroll
-        for (int ii = 0; ii < 8; ++ii)
+      for (int q = 0; q < 16; q += 2) {
+        // columns up to this warp's last row, two groups in flight (the entries above the diagonal are
+        // updated too: nothing reads them; a group behind the last column meets a dead register pair)
+        if (jb + 1 + q <= 2 * warp + 1) {
+          f32x2 v[4] = {a[2 * q + 2], a[2 * q + 3], q < 14 ? a[q < 14 ? 2 * q + 4 : 0] : 0ull,
+                        q < 14 ? a[q < 14 ? 2 * q + 5 : 0] : 0ull};
 #pragma unroll
-          for (int cc = 0; cc < 8; ++cc) a[ii][cc] = fmaf(-rc[ii], cv[cc], a[ii][cc]);
+          for (int j = 0; j < 8; ++j) {
+            const float4 t = *reinterpret_cast<const float4*>(lp + j * LP + 8 * q);
+            const float4 u = *reinterpret_cast<const float4*>(lp + j * LP + 8 * q + 8);
+            v[0] = fma2(ny[j], pack2(t.x, t.y), v[0]);
+            v[1] = fma2(ny[j], pack2(t.z, t.w), v[1]);
+            v[2] = fma2(ny[j], pack2(u.x, u.y), v[2]);
+            v[3] = fma2(ny[j], pack2(u.z, u.w), v[3]);
+          }
+          a[2 * q] = v[0]; a[2 * q + 1] = v[1];
+          a[2 * q + 2] = v[2]; a[2 * q + 3] = v[3];
+          if (q == 0 && (r >> 3) == jb + 1) {
+            const float2 lo = unpack2(v[0]), hi = unpack2(v[1]);
+            *reinterpret_cast<float4*>(&Pv[r & 7][4 * h]) = make_float4(lo.x, lo.y, hi.x, hi.y);
+          }
+        }
       }
     }
-  }
-  // L goes back over the lower part and, transposed, over the upper part (nothing reads the upper
-  // part of a diagonal block of A as matrix data; the panel solve loads L^T from there)
-  __syncthreads();
-#pragma unroll
-  for (int ii = 0; ii < 8; ++ii) {
-    float v[8];
-#pragma unroll
-    for (int cc = 0; cc < 8; ++cc) v[cc] = (c0 + cc <= r0 + ii) ? a[ii][cc] : 0.f;
-    *reinterpret_cast<float4*>(&St[ii * 16 + ty][c0]) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(&St[ii * 16 + ty][c0 + 4]) = make_float4(v[4], v[5], v[6], v[7]);
-  }
-  __syncthreads();
-  // row r of the result: L[r][c] for c <= r, L[c][r] for c > r
-  for (int e = tid; e < NB * NB; e += 256) {
-    const int r = e / NB, c = e % NB;
-    if (r < nb && c < nb) {
-      const int hi = max(r, c), lo = min(r, c);
-      Ab[(long long)r * lda + c] = St[(hi & 7) * 16 + (hi >> 3)][lo];
-    }
+    __syncthreads();
   }
 }
 
 // ---- panel solve: P <- P * L^-T for the rows below a factored diagonal block -----------------
 // L = the 128 x 128 lower block at (k0, k0), P = the `rest` rows below it (same columns).  Row r of
 // the result is the forward substitution y_j = (p_j - sum_{i<j} y_i L[j][i]) / L[j][j]: rows are
-// independent.  A CTA takes 128 rows, two threads per row: eight columns at a time, each thread
-// sums over every other earlier column, the pair combines with one shuffle per column and both
+// independent.  Two threads per row: eight columns at a time, one sums over the even and one over the
+// odd earlier columns, the pair combines with one shuffle per column and both
 // finish the 8 x 8 diagonal step.  The block kernel left L^T in the upper triangle of the
 // diagonal block, so the tile loads as it is (coalesced, no transposition) and the inner loop
-// reads eight consecutive entries L[j0..j0+7][i] as two broadcast vector loads.  Plain fp32 FMAs:
-// this is the step that used to need the explicit inverse of the diagonal block on the critical
-// path.
-constexpr int TR = 128;                    // rows per CTA
-constexpr int TPR = 2;                     // threads per row (four were measured slower: the 8 x 8
-                                           // diagonal step is repeated by every thread of a row)
-constexpr int TRT = TPR * TR;              // threads per CTA
-constexpr int LPITCH = NB + 4, YPITCH = NB + 2;   // YPITCH = 2 mod 32: a warp's rows hit distinct banks
-constexpr int TRSM_SMEM = (NB * LPITCH + TR * YPITCH + NB) * (int)sizeof(float);
+// reads eight consecutive entries L[j0..j0+7][i] as two broadcast vector loads.  Plain fp32 FMAs.
+//
+// Bound by shared-memory loads (a 16-byte broadcast costs as much as four of 4 bytes, and an entry of L
+// serves one row of a lane) and by the latency of the chain over columns.  With few rows (TR 32) every
+// SM gets its share of them: 13 to 14 us up to 9472 rows, where 128 rows per CTA on a quarter of the SMs
+// took 21.  With more rows two CTAs of 64 share an SM: 23 us for 9472 to 14208 rows, as before (two rows
+// per thread pair, which halve the loads of L, were slower for want of warps: 25 us).  Even and odd columns
+// of a row lie apart in shared memory: a thread reads four of its own at once.
+constexpr int TRT = 256;                   // threads per CTA (the first 2 * TR solve, all of them load)
+constexpr int LPITCH = NB + 4, YPITCH = NB + 4;
+template <int TR> constexpr int TRSM_SMEM = (NB * LPITCH + TR * YPITCH + NB) * (int)sizeof(float);
+template <int TR>                          // rows per CTA
 __global__ void __launch_bounds__(TRT) trsm_panel_kernel(float* __restrict__ A, long long lda, int k0, int rest,
                                                          long long sW) {
   A += (long long)blockIdx.y * sW;
   extern __shared__ __align__(16) float sm[];
   float* Lt = sm;                           // Lt[i * LPITCH + j] = L[j][i] for j >= i
-  float* Ys = sm + NB * LPITCH;             // this CTA's rows, YPITCH apart
+  float* Ys = sm + NB * LPITCH;             // this CTA's rows: 64 even columns, then 64 odd ones
   float* dinv = Ys + TR * YPITCH;
   const int tid = threadIdx.x;
   const float* Lkk = A + (long long)k0 * lda + k0;
@@ -355,52 +374,57 @@ __global__ void __launch_bounds__(TRT) trsm_panel_kernel(float* __restrict__ A, 
     const int e = it * TRT + tid, r = e / (NB / 4), c4 = e % (NB / 4);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (r < rows) v = *reinterpret_cast<const float4*>(P + (long long)(row0 + r) * lda + 4 * c4);
-    float2* dst = reinterpret_cast<float2*>(Ys + r * YPITCH + 4 * c4);
-    dst[0] = make_float2(v.x, v.y);
-    dst[1] = make_float2(v.z, v.w);
+    *reinterpret_cast<float2*>(Ys + r * YPITCH + 2 * c4) = make_float2(v.x, v.z);
+    *reinterpret_cast<float2*>(Ys + r * YPITCH + NB / 2 + 2 * c4) = make_float2(v.y, v.w);
   }
   __syncthreads();
   if (tid < NB) dinv[tid] = 1.f / Lt[tid * LPITCH + tid];
   __syncthreads();
-  {
-    const int r = tid / TPR, part = tid % TPR;
-    float* y = Ys + r * YPITCH;
+  if (tid < 2 * TR) {
+    const int part = tid & 1;
+    float* y = Ys + (tid >> 1) * YPITCH;
     for (int j0 = 0; j0 < NB; j0 += 8) {
-      float acc[8];
+      const float4 ev = *reinterpret_cast<const float4*>(y + j0 / 2);
+      const float4 od = *reinterpret_cast<const float4*>(y + NB / 2 + j0 / 2);
+      f32x2 acc2[4] = {part ? 0ull : pack2(ev.x, od.x), part ? 0ull : pack2(ev.y, od.y),
+                       part ? 0ull : pack2(ev.z, od.z), part ? 0ull : pack2(ev.w, od.w)};
+      const float* lt = Lt + part * LPITCH + j0;
+#pragma unroll 1
+      for (int i4 = 0; i4 < j0 / 2; i4 += 4) {      // this thread's columns 2 (i4 + k) + part
+        const float4 yv = *reinterpret_cast<const float4*>(y + part * (NB / 2) + i4);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[c] = part ? 0.f : y[j0 + c];
-#pragma unroll 4
-      for (int i = part; i < j0; i += TPR) {
-        const float yi = y[i];
-        const float4 l0 = *reinterpret_cast<const float4*>(Lt + i * LPITCH + j0);
-        const float4 l1 = *reinterpret_cast<const float4*>(Lt + i * LPITCH + j0 + 4);
-        acc[0] = fmaf(-yi, l0.x, acc[0]); acc[1] = fmaf(-yi, l0.y, acc[1]);
-        acc[2] = fmaf(-yi, l0.z, acc[2]); acc[3] = fmaf(-yi, l0.w, acc[3]);
-        acc[4] = fmaf(-yi, l1.x, acc[4]); acc[5] = fmaf(-yi, l1.y, acc[5]);
-        acc[6] = fmaf(-yi, l1.z, acc[6]); acc[7] = fmaf(-yi, l1.w, acc[7]);
-      }
+        for (int k = 0; k < 4; ++k) {
+          const float4 l0 = *reinterpret_cast<const float4*>(lt + 2 * (i4 + k) * LPITCH);
+          const float4 l1 = *reinterpret_cast<const float4*>(lt + 2 * (i4 + k) * LPITCH + 4);
+          const f32x2 l[4] = {pack2(l0.x, l0.y), pack2(l0.z, l0.w), pack2(l1.x, l1.y), pack2(l1.z, l1.w)};
+          const float yk = k == 0 ? yv.x : k == 1 ? yv.y : k == 2 ? yv.z : yv.w;
+          const f32x2 ny = pack2(-yk, -yk);
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
-        if (TPR == 4) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
-      }
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float yc = acc[c] * dinv[j0 + c];
-        acc[c] = yc;
-        if (c < 7) {
-          const float4 l0 = *reinterpret_cast<const float4*>(Lt + (j0 + c) * LPITCH + j0);
-          const float4 l1 = *reinterpret_cast<const float4*>(Lt + (j0 + c) * LPITCH + j0 + 4);
-          const float lr[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
-#pragma unroll
-          for (int c2 = c + 1; c2 < 8; ++c2) acc[c2] = fmaf(-yc, lr[c2], acc[c2]);
+          for (int c = 0; c < 4; ++c) acc2[c] = fma2(ny, l[c], acc2[c]);
         }
       }
-      if (part == 0) {
+      float acc[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) y[j0 + c] = acc[c];
+      for (int c = 0; c < 4; ++c) {
+        const float2 v = unpack2(acc2[c]);
+        acc[2 * c] = v.x + __shfl_xor_sync(0xffffffffu, v.x, 1);
+        acc[2 * c + 1] = v.y + __shfl_xor_sync(0xffffffffu, v.y, 1);
       }
-      __syncwarp();          // the partners read these eight values in the next step
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float di = dinv[j0 + c];
+        const float4 l0 = *reinterpret_cast<const float4*>(Lt + (j0 + c) * LPITCH + j0);
+        const float4 l1 = *reinterpret_cast<const float4*>(Lt + (j0 + c) * LPITCH + j0 + 4);
+        const float lr[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+        const float yc = acc[c] * di;
+        acc[c] = yc;
+#pragma unroll
+        for (int c2 = c + 1; c2 < 8; ++c2) acc[c2] = fmaf(-yc, lr[c2], acc[c2]);
+      }
+      // each partner keeps its own columns
+      *reinterpret_cast<float4*>(y + part * (NB / 2) + j0 / 2) =
+          part ? make_float4(acc[1], acc[3], acc[5], acc[7]) : make_float4(acc[0], acc[2], acc[4], acc[6]);
+      __syncwarp();
     }
   }
   __syncthreads();
@@ -408,11 +432,19 @@ __global__ void __launch_bounds__(TRT) trsm_panel_kernel(float* __restrict__ A, 
   for (int it = 0; it < TR * NB / 4 / TRT; ++it) {
     const int e = it * TRT + tid, r = e / (NB / 4), c4 = e % (NB / 4);
     if (r < rows) {
-      const float2* src = reinterpret_cast<const float2*>(Ys + r * YPITCH + 4 * c4);
-      const float2 a = src[0], b = src[1];
-      *reinterpret_cast<float4*>(P + (long long)(row0 + r) * lda + 4 * c4) = make_float4(a.x, a.y, b.x, b.y);
+      const float2 ev = *reinterpret_cast<const float2*>(Ys + r * YPITCH + 2 * c4);
+      const float2 od = *reinterpret_cast<const float2*>(Ys + r * YPITCH + NB / 2 + 2 * c4);
+      *reinterpret_cast<float4*>(P + (long long)(row0 + r) * lda + 4 * c4) = make_float4(ev.x, od.x, ev.y, od.y);
     }
   }
+}
+
+template <int TR>
+int launch_trsm(float* A, long long ld, int k0, int rest, int batch, long long sW, cudaStream_t stream) {
+  OC_OPT_IN_SMEM(trsm_panel_kernel<TR>, TRSM_SMEM<TR>);
+  trsm_panel_kernel<TR><<<dim3(oc_div_up(rest, TR), batch), TRT, TRSM_SMEM<TR>, stream>>>(A, ld, k0, rest, sW);
+  OC_CHECK_LAUNCH();
+  return OC_OK;
 }
 
 // ---- inverses of all diagonal blocks of L, one CTA per block (off the critical path) ----------
@@ -556,8 +588,6 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
   OC_CHECK_LAUNCH();
 
   // ---- blocked right-looking Cholesky --------------------------------------------------
-  OC_OPT_IN_SMEM(potrf_block_kernel, POTRF_SMEM);
-  OC_OPT_IN_SMEM(trsm_panel_kernel, TRSM_SMEM);
   OC_OPT_IN_SMEM(diag_inverse_kernel, DINV_SMEM);
   auto batched = [&](OcGemm& g) { g.batch = batch; g.strideA = sW; g.strideB = sW; g.strideC = sW; };
   // Two levels: inside an outer block of OB columns every 128-column panel updates only the
@@ -569,14 +599,17 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     const int kend = min(n, K0 + OB);
     for (int k0 = K0; k0 < kend; k0 += NB) {
       const int nb = min(NB, n - k0);
-      potrf_block_kernel<<<batch, 256, POTRF_SMEM, stream>>>(A, ld, k0, nb, status, sW);
+      potrf_block_kernel<<<batch, 256, 0, stream>>>(A, ld, k0, nb, status, sW);
       OC_CHECK_LAUNCH();
       const int rest = n - k0 - nb;
       if (rest <= 0) break;
       float* panel = A + (long long)(k0 + nb) * ld + k0;
       OC_REQUIRE(nb == NB, "hinv_factor: a panel with rows below it is a full panel");
-      trsm_panel_kernel<<<dim3(oc_div_up(rest, TR), batch), TRT, TRSM_SMEM, stream>>>(A, ld, k0, rest, sW);
-      OC_CHECK_LAUNCH();
+      // the fewer rows per CTA, the shorter its time, as long as all CTAs run at once (one or two per SM)
+      const long long row_sets = (long long)oc_div_up(rest, 32) * batch;
+      const int rc_t = row_sets <= 2 * 148 ? launch_trsm<32>(A, ld, k0, rest, batch, sW, stream)
+                                           : launch_trsm<64>(A, ld, k0, rest, batch, sW, stream);
+      if (rc_t) return rc_t;
       const int inner = kend - (k0 + nb);
       if (inner <= 0) continue;
       // columns [k0+nb, kend) of all rows below the panel's diagonal block (lower tiles only)
