@@ -343,15 +343,15 @@ __global__ void __launch_bounds__(256, 1) potrf_block_kernel(float* __restrict__
 //
 // Bound by shared-memory loads (a 16-byte broadcast costs as much as four of 4 bytes, and an entry of L
 // serves one row of a lane) and by the latency of the chain over columns.  With few rows (TR 32) every
-// SM gets its share of them: 13 to 14 us up to 9472 rows, where 128 rows per CTA on a quarter of the SMs
-// took 21.  With more rows two CTAs of 64 share an SM: 23 us for 9472 to 14208 rows, as before (two rows
+// SM gets its share of them: 12 to 13 us up to 9472 rows, where 128 rows per CTA on a quarter of the SMs
+// took 21.  With more rows two CTAs of 64 share an SM: 21 us for 9472 to 14208 rows, as before (two rows
 // per thread pair, which halve the loads of L, were slower for want of warps: 25 us).  Even and odd columns
 // of a row lie apart in shared memory: a thread reads four of its own at once.
 constexpr int TRT = 256;                   // threads per CTA (the first 2 * TR solve, all of them load)
 constexpr int LPITCH = NB + 4, YPITCH = NB + 4;
 template <int TR> constexpr int TRSM_SMEM = (NB * LPITCH + TR * YPITCH + NB) * (int)sizeof(float);
 template <int TR>                          // rows per CTA
-__global__ void __launch_bounds__(TRT) trsm_panel_kernel(float* __restrict__ A, long long lda, int k0, int rest,
+__global__ void __launch_bounds__(TRT, 2) trsm_panel_kernel(float* __restrict__ A, long long lda, int k0, int rest,
                                                          long long sW) {
   A += (long long)blockIdx.y * sW;
   extern __shared__ __align__(16) float sm[];
@@ -389,14 +389,19 @@ __global__ void __launch_bounds__(TRT) trsm_panel_kernel(float* __restrict__ A, 
       f32x2 acc2[4] = {part ? 0ull : pack2(ev.x, od.x), part ? 0ull : pack2(ev.y, od.y),
                        part ? 0ull : pack2(ev.z, od.z), part ? 0ull : pack2(ev.w, od.w)};
       const float* lt = Lt + part * LPITCH + j0;
-#pragma unroll 1
+#pragma unroll 2
       for (int i4 = 0; i4 < j0 / 2; i4 += 4) {      // this thread's columns 2 (i4 + k) + part
         const float4 yv = *reinterpret_cast<const float4*>(y + part * (NB / 2) + i4);
+        float4 lv[4][2];                             // all loads of the step before its arithmetic
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const float4 l0 = *reinterpret_cast<const float4*>(lt + 2 * (i4 + k) * LPITCH);
-          const float4 l1 = *reinterpret_cast<const float4*>(lt + 2 * (i4 + k) * LPITCH + 4);
-          const f32x2 l[4] = {pack2(l0.x, l0.y), pack2(l0.z, l0.w), pack2(l1.x, l1.y), pack2(l1.z, l1.w)};
+          lv[k][0] = *reinterpret_cast<const float4*>(lt + 2 * (i4 + k) * LPITCH);
+          lv[k][1] = *reinterpret_cast<const float4*>(lt + 2 * (i4 + k) * LPITCH + 4);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const f32x2 l[4] = {pack2(lv[k][0].x, lv[k][0].y), pack2(lv[k][0].z, lv[k][0].w),
+                              pack2(lv[k][1].x, lv[k][1].y), pack2(lv[k][1].z, lv[k][1].w)};
           const float yk = k == 0 ? yv.x : k == 1 ? yv.y : k == 2 ? yv.z : yv.w;
           const f32x2 ny = pack2(-yk, -yk);
 #pragma unroll
