@@ -183,8 +183,9 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // the update itself, so one loop body serves all micro-panels.  The operations on an entry are those of a
 // column-by-column elimination, in its order.
 // With 8 x 8 register blocks per thread, a single lane factoring the pivot block and half of the
-// lanes idle above the diagonal this took 31.5 us; now 25 us (per micro-panel 0.5 us of pivot chain, 0.6 us of
-// update, which shared-memory broadcasts bound: an entry of L loaded serves one row per lane).
+// lanes idle above the diagonal this took 31.5 us; now 25 us, of which the chain
+// from pivot to pivot is half (100 cycles a column) and the waits of the update (loads, eight dependent FMAs)
+// most of the rest.
 constexpr int LP = NB + 4;     // pitch of the published columns
 __global__ void __launch_bounds__(256, 1) potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb,
                                                           int* __restrict__ status, long long sW) {
@@ -341,9 +342,9 @@ __global__ void __launch_bounds__(256, 1) potrf_block_kernel(float* __restrict__
 // diagonal block, so the tile loads as it is (coalesced, no transposition) and the inner loop
 // reads eight consecutive entries L[j0..j0+7][i] as two broadcast vector loads.  Plain fp32 FMAs.
 //
-// Bound by shared-memory loads (a 16-byte broadcast costs as much as four of 4 bytes, and an entry of L
-// serves one row of a lane) and by the latency of the chain over columns.  With few rows (TR 32) every
-// SM gets its share of them: 12 to 13 us up to 9472 rows, where 128 rows per CTA on a quarter of the SMs
+// Bound by the latency of the chain over columns and by shared-memory loads (an entry of L serves one row
+// of a lane).  With few rows (TR 32) every SM gets its share of them: 12 to 13 us up to 9472 rows, where
+// 128 rows per CTA on a quarter of the SMs
 // took 21.  With more rows two CTAs of 64 share an SM: 21 us for 9472 to 14208 rows, as before (two rows
 // per thread pair, which halve the loads of L, were slower for want of warps: 25 us).  Even and odd columns
 // of a row lie apart in shared memory: a thread reads four of its own at once.
