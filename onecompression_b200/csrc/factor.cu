@@ -175,81 +175,62 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // from there).  A non-positive or non-finite pivot records (global index + 1) in *status (first one
 // wins); what is computed behind it means nothing, and no kernel of the chain waits for a value.
 //
-// A serial chain on one SM, 16 micro-panels of eight columns.  Two threads hold a row, in registers,
-// each every other group of four columns.  Per micro-panel the eight pivot rows publish their
-// 8 x 8 block; every thread factors it for itself (36 values, no further exchange) and solves its row
-// against it; the eight new columns go to shared memory, and every thread updates the rest of its
-// row, two columns per FMA instruction (fma.f32x2).  The register file moves eight columns to the left in
-// the update itself, so one loop body serves all micro-panels.  The operations on an entry are those of a
-// column-by-column elimination, in its order.
-// With 8 x 8 register blocks per thread, a single lane factoring the pivot block and half of the
-// lanes idle above the diagonal this took 31.5 us; now 25 us, of which the chain
-// from pivot to pivot is half (100 cycles a column) and the waits of the update (loads, eight dependent FMAs)
-// most of the rest.
+// A serial chain on one SM, 16 micro-panels of eight columns.  Its core is the chain from pivot block to
+// pivot block (factor 8 x 8, solve the next eight rows against it, update their own 8 x 8 block, factor
+// that), about 1000 cycles a step: a ninth warp walks it alone, one step ahead.  Of the other eight, two
+// threads hold a row in registers, each every other group of four columns: they solve their row against the
+// published pivot block, publish the eight new columns and update the rest of the row (two columns per
+// FMA instruction, fma.f32x2), beginning with the two groups that the pivot warp needs next.  The
+// register file moves eight columns to the left in the update itself, so one loop body serves all
+// micro-panels.  The operations on an entry are those of a column-by-column elimination, in its order.
+// With 8 x 8 register blocks per thread and a single lane factoring the pivot block this took 31.5 us, with
+// every thread factoring it for itself 25 us; now 17 us, about 1050 cycles a step on the pivot warp and up to
+// 2000 in the first steps on the rows (an entry of L that is loaded, 4 bytes to 32 lanes a cycle, serves one row).
 constexpr int LP = NB + 4;     // pitch of the published columns
-__global__ void __launch_bounds__(256, 1) potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb,
-                                                          int* __restrict__ status, long long sW) {
+constexpr int ROW_THREADS = 256;
+
+// reads the lower part of an 8 x 8 block
+__device__ __forceinline__ void load_block8(const float (*m)[8], float (&l)[8][8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float4 lo = *reinterpret_cast<const float4*>(&m[i][0]);
+    l[i][0] = lo.x; l[i][1] = lo.y; l[i][2] = lo.z; l[i][3] = lo.w;
+    if (i >= 4) {
+      const float4 hi = *reinterpret_cast<const float4*>(&m[i][4]);
+      l[i][4] = hi.x; l[i][5] = hi.y; l[i][6] = hi.z; l[i][7] = hi.w;
+    }
+  }
+}
+
+// y <- y L^-T for one row of eight entries; the diagonal of l holds the reciprocals of L's
+__device__ __forceinline__ void solve_row8(float (&y)[8], const float (&l)[8][8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    y[j] *= l[j][j];
+#pragma unroll
+    for (int c = j + 1; c < 8; ++c) y[c] = fmaf(-y[j], l[c][j], y[c]);
+  }
+}
+
+__global__ void __launch_bounds__(ROW_THREADS + 32, 1)
+potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb, int* __restrict__ status, long long sW) {
   A += (long long)blockIdx.x * sW;
   status += blockIdx.x;
-  __shared__ __align__(16) float Lp[8 * LP + 16];   // the micro-panel's columns, [8][row]
-  __shared__ __align__(16) float Pv[8][8];     // its pivot block
+  __shared__ __align__(16) float Lp[8 * LP + 16];  // the micro-panel's columns, [8][row]
+  __shared__ __align__(16) float L8[2][8][8];      // its factored pivot block, reciprocals on the diagonal
+  __shared__ __align__(16) float Qs[2][8][8];      // the next pivot rows: their entries in the micro-panel,
+  __shared__ __align__(16) float Pre[2][8][8];     //   and their own block, without this micro-panel's update
+  __shared__ __align__(16) float Xs[8][8], Nv[8][8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = lane >> 4, r = warp * 16 + (lane & 15);    // this thread: row r, columns 8q + 4h .. 8q + 4h + 3
-  float* Ab = A + (long long)k0 * lda + k0;
-  float* Ar = Ab + (long long)r * lda;
 
-  f32x2 a[32];                                 // a[2q], a[2q + 1]: group q of the remaining columns
-#pragma unroll
-  for (int q = 0; q < 16; ++q) {
-    const int c = 8 * q + 4 * h;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c <= r) {
-      if (nb == NB) v = *reinterpret_cast<const float4*>(Ar + c);
-      else if (r < nb) {
-        v.x = Ar[c];                           // c <= r < nb
-        if (c + 1 < nb) v.y = Ar[c + 1];
-        if (c + 2 < nb) v.z = Ar[c + 2];
-        if (c + 3 < nb) v.w = Ar[c + 3];
-      } else if (r - c < 4) {                  // rows behind the block: identity
-        v.x = r == c ? 1.f : 0.f; v.y = r == c + 1 ? 1.f : 0.f; v.z = r == c + 2 ? 1.f : 0.f; v.w = r == c + 3 ? 1.f : 0.f;
-      }
-    }
-    a[2 * q] = pack2(v.x, v.y);
-    a[2 * q + 1] = pack2(v.z, v.w);
-  }
-  if (r < 8) {
-    const float2 lo = unpack2(a[0]), hi = unpack2(a[1]);
-    *reinterpret_cast<float4*>(&Pv[r][4 * h]) = make_float4(lo.x, lo.y, hi.x, hi.y);
-  }
-  __syncthreads();
-
+  if (warp == ROW_THREADS / 32) {
+    // ---- pivot warp: every lane factors the pivot block for itself ----
+    __syncthreads();                               // Nv (block 0), Qs[0], Pre[0] are there
 #pragma unroll 1
-  for (int jb = 0; jb < NB / 8; ++jb) {
-    const int j0 = 8 * jb;
-    float y[8];
-    const bool live = warp * 16 + 15 >= j0;    // the same for the whole warp
-    if (live) {
+    for (int jb = 0; jb < NB / 8; ++jb) {
       float l[8][8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 lo = *reinterpret_cast<const float4*>(&Pv[i][0]);
-        l[i][0] = lo.x; l[i][1] = lo.y; l[i][2] = lo.z; l[i][3] = lo.w;
-        if (i >= 4) {
-          const float4 hi = *reinterpret_cast<const float4*>(&Pv[i][4]);
-          l[i][4] = hi.x; l[i][5] = hi.y; l[i][6] = hi.z; l[i][7] = hi.w;
-        }
-      }
-      {
-        const float2 m0 = unpack2(a[0]), m1 = unpack2(a[1]);
-        const float mine[4] = {m0.x, m0.y, m1.x, m1.y};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float other = __shfl_xor_sync(0xffffffffu, mine[i], 16);
-          y[i] = h ? other : mine[i];
-          y[4 + i] = h ? mine[i] : other;
-        }
-      }
-      int bad = 8;                             // first column with an unusable pivot
+      load_block8(Nv, l);
+      int bad = 8;                                 // first column with an unusable pivot
 #pragma unroll
       for (int jj = 0; jj < 8; ++jj) {
         // (selections, not branches: the eight columns are one stretch of code, whose instructions
@@ -261,44 +242,122 @@ __global__ void __launch_bounds__(256, 1) potrf_block_kernel(float* __restrict__
         // root followed by IEEE divisions
         float inv = rsqrtf(p);
         inv = inv * fmaf(-0.5f * p * inv, inv, 1.5f);
+        l[jj][jj] = inv;
 #pragma unroll
         for (int ii = jj + 1; ii < 8; ++ii) l[ii][jj] *= inv;
 #pragma unroll
         for (int cc = jj + 1; cc < 8; ++cc)
 #pragma unroll
           for (int ii = cc; ii < 8; ++ii) l[ii][cc] = fmaf(-l[ii][jj], l[cc][jj], l[ii][cc]);
-        // this row's entry of column jj, then its part in the columns behind
-        y[jj] *= inv;
-        if (r == j0 + jj) y[jj] = p * inv;
-#pragma unroll
-        for (int cc = jj + 1; cc < 8; ++cc) y[cc] = fmaf(-y[jj], l[cc][jj], y[cc]);
       }
-      if (bad < 8 && r == j0 && h == 0) atomicCAS(status, 0, k0 + j0 + bad + 1);
+      if (bad < 8 && lane == 0) atomicCAS(status, 0, k0 + 8 * jb + bad + 1);
+      if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          *reinterpret_cast<float4*>(&L8[jb & 1][i][0]) = make_float4(l[i][0], l[i][1], l[i][2], l[i][3]);
+          if (i >= 4) *reinterpret_cast<float4*>(&L8[jb & 1][i][4]) = make_float4(l[i][4], l[i][5], l[i][6], l[i][7]);
+        }
+      }
+      __syncthreads();                             // L8(jb) to the rows; Qs(jb), Pre(jb) from them
+      if (jb == NB / 8 - 1) break;
+      float x[8];
+      {
+        const float4 lo = *reinterpret_cast<const float4*>(&Qs[jb & 1][lane & 7][0]);
+        const float4 hi = *reinterpret_cast<const float4*>(&Qs[jb & 1][lane & 7][4]);
+        x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w; x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+      }
+      solve_row8(x, l);
+      if (lane < 8) {
+        *reinterpret_cast<float4*>(&Xs[lane][0]) = make_float4(x[0], x[1], x[2], x[3]);
+        *reinterpret_cast<float4*>(&Xs[lane][4]) = make_float4(x[4], x[5], x[6], x[7]);
+      }
+      __syncwarp();
+      // entries (r, c) and (r + 4, c) of the next pivot block
+      const int r = lane >> 3, c = lane & 7;
+      float v0 = Pre[jb & 1][r][c], v1 = Pre[jb & 1][r + 4][c];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 a0 = *reinterpret_cast<const float4*>(&Xs[r][4 * h]);
+        const float4 a1 = *reinterpret_cast<const float4*>(&Xs[r + 4][4 * h]);
+        const float4 bc = *reinterpret_cast<const float4*>(&Xs[c][4 * h]);
+        v0 = fmaf(-a0.x, bc.x, v0); v1 = fmaf(-a1.x, bc.x, v1);
+        v0 = fmaf(-a0.y, bc.y, v0); v1 = fmaf(-a1.y, bc.y, v1);
+        v0 = fmaf(-a0.z, bc.z, v0); v1 = fmaf(-a1.z, bc.z, v1);
+        v0 = fmaf(-a0.w, bc.w, v0); v1 = fmaf(-a1.w, bc.w, v1);
+      }
+      Nv[r][c] = v0;
+      Nv[r + 4][c] = v1;
+      __syncwarp();
+    }
+    return;
+  }
+
+  // ---- row threads: row r, columns 8q + 4h .. 8q + 4h + 3 ----
+  const int h = lane >> 4, r = warp * 16 + (lane & 15);
+  float* Ab = A + (long long)k0 * lda + k0;
+  float* Ar = Ab + (long long)r * lda;
+  f32x2 a[32];                                 // a[2q], a[2q + 1]: group q of the remaining columns
+  if (nb == NB) {
+    float4 v[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (8 * q + 4 * h <= r) v[q] = *reinterpret_cast<const float4*>(Ar + 8 * q + 4 * h);
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) { a[2 * q] = pack2(v[q].x, v[q].y); a[2 * q + 1] = pack2(v[q].z, v[q].w); }
+  } else {                                     // rows and columns behind the block: identity
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      float v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int c = 8 * q + 4 * h + i;
+        v[i] = (c <= r && r < nb) ? Ar[c] : (r == c ? 1.f : 0.f);
+      }
+      a[2 * q] = pack2(v[0], v[1]);
+      a[2 * q + 1] = pack2(v[2], v[3]);
+    }
+  }
+  auto publish = [&](float (*to)[8], f32x2 v0, f32x2 v1) {
+    const float2 lo = unpack2(v0), hi = unpack2(v1);
+    *reinterpret_cast<float4*>(&to[r & 7][4 * h]) = make_float4(lo.x, lo.y, hi.x, hi.y);
+  };
+  if (r < 8) publish(Nv, a[0], a[1]);
+  else if (r < 16) {
+    publish(Qs[0], a[0], a[1]);
+    publish(Pre[0], a[2], a[3]);
+  }
+  __syncthreads();
+
+#pragma unroll 1
+  for (int jb = 0; jb < NB / 8; ++jb) {
+    const int j0 = 8 * jb;
+    float y[8];
+    const bool live = warp * 16 + 15 >= j0;    // the same for the whole warp
+    __syncthreads();                           // L8(jb) from the pivot warp; the rows' columns are up to date
+    if (live) {
+      float l[8][8];
+      load_block8(L8[jb & 1], l);
+      {
+        const float2 m0 = unpack2(a[0]), m1 = unpack2(a[1]);
+        const float mine[4] = {m0.x, m0.y, m1.x, m1.y};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float other = __shfl_xor_sync(0xffffffffu, mine[i], 16);
+          y[i] = h ? other : mine[i];
+          y[4 + i] = h ? mine[i] : other;
+        }
+      }
+      solve_row8(y, l);
       const float4 m = h ? make_float4(y[4], y[5], y[6], y[7]) : make_float4(y[0], y[1], y[2], y[3]);
       const float mv[4] = {m.x, m.y, m.z, m.w};
-      const int c = j0 + 4 * h;                // columns c .. c + 3 are this thread's to store
       if (r >= j0 + 8) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) Lp[(4 * h + i) * LP + r] = mv[i];
-        if (nb == NB) *reinterpret_cast<float4*>(Ar + c) = m;
-        else if (r < nb) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) Ar[c + i] = mv[i];       // c + i < r < nb
-        }
-        if (r < nb) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) Ab[(long long)(c + i) * lda + r] = mv[i];
-        }
-      } else if (r >= j0 && r < nb) {          // pivot rows: up to the diagonal
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (c + i <= r) {
-            Ar[c + i] = mv[i];
-            Ab[(long long)(c + i) * lda + r] = mv[i];
-          }
       }
     }
-    __syncthreads();
+    asm volatile("bar.sync 1, 256;" ::: "memory");     // the row threads: Lp is there
     if (live) {
       f32x2 ny[8];
 #pragma unroll
@@ -322,14 +381,34 @@ __global__ void __launch_bounds__(256, 1) potrf_block_kernel(float* __restrict__
           }
           a[2 * q] = v[0]; a[2 * q + 1] = v[1];
           a[2 * q + 2] = v[2]; a[2 * q + 3] = v[3];
-          if (q == 0 && (r >> 3) == jb + 1) {
-            const float2 lo = unpack2(v[0]), hi = unpack2(v[1]);
-            *reinterpret_cast<float4*>(&Pv[r & 7][4 * h]) = make_float4(lo.x, lo.y, hi.x, hi.y);
+          if (q == 0 && (r >> 3) == jb + 2) {
+            publish(Qs[(jb + 1) & 1], v[0], v[1]);
+            publish(Pre[(jb + 1) & 1], v[2], v[3]);
           }
         }
       }
+      // the new columns go to global memory while the pivot warp is at work
+      const int c = j0 + 4 * h;                // columns c .. c + 3 are this thread's to store
+      const float mv[4] = {h ? y[4] : y[0], h ? y[5] : y[1], h ? y[6] : y[2], h ? y[7] : y[3]};
+      if (r >= j0 + 8) {
+        if (nb == NB) *reinterpret_cast<float4*>(Ar + c) = make_float4(mv[0], mv[1], mv[2], mv[3]);
+        else if (r < nb) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) Ar[c + i] = mv[i];       // c + i < r < nb
+        }
+        if (r < nb) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) Ab[(long long)(c + i) * lda + r] = mv[i];
+        }
+      } else if (r >= j0 && r < nb) {          // pivot rows: up to the diagonal
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (c + i <= r) {
+            Ar[c + i] = mv[i];
+            Ab[(long long)(c + i) * lda + r] = mv[i];
+          }
+      }
     }
-    __syncthreads();
   }
 }
 
@@ -605,7 +684,7 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     const int kend = min(n, K0 + OB);
     for (int k0 = K0; k0 < kend; k0 += NB) {
       const int nb = min(NB, n - k0);
-      potrf_block_kernel<<<batch, 256, 0, stream>>>(A, ld, k0, nb, status, sW);
+      potrf_block_kernel<<<batch, ROW_THREADS + 32, 0, stream>>>(A, ld, k0, nb, status, sW);
       OC_CHECK_LAUNCH();
       const int rest = n - k0 - nb;
       if (rest <= 0) break;
