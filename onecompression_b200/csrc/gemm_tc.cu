@@ -308,13 +308,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       const int n_chunks = max(1, (n_stages + CHAIN_STAGES - 1) / CHAIN_STAGES);
       const bool in_use = half == 0 || upper_half_in_use<BN>(p, m0, n0);
       float* out_tile = p.C + (long long)z * p.strideC;
-      if (p.beta != 0.f && in_use && m0 + quarter * 32 + lane < p.M) {
-        // the rows of C that this warp will read are on their way from HBM during the products
-        const float* c_row = out_tile + (long long)(m0 + quarter * 32 + lane) * p.ldc;
-#pragma unroll
-        for (int c = 0; c < DW; c += 32)
-          if (n0 + half * DW + c < p.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(c_row + n0 + half * DW + c));
-      }
+      if (in_use && p.beta != 0.f) prefetch_tile<DW>(out_tile, p.ldc, p.M, p.N, m0 + quarter * 32, n0 + half * DW, lane);
       float acc[DW];
 #pragma unroll
       for (int i = 0; i < DW; ++i) acc[i] = 0.f;
@@ -339,70 +333,9 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
       if (!ok) break;
       if (!in_use) continue;
-      // Epilogue.  A drain thread holds one row of the tile, so writing from the registers would
-      // touch 32 rows per instruction.  Each warp instead passes 32 x 32 slices through 4 KB of
-      // shared memory of its own (16-byte chunks swizzled by row, conflict-free both ways) and
-      // reads / writes C with four full 128-byte row segments per instruction.
       float4* stg = reinterpret_cast<float4*>(stage_ptr + STAGES * STAGE_BYTES) + (warp - S::FIRST_DRAIN) * 256;
-      const float alpha = p.alpha, beta = p.beta;
-      const int sub = lane >> 3, chunk = lane & 7;
-      // What bounds a product with few k-values is this epilogue: it waited for the old values of C eight
-      // times a tile, from HBM.  They are now in L2 by then (prefetched above), fetched AHEAD groups (16
-      // rows of a slice) before they are needed, and narrow tiles have eight drain warps instead of four:
-      // 28672 x 384 x 128 43.6 -> 36.4 us, rank-512 update of 3584 x 3584 73.9 -> 63.7 us.
-      constexpr int GROUPS = DW / 32 * 2, AHEAD = S::EPILOGUE_AHEAD;
-      float4 old[AHEAD][4];
-      auto fetch_old = [&](int grp, float4 (&to)[4]) {
-        const int col = n0 + half * DW + (grp >> 1) * 32 + chunk * 4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = m0 + quarter * 32 + ((grp & 1) * 4 + i) * 4 + sub;
-          to[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (beta != 0.f && row < p.M && col + 3 < p.N)
-            to[i] = *reinterpret_cast<const float4*>(out_tile + (long long)row * p.ldc + col);
-        }
-      };
-#pragma unroll
-      for (int g = 0; g < AHEAD; ++g) fetch_old(g, old[g]);
-#pragma unroll
-      for (int g = 0; g < GROUPS; ++g) {
-        const int c = g >> 1;
-        if ((g & 1) == 0) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float4 o;
-            o.x = alpha * acc[c * 32 + j * 4 + 0]; o.y = alpha * acc[c * 32 + j * 4 + 1];
-            o.z = alpha * acc[c * 32 + j * 4 + 2]; o.w = alpha * acc[c * 32 + j * 4 + 3];
-            stg[lane * 8 + (j ^ (lane & 7))] = o;
-          }
-          __syncwarp();
-        }
-        const int col = n0 + half * DW + c * 32 + chunk * 4;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int r = ((g & 1) * 4 + i) * 4 + sub;
-          const int row = m0 + quarter * 32 + r;
-          const float4 o = stg[r * 8 + (chunk ^ (r & 7))];
-          if (row >= p.M) continue;
-          float* out = out_tile + (long long)row * p.ldc + col;
-          if (col + 3 < p.N) {
-            float4 v = o;
-            if (beta != 0.f) {
-              const float4 q = old[g % AHEAD][i];
-              v.x = fmaf(beta, q.x, v.x); v.y = fmaf(beta, q.y, v.y);
-              v.z = fmaf(beta, q.z, v.z); v.w = fmaf(beta, q.w, v.w);
-            }
-            *reinterpret_cast<float4*>(out) = v;
-          } else {
-            const float e[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              if (col + j < p.N) out[j] = (beta != 0.f) ? fmaf(beta, out[j], e[j]) : e[j];
-          }
-        }
-        if (g + AHEAD < GROUPS) fetch_old(g + AHEAD, old[g % AHEAD]);
-        if (g & 1) __syncwarp();
-      }
+      store_tile<DW, S::EPILOGUE_AHEAD>(out_tile, p.ldc, p.M, p.N, p.alpha, p.beta, acc, stg, m0 + quarter * 32,
+                                        n0 + half * DW, lane);
     }
   }
 

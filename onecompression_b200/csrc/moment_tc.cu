@@ -48,7 +48,7 @@ constexpr int TILE_M = 128, TILE_N = 256, BK = 64, STAGES = 4;
 constexpr int ATOM_BYTES = BK * 128;                     // one 64-column x BK-token box
 constexpr int A_ATOMS = TILE_M / 64, B_ATOMS = TILE_N / 64;
 constexpr int STAGE_BYTES = (A_ATOMS + B_ATOMS) * ATOM_BYTES;
-constexpr int SMEM_DYN = STAGES * STAGE_BYTES + 1024;
+constexpr int SMEM_DYN = STAGES * STAGE_BYTES + 1024 + 8 * 4096;   // ring, its alignment, 4 KB per drain warp
 constexpr int NUM_THREADS = 320;
 constexpr uint32_t IDESC = (1u << 4) | (1u << 15) | (1u << 16) | ((TILE_N >> 3) << 17) | ((TILE_M >> 4) << 24);
 
@@ -221,11 +221,14 @@ moment_tc_kernel(const __grid_constant__ CUtensorMap map_xq, const __grid_consta
     const int e = warp - 2;
     const int quarter = warp & 3;
     const int half = e >> 2;
+    float4* stg = reinterpret_cast<float4*>(smem_raw + (stage_base - smem_u32(smem_raw)) + STAGES * STAGE_BYTES) + e * 256;
     uint32_t cc = 0;
     bool ok = true;
     for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
       int is_c, m0, n0;
       decode_item(p, item, is_c, m0, n0);
+      float* out = is_c ? p.C : p.H;
+      if (p.a_old != 0.f) prefetch_tile<128>(out, p.ldh, p.d, p.d, m0 + quarter * 32, n0 + half * 128, lane);
       float acc[128];
 #pragma unroll
       for (int i = 0; i < 128; ++i) acc[i] = 0.f;
@@ -251,26 +254,10 @@ moment_tc_kernel(const __grid_constant__ CUtensorMap map_xq, const __grid_consta
         if (lane == 0) mbar_arrive(smem_u32(&bar_acc_empty[buf]));
       }
       if (!ok) break;
-      const int row = m0 + quarter * 32 + lane;
-      if (row < p.d) {
-        float* out = (is_c ? p.C : p.H) + (long long)row * p.ldh;
-        const int cbase = n0 + half * 128;
-#pragma unroll
-        for (int c4 = 0; c4 < 32; ++c4) {
-          const int col = cbase + c4 * 4;
-          if (col < p.d) {  // d is a multiple of 8, so a float4 is inside or outside as a whole
-            float4 o;
-            o.x = p.a_new * acc[c4 * 4 + 0]; o.y = p.a_new * acc[c4 * 4 + 1];
-            o.z = p.a_new * acc[c4 * 4 + 2]; o.w = p.a_new * acc[c4 * 4 + 3];
-            if (p.a_old != 0.f) {
-              const float4 old = *reinterpret_cast<const float4*>(out + col);
-              o.x = fmaf(p.a_old, old.x, o.x); o.y = fmaf(p.a_old, old.y, o.y);
-              o.z = fmaf(p.a_old, old.z, o.z); o.w = fmaf(p.a_old, old.w, o.w);
-            }
-            *reinterpret_cast<float4*>(out + col) = o;
-          }
-        }
-      }
+      // Whole row segments instead of 16 bytes of 32 rows an instruction, old values on their way from HBM
+      // meanwhile: H and C at d = 5120, two chunks of 4096 tokens, 1004 -> 897 us.
+      // (d is a multiple of 8 and rows are 16-byte aligned: four columns are inside or outside as a whole)
+      store_tile<128, 1>(out, p.ldh, p.d, p.d, p.a_new, p.a_old, acc, stg, m0 + quarter * 32, n0 + half * 128, lane);
     }
   }
 

@@ -66,8 +66,11 @@ class MomentAccumulator:
         self.device = torch.device(device)
         if self.device.type != "cuda":
             raise RuntimeError("MomentAccumulator needs a CUDA device (no CPU path)")
-        self.H = torch.zeros((d, d), dtype=torch.float32, device=self.device)
-        self.C = torch.zeros((d, d), dtype=torch.float32, device=self.device) if cross else None
+        # not cleared: the first chunk enters with weight 0 for what was there, which the kernels
+        # take as "do not read it"
+        self._h = torch.empty((d, d), dtype=torch.float32, device=self.device)
+        self._c = torch.empty((d, d), dtype=torch.float32, device=self.device) if cross else None
+        self._written = False
         self.nsamples = 0
         self.chunk_tokens = chunk_tokens
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
@@ -78,6 +81,23 @@ class MomentAccumulator:
         self._scratch = None
         self._needs_mirror = False
 
+    def _clear_unwritten(self):
+        if not self._written:
+            self._h.zero_()
+            if self._c is not None:
+                self._c.zero_()
+            self._written = True
+
+    @property
+    def H(self):
+        self._clear_unwritten()
+        return self._h
+
+    @property
+    def C(self):
+        self._clear_unwritten()
+        return self._c
+
     def add(self, xq: torch.Tensor, xf: Optional[torch.Tensor] = None):
         """Fold a chunk of activations ([..., d], fp16) into the moments."""
         if xq.shape[-1] != self.d:
@@ -86,7 +106,7 @@ class MomentAccumulator:
         t = xq.shape[0]
         if t == 0:
             return
-        cross = self.C is not None
+        cross = self._c is not None
         if cross:
             if xf is None:
                 raise ValueError("this accumulator also builds the cross term: pass xf")
@@ -112,9 +132,10 @@ class MomentAccumulator:
         with torch.cuda.device(self.device):
             call(
                 "oc_moment_accum", ptr(xq), ptr(xf) if cross else None, ptr(scratch), t, self.d,
-                xq.stride(0), ptr(self.H), ptr(self.C), self.d, a_old, a_new, self.chunk_tokens,
+                xq.stride(0), ptr(self._h), ptr(self._c), self.d, a_old, a_new, self.chunk_tokens,
                 sm_count(self.device), self.engine, _DTYPES[xq.dtype], ptr(self.status), stream_handle(),
             )
+        self._written = True
         self._needs_mirror = not self.force_simt
 
     def _as_rows(self, x: torch.Tensor) -> torch.Tensor:
@@ -128,16 +149,17 @@ class MomentAccumulator:
 
     def finalize(self, check: bool = True):
         """Complete H (mirror the upper triangle) and return (H, C, nsamples)."""
+        self._clear_unwritten()
         if self._needs_mirror:
             with torch.cuda.device(self.device):
-                call("oc_mirror_upper", ptr(self.H), self.d, self.d, stream_handle())
+                call("oc_mirror_upper", ptr(self._h), self.d, self.d, stream_handle())
             self._needs_mirror = False
         if check:
             code = int(self.status.item())
             if code != 0:
                 raise RuntimeError(f"moment kernel: a bounded pipeline wait expired (code {code})")
         self._scratch = None
-        return self.H, self.C, self.nsamples
+        return self._h, self._c, self.nsamples
 
 
 def hessian_from_activations(x: torch.Tensor, seqs_per_slice: int = 8, **kw):

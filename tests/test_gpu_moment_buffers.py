@@ -1,0 +1,48 @@
+"""Moments into buffers that were not cleared: odd widths on both engines, no tokens at all, mirrored lower part."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d", [8, 60, 64, 72, 200, 264, 1000, 57])
+@pytest.mark.parametrize("cross", [False, True])
+@pytest.mark.parametrize("chunks", [(), (1,), (700,), (64, 0, 129)])
+def test_moments_do_not_read_what_was_there(d, cross, chunks):
+    from onecompression_b200 import kernels as K
+
+    dev = torch.device("cuda:0")
+    # leave NaNs where the accumulator is going to be allocated
+    junk = [torch.full((d, d), float("nan"), device=dev) for _ in range(3)]
+    del junk
+    g = torch.Generator().manual_seed(d)
+    acc = K.MomentAccumulator(d, dev, cross=cross)
+    xs = [(torch.randn(t, d, generator=g).half(), torch.randn(t, d, generator=g).half()) for t in chunks]
+    for xq, xf in xs:
+        acc.add(xq.to(dev), xf.to(dev) if cross else None)
+    h, c, n = acc.finalize()
+    assert n == sum(chunks)
+    xq = torch.cat([x for x, _ in xs] + [torch.zeros(0, d).half()]).double()
+    xf = torch.cat([x for _, x in xs] + [torch.zeros(0, d).half()]).double()
+    want = 2 / max(n, 1) * xq.t() @ xq
+    assert torch.equal(h, h.t())
+    # sums of n products in fp32 and truncating tensor-core chains of at most 512 tokens
+    bound = 1e-5 * max(1.0, float(want.abs().max()))
+    assert (h.cpu().double() - want).abs().max() <= bound
+    if cross:
+        want = 2 / max(n, 1) * (xf - xq).t() @ xq
+        assert (c.cpu().double() - want).abs().max() <= 1e-5 * max(1.0, float(want.abs().max()))
+    fresh = K.MomentAccumulator(d, dev, cross=cross)
+    assert not fresh.H.any() and (fresh.C is None or not fresh.C.any())
+
+
+@pytest.mark.parametrize("n,pad", [(1, 0), (3, 1), (64, 0), (65, 3), (130, 2), (1000, 0), (1000, 1)])
+def test_mirror(n, pad):
+    from onecompression_b200._lib import call, ptr, stream_handle
+
+    m = torch.randn(n, n + pad, device="cuda")
+    want = m.clone()
+    want[:, :n] = torch.triu(m[:, :n]) + torch.triu(m[:, :n], 1).t()
+    call("oc_mirror_upper", ptr(m), n + pad, n, stream_handle())
+    assert torch.equal(m, want)
