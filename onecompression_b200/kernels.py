@@ -33,6 +33,26 @@ def sm_count(device) -> int:
     return _sm_count_cache[idx]
 
 
+class _on:
+    """``torch.cuda.device`` for the calls below, at little cost when ``device`` is current already (a
+    call is often shorter than the context manager)."""
+
+    __slots__ = ("_other",)
+
+    def __init__(self, device):
+        device = torch.device(device)
+        same = device.type == "cuda" and (device.index is None or device.index == torch.cuda.current_device())
+        self._other = None if same else torch.cuda.device(device)
+
+    def __enter__(self):
+        if self._other is not None:
+            self._other.__enter__()
+
+    def __exit__(self, *exc):
+        if self._other is not None:
+            self._other.__exit__(*exc)
+
+
 def _require_cuda(t: torch.Tensor, what: str):
     if not t.is_cuda:
         raise RuntimeError(
@@ -129,7 +149,7 @@ class MomentAccumulator:
             if self._scratch is None or self._scratch.numel() < need or self._scratch.dtype != xq.dtype:
                 self._scratch = torch.empty(need, dtype=xq.dtype, device=self.device)
             scratch = self._scratch
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             call(
                 "oc_moment_accum", ptr(xq), ptr(xf) if cross else None, ptr(scratch), t, self.d,
                 xq.stride(0), ptr(self._h), ptr(self._c), self.d, a_old, a_new, self.chunk_tokens,
@@ -151,7 +171,7 @@ class MomentAccumulator:
         """Complete H (mirror the upper triangle) and return (H, C, nsamples)."""
         self._clear_unwritten()
         if self._needs_mirror:
-            with torch.cuda.device(self.device):
+            with _on(self.device):
                 call("oc_mirror_upper", ptr(self._h), self.d, self.d, stream_handle())
             self._needs_mirror = False
         if check:
@@ -236,7 +256,7 @@ def factor_hessian(h: torch.Tensor, percdamp: float, actorder: bool, max_retries
     dead = torch.empty(d, dtype=torch.uint8, device=dev)
     damp = torch.empty(2, dtype=torch.float32, device=dev)
     status = torch.empty(1, dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         nbytes = _lib.load().oc_hinv_workspace_bytes(d)
         ws = _workspace(nbytes, dev)
         rel, mult = 1.0, 1.0
@@ -281,7 +301,7 @@ def factor_hessians_batched(hs: torch.Tensor, percdamp: float, actorder: bool) -
            "dead": torch.empty((batch, n), dtype=torch.uint8, device=dev),
            "damp": torch.empty((batch, 2), dtype=torch.float32, device=dev),
            "status": torch.empty(batch, dtype=torch.int32, device=dev)}
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws = _workspace(_lib.load().oc_hinv_workspace_bytes(n) * batch, dev)
         call("oc_hinv_factor_batched", batch, ptr(hs), n, float(percdamp), 1 if actorder else 0, ptr(out["u"]),
              ptr(out["perm"]), ptr(out["invperm"]), ptr(out["dead"]), ptr(out["damp"]), ptr(out["status"]),
@@ -310,7 +330,7 @@ def factor_hessian_launch(h: torch.Tensor, percdamp: float, actorder: bool, buff
         "status": torch.empty(1, dtype=torch.int32, device=dev),
         "percdamp": float(percdamp), "actorder": bool(actorder),
     }
-    with torch.cuda.device(dev):
+    with _on(dev):
         ws = _workspace(_lib.load().oc_hinv_workspace_bytes(d), dev)
         call("oc_hinv_factor", ptr(h), h.stride(0), d, float(percdamp), 1.0, 1 if actorder else 0, 0,
              ptr(out["u"]), d, ptr(out["perm"]), ptr(out["invperm"]), ptr(out["dead"]), ptr(out["damp"]),
@@ -401,7 +421,7 @@ def gptq_quantize(
     if want_dequantized and "dequantized" not in outputs:
         outputs["dequantized"] = torch.empty((out, d), dtype=weight.dtype, device=dev)
     deq = outputs.get("dequantized")
-    with torch.cuda.device(dev):
+    with _on(dev):
         nbytes = _lib.load().oc_gptq_workspace_bytes(out, d, groupsize)
         ws = _workspace(nbytes, dev)
         call(
@@ -446,7 +466,7 @@ def gptq_quantize_batched(weights: torch.Tensor, u: torch.Tensor, dead: torch.Te
         res["qzeros"] = torch.empty((batch, groups, out * wbits // 32), dtype=torch.int32, device=dev)
     else:
         res["codes"] = torch.empty((batch, out, d), dtype=torch.int32, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         nbytes = _lib.load().oc_gptq_workspace_bytes(out, d, groupsize) * batch
         ws = _workspace(nbytes, dev)
         call("oc_gptq_quantize_batched", batch, ptr(weights), d, out, d, ptr(u), d, ptr(perm), ptr(invperm),
@@ -471,7 +491,7 @@ def qep_adjust(weight: torch.Tensor, c: torch.Tensor, factor: HessianFactor, per
         c = c.float().contiguous()
     out, d = weight.shape
     dev = weight.device
-    with torch.cuda.device(dev):
+    with _on(dev):
         for r0 in range(0, out, 65535 // 32 * 32):
             rows = min(65535 // 32 * 32, out - r0)
             nbytes = _lib.load().oc_qep_workspace_bytes(rows, d)
@@ -505,7 +525,7 @@ def rtn_quantize(weight: torch.Tensor, wbits: int, groupsize: int, sym: bool):
         "zeros": torch.empty((out, groups), dtype=torch.float32, device=dev),
         "dequantized": torch.empty((out, d), dtype=weight.dtype, device=dev),
     }
-    with torch.cuda.device(dev):
+    with _on(dev):
         call("oc_rtn_quantize", ptr(weight), weight.stride(0), out, d, wbits, groupsize, 1 if sym else 0,
              ptr(res["scales"]), ptr(res["zeros"]), ptr(res["codes"]), ptr(res["dequantized"]),
              _DTYPES[weight.dtype], stream_handle())
@@ -533,7 +553,7 @@ def pack_qweight(codes: torch.Tensor, wbits: int) -> torch.Tensor:
         assert d % f == 0, f"rows ({d}) must be divisible by pack_factor ({f})"
     codes = codes.to(torch.int32).contiguous()
     q = torch.empty((d * wbits // 32, out), dtype=torch.int32, device=codes.device)
-    with torch.cuda.device(codes.device):
+    with _on(codes.device):
         call("oc_pack_qweight", ptr(codes), out, d, wbits, ptr(q), stream_handle())
     return q
 
@@ -544,7 +564,7 @@ def unpack_qweight(qweight: torch.Tensor, wbits: int, shape) -> torch.Tensor:
     out, d = int(shape[0]), int(shape[1])
     qweight = qweight.to(torch.int32).contiguous()
     codes = torch.empty((out, d), dtype=torch.int32, device=qweight.device)
-    with torch.cuda.device(qweight.device):
+    with _on(qweight.device):
         call("oc_unpack_qweight", ptr(qweight), out, d, wbits, ptr(codes), stream_handle())
     return codes
 
@@ -559,7 +579,7 @@ def pack_qzeros(zeros: torch.Tensor, wbits: int, add: int = 0) -> torch.Tensor:
         assert out % f == 0, f"rows ({out}) must be divisible by pack_factor ({f})"
     zeros = zeros.to(torch.int32).contiguous()
     q = torch.empty((groups, out * wbits // 32), dtype=torch.int32, device=zeros.device)
-    with torch.cuda.device(zeros.device):
+    with _on(zeros.device):
         call("oc_pack_qzeros", ptr(zeros), groups, out, wbits, add, ptr(q), stream_handle())
     return q
 
@@ -570,7 +590,7 @@ def unpack_qzeros(qzeros: torch.Tensor, wbits: int, out_features: int, add: int 
     qzeros = qzeros.to(torch.int32).contiguous()
     groups = qzeros.shape[0]
     z = torch.empty((groups, out_features), dtype=torch.int32, device=qzeros.device)
-    with torch.cuda.device(qzeros.device):
+    with _on(qzeros.device):
         call("oc_unpack_qzeros", ptr(qzeros), groups, out_features, wbits, add, ptr(z), stream_handle())
     return z
 
@@ -585,7 +605,7 @@ def dequantize_packed(qweight, qzeros, scales, g_idx, wbits: int, shape) -> torc
     if g_idx is not None:
         g_idx = g_idx.to(device=dev, dtype=torch.int32).contiguous()
     w = torch.empty((out, d), dtype=torch.float16, device=dev)
-    with torch.cuda.device(dev):
+    with _on(dev):
         call("oc_dequantize_packed", ptr(qweight), ptr(qzeros), ptr(scales), ptr(g_idx), out, d,
              wbits, ptr(w), d, stream_handle())
     return w
@@ -628,7 +648,7 @@ def packed_linear(x: torch.Tensor, qweight, qzeros, scales, g_idx, bias, wbits: 
     if dev == torch.cuda.current_device():
         call("oc_packed_linear", *args, stream_handle())
     else:
-        with torch.cuda.device(dev):
+        with _on(dev):
             call("oc_packed_linear", *args, stream_handle())
     return y
 
@@ -643,7 +663,7 @@ def rmsnorm_f16(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tens
     if x2.stride(1) != 1:
         x2 = x2.contiguous()
     y = torch.empty((x2.shape[0], d), dtype=torch.float16, device=x.device)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         call("oc_rmsnorm_f16", ptr(x2), x2.stride(0), ptr(weight), float(eps), x2.shape[0], d, ptr(y), d,
              stream_handle())
     return y.view(x.shape)
@@ -683,7 +703,7 @@ def rope_f16(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Ten
         raise TypeError("rope_f16: could not allocate an output with the input's layout")
     b, h, s_len, d = x.shape
     cb = 0 if cos.shape[0] == 1 else cos.stride(0)
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         call("oc_rope_f16", ptr(x), ptr(y), ptr(cos), ptr(sin), b, h, s_len, d, x.stride(0), x.stride(1),
              x.stride(2), y.stride(0), y.stride(1), y.stride(2), cb, cos.stride(1), sm_count(x.device),
              stream_handle())
@@ -698,7 +718,7 @@ def swiglu_f16(gate: torch.Tensor, up: torch.Tensor, inplace: bool = False) -> t
             or not gate.is_contiguous() or not up.is_contiguous() or up.device != gate.device):
         raise TypeError("swiglu_f16 expects two contiguous fp16 tensors of equal shape on one device")
     y = gate if inplace else torch.empty_like(gate)
-    with torch.cuda.device(gate.device):
+    with _on(gate.device):
         call("oc_swiglu_f16", ptr(gate), ptr(up), ptr(y), gate.numel(), sm_count(gate.device), stream_handle())
     return y
 
@@ -764,7 +784,7 @@ class _HostCopier:
             self._bufs[slot] = buf
         pairs, off = [], 0
         # the copies and the event that guards them go to the tensors' own device
-        with torch.cuda.device(todo[0][1].device):
+        with _on(todo[0][1].device):
             for (i, t), sz in zip(todo, sizes):
                 nbytes = t.numel() * t.element_size()
                 view = buf[off : off + nbytes].view(t.dtype).view(t.shape)
@@ -803,13 +823,13 @@ class LayerTimer:
 
     def __init__(self, device):
         self.device = torch.device(device)
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             self.begin = torch.cuda.Event(enable_timing=True)
             self.begin.record()
 
     def stop(self, shares):
         """``shares``: [(result, fraction of the elapsed time that belongs to it)]."""
-        with torch.cuda.device(self.device):
+        with _on(self.device):
             end = torch.cuda.Event(enable_timing=True)
             end.record()
         entry = (self.begin, end, list(shares))
@@ -891,7 +911,7 @@ def gemm_f32(a, b, c=None, alpha=1.0, beta=0.0, trans_a=False, trans_b=False, fl
     n = b.shape[0] if trans_b else b.shape[1]
     if c is None:
         c = torch.zeros((m, n), dtype=torch.float32, device=a.device)
-    with torch.cuda.device(a.device):
+    with _on(a.device):
         call("oc_gemm_f32", ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(c), c.stride(0), m, n, k,
              float(alpha), float(beta), int(trans_a), int(trans_b), int(flags), stream_handle())
     return c
