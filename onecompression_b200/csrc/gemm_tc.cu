@@ -43,18 +43,19 @@ struct Shape {
   static constexpr int SMEM_DYN = STAGES * STAGE_BYTES + 1024 + DRAIN_WARPS * 4096;
   static constexpr int FIRST_DRAIN = FIRST_SPLIT + SPLIT_WARPS;
   // With 16 warps the register file gives 128 registers per thread at launch, fewer than a drain
-  // thread needs for its 128 partial sums: the warpgroups then trade registers (setmaxnreg).
-  static constexpr bool TRADE_REGISTERS = FIRST_SPLIT == 4;
+  // thread needs for its partial sums and the values of C on their way: the warpgroups trade registers
+  // (setmaxnreg).  Six split warps instead of four were measured slower on long products (4096^3 560 -> 646 us).
   static constexpr int THREADS = 32 * (FIRST_DRAIN + DRAIN_WARPS);
   static constexpr int SPLIT_THREADS = 32 * SPLIT_WARPS;
   static constexpr int TMEM_COLS = 2 * BN;
   // groups of 16 rows x 32 columns of C fetched ahead in the epilogue, as far as registers go
-  static constexpr int EPILOGUE_AHEAD = TRADE_REGISTERS ? 1 : 2;
+  static constexpr int EPILOGUE_AHEAD = BN == 256 ? 1 : 3;
   static_assert(BK == 32 || BK == 16, "K-major rows are one 128- or 64-byte swizzle span");
   static_assert(BN == 128 || BN == 256, "one or two 128-column halves");
 };
-using Narrow = Shape<128, 32, 3, 2>;   // warps: TMA, MMA, 4 split, 8 drain
-using Wide = Shape<256, 16, 4, 4>;     // warps: TMA, MMA, 2 idle | 4 split | 8 drain (four warpgroups)
+// warps of both: TMA, MMA, 2 idle | 4 split | 8 drain (four warpgroups)
+using Narrow = Shape<128, 32, 3, 4>;
+using Wide = Shape<256, 16, 4, 4>;
 
 struct TcGemmParams {
   float* C; long long ldc; long long strideC;
@@ -193,7 +194,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   const int total_items = p.batch * p.tiles_m * p.tiles_n;
 
   if (warp < S::FIRST_SPLIT) {
-  if (S::TRADE_REGISTERS) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
     if (lane == 0) {
       uint32_t stage = 0, phase = 1;
@@ -259,10 +260,10 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       }
     }
     __syncwarp();
-  }  // further warps of the first warpgroup (wide shape) idle
+  }  // further warps of the first warpgroup idle
   } else if (warp < S::FIRST_DRAIN) {
     // split warps
-    if (S::TRADE_REGISTERS) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     const int st = tid - 32 * S::FIRST_SPLIT;
     uint32_t stage = 0, phase = 0;
     bool ok = true;
@@ -295,7 +296,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   } else {
     // drain warps: TMEM lane quarter = warp % 4; a second set of four warps takes the upper half of
     // the columns
-    if (S::TRADE_REGISTERS) asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
     const int quarter = warp & 3;
     const int half = (warp - S::FIRST_DRAIN) >> 2;
     constexpr int DW = S::DW;

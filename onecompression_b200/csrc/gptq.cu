@@ -397,7 +397,8 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
 // owners wait for after each window, a block took 20 us at 4096 rows; now 14 us.  It is for up to
 // two row sets per SM: a load from shared memory delivers 32 lanes 4 bytes each a cycle, broadcast or not,
 // and one entry of U per row and column is twice what the arithmetic of the updates takes, so with many
-// rows the general kernel's is the better split (28672 rows: 44 us there, 55 to 73 us here).
+// rows the general kernel's is the better split (28672 rows: 44 us there, 73 us here with
+// two rows per lane).
 
 // one column with IEEE divisions: (error, level = q - zero)
 __device__ __noinline__ float2 exact_column(float x, float scale, float zero, float maxqf, float u) {
