@@ -159,9 +159,16 @@ class GPTQLinear(torch.nn.Module):
                 or torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack()
                 or torch._C._functorch.peek_interpreter_stack() is not None):
             return None
+        # what the general path reads as attributes (looked up where they usually are: an attribute of a
+        # module costs more than the rest of this function)
         b = self._buffers
-        return kernels.packed_linear(x, b["qweight"], b["qzeros"], b["scales"], b["g_idx"], b.get("bias"),
-                                     self.wbits, self.out_features, self.in_features)
+        try:
+            qweight, qzeros, scales, g_idx = b["qweight"], b["qzeros"], b["scales"], b["g_idx"]
+        except KeyError:    # one of them became a parameter or a plain attribute
+            qweight, qzeros, scales, g_idx = self.qweight, self.qzeros, self.scales, self.g_idx
+        bias = b["bias"] if "bias" in b else self.bias
+        return kernels.packed_linear(x, qweight, qzeros, scales, g_idx, bias, self.wbits, self.out_features,
+                                     self.in_features)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         y = self._decoded_in_product(x)

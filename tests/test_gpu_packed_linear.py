@@ -67,3 +67,21 @@ def test_packed_linear_keeps_the_general_path():
         assert m._decoded_in_product(view) is None
         assert torch.allclose(m(view), y, rtol=1e-2, atol=1e-2)
     assert m(x[:0]).shape == (0, 64)
+
+
+@pytest.mark.parametrize("kind", ["tensor", "parameter"])
+def test_bias_and_scales_assigned_later(kind):
+    """A bias given after construction, and scales that became a parameter, count for few tokens as for many."""
+    wrap = (lambda t: torch.nn.Parameter(t, requires_grad=False)) if kind == "parameter" else (lambda t: t)
+    m, w = layer(64, 256, 4, 64, False, False)
+    bias = torch.linspace(-4, 4, 64).half()
+    m.bias = wrap(bias.cuda())
+    scales = m.scales
+    del m.scales
+    m.scales = wrap(scales)
+    x = torch.randn(17, 256, generator=torch.Generator().manual_seed(3)).half()
+    want = x.double() @ w.double().t() + bias.double()
+    bound = 256 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + 2.0 ** -11 * want.abs() + 2.0 ** -25
+    for tokens in (4, 16, 17):
+        assert (m._decoded_in_product(x[:tokens].cuda()) is not None) == (tokens <= 16)
+        assert ((m(x[:tokens].cuda()).cpu().double() - want[:tokens]).abs() <= bound[:tokens]).all()

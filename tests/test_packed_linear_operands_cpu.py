@@ -1,0 +1,82 @@
+"""Which operands the packed layer's one-kernel path takes, and when it leaves a call to the general path.
+The kernels are replaced by the same sums in torch."""
+
+import pytest
+import torch
+
+from onecompression_b200 import kernels
+from onecompression_b200.quantizer.gptq.gptq_layer import GPTQLinear
+
+OUT, D = 8, 16
+
+
+def decoded(qweight, qzeros, scales, g_idx, wbits, shape):
+    assert wbits == 4
+    nibble = 4 * torch.arange(8, dtype=torch.int32)
+    q = ((qweight[:, None, :] >> nibble[None, :, None]) & 15).reshape(shape[1], shape[0])
+    z = (((qzeros[:, :, None] >> nibble) & 15).reshape(-1, shape[0]) + 1) & 15
+    g = g_idx.long()
+    return (scales[g].float() * (q - z[g]).float()).t().half()
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    seen = []
+
+    def packed_linear(x, qweight, qzeros, scales, g_idx, bias, wbits, out, d):
+        if x.numel() // d > kernels.PACKED_LINEAR_TOKENS:
+            return None
+        seen.append((qweight, qzeros, scales, g_idx, bias))
+        y = x.float() @ decoded(qweight, qzeros, scales, g_idx, wbits, (out, d)).float().t()
+        return (y if bias is None else y + bias.float()).half().detach()
+
+    monkeypatch.setattr(kernels, "packed_linear", packed_linear)
+    monkeypatch.setattr(kernels, "dequantize_packed", decoded)
+    return seen
+
+
+def layer(bias=None):
+    g = torch.Generator().manual_seed(1)
+    word = lambda *shape: torch.randint(-2 ** 31, 2 ** 31 - 1, shape, generator=g, dtype=torch.int64).int()
+    return GPTQLinear(D, OUT, 4, 8, False, word(D // 8, OUT), torch.rand(2, OUT, generator=g).half() * 0.1,
+                      word(2, OUT // 8), bias=bias, device="cpu", input_weight_is_packed=True,
+                      input_zero_is_packed=True)
+
+
+def check(m, calls, short=True):
+    """The first four of 17 tokens, alone and in the long call (which takes the general path)."""
+    x = torch.randn(17, D, generator=torch.Generator().manual_seed(2)).half()
+    before = len(calls)
+    got = m(x[:4])
+    assert len(calls) == before + (1 if short else 0)
+    want = m(x)[:4]
+    assert len(calls) == before + (1 if short else 0)
+    assert torch.allclose(got, want, rtol=2e-3, atol=2e-3)
+    return got
+
+
+BIAS = torch.linspace(-3, 3, OUT).half()
+
+
+@pytest.mark.parametrize("built_with", [None, torch.zeros(OUT)])
+@pytest.mark.parametrize("assigned", ["tensor", "parameter", "none"])
+def test_bias_assigned_after_construction(calls, built_with, assigned):
+    m = layer(built_with)
+    plain = check(layer(), calls)
+    m.bias = {"tensor": BIAS, "parameter": torch.nn.Parameter(BIAS, requires_grad=False), "none": None}[assigned]
+    got = check(m, calls)
+    assert torch.allclose(got - plain, torch.zeros(OUT).half() if assigned == "none" else BIAS, atol=5e-3)
+
+
+@pytest.mark.parametrize("name", ["qweight", "qzeros", "scales", "g_idx"])
+def test_operand_replaced_by_a_parameter_or_a_plain_attribute(calls, name):
+    want = check(layer(), calls)
+    m = layer()
+    t = getattr(m, name)
+    delattr(m, name)
+    m.register_parameter(name, torch.nn.Parameter(t, requires_grad=False))
+    assert torch.equal(check(m, calls), want) and calls[-1][["qweight", "qzeros", "scales", "g_idx"].index(name)] is getattr(m, name)
+    m = layer()
+    delattr(m, name)
+    setattr(m, name, t)
+    assert torch.equal(check(m, calls), want)
