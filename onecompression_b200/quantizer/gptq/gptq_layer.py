@@ -154,7 +154,7 @@ class GPTQLinear(torch.nn.Module):
         or transforms the operators of the forward pass (autograd, autocast, function transforms,
         tracing, dispatch modes) keeps the dequantized weight and ``linear``."""
         if (not self._weight_is_packed or type(x) is not torch.Tensor
-                or (x.requires_grad and torch.is_grad_enabled()) or forward_ad._current_level >= 0
+                or forward_ad._current_level >= 0
                 or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling()
                 or torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack()
                 or torch._C._functorch.peek_interpreter_stack() is not None):
@@ -167,6 +167,9 @@ class GPTQLinear(torch.nn.Module):
         except KeyError:    # one of them became a parameter or a plain attribute
             qweight, qzeros, scales, g_idx = self.qweight, self.qzeros, self.scales, self.g_idx
         bias = b["bias"] if "bias" in b else self.bias
+        if torch.is_grad_enabled() and (x.requires_grad or scales.requires_grad
+                                        or (bias is not None and bias.requires_grad)):
+            return None
         return kernels.packed_linear(x, qweight, qzeros, scales, g_idx, bias, self.wbits, self.out_features,
                                      self.in_features)
 

@@ -85,3 +85,14 @@ def test_bias_and_scales_assigned_later(kind):
     for tokens in (4, 16, 17):
         assert (m._decoded_in_product(x[:tokens].cuda()) is not None) == (tokens <= 16)
         assert ((m(x[:tokens].cuda()).cpu().double() - want[:tokens]).abs() <= bound[:tokens]).all()
+
+
+def test_trainable_bias_gets_its_gradient():
+    m, _ = layer(64, 256, 4, 64, False, False)
+    m.bias = torch.nn.Parameter(torch.zeros(64, device="cuda").half())
+    for tokens in (4, 17):
+        m.bias.grad = None
+        m(torch.ones(tokens, 256, device="cuda").half()).sum().backward()
+        assert torch.equal(m.bias.grad, torch.full_like(m.bias, tokens))
+    with torch.no_grad():
+        assert m._decoded_in_product(torch.ones(4, 256, device="cuda").half()) is not None

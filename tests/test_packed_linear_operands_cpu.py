@@ -80,3 +80,20 @@ def test_operand_replaced_by_a_parameter_or_a_plain_attribute(calls, name):
     delattr(m, name)
     setattr(m, name, t)
     assert torch.equal(check(m, calls), want)
+
+
+@pytest.mark.parametrize("name", ["bias", "scales"])
+def test_trainable_operands_keep_the_general_path(calls, name):
+    m = layer(BIAS)
+    t = getattr(m, name)
+    delattr(m, name)
+    m.register_parameter(name, torch.nn.Parameter(t))
+    x = torch.ones(4, D).half()
+    with torch.no_grad():
+        want = check(m, calls)                       # no graph to build: one kernel
+    assert torch.allclose(check(m, calls, short=False), want, rtol=2e-3, atol=2e-3)
+    m(x).sum().backward()
+    if name == "bias":
+        assert torch.equal(m.bias.grad, torch.full((OUT,), 4.0).half())
+    m.requires_grad_(False)
+    assert torch.equal(check(m, calls), want)
