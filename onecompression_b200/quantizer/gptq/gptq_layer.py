@@ -152,8 +152,10 @@ class GPTQLinear(torch.nn.Module):
     def _decoded_in_product(self, x):
         """The layer as one kernel, for a plain call on a few tokens; None otherwise.  Whatever watches
         or transforms the operators of the forward pass (autograd, autocast, function transforms,
-        tracing, dispatch modes) keeps the dequantized weight and ``linear``."""
+        tracing, dispatch modes) keeps the dequantized weight and ``linear``, and so does a decoding of
+        the layer's own (a subclass or an instance that replaces ``dequantized_weight``)."""
         if (not self._weight_is_packed or type(x) is not torch.Tensor
+                or type(self).dequantized_weight is not _decoding or "dequantized_weight" in self.__dict__
                 or forward_ad._current_level >= 0
                 or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling()
                 or torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack()
@@ -194,3 +196,6 @@ class GPTQLinear(torch.nn.Module):
         self.register_buffer("qweight", pack_int_weights(self.qweight.to(torch.int32), self.wbits))
         self.register_buffer("qzeros", pack_zeros(self.qzeros.to(torch.int32).contiguous(), self.wbits))
         self._weight_is_packed = True
+
+
+_decoding = GPTQLinear.dequantized_weight   # what the one-kernel path stands for

@@ -97,3 +97,18 @@ def test_trainable_operands_keep_the_general_path(calls, name):
         assert torch.equal(m.bias.grad, torch.full((OUT,), 4.0).half())
     m.requires_grad_(False)
     assert torch.equal(check(m, calls), want)
+
+
+def test_a_decoding_of_its_own_is_used_for_a_few_tokens_too(calls):
+    class Doubled(GPTQLinear):
+        def dequantized_weight(self):
+            return 2 * super().dequantized_weight()
+
+    m = layer()
+    plain = check(m, calls)
+    m.__class__ = Doubled
+    assert torch.allclose(check(m, calls, short=False), 2 * plain, rtol=2e-3, atol=2e-3)
+    m = layer()
+    original = m.dequantized_weight
+    m.dequantized_weight = lambda: 3 * original()
+    assert torch.allclose(check(m, calls, short=False), 3 * plain, rtol=2e-3, atol=2e-3)
