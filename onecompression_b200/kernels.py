@@ -621,7 +621,8 @@ def packed_linear(x: torch.Tensor, qweight, qzeros, scales, g_idx, bias, wbits: 
     layout, alignment, token count): dequantize and multiply then."""
     # (a decode step makes hundreds of these calls, each a few microseconds on the GPU: the checks are
     # written for little host time)
-    if x.dtype != torch.float16 or not x.is_cuda or x.dim() == 0 or x.shape[-1] != d or not x.is_contiguous():
+    if (x.dtype != torch.float16 or not x.is_cuda or x.dim() == 0 or x.shape[-1] != d or not x.is_contiguous()
+            or g_idx is None):
         return None
     tokens = x.numel() // d
     dev = x.get_device()

@@ -96,3 +96,13 @@ def test_trainable_bias_gets_its_gradient():
         assert torch.equal(m.bias.grad, torch.full_like(m.bias, tokens))
     with torch.no_grad():
         assert m._decoded_in_product(torch.ones(4, 256, device="cuda").half()) is not None
+
+
+def test_one_group_without_g_idx():
+    """dequantize_packed takes a missing g_idx as one group; so does the layer, for few tokens and many."""
+    m, w = layer(64, 256, 4, -1, False, False)
+    x = torch.randn(17, 256, generator=torch.Generator().manual_seed(4)).half()
+    want = (x.double() @ w.double().t())
+    m.g_idx = None
+    for tokens in (4, 17):
+        assert torch.allclose(m(x[:tokens].cuda()).cpu().double(), want[:tokens], rtol=1e-2, atol=1e-2)

@@ -112,3 +112,15 @@ def test_a_decoding_of_its_own_is_used_for_a_few_tokens_too(calls):
     original = m.dequantized_weight
     m.dequantized_weight = lambda: 3 * original()
     assert torch.allclose(check(m, calls, short=False), 3 * plain, rtol=2e-3, atol=2e-3)
+
+
+def test_the_kernel_is_not_offered_a_layer_without_g_idx():
+    class OnGpu:                  # what packed_linear asks of its input before it looks at the operands
+        dtype, is_cuda, shape = torch.float16, True, torch.Size([4, D])
+        dim = lambda self: 2
+        is_contiguous = lambda self: True
+        numel = lambda self: 4 * D
+        get_device = lambda self: 0
+
+    m = layer()
+    assert kernels.packed_linear(OnGpu(), m.qweight, m.qzeros, m.scales, None, None, 4, OUT, D) is None
