@@ -99,4 +99,6 @@ def ptr(t):
 def stream_handle():
     import torch
 
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # (the internal name saves building a Stream object; a torch without it has the public way)
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream

@@ -73,6 +73,20 @@ def make_g_idx(perm: Optional[torch.Tensor], groupsize: int, in_features: int, d
     return g.to(torch.int32)
 
 
+def _watchers():
+    """What tells that modes or function transforms are active.  None where this torch lacks one of these
+    internal names: the one-kernel path of the layer stays off then."""
+    try:
+        forward_ad._current_level
+        return (torch._C._len_torch_function_stack, torch._C._len_torch_dispatch_stack,
+                torch._C._functorch.peek_interpreter_stack)
+    except AttributeError:
+        return None
+
+
+_WATCHERS = _watchers()
+
+
 class GPTQLinear(torch.nn.Module):
     """Inference layer over a GPTQ result in the AutoGPTQ (v1) tensor layout - the consumer of
     what the column loop packs (reference: GPTQLinear, onecomp/quantizer/gptq/gptq_layer.py:247-714).
@@ -154,12 +168,13 @@ class GPTQLinear(torch.nn.Module):
         or transforms the operators of the forward pass (autograd, autocast, function transforms,
         tracing, dispatch modes) keeps the dequantized weight and ``linear``, and so does a decoding of
         the layer's own (a subclass or an instance that replaces ``dequantized_weight``)."""
-        if (not self._weight_is_packed or type(x) is not torch.Tensor
+        if (not self._weight_is_packed or type(x) is not torch.Tensor or torch.compiler.is_compiling()
                 or type(self).dequantized_weight is not _decoding or "dequantized_weight" in self.__dict__
-                or forward_ad._current_level >= 0
-                or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing() or torch.compiler.is_compiling()
-                or torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack()
-                or torch._C._functorch.peek_interpreter_stack() is not None):
+                or _WATCHERS is None or forward_ad._current_level >= 0
+                or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing()):
+            return None
+        function_modes, dispatch_modes, transforms = _WATCHERS
+        if function_modes() or dispatch_modes() or transforms() is not None:
             return None
         # what the general path reads as attributes (looked up where they usually are: an attribute of a
         # module costs more than the rest of this function)

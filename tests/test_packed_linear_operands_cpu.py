@@ -4,7 +4,8 @@ The kernels are replaced by the same sums in torch."""
 import pytest
 import torch
 
-from onecompression_b200 import kernels
+from onecompression_b200 import _lib, kernels
+from onecompression_b200.quantizer.gptq import gptq_layer
 from onecompression_b200.quantizer.gptq.gptq_layer import GPTQLinear
 
 OUT, D = 8, 16
@@ -124,3 +125,34 @@ def test_the_kernel_is_not_offered_a_layer_without_g_idx():
 
     m = layer()
     assert kernels.packed_linear(OnGpu(), m.qweight, m.qzeros, m.scales, None, None, 4, OUT, D) is None
+
+
+@pytest.mark.parametrize("holder,name", [(torch._C, "_len_torch_function_stack"), (torch._C, "_len_torch_dispatch_stack"),
+                                         (torch._C._functorch, "peek_interpreter_stack"),
+                                         (torch.autograd.forward_ad, "_current_level")])
+def test_a_torch_without_an_internal_name_has_the_general_path(calls, monkeypatch, holder, name):
+    with monkeypatch.context() as m:
+        m.delattr(holder, name)
+        found = gptq_layer._watchers()
+    assert found is None
+    monkeypatch.setattr(gptq_layer, "_WATCHERS", found)
+    check(layer(), calls, short=False)
+
+
+def test_stream_handle_without_the_internal_name(monkeypatch):
+    class Stream:
+        cuda_stream = 7
+
+    monkeypatch.setattr(torch.cuda, "current_stream", Stream)
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    assert _lib.stream_handle() == 7
+
+
+def test_compiled_layer(calls):
+    """A compiler sees the general path."""
+    m = layer(BIAS)
+    x = torch.randn(4, D, generator=torch.Generator().manual_seed(2)).half()
+    want = m(x)
+    before = len(calls)
+    got = torch.compile(m, backend="eager")(x)
+    assert len(calls) == before and torch.allclose(got, want, rtol=2e-3, atol=2e-3)
