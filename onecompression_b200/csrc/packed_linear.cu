@@ -196,12 +196,14 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) packed_linear_kernel(const L
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[t][n][i] = 0.f;
 
-  int group = -1;
+  constexpr int NO_GROUP = -2, BEHIND = -1;   // BEHIND: columns behind the last one, whose weights are zero
+  int group = NO_GROUP;
   __half2 s2[4], z2[4];
   auto load_group = [&](int gi) {
     unsigned z[4] = {0u, 0u, 0u, 0u};
     uint2 sv = make_uint2(0u, 0u);
-    if (a.staged) {
+    if (gi == BEHIND) {                    // (a group's own parameters could make them infinite, and 0 * inf a NaN)
+    } else if (a.staged) {
       sv = *reinterpret_cast<const uint2*>(par_s + gi * ROWS + 4 * g);
       const unsigned zb = *reinterpret_cast<const unsigned*>(par_z + gi * ROWS + 4 * g);
 #pragma unroll
@@ -224,8 +226,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) packed_linear_kernel(const L
     for (int h = 0; h < 2; ++h) {
       const int unit = unit0 + 4 * h;
       const int4 w0 = cur->w[h][0][lane], w1 = F::WORDS > 1 ? cur->w[h][F::WORDS - 1][lane] : make_int4(0, 0, 0, 0);
-      // (behind the last column: group 0, whose x is zero)
-      const int ug = unit < units ? (int)ugroup[unit] : 0;
+      const int ug = unit < units ? (int)ugroup[unit] : BEHIND;
       const unsigned wr[4][2] = {{(unsigned)w0.x, (unsigned)w1.x}, {(unsigned)w0.y, (unsigned)w1.y},
                                  {(unsigned)w0.z, (unsigned)w1.z}, {(unsigned)w0.w, (unsigned)w1.w}};
       __half2 v[4][4];    // [row][pair]: weights of columns (k, k + 4) of the unit
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) packed_linear_kernel(const L
             v[i][k] = __hmul2(__lows2half2(sa[i], s2[i]),
                               __hsub2(as_half2(F::pair(wr[i], unit, k) | 0x64006400u), __lows2half2(za[i], z2[i])));
         }
-        group = -1;
+        group = NO_GROUP;
       }
       __syncwarp();
 #pragma unroll

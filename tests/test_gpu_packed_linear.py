@@ -106,3 +106,26 @@ def test_one_group_without_g_idx():
     m.g_idx = None
     for tokens in (4, 17):
         assert torch.allclose(m(x[:tokens].cuda()).cpu().double(), want[:tokens], rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("bits,d", [(4, 8), (4, 1048), (8, 72), (2, 80), (3, 96), (4, 4096)])
+@pytest.mark.parametrize("act", [False, True])
+def test_columns_behind_the_last_one_count_for_nothing(bits, d, act):
+    """Codes equal to a large zero point: the weights are zero, the zero point alone times the scale is not finite."""
+    from onecompression_b200.quantizer.gptq.gptq_layer import GPTQLinear
+
+    out, top = 96, 2 ** bits - 1
+    codes = torch.full((out, d), top, dtype=torch.int32)
+    codes[1::2] -= torch.arange(d, dtype=torch.int32) % 2            # 0 and one negative step
+    groups = (d + 31) // 32
+    scale = torch.full((groups, out), 60000.0)
+    zero = torch.full((groups, out), top, dtype=torch.int32)
+    perm = torch.randperm(d, generator=torch.Generator().manual_seed(d)) if act else None
+    m = GPTQLinear(d, out, bits, 32, act, codes, scale, zero, perm=perm)
+    w = (60000.0 * (codes - top)).half()
+    x = torch.randn(16, d, generator=torch.Generator().manual_seed(5)).mul(2.0 ** -14).half()
+    want = x.double() @ w.double().t()
+    bound = d * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t()) + 2.0 ** -11 * want.abs() + 2.0 ** -25
+    for tokens in (1, 16):
+        got = m._decoded_in_product(x[:tokens].cuda()).cpu().double()
+        assert ((got - want[:tokens]).abs() <= bound[:tokens]).all()
