@@ -96,9 +96,22 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-def stream_handle():
+_current_stream = None
+
+
+def _stream_source():
+    """What gives the current stream: an internal name that saves building a Stream object, the public way
+    in a torch without it."""
     import torch
 
-    # (the internal name saves building a Stream object; a torch without it has the public way)
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), torch.cuda.current_device
+    if raw is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
+
+
+def stream_handle():
+    global _current_stream
+    if _current_stream is None:
+        _current_stream = _stream_source()
+    return _current_stream()

@@ -184,8 +184,8 @@ class GPTQLinear(torch.nn.Module):
         except KeyError:    # one of them became a parameter or a plain attribute
             qweight, qzeros, scales, g_idx = self.qweight, self.qzeros, self.scales, self.g_idx
         bias = b["bias"] if "bias" in b else self.bias
-        if torch.is_grad_enabled() and (x.requires_grad or scales.requires_grad
-                                        or (bias is not None and bias.requires_grad)):
+        if ((x.requires_grad or scales.requires_grad or (bias is not None and bias.requires_grad))
+                and torch.is_grad_enabled()):
             return None
         return kernels.packed_linear(x, qweight, qzeros, scales, g_idx, bias, self.wbits, self.out_features,
                                      self.in_features)

@@ -145,6 +145,7 @@ def test_stream_handle_without_the_internal_name(monkeypatch):
 
     monkeypatch.setattr(torch.cuda, "current_stream", Stream)
     monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+    monkeypatch.setattr(_lib, "_current_stream", None)
     assert _lib.stream_handle() == 7
 
 
