@@ -54,15 +54,18 @@ __global__ void diag_stats_kernel(const float* __restrict__ H, long long ld, int
 }
 
 // ---- act-order: stable descending argsort by counting ranks ---------------------
+// A NaN counts as +infinity: without a total order two columns would share a rank, and entries of perm,
+// which every later pass uses as an index, would keep what was in memory.
+__device__ __forceinline__ float rank_key(float v) { return v == v ? v : __int_as_float(0x7f800000); }
 __global__ void rank_sort_kernel(const float* __restrict__ key, int n, int* __restrict__ perm, long long sW) {
   key += (long long)blockIdx.y * sW;
   perm += (long long)blockIdx.y * n;
   __shared__ float tile[1024];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const float ki = (i < n) ? key[i] : 0.f;
+  const float ki = (i < n) ? rank_key(key[i]) : 0.f;
   int rank = 0;
   for (int base = 0; base < n; base += 1024) {
-    for (int t = threadIdx.x; t < 1024; t += blockDim.x) tile[t] = (base + t < n) ? key[base + t] : 0.f;
+    for (int t = threadIdx.x; t < 1024; t += blockDim.x) tile[t] = (base + t < n) ? rank_key(key[base + t]) : 0.f;
     __syncthreads();
     const int lim = min(1024, n - base);
     for (int t = 0; t < lim; ++t) {
