@@ -696,10 +696,12 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
   }
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   const bool vec_h = n % 4 == 0 && ldh % 4 == 0 && sH % 4 == 0 && aligned(H);
-  const bool staged = actorder && n <= BUILD_STAGED_N;
+  // (with reuse_perm the caller's perm counts, whatever actorder says)
+  const int permuted = actorder || reuse_perm;
+  const bool staged = permuted && n <= BUILD_STAGED_N;
   if (staged) OC_OPT_IN_SMEM(build_reversed_kernel, BUILD_STAGED_N * 4);
   build_reversed_kernel<<<dim3(n, batch), 256, staged ? n * 4 : 0, stream>>>(
-      H, ldh, n, perm, actorder, diagv, damp_out, rel_shift, A, ld, sH, sW, vec_h, staged);
+      H, ldh, n, perm, permuted, diagv, damp_out, rel_shift, A, ld, sH, sW, vec_h, staged);
   OC_CHECK_LAUNCH();
 
   // ---- blocked right-looking Cholesky --------------------------------------------------
