@@ -13,7 +13,8 @@
  *     says otherwise; matrices are row-major with an explicit leading dimension
  *     in elements;
  *   - nothing here allocates: scratch is passed in, its size comes from the
- *     matching *_workspace_bytes function;
+ *     matching *_workspace_bytes function; a workspace starts at a multiple of 4 bytes, better
+ *     16 (other starts take slower paths; the factor of 128 and more columns refuses them);
  *   - every call is asynchronous on `stream` (a cudaStream_t passed as void*);
  *   - the return value is 0 on success or a negative OC_ERR_* code, with a
  *     message available from oc_last_error() (per host thread);

@@ -671,6 +671,9 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
   OC_REQUIRE(H && U && perm && invperm && dead && damp_out && status && workspace, "hinv_factor: null pointer");
   OC_REQUIRE(n > 0 && ldh >= n && ldu >= n, "hinv_factor: bad dimensions");
   OC_REQUIRE(batch >= 1 && batch <= 65535, "hinv_factor: batch must be in 1..65535");
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  // (full panels are read and written 16 bytes at a time)
+  OC_REQUIRE(n < NB || aligned(workspace), "hinv_factor: the workspace must be 16-byte aligned");
   const long long sW = factor_ws_floats(n);
   if (workspace_bytes < sW * 4 * batch) {
     oc_set_last_error("hinv_factor: workspace too small");
@@ -694,8 +697,7 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     invert_perm_kernel<<<dim3(gb, batch), tb, 0, stream>>>(perm, invperm, n);
     OC_CHECK_LAUNCH();
   }
-  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  const bool vec_h = n % 4 == 0 && ldh % 4 == 0 && sH % 4 == 0 && aligned(H);
+  const bool vec_h = n % 4 == 0 && ldh % 4 == 0 && sH % 4 == 0 && aligned(H) && aligned(A);
   // (with reuse_perm the caller's perm counts, whatever actorder says)
   const int permuted = actorder || reuse_perm;
   const bool staged = permuted && n <= BUILD_STAGED_N;
@@ -806,7 +808,7 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
       if (rc) return rc;
     }
   }
-  const bool vec_u = n % 4 == 0 && ldu % 4 == 0 && sU % 4 == 0 && aligned(U);
+  const bool vec_u = n % 4 == 0 && ldu % 4 == 0 && sU % 4 == 0 && aligned(U) && aligned(X);
   reverse_upper_kernel<<<dim3(n, batch), 256, 0, stream>>>(X, ld, n, U, ldu, sW, sU, vec_u);
   OC_CHECK_LAUNCH();
   return OC_OK;

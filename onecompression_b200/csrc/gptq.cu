@@ -1017,7 +1017,8 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
 
   OC_REQUIRE(!mse || (q_grid >= 1 && q_norm > 0.f), "gptq_quantize: mse needs q_grid >= 1 and q_norm > 0");
   const int mse_steps = mse ? (int)(0.8 * q_grid) : 0;   // maxshrink = 0.8 as in the reference
-  const bool vec = d % 8 == 0 && ldw_in % 8 == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 &&
+  const bool vec = d % 8 == 0 && ldw_in % 8 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(Wf)) & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(dead) & 7) == 0;
   const bool staged = perm && d <= PREPARE_STAGED_D;
   if (staged) OC_OPT_IN_SMEM(gptq_prepare_kernel, PREPARE_STAGED_D * 4);

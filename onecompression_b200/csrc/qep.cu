@@ -121,7 +121,7 @@ extern "C" int oc_qep_adjust(void* W_, long long ldw_io, int out, int d, const f
   const int tb = 256;
   dim3 grid(oc_div_up(d, tb), out);
   const bool vec = d % 4 == 0 && ldw_io % 4 == 0 && (reinterpret_cast<uintptr_t>(W) & 7) == 0 &&
-                   (reinterpret_cast<uintptr_t>(dead) & 3) == 0;
+                   (reinterpret_cast<uintptr_t>(Wf) & 15) == 0 && (reinterpret_cast<uintptr_t>(dead) & 3) == 0;
   const dim3 grid4(oc_div_up(d, 4 * tb), out);
   qep_load_kernel<<<vec ? grid4 : grid, tb, 0, stream>>>(W, ldw_io, out, d, dead, Wf, ld, bf16, vec);
   OC_CHECK_LAUNCH();
