@@ -113,10 +113,20 @@ class MomentAccumulator:
         self._clear_unwritten()
         return self._h
 
+    @H.setter
+    def H(self, value):
+        self._clear_unwritten()   # (C counts as zero from now on)
+        self._h = value
+
     @property
     def C(self):
         self._clear_unwritten()
         return self._c
+
+    @C.setter
+    def C(self, value):
+        self._clear_unwritten()
+        self._c = value
 
     def add(self, xq: torch.Tensor, xf: Optional[torch.Tensor] = None):
         """Fold a chunk of activations ([..., d], fp16) into the moments."""

@@ -46,3 +46,42 @@ def test_mirror(n, pad):
     want[:, :n] = torch.triu(m[:, :n]) + torch.triu(m[:, :n], 1).t()
     call("oc_mirror_upper", ptr(m), n + pad, n, stream_handle())
     assert torch.equal(m, want)
+
+
+def chunk(t, d, seed):
+    g = torch.Generator().manual_seed(seed)
+    return torch.randn(t, d, generator=g).half().cuda(), torch.randn(t, d, generator=g).half().cuda()
+
+
+def same(got, want):
+    return torch.allclose(got, want, rtol=0, atol=1e-5 * max(1.0, float(want.abs().max())))
+
+
+@pytest.mark.parametrize("d", [57, 264])
+def test_moments_are_saved_and_put_back(d):
+    """H, C and nsamples of one accumulator, assigned to another that goes on, or added to its own."""
+    from onecompression_b200 import kernels as K
+
+    (q0, f0), (q1, f1) = chunk(100, d, 0), chunk(60, d, 1)
+    whole, first = K.MomentAccumulator(d, "cuda", cross=True), K.MomentAccumulator(d, "cuda", cross=True)
+    whole.add(q0, f0)
+    whole.add(q1, f1)
+    first.add(q0, f0)
+    saved = [t.clone() for t in first.finalize()[:2]]
+    junk = [torch.full((d, d), float("nan"), device="cuda") for _ in range(3)]
+    del junk
+    rest = K.MomentAccumulator(d, "cuda", cross=True)
+    rest.H, rest.C, rest.nsamples = saved[0], saved[1], 100
+    rest.add(q1, f1)
+    h, c, n = whole.finalize()
+    h2, c2, n2 = rest.finalize()
+    assert n2 == n and same(h2, h) and same(c2, c)
+    # what one of the two assignments leaves out is zero
+    junk = torch.full((d, d), float("nan"), device="cuda")
+    del junk
+    half = K.MomentAccumulator(d, "cuda", cross=True)
+    half.H = torch.eye(d, device="cuda")
+    assert torch.equal(half.H, torch.eye(d, device="cuda")) and not half.C.any()
+    half.C += 2
+    half.H *= 3
+    assert torch.equal(half.H, 3 * torch.eye(d, device="cuda")) and bool((half.C == 2).all())
