@@ -151,7 +151,8 @@ class MomentAccumulator:
         n = self.nsamples
         a_old = n / (n + t)
         a_new = 2.0 / (n + t)
-        self.nsamples = n + t
+        if n:   # (nothing of the buffers is read otherwise; nsamples may have been set from outside)
+            self._clear_unwritten()
         scratch = None
         if cross and not self.force_simt:
             # Xf - Xq as two 16-bit terms, rows packed: [2, t, d]
@@ -165,6 +166,7 @@ class MomentAccumulator:
                 xq.stride(0), ptr(self._h), ptr(self._c), self.d, a_old, a_new, self.chunk_tokens,
                 sm_count(self.device), self.engine, _DTYPES[xq.dtype], ptr(self.status), stream_handle(),
             )
+        self.nsamples = n + t
         self._written = True
         self._needs_mirror = not self.force_simt
 

@@ -85,3 +85,47 @@ def test_moments_are_saved_and_put_back(d):
     half.C += 2
     half.H *= 3
     assert torch.equal(half.H, 3 * torch.eye(d, device="cuda")) and bool((half.C == 2).all())
+
+
+@pytest.mark.parametrize("d", [57, 264])
+def test_an_add_that_failed_counts_for_nothing(d, monkeypatch):
+    """No scratch memory, then a launch that is refused: the next chunk is the first one."""
+    from onecompression_b200 import kernels as K
+
+    q, f = chunk(64, d, 2)
+    want = K.MomentAccumulator(d, "cuda", cross=True)
+    want.add(q, f)
+    junk = [torch.full((d, d), float("nan"), device="cuda") for _ in range(3)]
+    del junk
+    acc = K.MomentAccumulator(d, "cuda", cross=True)
+
+    def refuse(*args, **kwargs):
+        raise RuntimeError("refused")
+
+    for name, holder in (("call", K), ("empty", torch)):
+        if name == "empty" and d % 8:
+            continue                     # the FMA engine needs no scratch
+        with monkeypatch.context() as m:
+            m.setattr(holder, name, refuse)
+            with pytest.raises(RuntimeError, match="refused"):
+                acc.add(torch.cat([q, q]), torch.cat([f, f]))
+        assert acc.nsamples == 0
+    acc.add(q, f)
+    for got, ref in zip(acc.finalize()[:2], want.finalize()[:2]):
+        assert torch.equal(got, ref)
+
+
+@pytest.mark.parametrize("d", [57, 264])
+def test_a_sample_count_set_from_outside_weighs_zeros(d):
+    from onecompression_b200 import kernels as K
+
+    q, f = chunk(64, d, 3)
+    want = K.MomentAccumulator(d, "cuda", cross=True)
+    want.add(q, f)
+    junk = [torch.full((d, d), float("nan"), device="cuda") for _ in range(3)]
+    del junk
+    acc = K.MomentAccumulator(d, "cuda", cross=True)
+    acc.nsamples = 64
+    acc.add(q, f)
+    for got, ref in zip(acc.finalize()[:2], want.finalize()[:2]):
+        assert same(2 * got, ref)
