@@ -100,6 +100,7 @@ class MomentAccumulator:
         self.engine = 1 if self.force_simt else self.ENGINES[engine]
         self._scratch = None
         self._needs_mirror = False
+        self._lower_stale = False   # the kernels write the upper part of H only
 
     def _clear_unwritten(self):
         if not self._written:
@@ -108,15 +109,25 @@ class MomentAccumulator:
                 self._c.zero_()
             self._written = True
 
+    def _mirror(self):
+        with _on(self.device):
+            call("oc_mirror_upper", ptr(self._h), self.d, self.d, stream_handle())
+        self._lower_stale = False
+
     @property
     def H(self):
+        """The second moments so far, both triangles.  (A later ``add`` brings the upper part of this
+        tensor up to date, the next access or ``finalize`` the lower one.)"""
         self._clear_unwritten()
+        if self._lower_stale:
+            self._mirror()
         return self._h
 
     @H.setter
     def H(self, value):
         self._clear_unwritten()   # (C counts as zero from now on)
         self._h = value
+        self._lower_stale = False
 
     @property
     def C(self):
@@ -168,7 +179,7 @@ class MomentAccumulator:
             )
         self.nsamples = n + t
         self._written = True
-        self._needs_mirror = not self.force_simt
+        self._needs_mirror = self._lower_stale = not self.force_simt
 
     def _as_rows(self, x: torch.Tensor) -> torch.Tensor:
         _require_cuda(x, "activations")
@@ -183,8 +194,7 @@ class MomentAccumulator:
         """Complete H (mirror the upper triangle) and return (H, C, nsamples)."""
         self._clear_unwritten()
         if self._needs_mirror:
-            with _on(self.device):
-                call("oc_mirror_upper", ptr(self._h), self.d, self.d, stream_handle())
+            self._mirror()
             self._needs_mirror = False
         if check:
             code = int(self.status.item())

@@ -129,3 +129,24 @@ def test_a_sample_count_set_from_outside_weighs_zeros(d):
     acc.add(q, f)
     for got, ref in zip(acc.finalize()[:2], want.finalize()[:2]):
         assert same(2 * got, ref)
+
+
+@pytest.mark.parametrize("d", [57, 264, 1000])
+def test_h_between_two_chunks(d):
+    """Both triangles, whatever was in memory; reading it changes nothing of what comes out in the end."""
+    from onecompression_b200 import kernels as K
+
+    (q0, _), (q1, _) = chunk(100, d, 4), chunk(60, d, 5)
+    want = K.MomentAccumulator(d, "cuda")
+    want.add(q0)
+    after_one = K.MomentAccumulator(d, "cuda")
+    after_one.add(q0)
+    want.add(q1)
+    junk = [torch.full((d, d), float("nan"), device="cuda") for _ in range(3)]
+    del junk
+    acc = K.MomentAccumulator(d, "cuda")
+    acc.add(q0)
+    assert torch.equal(acc.H, after_one.finalize()[0]) and torch.equal(acc.H, acc.H.t())
+    acc.add(q1)
+    assert torch.equal(acc.H, acc.H.t())
+    assert torch.equal(acc.finalize()[0], want.finalize()[0])
