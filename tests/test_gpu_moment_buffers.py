@@ -26,7 +26,11 @@ def test_moments_do_not_read_what_was_there(d, cross, chunks):
     xq = torch.cat([x for x, _ in xs] + [torch.zeros(0, d).half()]).double()
     xf = torch.cat([x for _, x in xs] + [torch.zeros(0, d).half()]).double()
     want = 2 / max(n, 1) * xq.t() @ xq
-    assert torch.equal(h, h.t())
+    if acc.force_simt:
+        # (slices of 256 tokens are added atomically, in any order: a rounding each of at most two partial sums)
+        assert (h - h.t()).abs().max() <= 4 * 2.0 ** -24 * h.abs().max() * 2
+    else:
+        assert torch.equal(h, h.t())
     # sums of n products in fp32 and truncating tensor-core chains of at most 512 tokens
     bound = 1e-5 * max(1.0, float(want.abs().max()))
     assert (h.cpu().double() - want).abs().max() <= bound
