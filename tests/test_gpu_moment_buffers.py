@@ -93,7 +93,7 @@ def test_moments_are_saved_and_put_back(d):
 
 @pytest.mark.parametrize("d", [57, 264])
 def test_an_add_that_failed_counts_for_nothing(d, monkeypatch):
-    """No scratch memory, then a launch that is refused: the next chunk is the first one."""
+    """No memory for the scratch, then a launch that is refused: the next chunk is the first one."""
     from onecompression_b200 import kernels as K
 
     q, f = chunk(64, d, 2)
@@ -106,7 +106,7 @@ def test_an_add_that_failed_counts_for_nothing(d, monkeypatch):
     def refuse(*args, **kwargs):
         raise RuntimeError("refused")
 
-    for name, holder in (("call", K), ("empty", torch)):
+    for name, holder in (("empty", torch), ("call", K)):
         if name == "empty" and d % 8:
             continue                     # the FMA engine needs no scratch
         with monkeypatch.context() as m:
