@@ -400,23 +400,22 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
 // rows the general kernel's is the better split (28672 rows: 44 us there, 73 us here with
 // two rows per lane).
 
-// one column with IEEE divisions: (error, level = q - zero)
+// one column with IEEE divisions: (error, code)
 __device__ __noinline__ float2 exact_column(float x, float scale, float zero, float maxqf, float u) {
   float q = __fadd_rn(rintf(__fdiv_rn(x, scale)), zero);
   q = fminf(fmaxf(q, 0.f), maxqf);
-  const float level = __fsub_rn(q, zero);
-  return make_float2(__fdiv_rn(__fsub_rn(x, __fmul_rn(scale, level)), u), level);
+  return make_float2(__fdiv_rn(__fsub_rn(x, __fmul_rn(scale, __fsub_rn(q, zero))), u), q);
 }
 
 constexpr int NWIN = BLK / SUB, CHUNK = 4;    // windows of a block; columns published at once
 
-// columns 4Q .. 4Q+3 of a window: errors to `es` (32 per column) and er, levels to lv.  False if a
+// columns 4Q .. 4Q+3 of a window: errors to `es` (32 per column) and er, codes to cd.  False if a
 // column of this lane has to be repeated with divisions.
 template <int Q, bool EXACT>
 __device__ __forceinline__ bool produce_chunk(float (&w)[SUB], const float* __restrict__ ublk,
                                               const float* __restrict__ rdiag, float scale, float rs, float lo,
                                               float hi, float zero, float maxqf, float* es, float (&er)[SUB],
-                                              float (&lv)[SUB]) {
+                                              float (&cd)[SUB]) {
   constexpr float RINT = 12582912.f;   // 1.5 * 2^23
   bool bad = !(fabsf(zero) < 65536.f);
 #pragma unroll
@@ -426,7 +425,7 @@ __device__ __forceinline__ bool produce_chunk(float (&w)[SUB], const float* __re
     if (EXACT) {
       const float2 v = exact_column(x, scale, zero, maxqf, u);
       er[i] = v.x;
-      lv[i] = v.y;
+      cd[i] = v.y;
     } else {
       const float t = __fmul_rn(x, rs);
       const float n = __fsub_rn(__fadd_rn(t, RINT), RINT);
@@ -440,7 +439,7 @@ __device__ __forceinline__ bool produce_chunk(float (&w)[SUB], const float* __re
       const float e = __fmaf_rn(__fmaf_rn(-q1, u, r), y, q1);
       bad |= !(fabsf(r) < SAFE_HI) || !(fabsf(e) < 0x1p120f);
       er[i] = e;
-      lv[i] = level;
+      cd[i] = __fadd_rn(level, zero);
     }
     es[c * 32] = er[i];
     propagate(w, i, er[i], ublk + i * BLK);
@@ -562,17 +561,17 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
 
   // this warp's own window
   const float* ublk = Us + wid * SUB * BLK + wid * SUB;
-  float er[SUB], lv[SUB];
+  float er[SUB], cd[SUB];
   auto step = [&](auto q_const) {
     constexpr int Q = decltype(q_const)::value;
     float* es = Es + Q * CHUNK * 32 + lane;
     float entry[SUB];
 #pragma unroll
     for (int m = Q * CHUNK; m < SUB; ++m) entry[m] = w[m];
-    if (!produce_chunk<Q, false>(w, ublk, rdiag + wid * SUB, scale, rs, lo, hi, zero, maxqf, es, er, lv)) {
+    if (!produce_chunk<Q, false>(w, ublk, rdiag + wid * SUB, scale, rs, lo, hi, zero, maxqf, es, er, cd)) {
 #pragma unroll
       for (int m = Q * CHUNK; m < SUB; ++m) w[m] = entry[m];
-      produce_chunk<Q, true>(w, ublk, rdiag + wid * SUB, scale, rs, lo, hi, zero, maxqf, es, er, lv);
+      produce_chunk<Q, true>(w, ublk, rdiag + wid * SUB, scale, rs, lo, hi, zero, maxqf, es, er, cd);
     }
     if (wid < NWIN - 1) {
       __syncwarp();
@@ -588,7 +587,7 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
   float* err_out = a.ErrT + (long long)(wid * SUB) * a.lde + row;
 #pragma unroll
   for (int i = 0; i < SUB; ++i) {
-    code_out[(long long)i * a.out] = (unsigned short)__fadd_rn(lv[i], zero);
+    code_out[(long long)i * a.out] = (unsigned short)cd[i];
     err_out[(long long)i * a.lde] = er[i];
   }
 }

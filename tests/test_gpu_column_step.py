@@ -65,3 +65,28 @@ def test_block_of_columns_is_exact(rows, wbits, gs, sym, case):
     assert torch.equal(got["scales_f32"].cpu(), want[1])
     assert torch.equal(got["zeros"].cpu(), want[2])
     assert torch.equal(got["codes"].cpu(), want[0])
+
+
+@pytest.mark.parametrize("rows", [8, 19000])
+def test_group_whose_scale_rounds_to_zero(rows):
+    """The zero point is infinite: the first code is the top one, and NaNs follow, for few rows as for many."""
+    from onecompression_b200 import kernels as K
+
+    d = 256
+    dev = torch.device("cuda:0")
+    w = torch.zeros(rows, d)
+    w[:, 0], w[:, 1] = 1.25, 15.0                  # scale 1, zero point 0, an error of 1/4 in column 0
+    u = torch.eye(d)
+    u[0, 128], u[0, 129] = -2.0 ** -147, 2.0 ** -147    # the second group: 2^-149, -2^-149, 0, 0, ...
+    iota = torch.arange(d, dtype=torch.int32, device=dev)
+    f = K.HessianFactor(u.to(dev), iota, iota, torch.zeros(d, dtype=torch.uint8, device=dev),
+                        torch.ones(2, device=dev), False, 0.01, 1.0, 1)
+    old = K._lib.load().oc_set_gemm_engine(1)      # the FMA engine keeps subnormal values
+    try:
+        got = K.gptq_quantize(w.half().to(dev), f, 4, 128, False, pack=False, want_codes=True, want_scales_f32=True)
+    finally:
+        K._lib.load().oc_set_gemm_engine(old)
+    want = torch.zeros(rows, d, dtype=torch.int32)
+    want[:, 0], want[:, 1], want[:, 128] = 1, 15, 15
+    assert not got["scales_f32"][1].any()
+    assert torch.equal(got["codes"].cpu(), want)
