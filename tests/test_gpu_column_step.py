@@ -90,3 +90,26 @@ def test_group_whose_scale_rounds_to_zero(rows):
     want[:, 0], want[:, 1], want[:, 128] = 1, 15, 15
     assert not got["scales_f32"][1].any()
     assert torch.equal(got["codes"].cpu(), want)
+
+
+@pytest.mark.parametrize("gs,act", [(48, False), (48, True), (80, False), (256, True), (256, False), (-1, False)])
+@pytest.mark.parametrize("mse", [False, True])
+def test_groups_across_blocks_do_not_depend_on_the_kernel(gs, act, mse):
+    """A group that crosses the end of a block, or holds several blocks, has its parameters handed between
+    the warps of the window kernel and from block to block.  96 rows take that kernel, 9600 the general one."""
+    from onecompression_b200 import kernels as K
+
+    d, out, dev = 640, 9600, torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(gs + 100)
+    x = torch.randn(2048, d, generator=g, device=dev).half()
+    x[:, ::37] *= 6
+    f = K.factor_hessian(K.hessian_from_activations(x)[0], 0.01, act)
+    w = (torch.randn(out, d, generator=g, device=dev) * 0.02).half()
+    args = dict(wbits=3, groupsize=gs, sym=False, pack=False, want_codes=True, want_scales_f32=True, mse=mse, q_grid=20)
+    whole = K.gptq_quantize(w, f, **args)
+    for r0 in (0, 4800, 9504):
+        part = K.gptq_quantize(w[r0:r0 + 96].contiguous(), f, **args)
+        for name in ("codes", "dequantized"):
+            assert torch.equal(part[name], whole[name][r0:r0 + 96])
+        for name in ("scales_f32", "scales", "zeros"):
+            assert torch.equal(part[name], whole[name][:, r0:r0 + 96])

@@ -1,5 +1,6 @@
 """The passes that bring matrices into and out of the column loop, the factor and the correction: odd
-sizes, strided rows and act-order, each against an equivalent call that takes another branch."""
+sizes, strided rows and act-order, each against an equivalent call whose passes take another branch (the
+column loop between them is the same on both sides)."""
 
 import pytest
 import torch
