@@ -96,22 +96,24 @@ def ptr(t):
     return None if t is None else t.data_ptr()
 
 
-_current_stream = None
+_raw_stream = None
 
 
 def _stream_source():
-    """What gives the current stream: an internal name that saves building a Stream object, the public way
-    in a torch without it."""
+    """What gives the stream of a device index: an internal name that saves building a Stream object, the
+    public way in a torch without it."""
     import torch
 
-    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), torch.cuda.current_device
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
     if raw is None:
-        return lambda: torch.cuda.current_stream().cuda_stream
-    return lambda: raw(device())
+        return torch.cuda.current_device, lambda index: torch.cuda.current_stream(index).cuda_stream
+    return torch.cuda.current_device, raw
 
 
-def stream_handle():
-    global _current_stream
-    if _current_stream is None:
-        _current_stream = _stream_source()
-    return _current_stream()
+def stream_handle(current=None):
+    """The current stream of the current device (whose index a caller may know already)."""
+    global _raw_stream
+    if _raw_stream is None:
+        _raw_stream = _stream_source()
+    device, raw = _raw_stream
+    return raw(device() if current is None else current)

@@ -25,12 +25,16 @@ _sm_count_cache: dict[int, int] = {}
 
 
 def sm_count(device) -> int:
-    idx = device if isinstance(device, int) else torch.device(device).index
+    idx = device if isinstance(device, int) else _as_device(device).index
     if idx is None:
         idx = torch.cuda.current_device()
     if idx not in _sm_count_cache:
         _sm_count_cache[idx] = torch.cuda.get_device_properties(idx).multi_processor_count
     return _sm_count_cache[idx]
+
+
+def _as_device(device) -> torch.device:
+    return device if type(device) is torch.device else torch.device(device)
 
 
 class _on:
@@ -40,7 +44,7 @@ class _on:
     __slots__ = ("_other",)
 
     def __init__(self, device):
-        device = torch.device(device)
+        device = _as_device(device)
         same = device.type == "cuda" and (device.index is None or device.index == torch.cuda.current_device())
         self._other = None if same else torch.cuda.device(device)
 
@@ -669,7 +673,7 @@ def packed_linear(x: torch.Tensor, qweight, qzeros, scales, g_idx, bias, wbits: 
     y = x.new_empty((*x.shape[:-1], out))
     args = (pq, qzeros.data_ptr(), ps, pg, out, d, groups, wbits, px, tokens, ptr(bias), y.data_ptr(), sm_count(dev))
     if dev == torch.cuda.current_device():
-        call("oc_packed_linear", *args, stream_handle())
+        call("oc_packed_linear", *args, stream_handle(dev))
     else:
         with _on(dev):
             call("oc_packed_linear", *args, stream_handle())

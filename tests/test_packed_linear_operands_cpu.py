@@ -141,12 +141,14 @@ def test_a_torch_without_an_internal_name_has_the_general_path(calls, monkeypatc
 
 def test_stream_handle_without_the_internal_name(monkeypatch):
     class Stream:
-        cuda_stream = 7
+        def __init__(self, index):
+            self.cuda_stream = 7 + index
 
     monkeypatch.setattr(torch.cuda, "current_stream", Stream)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
     monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
-    monkeypatch.setattr(_lib, "_current_stream", None)
-    assert _lib.stream_handle() == 7
+    monkeypatch.setattr(_lib, "_raw_stream", None)
+    assert _lib.stream_handle() == 8 and _lib.stream_handle(2) == 9
 
 
 def test_compiled_layer(calls):
