@@ -95,7 +95,7 @@ struct LinearArgs {
   const int* qweight; const int* qzeros; const __half* scales; const int* g_idx;
   const __half* x; const __half* bias; __half* y;
   int out, d, tokens, groups;
-  int staged;                // groups whose parameters fit in shared memory: all of them, or none
+  int staged;                // groups whose parameters lie in shared memory: all of them and one of zeros, or none
   long long ldz;
 };
 
@@ -109,8 +109,9 @@ template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.
 // one warp's slot of the ring: packed words and x of one iteration (two times 32 columns)
 template <int WORDS, int NT> struct __align__(16) Slot { int4 w[2][WORDS][32]; uint4 x[2][NT][32]; };
 
-constexpr int STAGED_BYTES = 40960;   // most shared memory that group parameters may take
 constexpr int PAR_BYTES = ROWS * 3;   // per group: 32 fp16 scales and 32 zero points of one byte
+constexpr int STAGED_GROUPS = 427;    // most groups whose parameters are staged, the one of zeros included
+constexpr int STAGED_BYTES = STAGED_GROUPS * PAR_BYTES;
 constexpr int MAX_UNITS = 8192;       // most eight-column units (two bytes each); wider layers are refused
 
 // NT * 8 tokens, WARPS column shares per CTA, DEPTH iterations of a warp in flight
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) packed_linear_kernel(const L
     const int gi = e / (ROWS / 4), r4 = e % (ROWS / 4) * 4, rr = blockIdx.x * ROWS + r4;
     unsigned z[4] = {0u, 0u, 0u, 0u};
     uint2 sv = make_uint2(0u, 0u);
-    if (rr < a.out) {
+    if (rr < a.out && gi < a.groups) {
       sv = *reinterpret_cast<const uint2*>(a.scales + (long long)gi * a.out + rr);
       load_zeros<BITS>(a.qzeros + gi * a.ldz, rr, z);
     }
@@ -196,19 +197,17 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) packed_linear_kernel(const L
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[t][n][i] = 0.f;
 
-  constexpr int NO_GROUP = -2, BEHIND = -1;   // BEHIND: columns behind the last one, whose weights are zero
-  int group = NO_GROUP;
+  int group = -1;
   __half2 s2[4], z2[4];
   auto load_group = [&](int gi) {
     unsigned z[4] = {0u, 0u, 0u, 0u};
     uint2 sv = make_uint2(0u, 0u);
-    if (gi == BEHIND) {                    // (a group's own parameters could make them infinite, and 0 * inf a NaN)
-    } else if (a.staged) {
+    if (a.staged) {
       sv = *reinterpret_cast<const uint2*>(par_s + gi * ROWS + 4 * g);
       const unsigned zb = *reinterpret_cast<const unsigned*>(par_z + gi * ROWS + 4 * g);
 #pragma unroll
       for (int i = 0; i < 4; ++i) z[i] = (zb >> (8 * i)) & 0xffu;
-    } else if (rows_ok) {
+    } else if (rows_ok && gi < a.groups) {
       sv = *reinterpret_cast<const uint2*>(a.scales + (long long)gi * a.out + r);
       load_zeros<BITS>(a.qzeros + gi * a.ldz, r, z);
     }
@@ -226,7 +225,9 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) packed_linear_kernel(const L
     for (int h = 0; h < 2; ++h) {
       const int unit = unit0 + 4 * h;
       const int4 w0 = cur->w[h][0][lane], w1 = F::WORDS > 1 ? cur->w[h][F::WORDS - 1][lane] : make_int4(0, 0, 0, 0);
-      const int ug = unit < units ? (int)ugroup[unit] : BEHIND;
+      // Columns behind the last one belong to a group of their own with a scale of zero: a group of the
+      // layer could make their weights infinite (scale * zero point beyond fp16), and 0 * inf a NaN.
+      const int ug = unit < units ? (int)ugroup[unit] : a.groups;
       const unsigned wr[4][2] = {{(unsigned)w0.x, (unsigned)w1.x}, {(unsigned)w0.y, (unsigned)w1.y},
                                  {(unsigned)w0.z, (unsigned)w1.z}, {(unsigned)w0.w, (unsigned)w1.w}};
       __half2 v[4][4];    // [row][pair]: weights of columns (k, k + 4) of the unit
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(WARPS * 32, CTAS) packed_linear_kernel(const L
             v[i][k] = __hmul2(__lows2half2(sa[i], s2[i]),
                               __hsub2(as_half2(F::pair(wr[i], unit, k) | 0x64006400u), __lows2half2(za[i], z2[i])));
         }
-        group = NO_GROUP;
+        group = -1;
       }
       __syncwarp();
 #pragma unroll
@@ -333,7 +334,7 @@ extern "C" int oc_packed_linear(const int* qweight, const int* qzeros, const voi
   OC_REQUIRE(d / 8 <= MAX_UNITS && groups < 0xffff, "packed_linear: too many columns or groups");
   OC_REQUIRE(groups >= 1 && (groups == 1 || g_idx), "packed_linear: several groups need g_idx");
   LinearArgs a{qweight, qzeros, (const __half*)scales16, g_idx, (const __half*)x16, (const __half*)bias16,
-               (__half*)y16, out, d, tokens, groups, groups <= STAGED_BYTES / PAR_BYTES ? groups : 0,
+               (__half*)y16, out, d, tokens, groups, groups < STAGED_GROUPS ? groups + 1 : 0,
                (bits == 3) ? out / 32 * 3 : out / f};
   if (sm_count <= 0) sm_count = 148;
   cudaStream_t s = (cudaStream_t)stream;
