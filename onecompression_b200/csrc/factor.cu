@@ -724,7 +724,8 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
       if (rest <= 0) break;
       float* panel = A + (long long)(k0 + nb) * ld + k0;
       OC_REQUIRE(nb == NB, "hinv_factor: a panel with rows below it is a full panel");
-      // the fewer rows per CTA, the shorter its time, as long as all CTAs run at once (one or two per SM)
+      // the fewer rows per CTA, the shorter its time, as long as all CTAs run at once (one or two on each
+      // of a B200's 148 SMs)
       const long long row_sets = (long long)oc_div_up(rest, 32) * batch;
       const int rc_t = row_sets <= 2 * 148 ? launch_trsm<32>(A, ld, k0, rest, batch, sW, stream)
                                            : launch_trsm<64>(A, ld, k0, rest, batch, sW, stream);

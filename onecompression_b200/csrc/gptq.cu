@@ -1,18 +1,21 @@
 // GPTQ column loop for one Linear weight, given the inverse-Hessian factor U.
 //
-// Follows run_gptq of the reference (onecomp/quantizer/gptq/_gptq.py:646-794)
-// operation for operation in fp32: true divides, round-half-to-even, the
-// rank-1 update as a rounded product followed by a rounded subtraction (this
-// file is compiled with -fmad=false and uses the _rn intrinsics besides).
+// Follows run_gptq of the reference (onecomp/quantizer/gptq/_gptq.py:646-794) in fp32 with its
+// roundings: quotients rounded like true divides (by a reciprocal and its correction where that
+// provably gives the same value, by a division where not), round-half-to-even, the rank-1 update as a
+// rounded product followed by a rounded subtraction (this file is compiled with -fmad=false and
+// uses the _rn intrinsics besides).
 //
-// Rows of W are independent given U, so one thread owns one row for a whole
-// block of up to 128 columns: the row's block lives in shared memory, 16
-// columns at a time in registers; the in-block error propagation needs no
-// inter-thread communication at all.  The lazy-batch trailing update
-// W[:, i2:] -= Err * U[i1:i2, i2:] is a launch of the fp32 GEMM engine with
-// the error block stored transposed (coalesced stores here, coalesced loads
-// there).  Codes are kept transposed ([column][row], 16 bit) until a final
-// pass packs them in original column order.
+// Rows of W are independent given U.  A block of up to 128 columns is worked off 16 columns (a
+// window) at a time in registers, by one of two kernels with the same bits:
+//   gptq_window_kernel  full blocks with up to two sets of 32 rows per SM: eight warps share 32 rows, one
+//                       warp per window; the errors of a window go to the later warps through shared
+//                       memory and named barriers
+//   gptq_block_kernel   everything else: one thread owns one row, whose block lives in shared memory;
+//                       in CTAs with few rows the other threads apply the updates behind the window
+// The lazy-batch trailing update W[:, i2:] -= Err * U[i1:i2, i2:] is a launch of the fp32 GEMM engine
+// with the error block stored transposed (coalesced stores here, coalesced loads there).  Codes are kept
+// transposed ([column][row], 16 bit) until a final pass packs them in original column order.
 #include "common.cuh"
 #include <type_traits>
 

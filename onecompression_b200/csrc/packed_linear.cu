@@ -1,7 +1,7 @@
 // y = x W^T (+ bias) for a few tokens, W in the packed AutoGPTQ layout, decoded inside the product.
 //
-// What bounds it: the packed weight is read once (bits / 8 bytes per weight) and nothing else of that
-// size moves, so HBM; decoding into an fp16 matrix first writes and reads 4 more bytes per weight.
+// The packed weight is read once (bits / 8 bytes per weight) and nothing else of that size moves;
+// decoding into an fp16 matrix first writes and reads 4 more bytes per weight.
 // The weights are the values of oc_dequantize_packed, bit for bit: scale * (q - z) is exact in fp32
 // (11 + 9 significant bits), so the fp16 product of the fp16 scale with the exact fp16 integer q - z is
 // its rounding.  Products and sums are fp32 (mma.sync m16n8k16; at these token counts the tensor
@@ -14,10 +14,16 @@
 // of one 16-byte load per token.  Rows are dealt to the two m16 tiles the same way.  The warps
 // of a CTA share the rows and split the columns; their sums meet in shared memory in a fixed order.
 //
-// Measured, 14336 x 4096, 4 bits, cold L2: 4 tokens 21.5 us, 16 tokens 29.5 us, against 77 us for decoding
+// Measured, 14336 x 4096, 4 bits, cold L2: 4 tokens 20 us, 16 tokens 29.5 us, against 77 us for decoding
 // and a library product (56 + 20); act-order 53 against 129 us.  4096 x 4096: 9 against 36 us.  At 16 tokens
 // it still takes less than half of the other way; more tokens are left to decoding once and a GEMM on
-// the tensor cores.  What is left is instructions (about 90 per warp for 32 x 32 weights), not HBM (1.4 TB/s).
+// the tensor cores.
+//
+// What bounds it at 4 tokens is latency: HBM delivers 1.3 TB/s (its floor is 5 us), and the 9.3 M warp instructions
+// are issued in 49 % of the cycles that an SM is active (74 % of the kernel's).  A CTA stages all group
+// parameters and the groups of all columns before its first product, and a warp has eleven iterations behind a
+// ring of two; the leading stalls are loads on their way (1.9 cycles per instruction) and the barrier
+// behind the staging (0.9).
 #include "common.cuh"
 
 namespace {
@@ -307,9 +313,9 @@ int launch(const LinearArgs& a, int grid, cudaStream_t stream) {
 template <int BITS>
 int launch_bits(const LinearArgs& a, int sm_count, cudaStream_t stream) {
   const int grid = oc_div_up(a.out, ROWS);
-  // With at most one CTA per SM the columns are split over 16 warps, with more over 6, so that four
-  // CTAs share an SM (14336 rows are 448 CTAs, just over three per SM): either way one wave of CTAs
-  // has the loads in flight that cover HBM's latency.
+  // With at most one CTA per SM the columns are split over 16 warps, with more over 6, so that several CTAs
+  // share an SM: four for up to 8 tokens (one wave up to 18944 rows; 14336 rows are 448 CTAs, just over
+  // three per SM), two for more tokens, whose sums take the registers (14336 rows are one and a half waves).
   const bool few = grid <= sm_count;
   if (a.tokens <= 8)
     return few ? launch<BITS, 1, 16, 2, 1>(a, grid, stream) : launch<BITS, 1, 6, 2, 4>(a, grid, stream);
