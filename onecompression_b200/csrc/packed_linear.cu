@@ -23,7 +23,7 @@
 // are issued in 49 % of the cycles that an SM is active (74 % of the kernel's).  A CTA stages all group
 // parameters and the groups of all columns before its first product, and a warp has eleven iterations behind a
 // ring of two; the leading stalls are loads on their way (1.9 cycles per instruction) and the barrier
-// behind the staging (0.9).
+// behind the staging (0.8).
 #include "common.cuh"
 
 namespace {
