@@ -197,7 +197,7 @@ class MomentAccumulator:
     def finalize(self, check: bool = True):
         """Complete H (mirror the upper triangle) and return (H, C, nsamples)."""
         self._clear_unwritten()
-        if self._needs_mirror:
+        if self._needs_mirror:   # (after a look at H too: what was added to it since may be an upper part)
             self._mirror()
             self._needs_mirror = False
         if check:

@@ -1,4 +1,4 @@
-"""Inputs of the factor that are no ordinary Hessian: NaNs on the diagonal with act-order."""
+"""The factor with NaNs on the diagonal and act-order, and with an order that the caller brings."""
 
 import pytest
 import torch
