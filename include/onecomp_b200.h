@@ -255,11 +255,20 @@ int oc_packed_linear(const int* qweight, const int* qzeros, const void* scales16
 int oc_gemm_f32(const float* A, long long lda, const float* B, long long ldb, float* C,
                 long long ldc, int M, int N, int K, float alpha, float beta, int transA,
                 int transB, int flags, void* stream);
+/* C = alpha*opA(A)*opB(B), or C += with `add`, as the factor, the column loop and the correction compute it: both operands are first
+ * written as two scaled fp16 planes (rows_scaled != 0: the rows of an untransposed A are scaled each for
+ * itself), then multiplied on the tensor cores, three products for one.  C 16-byte aligned, ldc a multiple
+ * of 4 (rows of C are written up to the next multiple of four columns); workspace: that many bytes, 256-byte aligned. */
+long long oc_gemm_split_workspace_bytes(int M, int N, int K, int transA, int transB);
+int oc_gemm_split_f32(const float* A, long long lda, const float* B, long long ldb, float* C, long long ldc,
+                      int M, int N, int K, float alpha, int add, int transA, int transB, int flags,
+                      int rows_scaled, void* workspace, void* stream);
 /* Engine behind every fp32 product of this library (oc_gemm_f32, the Cholesky and inverse
- * updates, the GPTQ trailing update, the QEP products): mode 0 (default) runs 16-byte aligned
- * operands on the tensor cores as 3xTF32 (fp32-grade accuracy), mode 1 always uses the fp32 FMA
+ * updates, the GPTQ trailing update, the QEP products): mode 0 (default) runs them on the tensor
+ * cores with fp32-grade accuracy (operands in two fp16 planes; 3xTF32 where operands are given as they are and
+ * for block sizes other than 128), 16-byte aligned operands and workspaces provided; mode 1 always uses the fp32 FMA
  * kernel.  Returns the previous mode.  oc_gemm_tc_status() is 0 unless a bounded pipeline wait
- * of the tensor-core engine expired on the current device (201..205). */
+ * of a tensor-core product expired on the current device (201..205, 301..304). */
 int oc_set_gemm_engine(int mode);
 int oc_gemm_tc_status(void);
 /* Output tile of the tensor-core engine for plain products (flags == 0): 0 (default) picks

@@ -22,6 +22,8 @@ SOURCES = {
     "errors.cu": [],
     "gemm.cu": [],
     "gemm_tc.cu": [],
+    "gemm_split.cu": [],
+    "split.cu": [],
     "factor.cu": [],
     "gptq.cu": ["-fmad=false"],
     "moment_simt.cu": [],

@@ -112,3 +112,11 @@ struct OcGemm {
 };
 
 int oc_gemm_f32_launch(const OcGemm& g, cudaStream_t stream);
+
+// What the tensor-core products need to know about the current device.
+struct OcGemmDevice {
+  int sms;
+  int* status;      // device word that records an expired pipeline wait
+  int tile_shape;   // the switch of oc_set_gemm_tile_shape
+};
+int oc_gemm_device(OcGemmDevice& d);

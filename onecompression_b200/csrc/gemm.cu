@@ -206,6 +206,8 @@ extern "C" int oc_set_gemm_engine(int mode) {
   return old;
 }
 
+bool oc_split_engine_on() { return g_engine_mode == 0; }
+
 int oc_gemm_f32_launch(const OcGemm& g, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return OC_OK;
   OC_REQUIRE(g.A && g.B && g.C && g.K >= 0, "gemm: null operand or negative K");

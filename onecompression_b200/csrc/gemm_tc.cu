@@ -385,7 +385,7 @@ int* g_status[OC_MAX_DEVICES] = {};
 int g_tile_shape = 0;   // 0: chosen per product; 1: narrow tiles only; 2: wide tiles wherever allowed
 
 template <class S>
-int launch_shape(const OcGemm& g, int dev, cudaStream_t stream) {
+int launch_shape(const OcGemm& g, const OcGemmDevice& dev, cudaStream_t stream) {
   CUtensorMap ma, mb;
   int rc = make_operand_map(&ma, g.A, g.transA != 0, g.M, g.K, g.lda, g.strideA, g.batch, BM, S::BK);
   if (rc) return rc;
@@ -395,10 +395,10 @@ int launch_shape(const OcGemm& g, int dev, cudaStream_t stream) {
   p.C = g.C; p.ldc = g.ldc; p.strideC = g.strideC; p.M = g.M; p.N = g.N; p.K = g.K;
   p.alpha = g.alpha; p.beta = g.beta; p.flags = g.flags; p.batch = g.batch;
   p.tiles_m = oc_div_up(g.M, BM); p.tiles_n = oc_div_up(g.N, S::BN);
-  p.status = g_status[dev];
+  p.status = dev.status;
   const long long items = (long long)p.batch * p.tiles_m * p.tiles_n;
   OC_REQUIRE(items < (1ll << 30), "gemm: too many tiles");
-  const int grid = (int)((items < g_sm_count[dev]) ? items : g_sm_count[dev]);
+  const int grid = (int)((items < dev.sms) ? items : dev.sms);
   const bool a_mn = g.transA != 0, b_mn = g.transB == 0;
   if (a_mn) return b_mn ? launch<true, true, S>(ma, mb, p, grid, stream) : launch<true, false, S>(ma, mb, p, grid, stream);
   return b_mn ? launch<false, true, S>(ma, mb, p, grid, stream) : launch<false, false, S>(ma, mb, p, grid, stream);
@@ -455,7 +455,7 @@ extern "C" int oc_gemm_tile_choice(int M, int N, int batch, int flags, int sms) 
   return cost_wide < cost_narrow ? 2 : 1;
 }
 
-int oc_gemm_tc_launch(const OcGemm& g, cudaStream_t stream) {
+int oc_gemm_device(OcGemmDevice& d) {
   OC_CURRENT_DEVICE(dev);
   if (!g_status[dev]) {
     void* p = nullptr;
@@ -465,7 +465,15 @@ int oc_gemm_tc_launch(const OcGemm& g, cudaStream_t stream) {
   if (g_sm_count[dev] == 0) {
     OC_CUDA(cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev));
   }
-  const bool wide = oc_gemm_tile_choice(g.M, g.N, g.batch, g.flags, g_sm_count[dev]) == 2;
+  d.sms = g_sm_count[dev]; d.status = g_status[dev]; d.tile_shape = g_tile_shape;
+  return OC_OK;
+}
+
+int oc_gemm_tc_launch(const OcGemm& g, cudaStream_t stream) {
+  OcGemmDevice dev;
+  const int rc = oc_gemm_device(dev);
+  if (rc) return rc;
+  const bool wide = oc_gemm_tile_choice(g.M, g.N, g.batch, g.flags, dev.sms) == 2;
   return wide ? launch_shape<Wide>(g, dev, stream) : launch_shape<Narrow>(g, dev, stream);
 }
 

@@ -4,9 +4,10 @@
 // The reference factors H + damp I and solves with potrf + potrs.  Here the
 // inverse-Hessian factor U of the same damped matrix (U^T U = (P H P^T + damp I)^-1,
 // P the act-order permutation or the identity) is already at hand for the GPTQ
-// column loop, so the solve becomes two triangular products on the fp32 GEMM
-// engine:   dW P^T = ((W C) P^T) U^T U.
-#include "common.cuh"
+// column loop, so the solve becomes two triangular products:   dW P^T = ((W C) P^T) U^T U.
+// The three products run on the tensor cores with operands in two fp16 planes (split.cuh); the weight, 16 bits
+// wide, needs one plane.
+#include "split.cuh"
 
 namespace {
 
@@ -51,6 +52,40 @@ __global__ void qep_load_kernel(const void* __restrict__ W, long long ldw_in, in
   Wf[(long long)r * ldw + c] = (dead && dead[c]) ? 0.f : v;
 }
 
+// W with dead columns zeroed as one fp16 plane: an fp16 weight as it is; a bf16 weight with every row of 128 columns
+// scaled by a power of two (table, entry chunk * out + row), which keeps its 8 bits.  One warp per row of 128.
+__global__ void __launch_bounds__(256) qep_plane_kernel(const void* __restrict__ W, long long ldw_in, int out, int d,
+                                                        const unsigned char* __restrict__ dead, __half* __restrict__ plane,
+                                                        long long ldp, float* __restrict__ table, int bf16, int vec) {
+  const int lane = threadIdx.x & 31, r = blockIdx.y * 8 + (threadIdx.x >> 5), c = blockIdx.x * 128 + lane * 4;
+  if (r >= out) return;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+  if (c < d) {
+    if (vec) {
+      const float4 t = load_masked(W, (long long)r * ldw_in + c, c, dead, bf16);
+      v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < d && !(dead && dead[c + j])) v[j] = oc_ld16(W, (long long)r * ldw_in + c + j, bf16);
+    }
+  }
+  if (bf16) {
+    float mx = fmaxf(fmaxf(oc_finite_abs(v[0]), oc_finite_abs(v[1])), fmaxf(oc_finite_abs(v[2]), oc_finite_abs(v[3])));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    float inv;
+    const float s = oc_split_scale(mx, inv);
+    if (lane == 0) table[(long long)blockIdx.x * out + r] = inv;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] *= s;
+  }
+  if (c >= d) return;
+  const __half2 a = __floats2half2_rn(v[0], v[1]), b = __floats2half2_rn(v[2], v[3]);
+  *reinterpret_cast<uint2*>(plane + (long long)r * ldp + c) =
+      make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+}
+
 __global__ void gather_cols_kernel(const float* __restrict__ src, long long lds, int out, int d,
                                    const int* __restrict__ perm, float* __restrict__ dst, long long ldd) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -93,10 +128,77 @@ __global__ void qep_store_kernel(const unsigned char* __restrict__ dead, const f
 
 long long round4(long long x) { return (x + 3) / 4 * 4; }
 
+long long round8(long long x) { return (x + 7) / 8 * 8; }
+long long blocks(long long x) { return (x + OC_SPLIT_BLOCK - 1) / OC_SPLIT_BLOCK; }
+
+// Workspace with split operands: the left operand's planes, an fp32 result, the planes of C (later those of U), and
+// their tables.
+struct QepWs {
+  long long ld, planes, result, right, tab_rows, tab, total;
+  QepWs(int out, int d) {
+    ld = round8(d);
+    planes = 4 * (long long)out * ld; result = 4 * (long long)out * ld; right = 4 * (long long)d * ld;
+    tab_rows = round8(blocks(d) * out) * 4; tab = round8(blocks(d) * blocks(d)) * 4;
+    total = planes + result + right + tab_rows + tab;
+  }
+};
+
+// dW P^T (fp32, ws.ld apart) into the workspace; returned in `delta`
+int split_products(const void* W, long long ldw_io, int out, int d, const float* C, long long ldc, const float* U,
+                   long long ldu, const int* perm, const unsigned char* dead, int bf16, int vec, char* workspace,
+                   float*& delta, cudaStream_t stream) {
+  const QepWs ws(out, d);
+  __half* Lp = (__half*)workspace;
+  float* R = (float*)(workspace + ws.planes);
+  __half* Rp = (__half*)(workspace + ws.planes + ws.result);
+  float* tabL = (float*)(workspace + ws.planes + ws.result + ws.right);
+  float* tabR = (float*)(workspace + ws.planes + ws.result + ws.right + ws.tab_rows);
+  const long long nb = blocks(d);
+  delta = R;
+  qep_plane_kernel<<<dim3((int)nb, oc_div_up(out, 8)), 256, 0, stream>>>(W, ldw_io, out, d, dead, Lp, ws.ld, tabL, bf16, vec);
+  OC_CHECK_LAUNCH();
+  OcSplitArgs right{};
+  right.rows = right.cols = d; right.planes = Rp; right.plane = d * ws.ld; right.ldp = ws.ld; right.table = tabR;
+  right.ldt = nb; right.nb1 = right.nb2 = 1;
+  right.src = C; right.ld = ldc;
+  int rc = oc_split_launch(right, stream);
+  if (rc) return rc;
+  OcSplitArgs left{};
+  left.src = R; left.ld = ws.ld; left.rows = out; left.cols = d; left.planes = Lp; left.plane = out * ws.ld;
+  left.ldp = ws.ld; left.table = tabL; left.ldt = out; left.per_row = 1; left.nb1 = left.nb2 = 1;
+  OcSplitGemm g{};
+  g.C = R; g.ldc = ws.ld; g.M = out; g.N = d; g.K = d; g.nb1 = g.nb2 = 1; g.alpha = 1.f;
+  g.A.planes = Lp; g.A.plane = left.plane; g.A.ld = ws.ld; g.A.scale_k = out; g.A.scale_r = OC_SPLIT_BLOCK; g.A.scale_row = 1;
+  g.B.planes = Rp; g.B.plane = right.plane; g.B.ld = ws.ld; g.B.terms = 2; g.B.scale = tabR;
+  // R = Wz C
+  g.A.terms = 1; g.A.scale = bf16 ? tabL : nullptr;
+  g.B.mn_major = 1; g.B.scale_k = nb; g.B.scale_r = 1;
+  rc = oc_gemm_split_launch(g, stream);
+  if (rc) return rc;
+  // T = R P^T U^T      (U upper: U[n][k] = 0 for k < n)
+  right.src = U; right.ld = ldu; right.region = OC_SPLIT_UPPER;
+  rc = oc_split_launch(right, stream);
+  if (rc) return rc;
+  left.perm = perm;
+  rc = oc_split_launch(left, stream);
+  if (rc) return rc;
+  g.A.terms = 2; g.A.scale = tabL;
+  g.B.mn_major = 0; g.B.scale_k = 1; g.B.scale_r = nb; g.flags = OC_GEMM_KLO_FROM_N;
+  rc = oc_gemm_split_launch(g, stream);
+  if (rc) return rc;
+  // dW P^T = T U       (U[k][n] = 0 for k > n)
+  left.perm = nullptr;
+  rc = oc_split_launch(left, stream);
+  if (rc) return rc;
+  g.B.mn_major = 1; g.B.scale_k = nb; g.B.scale_r = 1; g.flags = OC_GEMM_KHI_FROM_N;
+  return oc_gemm_split_launch(g, stream);
+}
+
 }  // namespace
 
 extern "C" long long oc_qep_workspace_bytes(int out, int d) {
-  return 3 * (long long)out * round4(d) * 4 + 256;
+  const long long plain = 3 * (long long)out * round4(d) * 4, split = QepWs(out, d).total;
+  return (plain > split ? plain : split) + 256;
 }
 
 // See include/onecomp_b200.h for the contract.
@@ -123,6 +225,18 @@ extern "C" int oc_qep_adjust(void* W_, long long ldw_io, int out, int d, const f
   const bool vec = d % 4 == 0 && ldw_io % 4 == 0 && (reinterpret_cast<uintptr_t>(W) & 7) == 0 &&
                    (reinterpret_cast<uintptr_t>(Wf) & 15) == 0 && (reinterpret_cast<uintptr_t>(dead) & 3) == 0;
   const dim3 grid4(oc_div_up(d, 4 * tb), out);
+  if (oc_split_engine_on() && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
+    float* delta = nullptr;
+    const bool vec_w = d % 4 == 0 && ldw_io % 4 == 0 && (reinterpret_cast<uintptr_t>(W) & 7) == 0 &&
+                       (reinterpret_cast<uintptr_t>(dead) & 3) == 0;
+    const int rc = split_products(W, ldw_io, out, d, C, ldc, U, ldu, perm, dead, bf16, vec_w, (char*)workspace, delta, stream);
+    if (rc) return rc;
+    const bool vec_st = vec_w && !perm;
+    qep_store_kernel<<<vec_st ? grid4 : grid, tb, 0, stream>>>(dead, delta, QepWs(out, d).ld, out, d, perm, perccorr, W,
+                                                              ldw_io, bf16, vec_st);
+    OC_CHECK_LAUNCH();
+    return OC_OK;
+  }
   qep_load_kernel<<<vec ? grid4 : grid, tb, 0, stream>>>(W, ldw_io, out, d, dead, Wf, ld, bf16, vec);
   OC_CHECK_LAUNCH();
   OcGemm g{};

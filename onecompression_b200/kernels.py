@@ -906,8 +906,8 @@ class deferred_host_copies:
 
 
 def set_gemm_engine(mode: int) -> int:
-    """0: fp32 products run on the tensor cores as 3xTF32 when their operands are 16-byte
-    aligned (default); 1: always the fp32 FMA kernel.  Returns the previous mode."""
+    """0: fp32 products run on the tensor cores in split operands when these are 16-byte aligned
+    (default); 1: always the fp32 FMA kernel.  Returns the previous mode."""
     return _lib.load().oc_set_gemm_engine(int(mode))
 
 
@@ -941,4 +941,20 @@ def gemm_f32(a, b, c=None, alpha=1.0, beta=0.0, trans_a=False, trans_b=False, fl
     with _on(a.device):
         call("oc_gemm_f32", ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(c), c.stride(0), m, n, k,
              float(alpha), float(beta), int(trans_a), int(trans_b), int(flags), stream_handle())
+    return c
+
+
+def gemm_split(a, b, c=None, alpha=1.0, add=False, trans_a=False, trans_b=False, flags=0, rows_scaled=False):
+    """Product of operands split into two fp16 planes, exposed for tests: C = alpha·op(A)·op(B), added to C with ``add``."""
+    _require_cuda(a, "a")
+    m = a.shape[1] if trans_a else a.shape[0]
+    k = a.shape[0] if trans_a else a.shape[1]
+    n = b.shape[0] if trans_b else b.shape[1]
+    if c is None:
+        c = torch.zeros((m, n), dtype=torch.float32, device=a.device)
+    with _on(a.device):
+        ws = _workspace(_lib.load().oc_gemm_split_workspace_bytes(m, n, k, int(trans_a), int(trans_b)), a.device)
+        call("oc_gemm_split_f32", ptr(a), a.stride(0), ptr(b), b.stride(0), ptr(c), c.stride(0), m, n, k,
+             float(alpha), int(add), int(trans_a), int(trans_b), int(flags), int(rows_scaled), ptr(ws),
+             stream_handle())
     return c
