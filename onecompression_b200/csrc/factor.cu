@@ -7,13 +7,17 @@
 //   A = J (P H P^T + damp I) J      (J reverses the index order, P is the act-order permutation)
 //   A = L L^T                       blocked right-looking Cholesky (two levels: 128 / 512), fp32:
 //                                   diagonal block on one SM, panel solve by forward substitution
-//                                   (fp32 FMAs, all SMs), updates on the tensor cores (3xTF32)
+//                                   (fp32 FMAs, all SMs), updates on the tensor cores (gemm_split.cu)
 //   X = L^-1                        diagonal blocks inverted in one launch, then joined level by
 //                                   level (recursive blocked triangular inverse), fp32
 //   U = J X J                       upper triangular, U^T U = (P H P^T + damp I)^-1
 //
 // because J L J is the upper factor V of H = V V^T and U = V^-1.
-#include "common.cuh"
+//
+// A is equilibrated: rows and columns are multiplied by powers of two that bring its diagonal into [1, 4), and the
+// columns of U are scaled back.  Nothing but exponents changes, and the entries of L are below 2 in
+// magnitude, so that the panels of L can be kept as two fp16 planes (split.cuh) under one fixed scale.
+#include "split.cuh"
 
 namespace {
 
@@ -25,14 +29,16 @@ constexpr int BUILD_STAGED_N = 49152;   // widest row that the act-order gather 
 // diagv[j] = H[j,j] (1 where it is 0), dead[j], damp_out[0] = percdamp * mean(diagv)
 // Batched launches: block index `b` of the batch dimension selects the problem; `sH`, `sW`, ... are
 // the element strides between consecutive problems.
-__global__ void diag_stats_kernel(const float* __restrict__ H, long long ld, int n, float percdamp,
+// equil[j] = 2^-e with (diagv[j] + shift) / 4^e in [1, 4)
+__global__ void diag_stats_kernel(const float* __restrict__ H, long long ld, int n, float percdamp, float rel_shift,
                                   float* __restrict__ diagv, unsigned char* __restrict__ dead,
-                                  float* __restrict__ damp_out, long long sH, long long sW) {
+                                  float* __restrict__ damp_out, float* __restrict__ equil, long long sH, long long sW) {
   {
     const long long b = blockIdx.x;
-    H += b * sH; diagv += b * sW; dead += b * n; damp_out += b * 2;
+    H += b * sH; diagv += b * sW; dead += b * n; damp_out += b * 2; equil += b * sW;
   }
   __shared__ double red[32];
+  __shared__ float damp_s;
   double s = 0.0;
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
     float v = H[(long long)j * ld + j];
@@ -48,8 +54,16 @@ __global__ void diag_stats_kernel(const float* __restrict__ H, long long ld, int
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int w = 0; w < (blockDim.x + 31) / 32; ++w) t += red[w];
-    damp_out[0] = percdamp * (float)(t / (double)n);
+    damp_out[0] = damp_s = percdamp * (float)(t / (double)n);
     damp_out[1] = (float)(t / (double)n);
+  }
+  __syncthreads();
+  const float shift = rel_shift * damp_s;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const float v = diagv[j] + shift;
+    const int e = ((int)(__float_as_uint(v) >> 23) - 127) >> 1;
+    const bool ok = v > 0.f && v <= 3.402823466e38f;       // (anything else ends in a bad pivot)
+    equil[j] = ok ? __uint_as_float((unsigned)(127 - e) << 23) : 1.f;
   }
 }
 
@@ -90,67 +104,77 @@ __global__ void invert_perm_kernel(const int* __restrict__ perm, int* __restrict
   if (i < n) inv[perm[i]] = i;
 }
 
-// ---- A = J (P Hfix P^T + shift I) J ------------------------------------------------
+// ---- A = J D (P Hfix P^T + shift I) D J, D = diag(equil) --------------------------------------
 // Only what the factorisation reads: every row up to the end of its diagonal block.  One CTA per row,
 // bound by HBM (4 bytes in, 2 out per entry of H with act-order, where the whole row of H passes
 // through shared memory and the permutation is a gather on chip; half of that without).  One global
 // access per entry before: 14336 with act-order 1042 us, 264 us now; 4096 67, 16 us.
+// equil_p[j] = equil[perm[j]]: what scales the columns of U back.
 __global__ void __launch_bounds__(256) build_reversed_kernel(
     const float* __restrict__ H, long long ldh, int n, const int* __restrict__ perm, int permuted,
-    const float* __restrict__ diagv, const float* __restrict__ damp, float rel_shift, float* __restrict__ A,
-    long long lda, long long sH, long long sW, int vec, int staged) {
+    const float* __restrict__ diagv, const float* __restrict__ damp, float rel_shift, const float* __restrict__ equil,
+    float* __restrict__ equil_p, float* __restrict__ A, long long lda, long long sH, long long sW, int vec, int staged) {
   extern __shared__ __align__(16) float row_s[];
   const int i = blockIdx.x;
   {
     const long long b = blockIdx.y;
-    H += b * sH; perm += b * n; diagv += b * sW; damp += b * 2; A += b * sW;
+    H += b * sH; perm += b * n; diagv += b * sW; damp += b * 2; A += b * sW; equil += b * sW; equil_p += b * sW;
   }
   const int pi = permuted ? perm[n - 1 - i] : n - 1 - i;
   const float* h = H + (long long)pi * ldh;
   float* a = A + (long long)i * lda;
+  const float di = equil[pi];
   const int end = min(n, (i / NB + 1) * NB);
   if (permuted && staged) {
     if (vec) {
-      for (int j = threadIdx.x * 4; j < n; j += 1024) *reinterpret_cast<float4*>(row_s + j) = *reinterpret_cast<const float4*>(h + j);
+      for (int j = threadIdx.x * 4; j < n; j += 1024) {
+        const float4 v = *reinterpret_cast<const float4*>(h + j), d = *reinterpret_cast<const float4*>(equil + j);
+        *reinterpret_cast<float4*>(row_s + j) = make_float4(v.x * di * d.x, v.y * di * d.y, v.z * di * d.z, v.w * di * d.w);
+      }
     } else {
-      for (int j = threadIdx.x; j < n; j += 256) row_s[j] = h[j];
+      for (int j = threadIdx.x; j < n; j += 256) row_s[j] = h[j] * di * equil[j];
     }
     __syncthreads();
     for (int j = threadIdx.x; j < end; j += 256) a[j] = row_s[perm[n - 1 - j]];
   } else if (permuted) {
-    for (int j = threadIdx.x; j < end; j += 256) a[j] = h[perm[n - 1 - j]];
+    for (int j = threadIdx.x; j < end; j += 256) { const int p = perm[n - 1 - j]; a[j] = h[p] * di * equil[p]; }
   } else if (vec) {           // n, ldh, lda multiples of 4, 16-byte aligned: so is `end`
     for (int j = threadIdx.x * 4; j < end; j += 1024) {
-      const float4 v = *reinterpret_cast<const float4*>(h + n - 4 - j);
-      *reinterpret_cast<float4*>(a + j) = make_float4(v.w, v.z, v.y, v.x);
+      const float4 v = *reinterpret_cast<const float4*>(h + n - 4 - j), d = *reinterpret_cast<const float4*>(equil + n - 4 - j);
+      *reinterpret_cast<float4*>(a + j) = make_float4(v.w * di * d.w, v.z * di * d.z, v.y * di * d.y, v.x * di * d.x);
     }
   } else {
-    for (int j = threadIdx.x; j < end; j += 256) a[j] = h[n - 1 - j];
+    for (int j = threadIdx.x; j < end; j += 256) a[j] = h[n - 1 - j] * di * equil[n - 1 - j];
   }
   __syncthreads();
-  if (threadIdx.x == 0) a[i] = diagv[pi] + rel_shift * damp[0];
+  if (threadIdx.x == 0) {
+    a[i] = (diagv[pi] + rel_shift * damp[0]) * di * di;
+    equil_p[n - 1 - i] = di;
+  }
 }
 
-// ---- U = J X J (upper part), zero below the diagonal ------------------------------------
+// ---- U = J X J D (upper part), zero below the diagonal ------------------------------------
 // One CTA per row, bound by HBM (2 bytes in, 4 out per entry).  One entry per access before: 14336
 // 619 us, 183 us now; 4096 50, 14 us.
 __global__ void __launch_bounds__(256) reverse_upper_kernel(const float* __restrict__ X, long long ldx, int n,
-                                                            float* __restrict__ U, long long ldu, long long sW,
-                                                            long long sU, int vec) {
+                                                            const float* __restrict__ equil_p, float* __restrict__ U,
+                                                            long long ldu, long long sW, long long sU, int vec) {
   const int i = blockIdx.x;
   const float* x = X + (long long)blockIdx.y * sW + (long long)(n - 1 - i) * ldx;
   float* u = U + (long long)blockIdx.y * sU + (long long)i * ldu;
+  equil_p += (long long)blockIdx.y * sW;
   if (vec) {
     for (int j = threadIdx.x * 4; j < n; j += 1024) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       if (j + 3 >= i) {
-        const float4 t = *reinterpret_cast<const float4*>(x + n - 4 - j);
-        v.x = j >= i ? t.w : 0.f; v.y = j + 1 >= i ? t.z : 0.f; v.z = j + 2 >= i ? t.y : 0.f; v.w = t.x;
+        const float4 t = *reinterpret_cast<const float4*>(x + n - 4 - j), d = *reinterpret_cast<const float4*>(equil_p + j);
+        v.x = j >= i ? t.w * d.x : 0.f; v.y = j + 1 >= i ? t.z * d.y : 0.f; v.z = j + 2 >= i ? t.y * d.z : 0.f;
+        v.w = t.x * d.w;
       }
       *reinterpret_cast<float4*>(u + j) = v;
     }
   } else {
-    for (int j = threadIdx.x; j < n; j += 256) u[j] = (j >= i) ? x[n - 1 - j] : 0.f;
+    for (int j = threadIdx.x; j < n; j += 256) u[j] = (j >= i) ? x[n - 1 - j] * equil_p[j] : 0.f;
   }
 }
 
@@ -433,10 +457,14 @@ potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb, int* __
 constexpr int TRT = 256;                   // threads per CTA (the first 2 * TR solve, all of them load)
 constexpr int LPITCH = NB + 4, YPITCH = NB + 4;
 template <int TR> constexpr int TRSM_SMEM = (NB * LPITCH + TR * YPITCH + NB) * (int)sizeof(float);
-template <int TR>                          // rows per CTA
+// With SPLIT the solved rows leave as two fp16 planes under the fixed scale L_SCALE (the products behind the
+// panel are all that reads them), without as fp32 in place.
+constexpr float L_SCALE = 8192.f;          // entries of L are below 2
+template <int TR, bool SPLIT>              // rows per CTA
 __global__ void __launch_bounds__(TRT, 2) trsm_panel_kernel(float* __restrict__ A, long long lda, int k0, int rest,
-                                                         long long sW) {
+                                                         long long sW, __half* __restrict__ planes, long long plane) {
   A += (long long)blockIdx.y * sW;
+  if (SPLIT) planes += (long long)blockIdx.y * sW * 2;
   extern __shared__ __align__(16) float sm[];
   float* Lt = sm;                           // Lt[i * LPITCH + j] = L[j][i] for j >= i
   float* Ys = sm + NB * LPITCH;             // this CTA's rows: 64 even columns, then 64 odd ones
@@ -522,15 +550,25 @@ __global__ void __launch_bounds__(TRT, 2) trsm_panel_kernel(float* __restrict__ 
     if (r < rows) {
       const float2 ev = *reinterpret_cast<const float2*>(Ys + r * YPITCH + 2 * c4);
       const float2 od = *reinterpret_cast<const float2*>(Ys + r * YPITCH + NB / 2 + 2 * c4);
-      *reinterpret_cast<float4*>(P + (long long)(row0 + r) * lda + 4 * c4) = make_float4(ev.x, od.x, ev.y, od.y);
+      if (SPLIT) {
+        uint2 hi, lo;
+        oc_split4(make_float4(ev.x * L_SCALE, od.x * L_SCALE, ev.y * L_SCALE, od.y * L_SCALE), hi, lo);
+        __half* to = planes + (long long)(k0 + NB + row0 + r) * lda + k0 + 4 * c4;
+        *reinterpret_cast<uint2*>(to) = hi;
+        *reinterpret_cast<uint2*>(to + plane) = lo;
+      } else {
+        *reinterpret_cast<float4*>(P + (long long)(row0 + r) * lda + 4 * c4) = make_float4(ev.x, od.x, ev.y, od.y);
+      }
     }
   }
 }
 
-template <int TR>
-int launch_trsm(float* A, long long ld, int k0, int rest, int batch, long long sW, cudaStream_t stream) {
-  OC_OPT_IN_SMEM(trsm_panel_kernel<TR>, TRSM_SMEM<TR>);
-  trsm_panel_kernel<TR><<<dim3(oc_div_up(rest, TR), batch), TRT, TRSM_SMEM<TR>, stream>>>(A, ld, k0, rest, sW);
+template <int TR, bool SPLIT>
+int launch_trsm(float* A, long long ld, int k0, int rest, int batch, long long sW, __half* planes, long long plane,
+                cudaStream_t stream) {
+  OC_OPT_IN_SMEM((trsm_panel_kernel<TR, SPLIT>), TRSM_SMEM<TR>);
+  trsm_panel_kernel<TR, SPLIT><<<dim3(oc_div_up(rest, TR), batch), TRT, TRSM_SMEM<TR>, stream>>>(A, ld, k0, rest, sW,
+                                                                                              planes, plane);
   OC_CHECK_LAUNCH();
   return OC_OK;
 }
@@ -544,7 +582,8 @@ constexpr int DINV_T = 512;
 constexpr int DINV_SMEM = (2 * NB * (NB + 1) + (NB / 2) * (NB / 2)) * (int)sizeof(float);
 __global__ void __launch_bounds__(DINV_T) diag_inverse_kernel(const float* __restrict__ A, long long lda,
                                                            float* __restrict__ X, long long ldx, int n,
-                                                           long long sW) {
+                                                           long long sW, __half* __restrict__ planes, long long plane,
+                                                           float* __restrict__ table, int ldt) {
   A += (long long)blockIdx.y * sW;
   X += (long long)blockIdx.y * sW;
   extern __shared__ __align__(16) float sm[];
@@ -643,23 +682,120 @@ __global__ void __launch_bounds__(DINV_T) diag_inverse_kernel(const float* __res
   // A product with the lower triangular X starts its k-range at its tile's first column; tiles are up
   // to 256 columns wide and start at even blocks, so they also read the block right of an even
   // diagonal block.  Nothing else above the diagonal blocks is ever read.
-  if ((blockIdx.x & 1) == 0) {
-    const int width = min(NB, n - k0 - NB);
+  const int width = (blockIdx.x & 1) == 0 ? min(NB, n - k0 - NB) : 0;
+  if (!planes) {
     for (int e = tid; e < nb * NB; e += DINV_T)
       if (e % NB < width) Xb[(long long)(e / NB) * ldx + NB + e % NB] = 0.f;
+    return;
+  }
+  // the products read the two planes of X (split.cuh; block scales)
+  planes += (long long)blockIdx.y * sW * 2 + (long long)k0 * ldx + k0;
+  table += (long long)blockIdx.y * sW + (long long)blockIdx.x * (ldt + 1);
+  float mx = 0.f;
+  for (int e = tid; e < NB * NB; e += DINV_T) mx = fmaxf(mx, oc_finite_abs(Y[e / NB][e % NB]));
+  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) T[tid >> 5] = mx;                // (the joins' scratch is free)
+  __syncthreads();
+  mx = 0.f;
+  for (int w = 0; w < DINV_T / 32; ++w) mx = fmaxf(mx, T[w]);
+  float inv;
+  const float sc = oc_split_scale(mx, inv);
+  if (tid == 0) {
+    table[0] = inv;
+    if (width > 0) table[1] = 1.f;
+  }
+#pragma unroll 4
+  for (int e = tid; e < NB * NB / 4; e += DINV_T) {
+    const int i = e / (NB / 4), j = e % (NB / 4) * 4;
+    if (i >= nb) break;
+    __half* to = planes + (long long)i * ldx + j;
+    uint2 hi, lo;
+    if (j < nb) {      // (entries behind the last column are zero, and rows are padded to groups of eight)
+      oc_split4(make_float4(Y[i][j] * sc, j + 1 < nb ? Y[i][j + 1] * sc : 0.f, j + 2 < nb ? Y[i][j + 2] * sc : 0.f,
+                            j + 3 < nb ? Y[i][j + 3] * sc : 0.f), hi, lo);
+      *reinterpret_cast<uint2*>(to) = hi;
+      *reinterpret_cast<uint2*>(to + plane) = lo;
+    }
+    if (j < width) {
+      *reinterpret_cast<uint2*>(to + NB) = make_uint2(0u, 0u);
+      *reinterpret_cast<uint2*>(to + NB + plane) = make_uint2(0u, 0u);
+    }
   }
 }
 
 }  // namespace
 
-// Workspace layout of one problem (floats): A[n*ld] | X[n*ld] | T[n*ld] | diagv[n] | pad;
-// ld = round_up(n,4).  A batch keeps the problems' workspaces one after another.
-static long long factor_ws_floats(int n) {
-  const long long ld = (n + 3) / 4 * 4;
-  return (3 * (long long)n * ld + ((n + 3) / 4 * 4) + 4 + 63) / 64 * 64;
-}
+// Workspace of one problem (floats, rows ld = round_up(n, 8) apart): A, X, T fp32; the fp16 planes of L and X (two planes
+// take the room of one fp32 matrix); vectors of n; block tables of X and T.  The planes of T take A's place:
+// behind the Cholesky factorisation nothing reads A.  A batch keeps the problems' workspaces one after another.
+struct FactorWs {
+  long long ld, mat, nblk, total;
+  explicit FactorWs(int n) {
+    ld = (n + 7) / 8 * 8; mat = (long long)n * ld; nblk = (n + NB - 1) / NB;
+    total = (5 * mat + 3 * ld + 2 * ((nblk * nblk + 3) / 4 * 4) + 63) / 64 * 64;
+  }
+  float* A(float* w) const { return w; }
+  float* X(float* w) const { return w + mat; }
+  float* T(float* w) const { return w + 2 * mat; }
+  __half* planesL(float* w) const { return reinterpret_cast<__half*>(w + 3 * mat); }
+  __half* planesX(float* w) const { return reinterpret_cast<__half*>(w + 4 * mat); }
+  __half* planesT(float* w) const { return reinterpret_cast<__half*>(w); }
+  float* diagv(float* w) const { return w + 5 * mat; }
+  float* equil(float* w) const { return w + 5 * mat + ld; }
+  float* equil_p(float* w) const { return w + 5 * mat + 2 * ld; }
+  float* tableX(float* w) const { return w + 5 * mat + 3 * ld; }
+  float* tableT(float* w) const { return w + 5 * mat + 3 * ld + (nblk * nblk + 3) / 4 * 4; }
+};
+static long long factor_ws_floats(int n) { return FactorWs(n).total; }
 
 extern "C" long long oc_hinv_workspace_bytes(int n) { return factor_ws_floats(n) * 4; }
+
+// `count` problems of one level of the blocked inverse, for `batch` matrices: T21 = L21 X11, X21 = -X22 T21 with
+// X11, X22 of s and `rows` rows, the first at row and column r0, `step` entries apart.  T and X21 (unless no level
+// follows) are split into planes for the products that read them.
+static int invert_level_split(const FactorWs& ws, float* w0, int s, long long r0, int rows, int count, long long step,
+                              int batch, long long sW, bool more, cudaStream_t stream) {
+  const long long ld = ws.ld, mid = r0 + s, at = mid * ld + r0;
+  const long long nblk = ws.nblk, tab_step = 2 * (s / NB) * (nblk + 1), tab_at = mid / NB * nblk + r0 / NB;
+  auto operand = [&](__half* planes, long long row, long long col, float* table) {
+    OcSplitOperand o{};
+    o.planes = planes + row * ld + col; o.plane = ws.mat; o.ld = ld; o.terms = 2;
+    o.stride1 = step; o.stride2 = 2 * sW;
+    if (table) {
+      o.scale = table + row / NB * nblk + col / NB; o.scale1 = tab_step; o.scale2 = sW;
+      o.scale_k = 1; o.scale_r = nblk;
+    }
+    return o;
+  };
+  auto stored_by_k = [](OcSplitOperand o) {
+    o.mn_major = 1;
+    const long long t = o.scale_k; o.scale_k = o.scale_r; o.scale_r = t;
+    return o;
+  };
+  auto split_block = [&](const float* src, __half* planes, float* table) {
+    OcSplitArgs a{};
+    a.src = src + at; a.ld = ld; a.rows = rows; a.cols = s;
+    a.planes = planes + at; a.plane = ws.mat; a.ldp = ld; a.table = table + tab_at; a.ldt = nblk;
+    a.nb1 = count; a.nb2 = batch;
+    a.src1 = a.dst1 = step; a.src2 = sW; a.dst2 = 2 * sW; a.tab1 = tab_step; a.tab2 = sW;
+    return oc_split_launch(a, stream);
+  };
+  OcSplitGemm g{};
+  g.ldc = ld; g.strideC1 = step; g.strideC2 = sW; g.nb1 = count; g.nb2 = batch; g.M = rows; g.N = s;
+  g.A = operand(ws.planesL(w0), mid, r0, nullptr);
+  g.B = stored_by_k(operand(ws.planesX(w0), r0, r0, ws.tableX(w0)));
+  g.C = ws.T(w0) + at; g.K = s; g.alpha = 1.f / L_SCALE; g.flags = OC_GEMM_KLO_FROM_N;
+  int rc = oc_gemm_split_launch(g, stream);
+  if (rc) return rc;
+  rc = split_block(ws.T(w0), ws.planesT(w0), ws.tableT(w0));
+  if (rc) return rc;
+  g.A = operand(ws.planesX(w0), mid, mid, ws.tableX(w0));
+  g.B = stored_by_k(operand(ws.planesT(w0), mid, r0, ws.tableT(w0)));
+  g.C = ws.X(w0) + at; g.K = rows; g.alpha = -1.f; g.flags = OC_GEMM_KHI_FROM_M;
+  rc = oc_gemm_split_launch(g, stream);
+  if (rc || !more) return rc;
+  return split_block(ws.X(w0), ws.planesX(w0), ws.tableX(w0));
+}
 
 // Factorisation of `batch` matrices of equal size laid out one after another (H [batch, n, ldh],
 // U [batch, n, ldu], perm / invperm / dead [batch, n], damp_out [batch, 2], status [batch]).  The
@@ -679,15 +815,16 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     oc_set_last_error("hinv_factor: workspace too small");
     return OC_ERR_WORKSPACE;
   }
-  const long long ld = (n + 3) / 4 * 4;
+  const FactorWs ws(n);
+  const long long ld = ws.ld;
   const long long sH = (long long)n * ldh, sU = (long long)n * ldu;
-  float* A = (float*)workspace;
-  float* X = A + (long long)n * ld;
-  float* T = X + (long long)n * ld;
-  float* diagv = T + (long long)n * ld;
+  float* w0 = (float*)workspace;
+  float *A = ws.A(w0), *X = ws.X(w0), *T = ws.T(w0);
+  float *diagv = ws.diagv(w0), *equil = ws.equil(w0), *equil_p = ws.equil_p(w0);
+  const bool split = oc_split_engine_on() && n > NB;     // (and then the workspace is aligned)
 
   OC_CUDA(cudaMemsetAsync(status, 0, sizeof(int) * batch, stream));
-  diag_stats_kernel<<<batch, 1024, 0, stream>>>(H, ldh, n, percdamp, diagv, dead, damp_out, sH, sW);
+  diag_stats_kernel<<<batch, 1024, 0, stream>>>(H, ldh, n, percdamp, rel_shift, diagv, dead, damp_out, equil, sH, sW);
   OC_CHECK_LAUNCH();
   const int tb = 256, gb = oc_div_up(n, tb);
   if (!reuse_perm) {
@@ -703,12 +840,31 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
   const bool staged = permuted && n <= BUILD_STAGED_N;
   if (staged) OC_OPT_IN_SMEM(build_reversed_kernel, BUILD_STAGED_N * 4);
   build_reversed_kernel<<<dim3(n, batch), 256, staged ? n * 4 : 0, stream>>>(
-      H, ldh, n, perm, permuted, diagv, damp_out, rel_shift, A, ld, sH, sW, vec_h, staged);
+      H, ldh, n, perm, permuted, diagv, damp_out, rel_shift, equil, equil_p, A, ld, sH, sW, vec_h, staged);
   OC_CHECK_LAUNCH();
 
   // ---- blocked right-looking Cholesky --------------------------------------------------
   OC_OPT_IN_SMEM(diag_inverse_kernel, DINV_SMEM);
-  auto batched = [&](OcGemm& g) { g.batch = batch; g.strideA = sW; g.strideB = sW; g.strideC = sW; };
+  __half* Lp = ws.planesL(w0);
+  // C -= P P^T for the rows of L below `r0`, columns [c0, c0 + k): lower tiles of the N columns from r0 on
+  auto update = [&](int r0, int c0, int k, int M, int N) {
+    if (split) {
+      OcSplitGemm g{};
+      g.A.planes = Lp + (long long)r0 * ld + c0; g.A.plane = ws.mat; g.A.ld = ld; g.A.terms = 2;
+      g.A.stride2 = 2 * sW;
+      g.B = g.A;
+      g.C = A + (long long)r0 * ld + r0; g.ldc = ld; g.strideC2 = sW;
+      g.M = M; g.N = N; g.K = k; g.nb1 = 1; g.nb2 = batch;
+      g.alpha = -1.f / (L_SCALE * L_SCALE); g.add = 1; g.flags = OC_GEMM_SKIP_UPPER_TILES;
+      return oc_gemm_split_launch(g, stream);
+    }
+    OcGemm g{};
+    g.A = A + (long long)r0 * ld + c0; g.lda = ld; g.B = g.A; g.ldb = ld; g.transB = 1;
+    g.C = A + (long long)r0 * ld + r0; g.ldc = ld;
+    g.M = M; g.N = N; g.K = k; g.alpha = -1.f; g.beta = 1.f; g.flags = OC_GEMM_SKIP_UPPER_TILES;
+    g.batch = batch; g.strideA = g.strideB = g.strideC = sW;
+    return oc_gemm_f32_launch(g, stream);
+  };
   // Two levels: inside an outer block of OB columns every 128-column panel updates only the
   // rest of that outer block (full height); the matrix behind the outer block is updated once per
   // outer block with K = OB, so it is read and written n/OB times instead of n/128 times.
@@ -722,95 +878,78 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
       OC_CHECK_LAUNCH();
       const int rest = n - k0 - nb;
       if (rest <= 0) break;
-      float* panel = A + (long long)(k0 + nb) * ld + k0;
       OC_REQUIRE(nb == NB, "hinv_factor: a panel with rows below it is a full panel");
       // the fewer rows per CTA, the shorter its time, as long as all CTAs run at once (one or two on each
       // of a B200's 148 SMs)
       const long long row_sets = (long long)oc_div_up(rest, 32) * batch;
-      const int rc_t = row_sets <= 2 * 148 ? launch_trsm<32>(A, ld, k0, rest, batch, sW, stream)
-                                           : launch_trsm<64>(A, ld, k0, rest, batch, sW, stream);
+      const bool few = row_sets <= 2 * 148;
+      const int rc_t = split ? (few ? launch_trsm<32, true>(A, ld, k0, rest, batch, sW, Lp, ws.mat, stream)
+                                    : launch_trsm<64, true>(A, ld, k0, rest, batch, sW, Lp, ws.mat, stream))
+                             : (few ? launch_trsm<32, false>(A, ld, k0, rest, batch, sW, nullptr, 0, stream)
+                                    : launch_trsm<64, false>(A, ld, k0, rest, batch, sW, nullptr, 0, stream));
       if (rc_t) return rc_t;
       const int inner = kend - (k0 + nb);
       if (inner <= 0) continue;
-      // columns [k0+nb, kend) of all rows below the panel's diagonal block (lower tiles only)
-      OcGemm s{};
-      s.A = panel; s.lda = ld; s.B = panel; s.ldb = ld;
-      s.C = A + (long long)(k0 + nb) * ld + (k0 + nb); s.ldc = ld;
-      s.M = rest; s.N = inner; s.K = nb; s.alpha = -1.f; s.beta = 1.f; s.transA = 0; s.transB = 1;
-      s.flags = OC_GEMM_SKIP_UPPER_TILES;
-      batched(s);
-      int rc = oc_gemm_f32_launch(s, stream);
+      // columns [k0+nb, kend) of all rows below the panel's diagonal block
+      const int rc = update(k0 + nb, k0, nb, rest, inner);
       if (rc) return rc;
     }
     const int rest2 = n - kend;
     if (rest2 <= 0) break;
-    // trailing <- trailing - P * P^T with P = L[kend.., K0..kend)  (lower tiles only)
-    float* P = A + (long long)kend * ld + K0;
-    OcGemm t{};
-    t.A = P; t.lda = ld; t.B = P; t.ldb = ld;
-    t.C = A + (long long)kend * ld + kend; t.ldc = ld;
-    t.M = rest2; t.N = rest2; t.K = kend - K0; t.alpha = -1.f; t.beta = 1.f; t.transA = 0; t.transB = 1;
-    t.flags = OC_GEMM_SKIP_UPPER_TILES;
-    batched(t);
-    const int rc2 = oc_gemm_f32_launch(t, stream);
+    // trailing <- trailing - P * P^T with P = L[kend.., K0..kend)
+    const int rc2 = update(kend, K0, kend - K0, rest2, rest2);
     if (rc2) return rc2;
   }
   // inverses of the diagonal blocks, all at once: the seeds of the blocked inverse below
-  diag_inverse_kernel<<<dim3(oc_div_up(n, NB), batch), DINV_T, DINV_SMEM, stream>>>(A, ld, X, ld, n, sW);
+  diag_inverse_kernel<<<dim3(oc_div_up(n, NB), batch), DINV_T, DINV_SMEM, stream>>>(
+      A, ld, X, ld, n, sW, split ? ws.planesX(w0) : nullptr, ws.mat, ws.tableX(w0), (int)ws.nblk);
   OC_CHECK_LAUNCH();
 
   // ---- recursive blocked inverse of L: X holds the inverted diagonal blocks -----------------
-  // One matrix: the uniform problems of a level form one batched product.  Several matrices: the
-  // batch dimension is taken by the matrices and the problems of a level are launched one by one.
+  // The uniform problems of a level form one batched product (of both batch dimensions: problems and
+  // matrices); a last problem with fewer rows has its own.
   for (long long s = NB; s < n; s *= 2) {
     const int nprob = (int)((n + 2 * s - 1) / (2 * s));
-    int nfull = 0;
-    for (int m = 0; m < nprob; ++m) {
-      const long long mid = 2 * s * m + s, end = 2 * s * m + 2 * s;
-      if (mid < n && end <= n) nfull = m + 1;
-    }
-    // (first problem, count as one launch, rows of the lower block)
+    const int nfull = (int)(n / (2 * s));
+    const long long mid_last = 2 * s * nfull + s;
+    // (first problem, count, rows of the lower block)
     struct Launch { int first, count, rows; };
-    Launch list[2 + 1];
+    Launch list[2];
     int nl = 0;
-    if (batch == 1) {
-      if (nfull > 0) list[nl++] = {0, nfull, (int)s};
-      const long long mid = 2 * s * nfull + s;
-      if (nfull < nprob && mid < n) list[nl++] = {nfull, 1, (int)(n - mid)};
-    }
-    const int total = (batch == 1) ? nl : nprob;
-    for (int li = 0; li < total; ++li) {
-      int first, count, rows;
-      if (batch == 1) { first = list[li].first; count = list[li].count; rows = list[li].rows; }
-      else {
-        first = li; count = 1;
-        const long long mid = 2 * s * first + s;
-        if (mid >= n) continue;
-        rows = (int)min((long long)s, n - mid);
+    if (nfull > 0) list[nl++] = {0, nfull, (int)s};
+    if (nfull < nprob && mid_last < n) list[nl++] = {nfull, 1, (int)(n - mid_last)};
+    for (int li = 0; li < nl; ++li) {
+      const int count = list[li].count, rows = list[li].rows;
+      const long long r0 = 2 * s * list[li].first, mid = r0 + s, step = 2 * s * (ld + 1);
+      if (split) {
+        const int rc = invert_level_split(ws, w0, (int)s, r0, rows, count, step, batch, sW, 2 * s < n, stream);
+        if (rc) return rc;
+        continue;
       }
-      const long long r0 = 2 * s * first, mid = r0 + s;
-      const long long stride = (batch == 1) ? 2 * s * (ld + 1) : sW;
-      const int nb_launch = (batch == 1) ? count : batch;
-      OcGemm g1{};  // T21 = L21 * X11   (X11 lower triangular)
-      g1.A = A + mid * ld + r0; g1.lda = ld; g1.strideA = stride;
-      g1.B = X + r0 * ld + r0; g1.ldb = ld; g1.strideB = stride;
-      g1.C = T + mid * ld + r0; g1.ldc = ld; g1.strideC = stride;
-      g1.M = rows; g1.N = (int)s; g1.K = (int)s; g1.alpha = 1.f; g1.beta = 0.f;
-      g1.flags = OC_GEMM_KLO_FROM_N; g1.batch = nb_launch;
-      int rc = oc_gemm_f32_launch(g1, stream);
-      if (rc) return rc;
-      OcGemm g2{};  // X21 = -X22 * T21  (X22 lower triangular)
-      g2.A = X + mid * ld + mid; g2.lda = ld; g2.strideA = stride;
-      g2.B = T + mid * ld + r0; g2.ldb = ld; g2.strideB = stride;
-      g2.C = X + mid * ld + r0; g2.ldc = ld; g2.strideC = stride;
-      g2.M = rows; g2.N = (int)s; g2.K = rows; g2.alpha = -1.f; g2.beta = 0.f;
-      g2.flags = OC_GEMM_KHI_FROM_M; g2.batch = nb_launch;
-      rc = oc_gemm_f32_launch(g2, stream);
-      if (rc) return rc;
+      // (the FMA engine has one batch dimension: the matrices of a batch one by one)
+      for (int b = 0; b < batch; ++b) {
+        float *Ab = A + b * sW, *Xb = X + b * sW, *Tb = T + b * sW;
+        OcGemm g1{};  // T21 = L21 * X11   (X11 lower triangular)
+        g1.A = Ab + mid * ld + r0; g1.lda = ld; g1.strideA = step;
+        g1.B = Xb + r0 * ld + r0; g1.ldb = ld; g1.strideB = step;
+        g1.C = Tb + mid * ld + r0; g1.ldc = ld; g1.strideC = step;
+        g1.M = rows; g1.N = (int)s; g1.K = (int)s; g1.alpha = 1.f; g1.beta = 0.f;
+        g1.flags = OC_GEMM_KLO_FROM_N; g1.batch = count;
+        int rc = oc_gemm_f32_launch(g1, stream);
+        if (rc) return rc;
+        OcGemm g2{};  // X21 = -X22 * T21  (X22 lower triangular)
+        g2.A = Xb + mid * ld + mid; g2.lda = ld; g2.strideA = step;
+        g2.B = Tb + mid * ld + r0; g2.ldb = ld; g2.strideB = step;
+        g2.C = Xb + mid * ld + r0; g2.ldc = ld; g2.strideC = step;
+        g2.M = rows; g2.N = (int)s; g2.K = rows; g2.alpha = -1.f; g2.beta = 0.f;
+        g2.flags = OC_GEMM_KHI_FROM_M; g2.batch = count;
+        rc = oc_gemm_f32_launch(g2, stream);
+        if (rc) return rc;
+      }
     }
   }
   const bool vec_u = n % 4 == 0 && ldu % 4 == 0 && sU % 4 == 0 && aligned(U) && aligned(X);
-  reverse_upper_kernel<<<dim3(n, batch), 256, 0, stream>>>(X, ld, n, U, ldu, sW, sU, vec_u);
+  reverse_upper_kernel<<<dim3(n, batch), 256, 0, stream>>>(X, ld, n, equil_p, U, ldu, sW, sU, vec_u);
   OC_CHECK_LAUNCH();
   return OC_OK;
 }
