@@ -16,7 +16,7 @@
 // One persistent CTA per SM walks a static list of 128 x 256 output tiles.
 //   warp 0      : TMA producer (4-stage ring, 6 boxes per stage)
 //   warp 1      : TMEM allocation, MMA issue (M=128, N=256, K=16; 4 per stage)
-//   warps 2..9  : drain.  Tokens are consumed in chunks (default 512); each
+//   warps 4..11 : drain.  Tokens are consumed in chunks (default 512); each
 //                 chunk accumulates in one of two 256-column TMEM buffers, and
 //                 the drain warps add finished chunks into fp32 registers with
 //                 round-to-nearest while the next chunk is in flight, so the
@@ -49,7 +49,9 @@ constexpr int ATOM_BYTES = BK * 128;                     // one 64-column x BK-t
 constexpr int A_ATOMS = TILE_M / 64, B_ATOMS = TILE_N / 64;
 constexpr int STAGE_BYTES = (A_ATOMS + B_ATOMS) * ATOM_BYTES;
 constexpr int SMEM_DYN = STAGES * STAGE_BYTES + 1024 + 8 * 4096;   // ring, its alignment, 4 KB per drain warp
-constexpr int NUM_THREADS = 320;
+// Three warpgroups: TMA, MMA and two idle warps; eight drain warps, each thread with 128 sums.  They trade registers
+// (setmaxnreg): ten warps of one size had 168 registers a thread, and the sums spilled.
+constexpr int FIRST_DRAIN = 4, NUM_THREADS = 32 * (FIRST_DRAIN + 8);
 constexpr uint32_t IDESC = (1u << 4) | (1u << 15) | (1u << 16) | ((TILE_N >> 3) << 17) | ((TILE_M >> 4) << 24);
 
 struct MomentParams {
@@ -144,6 +146,8 @@ moment_tc_kernel(const __grid_constant__ CUtensorMap map_xq, const __grid_consta
   const int total_stages = (int)((p.n_tok + BK - 1) / BK);
   const int n_chunks = (total_stages + p.chunk_stages - 1) / p.chunk_stages;
 
+  if (warp < FIRST_DRAIN) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
   if (warp == 0) {
     if (lane == 0) {
       uint32_t stage = 0, phase = 1;
@@ -216,9 +220,11 @@ moment_tc_kernel(const __grid_constant__ CUtensorMap map_xq, const __grid_consta
       }
     }
     __syncwarp();
+  }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
     // drain warps: TMEM lane quarter = warp % 4; columns [half*128, half*128+128)
-    const int e = warp - 2;
+    const int e = warp - FIRST_DRAIN;
     const int quarter = warp & 3;
     const int half = e >> 2;
     float4* stg = reinterpret_cast<float4*>(smem_raw + (stage_base - smem_u32(smem_raw)) + STAGES * STAGE_BYTES) + e * 256;
@@ -257,7 +263,7 @@ moment_tc_kernel(const __grid_constant__ CUtensorMap map_xq, const __grid_consta
       // Whole row segments instead of 16 bytes of 32 rows an instruction, old values on their way from HBM
       // meanwhile: H and C at d = 5120, two chunks of 4096 tokens, 1004 -> 897 us.
       // (d is a multiple of 8 and rows are 16-byte aligned: four columns are inside or outside as a whole)
-      store_tile<128, 1>(out, p.ldh, p.d, p.d, p.a_new, p.a_old, acc, stg, m0 + quarter * 32, n0 + half * 128, lane);
+      store_tile<128, 3>(out, p.ldh, p.d, p.d, p.a_new, p.a_old, acc, stg, m0 + quarter * 32, n0 + half * 128, lane);
     }
   }
 
