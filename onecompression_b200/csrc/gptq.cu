@@ -13,10 +13,12 @@
 //                       memory and named barriers
 //   gptq_block_kernel   everything else: one thread owns one row, whose block lives in shared memory;
 //                       in CTAs with few rows the other threads apply the updates behind the window
-// The lazy-batch trailing update W[:, i2:] -= Err * U[i1:i2, i2:] is a launch of the fp32 GEMM engine
-// with the error block stored transposed (coalesced stores here, coalesced loads there).  Codes are kept
+// The lazy-batch trailing update W[:, i2:] -= Err * U[i1:i2, i2:] is a tensor-core product of operands in two fp16
+// planes each (split.cuh): U is split once per call, the column kernels leave the errors of a block of 128
+// columns split, transposed, every row under a scale of its own.  Other block sizes, unaligned workspaces and the FMA
+// engine take fp32 errors and oc_gemm_f32_launch.  Codes are kept
 // transposed ([column][row], 16 bit) until a final pass packs them in original column order.
-#include "common.cuh"
+#include "split.cuh"
 #include <type_traits>
 
 namespace {
@@ -30,15 +32,32 @@ struct ColArgs {
   const float* Wf; long long ldw;
   int out, d, i1, count;
   const float* U; long long ldu;
-  float* ErrT; long long lde;
+  float* ErrT; long long lde;   // errors [column][row], fp32; not used when they leave as planes
+  __half* errp; long long err_plane; float* err_scale;   // planes [column][row] and 2^-e per row; null: fp32
   unsigned short* codesT;
   float* scales; float* zeros;  // [G][out] fp32 (G = 1 for per-channel)
   int gs, maxq, sym;
   int mse_steps; float mse_grid, mse_norm;   // mse_steps = 0: plain min/max fit
   // batched problems (blockIdx.y): element strides between consecutive problems, 0 for one problem
   long long sW, sU, sE, sC, sS;
+  long long sEp, sEs;
   int batch;
 };
+
+// columns c .. c + 3 of a row's errors to their planes
+__device__ __forceinline__ void store_halves(__half* to, long long lde, long long plane, uint2 hi, uint2 lo) {
+  const unsigned h[2] = {hi.x, hi.y}, l[2] = {lo.x, lo.y};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    to[j * lde] = __ushort_as_half((unsigned short)(h[j >> 1] >> (16 * (j & 1))));
+    to[plane + j * lde] = __ushort_as_half((unsigned short)(l[j >> 1] >> (16 * (j & 1))));
+  }
+}
+__device__ __forceinline__ void store_split4(__half* to, long long lde, long long plane, float4 v, float s) {
+  uint2 hi, lo;
+  oc_split4(make_float4(v.x * s, v.y * s, v.z * s, v.w * s), hi, lo);
+  store_halves(to, lde, plane, hi, lo);
+}
 
 // scale / zero over the values v[0..n), reference: GPTQExcecutor.find_params
 // (onecomp/quantizer/gptq/_gptq.py:886-972, perchannel=True, mse=False)
@@ -170,7 +189,7 @@ template <int NROWS>
 __device__ __forceinline__ bool fast_window(const float* __restrict__ wcols, const float* __restrict__ ublk,
                                             const float* __restrict__ rdiag, float scale, float zero, float maxqf,
                                             unsigned short* code_out, long long ldc, float* err_out, long long lde,
-                                            float (&er)[SUB]) {
+                                            bool fp32_errors, float (&er)[SUB]) {
   constexpr float RINT = 12582912.f;   // 1.5 * 2^23
   float w[SUB];
 #pragma unroll
@@ -197,7 +216,7 @@ __device__ __forceinline__ bool fast_window(const float* __restrict__ wcols, con
     bad |= !(fabsf(r) < SAFE_HI) || !(fabsf(e) < 0x1p120f);
     er[i] = e;
     code_out[i * ldc] = (unsigned short)__fadd_rn(level, zero);
-    err_out[i * lde] = e;
+    if (fp32_errors) err_out[i * lde] = e;
     propagate(w, i, e, ublk + i * BLK);
   }
   return !bad;
@@ -222,6 +241,7 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
     const long long b = blockIdx.y;      // problem of a batch
     a.Wf += b * a.sW; a.U += b * a.sU; a.ErrT += b * a.sE; a.codesT += b * a.sC;
     a.scales += b * a.sS; a.zeros += b * a.sS;
+    if (a.errp) { a.errp += b * a.sEp; a.err_scale += b * a.sEs; }
   }
 
   // whole block, 16-byte aligned rows: vector loads (the part of U below the diagonal is never used)
@@ -303,7 +323,7 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
         if (!exact)
           exact = !fast_window<NROWS>(wrow + cb, Us + cb * BLK + cb, rdiag + cb, scale, zero, maxqf,
                                       code_out + (long long)cb * a.out, a.out, err_out + (long long)cb * a.lde,
-                                      a.lde, er);
+                                      a.lde, a.errp == nullptr, er);
       }
       if (exact) {
         float w[SUB];
@@ -325,10 +345,16 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
             const float e = __fdiv_rn(__fsub_rn(x, dq), Us[ci * BLK + ci]);
             er[i] = e;
             code_out[(long long)ci * a.out] = (unsigned short)q;
-            err_out[(long long)ci * a.lde] = e;
+            if (!a.errp) err_out[(long long)ci * a.lde] = e;
             propagate(w, i, e, Us + ci * BLK + cb);
           }
         }
+      }
+      if (a.errp) {
+        // the columns of the tile that are done with hold their errors
+#pragma unroll
+        for (int v = 0; v < SUB / 4; ++v)
+          *reinterpret_cast<float4*>(wrow + cb + 4 * v) = make_float4(er[4 * v], er[4 * v + 1], er[4 * v + 2], er[4 * v + 3]);
       }
       if (helped) {
 #pragma unroll
@@ -383,6 +409,20 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
         }
       }
     }
+  }
+  if (a.errp && owner) {        // a full block
+    float mx = 0.f;
+#pragma unroll 4
+    for (int c = 0; c < BLK; c += 4) {
+      const float4 v = *reinterpret_cast<const float4*>(wrow + c);
+      mx = fmaxf(mx, fmaxf(fmaxf(oc_finite_abs(v.x), oc_finite_abs(v.y)), fmaxf(oc_finite_abs(v.z), oc_finite_abs(v.w))));
+    }
+    float inv;
+    const float s = oc_split_scale(mx, inv);
+    a.err_scale[row] = inv;
+#pragma unroll 4
+    for (int c = 0; c < BLK; c += 4)
+      store_split4(a.errp + (long long)c * a.lde + row, a.lde, a.err_plane, *reinterpret_cast<const float4*>(wrow + c), s);
   }
 }
 
@@ -450,6 +490,65 @@ __device__ __forceinline__ bool produce_chunk(float (&w)[SUB], const float* __re
   return !bad;
 }
 
+// The chain over the columns of a block, from the view of warp `wid`: w becomes the block-entry window with the updates
+// of the earlier windows, then er and cd the errors and codes of the warp's own.
+__device__ __forceinline__ void window_chain(int wid, int lane, float (&w)[SUB], const float* __restrict__ Us,
+                                             const float* __restrict__ rdiag, float* Es, float scale, float zero,
+                                             float maxqf, float (&er)[SUB], float (&cd)[SUB]) {
+  const float rs = safe_reciprocal(scale);
+  const float lo = __fsub_rn(0.f, zero), hi = __fsub_rn(maxqf, zero);
+
+  // the windows before this warp's own: their errors, as they are published.  Named barriers 1 .. 4 stand for
+  // the four chunks of a window (its producer arrives, the warps of later windows wait), barrier 5 for
+  // the end of a window, behind which the next one may publish.
+#pragma unroll 1
+  for (int pw = 0; pw < wid; ++pw) {
+    const int threads = 32 * (NWIN - pw);
+#pragma unroll 1
+    for (int q = 0; q < SUB / CHUNK; ++q) {
+      asm volatile("bar.sync %0, %1;" ::"r"(q + 1), "r"(threads) : "memory");
+      const float* es = Es + q * CHUNK * 32 + lane;
+      const float* ur = Us + (pw * SUB + q * CHUNK) * BLK + wid * SUB;
+#pragma unroll
+      for (int c = 0; c < CHUNK; ++c) {
+        const float e = es[c * 32];
+#pragma unroll
+        for (int v = 0; v < SUB / 4; ++v) {
+          const float4 u = *reinterpret_cast<const float4*>(ur + c * BLK + 4 * v);
+          w[4 * v] = __fsub_rn(w[4 * v], __fmul_rn(e, u.x));
+          w[4 * v + 1] = __fsub_rn(w[4 * v + 1], __fmul_rn(e, u.y));
+          w[4 * v + 2] = __fsub_rn(w[4 * v + 2], __fmul_rn(e, u.z));
+          w[4 * v + 3] = __fsub_rn(w[4 * v + 3], __fmul_rn(e, u.w));
+        }
+      }
+    }
+    asm volatile("bar.sync 5, %0;" ::"r"(threads - 32) : "memory");
+  }
+
+  // this warp's own window
+  const float* ublk = Us + wid * SUB * BLK + wid * SUB;
+  auto step = [&](auto q_const) {
+    constexpr int Q = decltype(q_const)::value;
+    float* es = Es + Q * CHUNK * 32 + lane;
+    float entry[SUB];
+#pragma unroll
+    for (int m = Q * CHUNK; m < SUB; ++m) entry[m] = w[m];
+    if (!produce_chunk<Q, false>(w, ublk, rdiag, scale, rs, lo, hi, zero, maxqf, es, er, cd)) {
+#pragma unroll
+      for (int m = Q * CHUNK; m < SUB; ++m) w[m] = entry[m];
+      produce_chunk<Q, true>(w, ublk, rdiag, scale, rs, lo, hi, zero, maxqf, es, er, cd);
+    }
+    if (wid < NWIN - 1) {
+      __syncwarp();
+      asm volatile("bar.arrive %0, %1;" ::"r"(Q + 1), "r"(32 * (NWIN - wid)) : "memory");
+    }
+  };
+  step(std::integral_constant<int, 0>{});
+  step(std::integral_constant<int, 1>{});
+  step(std::integral_constant<int, 2>{});
+  step(std::integral_constant<int, 3>{});
+}
+
 __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
   extern __shared__ __align__(16) float sm[];
   float* Us = sm;                                // [BLK][BLK], upper triangle of the diagonal block of U
@@ -463,6 +562,7 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
     const long long b = blockIdx.y;      // problem of a batch
     a.Wf += b * a.sW; a.U += b * a.sU; a.ErrT += b * a.sE; a.codesT += b * a.sC;
     a.scales += b * a.sS; a.zeros += b * a.sS;
+    if (a.errp) { a.errp += b * a.sEp; a.err_scale += b * a.sEs; }
   }
   // everything that comes from global memory is requested before anything is waited for
 #pragma unroll
@@ -532,67 +632,35 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
       zero = pz[(opened - i1) / SUB * 32 + lane];
     }
   }
-  const float rs = safe_reciprocal(scale), maxqf = (float)a.maxq;
-  const float lo = __fsub_rn(0.f, zero), hi = __fsub_rn(maxqf, zero);
-
-  // the windows before this warp's own: their errors, as they are published.  Named barriers 1 .. 4 stand for
-  // the four chunks of a window (its producer arrives, the warps of later windows wait), barrier 5 for
-  // the end of a window, behind which the next one may publish.
-#pragma unroll 1
-  for (int pw = 0; pw < wid; ++pw) {
-    const int threads = 32 * (NWIN - pw);
-#pragma unroll 1
-    for (int q = 0; q < SUB / CHUNK; ++q) {
-      asm volatile("bar.sync %0, %1;" ::"r"(q + 1), "r"(threads) : "memory");
-      const float* es = Es + q * CHUNK * 32 + lane;
-      const float* ur = Us + (pw * SUB + q * CHUNK) * BLK + wid * SUB;
-#pragma unroll
-      for (int c = 0; c < CHUNK; ++c) {
-        const float e = es[c * 32];
-#pragma unroll
-        for (int v = 0; v < SUB / 4; ++v) {
-          const float4 u = *reinterpret_cast<const float4*>(ur + c * BLK + 4 * v);
-          w[4 * v] = __fsub_rn(w[4 * v], __fmul_rn(e, u.x));
-          w[4 * v + 1] = __fsub_rn(w[4 * v + 1], __fmul_rn(e, u.y));
-          w[4 * v + 2] = __fsub_rn(w[4 * v + 2], __fmul_rn(e, u.z));
-          w[4 * v + 3] = __fsub_rn(w[4 * v + 3], __fmul_rn(e, u.w));
-        }
-      }
-    }
-    asm volatile("bar.sync 5, %0;" ::"r"(threads - 32) : "memory");
-  }
-
-  // this warp's own window
-  const float* ublk = Us + wid * SUB * BLK + wid * SUB;
   float er[SUB], cd[SUB];
-  auto step = [&](auto q_const) {
-    constexpr int Q = decltype(q_const)::value;
-    float* es = Es + Q * CHUNK * 32 + lane;
-    float entry[SUB];
+  window_chain(wid, lane, w, Us, rdiag + wid * SUB, Es, scale, zero, (float)a.maxq, er, cd);
+  if (live) {
+    unsigned short* code_out = a.codesT + (long long)col0 * a.out + row;
 #pragma unroll
-    for (int m = Q * CHUNK; m < SUB; ++m) entry[m] = w[m];
-    if (!produce_chunk<Q, false>(w, ublk, rdiag + wid * SUB, scale, rs, lo, hi, zero, maxqf, es, er, cd)) {
+    for (int i = 0; i < SUB; ++i) code_out[(long long)i * a.out] = (unsigned short)cd[i];
+    if (!a.errp) {
+      float* err_out = a.ErrT + (long long)(wid * SUB) * a.lde + row;
 #pragma unroll
-      for (int m = Q * CHUNK; m < SUB; ++m) w[m] = entry[m];
-      produce_chunk<Q, true>(w, ublk, rdiag + wid * SUB, scale, rs, lo, hi, zero, maxqf, es, er, cd);
+      for (int i = 0; i < SUB; ++i) err_out[(long long)i * a.lde] = er[i];
     }
-    if (wid < NWIN - 1) {
-      __syncwarp();
-      asm volatile("bar.arrive %0, %1;" ::"r"(Q + 1), "r"(32 * (NWIN - wid)) : "memory");
-    }
-  };
-  step(std::integral_constant<int, 0>{});
-  step(std::integral_constant<int, 1>{});
-  step(std::integral_constant<int, 2>{});
-  step(std::integral_constant<int, 3>{});
-  if (!live) return;
-  unsigned short* code_out = a.codesT + (long long)col0 * a.out + row;
-  float* err_out = a.ErrT + (long long)(wid * SUB) * a.lde + row;
-#pragma unroll
-  for (int i = 0; i < SUB; ++i) {
-    code_out[(long long)i * a.out] = (unsigned short)cd[i];
-    err_out[(long long)i * a.lde] = er[i];
   }
+  if (!a.errp) return;
+  // the errors of a row leave under one scale, which is known when the last window is done
+  float mxe = 0.f;
+#pragma unroll
+  for (int i = 0; i < SUB; ++i) mxe = fmaxf(mxe, oc_finite_abs(er[i]));
+  mm_hi[wid * 32 + lane] = mxe;      // (its ranges were read before the chain)
+  __syncthreads();
+#pragma unroll
+  for (int v = 0; v < NWIN; ++v) mxe = fmaxf(mxe, mm_hi[v * 32 + lane]);
+  float inv;
+  const float se = oc_split_scale(mxe, inv);
+  if (!live) return;
+  if (wid == 0) a.err_scale[row] = inv;
+#pragma unroll
+  for (int i = 0; i < SUB; i += 4)
+    store_split4(a.errp + (long long)(wid * SUB + i) * a.lde + row, a.lde, a.err_plane,
+                 make_float4(er[i], er[i + 1], er[i + 2], er[i + 3]), se);
 }
 
 int launch_windows(const ColArgs& a, cudaStream_t stream) {
@@ -954,6 +1022,8 @@ int launch_block(const ColArgs& a, cudaStream_t stream) {
 }
 
 long long round4(long long x) { return (x + 3) / 4 * 4; }
+long long round8(long long x) { return (x + 7) / 8 * 8; }
+long long u_blocks(int d) { return (d + OC_SPLIT_BLOCK - 1) / OC_SPLIT_BLOCK; }
 
 constexpr int PREPARE_STAGED_D = 49152;   // widest row that the act-order gather keeps in shared memory
 
@@ -963,7 +1033,10 @@ extern "C" long long oc_gptq_workspace_bytes(int out, int d, int groupsize) {
   const long long G = (groupsize == -1) ? 1 : (d + groupsize - 1) / groupsize;
   long long b = 0;
   b += (long long)out * round4(d) * 4;       // Wf
-  b += (long long)SUPER * BLK * round4(out) * 4;  // ErrT
+  b += (long long)SUPER * BLK * round8(out) * 4;  // errors, fp32 or as two planes
+  b += SUPER * round8(out) * 4;              // their scales
+  b += 4 * (long long)d * round8(d);         // planes of U
+  b += round4(u_blocks(d) * u_blocks(d)) * 4;     // their scales
   b += round4((long long)d * out * 2);       // codesT
   b += 2 * G * (long long)out * 4;           // scales, zeros fp32
   return b + 256;
@@ -1004,13 +1077,16 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   }
   if (ld_out < out) ld_out = out;
   const int G = (groupsize == -1) ? 1 : (d + groupsize - 1) / groupsize;
-  const long long ldw = round4(d), lde = round4(out);
+  const long long ldw = round4(d), lde = round8(out), ldu_p = round8(d);
   // workspace: all problems' Wf, then all ErrT, codesT, scales, zeros (each contiguous over the batch)
   const long long nWf = (long long)out * ldw, nErr = (long long)SUPER * BLK * lde;
   const long long nCodes = round4((long long)d * out * 2) / 2, nPar = (long long)G * out;
   char* ws = (char*)workspace;
   float* Wf = (float*)ws;                       ws += nWf * 4 * batch;
   float* ErrT = (float*)ws;                     ws += nErr * 4 * batch;
+  float* err_scale = (float*)ws;                ws += SUPER * lde * 4 * batch;
+  __half* Up = (__half*)ws;                     ws += 2 * d * ldu_p * 2 * batch;
+  float* u_table = (float*)ws;                  ws += round4(u_blocks(d) * u_blocks(d)) * 4 * batch;
   unsigned short* codesT = (unsigned short*)ws; ws += nCodes * 2 * batch;
   float* scales = (float*)ws;                   ws += nPar * 4 * batch;
   float* zeros = (float*)ws;
@@ -1039,38 +1115,74 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   // the same updates, grouped differently in the fp32 sum.
   // A group's parameters are fitted on columns that must carry every earlier update, so the
   // far update may only be postponed when no group reaches across the end of a block group.
+  // Full blocks of 128 columns with something behind them leave their errors split.
+  const bool split = oc_split_engine_on() && blocksize == BLK && d > BLK && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
+  const long long nb_u = u_blocks(d), nTab = round4(nb_u * nb_u), nErrP = SUPER * BLK * lde;
+  if (split) {
+    OcSplitArgs us{};
+    us.src = U; us.ld = ldu; us.rows = us.cols = d; us.planes = Up; us.plane = d * ldu_p; us.ldp = ldu_p;
+    us.table = u_table; us.ldt = nb_u; us.region = OC_SPLIT_UPPER;
+    us.nb1 = batch; us.nb2 = 1; us.src1 = sU; us.dst1 = 2 * us.plane; us.tab1 = nTab;
+    const int rc = oc_split_launch(us, stream);
+    if (rc) return rc;
+  }
   const bool two_level = (groupsize == -1) || ((SUPER * blocksize) % groupsize == 0);
   const int super_cols = (two_level ? SUPER : 1) * blocksize;
-  for (int i1 = 0; i1 < d; i1 += blocksize) {
-    const int count = min(blocksize, d - i1);
+  OcSplitOperand u_op{};
+  u_op.planes = Up; u_op.plane = d * ldu_p; u_op.ld = ldu_p; u_op.mn_major = 1; u_op.terms = 2; u_op.stride1 = 2 * d * ldu_p;
+  u_op.scale = u_table; u_op.scale_k = nb_u; u_op.scale_r = 1; u_op.scale1 = nTab;
+  auto col_args = [&](int i1, int count, float* err_rows, __half* err_planes, float* err_sc) {
+    return ColArgs{Wf, ldw, out, d, i1, count, U, ldu, err_rows, lde, err_planes, nErrP, err_sc, codesT, scales, zeros,
+                   groupsize, maxq, sym, mse_steps, (float)q_grid, q_norm, nWf, sU, nErr, nCodes, nPar, 2 * nErrP,
+                   SUPER * lde, batch};
+  };
+  // W[:, n0 .. n1) -= Err U[k0 .. k0 + k, n0 .. n1), Err the planes of the group that starts at column s0
+  auto split_update = [&](int s0, int k0, int k, int n0, int n1) {
+    OcSplitGemm g{};
+    g.A.planes = (__half*)ErrT + (long long)(k0 - s0) * lde; g.A.plane = nErrP; g.A.ld = lde; g.A.mn_major = 1;
+    g.A.terms = 2; g.A.stride1 = 2 * nErrP;
+    g.A.scale = err_scale + (k0 - s0) / BLK * lde; g.A.scale_k = lde; g.A.scale_r = BLK; g.A.scale_row = 1;
+    g.A.scale1 = SUPER * lde;
+    g.B = u_op;
+    g.B.planes += (long long)k0 * ldu_p + n0; g.B.scale += k0 / BLK * nb_u + n0 / BLK;
+    g.C = Wf + n0; g.ldc = ldw; g.strideC1 = nWf;
+    g.M = out; g.N = n1 - n0; g.K = k; g.nb1 = batch; g.nb2 = 1; g.alpha = -1.f; g.add = 1;
+    return oc_gemm_split_launch(g, stream);
+  };
+  for (int i1 = 0, i2; i1 < d; i1 = i2) {
     const int s0 = (i1 / super_cols) * super_cols;          // first column of the group
     const int s1 = min(d, s0 + super_cols);                 // one past its last column
-    float* err_rows = ErrT + (long long)(i1 - s0) * lde;
-    ColArgs a{Wf, ldw, out, d, i1, count, U, ldu, err_rows, lde, codesT, scales, zeros, groupsize, maxq, sym,
-              mse_steps, (float)q_grid, q_norm, nWf, sU, nErr, nCodes, nPar, batch};
     int rc;
+    const int count = min(blocksize, d - i1);
+    i2 = i1 + count;
+    float* err_rows = ErrT + (long long)(i1 - s0) * lde;
+    const ColArgs a = col_args(i1, count, err_rows, split && i2 < d ? (__half*)ErrT + (long long)(i1 - s0) * lde : nullptr,
+                               err_scale + (i1 - s0) / BLK * lde);
     if (per_sm <= 2 && windows_fit(a)) rc = launch_windows(a, stream);
     else if (per_sm <= 1) rc = launch_block<1>(a, stream);
     else if (per_sm <= 2) rc = launch_block<2>(a, stream);
     else if (per_sm <= 4) rc = launch_block<4>(a, stream);
     else rc = launch_block<8>(a, stream);
     if (rc) return rc;
-    const int i2 = i1 + count;
-    OcGemm g{};
-    g.lda = lde; g.transA = 1; g.ldb = ldu; g.transB = 0; g.ldc = ldw;
-    g.M = out; g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
-    g.batch = batch; g.strideA = nErr; g.strideB = sU; g.strideC = nWf;
-    if (i2 < s1) {
-      g.A = err_rows; g.K = count;
-      g.B = U + (long long)i1 * ldu + i2; g.C = Wf + i2; g.N = s1 - i2;
+    if (i2 >= d) break;
+    // near: the rest of the group, behind this block; far: everything behind the group, at its end
+    const bool near = i2 < s1;
+    if (split) rc = near ? split_update(s0, i1, count, i2, s1) : split_update(s0, s0, s1 - s0, s1, d);
+    else {
+      OcGemm g{};
+      g.lda = lde; g.transA = 1; g.ldb = ldu; g.transB = 0; g.ldc = ldw;
+      g.M = out; g.alpha = -1.f; g.beta = 1.f; g.flags = 0;
+      g.batch = batch; g.strideA = nErr; g.strideB = sU; g.strideC = nWf;
+      if (near) {
+        g.A = err_rows; g.K = count;
+        g.B = U + (long long)i1 * ldu + i2; g.C = Wf + i2; g.N = s1 - i2;
+      } else {
+        g.A = ErrT; g.K = s1 - s0;
+        g.B = U + (long long)s0 * ldu + s1; g.C = Wf + s1; g.N = d - s1;
+      }
       rc = oc_gemm_f32_launch(g, stream);
-      if (rc) return rc;
-    } else if (i2 < d) {
-      g.A = ErrT; g.K = s1 - s0;
-      g.B = U + (long long)s0 * ldu + s1; g.C = Wf + s1; g.N = d - s1;
-      rc = oc_gemm_f32_launch(g, stream);
-      if (rc) return rc;
     }
+    if (rc) return rc;
   }
 
   const int tb = 128;

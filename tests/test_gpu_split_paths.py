@@ -1,0 +1,117 @@
+"""The callers of the split products where their shapes can go wrong: partial blocks and panels, one or two blocks,
+16-bit types, act-order, rows and diagonals of very different size."""
+
+import pytest
+import torch
+
+from onecompression_b200 import kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+def gen(seed):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def moment(n, seed, tokens=4):
+    x = torch.randn(tokens * n, n, generator=gen(seed), device="cuda")
+    return x.t() @ x / (tokens * n)
+
+
+def factor64(h, percdamp, perm):
+    a = h.double()[perm][:, perm]
+    diag = torch.diagonal(a)
+    diag += percdamp * diag.mean()
+    return torch.linalg.cholesky(torch.cholesky_inverse(torch.linalg.cholesky(a)), upper=True)
+
+
+def as_factor(u, h, perm=None):
+    n = u.shape[0]
+    iota = torch.arange(n, device="cuda")
+    p = iota if perm is None else perm
+    mean = torch.diagonal(h).mean()
+    return K.HessianFactor(u.float().contiguous(), p.int(), torch.argsort(p).int(),
+                           torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.stack([0.01 * mean, mean]).float(),
+                           perm is not None, 0.01, 1.0, 1)
+
+
+@pytest.mark.parametrize("act", [False, True])
+@pytest.mark.parametrize("n", [128, 129, 255, 256, 257, 384, 513, 777, 1027])
+def test_factor(n, act):
+    """Bound: n * 2^-24 * cond; the moments of 4 n tokens have a condition of 9."""
+    h = moment(n, n)
+    f = K.factor_hessian(h, 0.01, act)
+    u = factor64(h, 0.01, f.perm.long())
+    assert (f.u.double() - u).norm() <= n * 2.0**-24 * 9 * u.norm()
+    assert torch.equal(f.u, f.u.triu())
+    hs = torch.stack([h, moment(n, n + 5000), h])
+    out = K.factor_hessians_batched(hs, 0.01, act)
+    assert torch.equal(out["u"][0], f.u) and torch.equal(out["u"][2], f.u) and not out["status"].any()
+
+
+@pytest.mark.parametrize("n", [300, 640])
+def test_factor_of_a_badly_scaled_matrix(n):
+    """H = D S D, D over 2^-20 .. 2^20: U D is the factor of S, to the accuracy of S alone."""
+    s = moment(n, 1)
+    d = torch.exp2(torch.randint(-20, 21, (n,), generator=gen(2), device="cuda").float())
+    f = K.factor_hessian(s * d[:, None] * d[None, :], 0.0, False)
+    u = factor64(s, 0.0, torch.arange(n, device="cuda"))
+    assert (f.u.double() * d.double() - u).norm() <= n * 2.0**-24 * 9 * u.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("act", [False, True])
+@pytest.mark.parametrize("out,d", [(1, 128), (5, 129), (40, 96), (128, 256), (130, 390), (300, 257)])
+def test_correction(out, d, act, dtype):
+    """Within one unit of the weight's type of the float64 result (the rounding to it, where fp32 sums meet a tie),
+    and a row does not depend on the others."""
+    h = moment(d, 3)
+    perm = torch.argsort(torch.diagonal(h), descending=True, stable=True) if act else None
+    u = factor64(h, 0.01, perm if act else torch.arange(d, device="cuda"))
+    f = as_factor(u, h, perm)
+    f.dead[d // 3] = 1
+    w = torch.randn(out, d, generator=gen(4), device="cuda") * 0.02
+    w[0] *= 2.0**-6
+    w = w.to(dtype)
+    c = 0.02 * h + 0.01 * torch.randn(d, d, generator=gen(5), device="cuda") / d**0.5
+    got = K.qep_adjust(w.clone(), c, f, 0.5)
+    w64 = w.double()
+    w64[:, d // 3] = 0
+    p = f.perm.long()
+    u64 = f.u.double()
+    delta = torch.empty_like(w64)
+    delta[:, p] = ((w64 @ c.double())[:, p] @ u64.t()) @ u64
+    want = w64 + 0.5 * delta
+    # (fp16 values below 2^-14 are 2^-24 apart)
+    ulp = want.abs() * 2.0**-10 + 2.0**-24 if dtype == torch.float16 else want.abs() * 2.0**-7
+    ulp = ulp + w64.norm(dim=1, keepdim=True) * 2.0**-24
+    assert ((got.double() - want).abs() <= ulp).all()
+    for r in {0, out // 2, out - 1}:
+        assert torch.equal(K.qep_adjust(w[r:r + 1].clone(), c, f, 0.5)[0], got[r])
+
+
+@pytest.mark.parametrize("act", [False, True])
+@pytest.mark.parametrize("out,d,gs", [(1, 256, 128), (40, 160, 32), (33, 640, 128), (260, 1184, -1), (9600, 288, 32),
+                                      (2000, 544, 96)])
+def test_column_loop(out, d, gs, act):
+    """Against the FMA engine on the same factor: sums in another order move a code where a weight lies next to the
+    middle between two, and what follows in its row (one row in fifty here at most)."""
+    h = moment(d, 6)
+    perm = torch.argsort(torch.diagonal(h), descending=True, stable=True) if act else None
+    f = as_factor(factor64(h, 0.01, perm if act else torch.arange(d, device="cuda")), h, perm)
+    w = (torch.randn(out, d, generator=gen(7), device="cuda") * 0.02)
+    w[out // 2] *= 2.0**-10
+    w = w.half()
+    new = K.gptq_quantize(w, f, 4, gs, False, pack=False, want_codes=True)
+    old_mode = K.set_gemm_engine(1)
+    try:
+        old = K.gptq_quantize(w, f, 4, gs, False, pack=False, want_codes=True)
+    finally:
+        K.set_gemm_engine(old_mode)
+    moved = (new["codes"] != old["codes"]).any(dim=1)
+    assert moved.sum() <= 1 + out // 50
+    assert torch.equal(new["dequantized"][~moved], old["dequantized"][~moved])
+    r = out // 2
+    alone = K.gptq_quantize(w[r:r + 1].contiguous(), f, 4, gs, False, pack=False, want_codes=True)
+    assert torch.equal(alone["codes"][0], new["codes"][r])
+    assert K.gemm_tc_status() == 0
