@@ -7,7 +7,9 @@
 // uses the _rn intrinsics besides).
 //
 // Rows of W are independent given U.  A block of up to 128 columns is worked off 16 columns (a
-// window) at a time in registers, by one of two kernels with the same bits:
+// window) at a time in registers, by one of three kernels with the same bits:
+//   gptq_group_kernel   up to four full blocks in one launch, one set of 32 rows per SM at most: the windows of
+//                       gptq_window_kernel, and the updates from block to block on the tensor core meanwhile
 //   gptq_window_kernel  full blocks with up to two sets of 32 rows per SM: eight warps share 32 rows, one
 //                       warp per window; the errors of a window go to the later warps through shared
 //                       memory and named barriers
@@ -18,7 +20,7 @@
 // columns split, transposed, every row under a scale of its own.  Other block sizes, unaligned workspaces and the FMA
 // engine take fp32 errors and oc_gemm_f32_launch.  Codes are kept
 // transposed ([column][row], 16 bit) until a final pass packs them in original column order.
-#include "split.cuh"
+#include "split_tc.cuh"
 #include <type_traits>
 
 namespace {
@@ -678,6 +680,279 @@ bool windows_fit(const ColArgs& a) {
          aligned(a.U) && aligned(a.Wf) && (a.batch == 1 || (a.sU % 4 == 0 && a.sW % 4 == 0));
 }
 
+// ---- up to four full blocks in one launch ---------------------------------------------------------
+// The blocks of one group of the lazy-batch update, 32 rows per CTA.  Between two blocks of gptq_window_kernel lie a
+// launch of the product that updates the rest of the group and the start of the next kernel, 24 us a block at 4096 rows,
+// of which the chain over the columns takes 11.  Here the update of the next 128 columns is 24 MMAs whose
+// operand from U has been waiting in shared memory since the chain began, and those of the columns behind run
+// while the next block's chain does.
+//
+// D^T = U^T Err^T: M = 128 columns of W, N = the CTA's 32 rows, K = the 128 columns just quantized, accumulated as in
+// gemm_split_kernel (same terms, order and chains: same bits), one accumulator of 32 TMEM columns for every pair
+// of source and target block.  A target block reads its columns of W once, subtracts the accumulators of its
+// sources in order and passes the result through shared memory to the windows.
+//   warps 0..7  windows; between blocks TMEM lane quarter = warp % 4, i.e. 32 columns, and half of the rows
+//   warp 8      TMA of U's planes, 32 k-values of 128 columns a stage
+//   warp 9      MMA
+// The group parameters are fitted on whole groups inside a block (128 a multiple of the group size) or given per channel.
+constexpr int GROUP_STAGES = 4, GROUP_STAGE_BYTES = 2 * octc::SPLIT_MN_ATOM;    // 128 columns of both planes
+constexpr int GROUP_ERR_BYTES = 2 * 32 * BLK * 2;                               // errors of 32 rows, both planes
+constexpr int GROUP_SMEM = 1024 + GROUP_STAGES * GROUP_STAGE_BYTES + GROUP_ERR_BYTES +
+                           (BLK * BLK + BLK * 33 + BLK + (2 * NWIN + SUB + SUPER) * 32) * 4;
+struct GroupArgs {
+  ColArgs c;                     // of the first block; errors of all blocks go to its planes, 128 rows a block
+  int blocks;
+  const float* u_table; long long u_tab_ld, u_tab_b;   // 2^-e of U's blocks
+  int store_errors;              // something lies behind the group
+  int* status;
+};
+
+__device__ __forceinline__ void bar_windows() { asm volatile("bar.sync 6, 256;" ::: "memory"); }
+
+__global__ void __launch_bounds__(320, 1)
+gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga) {
+  using namespace octc;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t bar_full[GROUP_STAGES], bar_empty[GROUP_STAGES], bar_err[SUPER], bar_acc[SUPER * SUPER];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag_s;
+  volatile int* abort_flag = &abort_flag_s;
+  ColArgs a = ga.c;
+  const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31, batch = blockIdx.y;
+  uint8_t* base = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  const uint32_t stage_base = smem_u32(base);
+  uint8_t* err_s = base + GROUP_STAGES * GROUP_STAGE_BYTES;    // [plane][k / 64][row][64 k], 128-byte swizzle
+  float* Us = reinterpret_cast<float*>(err_s + GROUP_ERR_BYTES);   // [BLK][BLK], upper triangle of the diagonal block of U
+  float* tile = Us + BLK * BLK;                                // [BLK][33] entry values of a block, column by column
+  float* rdiag = tile + BLK * 33;
+  float* mm_lo = rdiag + BLK, *mm_hi = mm_lo + NWIN * 32;
+  float* Es = mm_hi + NWIN * 32;                               // [SUB][32]
+  float* inv_s = Es + SUB * 32;                                // [SUPER][32] 2^-e of the blocks' errors
+
+  if (tid == 0) {
+    for (int s = 0; s < GROUP_STAGES; ++s) { mbar_init(smem_u32(&bar_full[s]), 1); mbar_init(smem_u32(&bar_empty[s]), 1); }
+    for (int j = 0; j < SUPER; ++j) mbar_init(smem_u32(&bar_err[j]), 1);
+    for (int j = 0; j < SUPER * SUPER; ++j) mbar_init(smem_u32(&bar_acc[j]), 1);
+    abort_flag_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (wid == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(&tmem_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_slot;
+  // accumulator of source block j and target block t
+  auto acc_at = [&](int j, int t) { return tmem_base + (uint32_t)(t * (t - 1) / 2 + j) * 32u; };
+
+  if (wid == 8) {
+    if (lane == 0) {
+      uint32_t stage = 0, phase = 1;
+      bool ok = true;
+      for (int j = 0; j < ga.blocks && ok; ++j)
+        for (int t = j + 1; t < ga.blocks && ok; ++t)
+          for (int ks = 0; ks < BLK / SPLIT_BK; ++ks) {
+            ok = mbar_wait(smem_u32(&bar_empty[stage]), phase, abort_flag, ga.status, 311);
+            if (!ok) break;
+            const uint32_t bar = smem_u32(&bar_full[stage]), dst = stage_base + stage * GROUP_STAGE_BYTES;
+            mbar_expect_tx(bar, GROUP_STAGE_BYTES);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+              tma_load_planes(dst + h * SPLIT_MN_ATOM, &map_u, a.i1 + t * BLK + h * 64, a.i1 + j * BLK + ks * SPLIT_BK, batch, 0, bar);
+            if (++stage == GROUP_STAGES) { stage = 0; phase ^= 1; }
+          }
+      if (!ok) {
+        // let copies already issued land before the CTA's shared memory is released
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 200000ull) { }
+      }
+    }
+    __syncwarp();
+  } else if (wid == 9) {
+    if (lane == 0) {
+      constexpr uint32_t ID = split_idesc(true, false, BLK, 32);
+      // errors: K-major rows of 64 k (128-byte swizzle), groups of 8 rows 1024 bytes apart
+      auto err_desc = [&](int plane, int k16) {
+        uint64_t d = (uint64_t)(((smem_u32(err_s) + plane * 8192 + (k16 >> 2) * 4096 + (k16 & 3) * 32) & 0x3FFFFu) >> 4);
+        d |= (uint64_t)1 << 16;
+        d |= (uint64_t)(1024 >> 4) << 32;
+        d |= 1ull << 46;
+        d |= 2ull << 61;
+        return d;
+      };
+      uint32_t stage = 0, phase = 0;
+      bool ok = true;
+      for (int j = 0; j + 1 < ga.blocks && ok; ++j) {
+        ok = mbar_wait(smem_u32(&bar_err[j]), 0, abort_flag, ga.status, 312);
+        tc_fence_after();
+        for (int t = j + 1; t < ga.blocks && ok; ++t) {
+          const uint32_t d = acc_at(j, t);
+          for (int ks = 0; ks < BLK / SPLIT_BK; ++ks) {
+            ok = mbar_wait(smem_u32(&bar_full[stage]), phase, abort_flag, ga.status, 313);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t u_hi = stage_base + stage * GROUP_STAGE_BYTES, u_lo = u_hi + SPLIT_MN_LO;
+#pragma unroll
+            for (int kk = 0; kk < SPLIT_BK / 16; ++kk) {
+              const uint64_t uh = split_desc_mn(u_hi, kk), ul = split_desc_mn(u_lo, kk);
+              const uint64_t eh = err_desc(0, ks * 2 + kk), el = err_desc(1, ks * 2 + kk);
+              umma_f16(d, ul, eh, ID, (ks > 0 || kk > 0) ? 1u : 0u);
+              umma_f16(d, uh, el, ID, 1u);
+              umma_f16(d, uh, eh, ID, 1u);
+            }
+            umma_commit(smem_u32(&bar_empty[stage]));
+            if (++stage == GROUP_STAGES) { stage = 0; phase ^= 1; }
+          }
+          if (ok) umma_commit(smem_u32(&bar_acc[j * SUPER + t]));
+        }
+      }
+    }
+    __syncwarp();
+  } else {
+    {
+      const long long b = batch;
+      a.Wf += b * a.sW; a.U += b * a.sU; a.codesT += b * a.sC; a.scales += b * a.sS; a.zeros += b * a.sS;
+      a.errp += b * a.sEp; a.err_scale += b * a.sEs;
+    }
+    const float* u_table = ga.u_table + (long long)batch * ga.u_tab_b;
+    const int row0 = blockIdx.x * 32, row = row0 + lane, gs = a.gs;
+    const bool live = row < a.out;
+    const int quarter = wid & 3, half = wid >> 2;       // of the columns / rows, between blocks
+    const float maxqf = (float)a.maxq;
+    float scale = 1.f, zero = 0.f;
+    if (gs == -1 && live) { scale = a.scales[row]; zero = a.zeros[row]; }
+    float wv[16], udiag = 0.f;
+    auto request = [&](int i1) {                        // what block i1 needs from global memory
+#pragma unroll
+      for (int it = 0; it < BLK * BLK / 4 / 256; ++it) {
+        const int e = it * 256 + tid, i = e / (BLK / 4), j4 = e % (BLK / 4);
+        if (4 * j4 + 3 >= i)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                       ::"r"(smem_u32(Us + i * BLK + 4 * j4)), "l"(a.U + (long long)(i1 + i) * a.ldu + i1 + 4 * j4) : "memory");
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {
+        const int rr = row0 + half * 16 + r;
+        wv[r] = rr < a.out ? a.Wf[(long long)rr * a.ldw + i1 + quarter * 32 + lane] : 0.f;
+      }
+      if (tid < BLK) udiag = a.U[(long long)(i1 + tid) * a.ldu + i1 + tid];
+    };
+    request(a.i1);
+
+#pragma unroll 1
+    for (int t = 0; t < ga.blocks; ++t) {
+      const int i1 = a.i1 + t * BLK, col0 = i1 + wid * SUB;
+      // ---- entry values: W minus the updates of the group's earlier blocks, in their order
+#pragma unroll 1
+      for (int j = 0; j < t; ++j) {
+        const float fu = u_table[(long long)(a.i1 / BLK + j) * ga.u_tab_ld + a.i1 / BLK + t];
+        mbar_wait(smem_u32(&bar_acc[j * SUPER + t]), 0, abort_flag, ga.status, 314);
+        tc_fence_after();
+        float v[16];
+        tmem_ld16(acc_at(j, t) + ((uint32_t)(quarter * 32) << 16) + half * 16, v);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) wv[r] = fmaf(-(inv_s[j * 32 + half * 16 + r] * fu), v[r], wv[r]);
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r) tile[(quarter * 32 + lane) * 33 + half * 16 + r] = wv[r];
+      if (tid < BLK) rdiag[tid] = safe_reciprocal(udiag);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      bar_windows();
+      float w[SUB], mn = 0.f, mx = 0.f;
+#pragma unroll
+      for (int i = 0; i < SUB; ++i) {
+        w[i] = tile[(wid * SUB + i) * 33 + lane];
+        mn = fminf(mn, w[i]);
+        mx = fmaxf(mx, w[i]);
+      }
+      if (gs != -1) {
+        // whole groups in the block: every window finds its group's parameters for itself
+        mm_lo[wid * 32 + lane] = mn;
+        mm_hi[wid * 32 + lane] = mx;
+        bar_windows();
+        const int g = col0 / gs, opened = g * gs, first = (opened - i1) / SUB, wins = gs / SUB;
+#pragma unroll
+        for (int v = 0; v < NWIN; ++v)
+          if (v < wins) {
+            mn = fminf(mn, mm_lo[(first + v) * 32 + lane]);
+            mx = fmaxf(mx, mm_hi[(first + v) * 32 + lane]);
+          }
+        params_from_range(mn, mx, a.maxq, a.sym, scale, zero);
+        if (opened == col0 && live) {
+          a.scales[(long long)g * a.out + row] = scale;
+          a.zeros[(long long)g * a.out + row] = zero;
+        }
+      }
+      float er[SUB], cd[SUB];
+      window_chain(wid, lane, w, Us, rdiag + wid * SUB, Es, scale, zero, maxqf, er, cd);
+      // ---- the errors of a row leave under one scale, which is known when the last window is done
+      float mxe = 0.f;
+#pragma unroll
+      for (int i = 0; i < SUB; ++i) mxe = fmaxf(mxe, oc_finite_abs(er[i]));
+      bar_windows();                     // (the ranges have been read by all)
+      mm_hi[wid * 32 + lane] = mxe;
+      bar_windows();
+      const bool more = t + 1 < ga.blocks;
+      if (more) request(i1 + BLK);       // (nobody reads this block of U any more)
+#pragma unroll
+      for (int v = 0; v < NWIN; ++v) mxe = fmaxf(mxe, mm_hi[v * 32 + lane]);
+      float inv;
+      const float se = oc_split_scale(mxe, inv);
+      uint2 hi[4], lo[4];
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        oc_split4(make_float4(er[4 * v] * se, er[4 * v + 1] * se, er[4 * v + 2] * se, er[4 * v + 3] * se), hi[v], lo[v]);
+      if (more) {
+        // (the MMAs that read the previous block's errors are done: its last target's accumulator, waited for here)
+        if (t > 0) mbar_wait(smem_u32(&bar_acc[(t - 1) * SUPER + ga.blocks - 1]), 0, abort_flag, ga.status, 315);
+        uint8_t* to = err_s + (wid >> 2) * 4096 + lane * 128;
+        const int c = (wid & 3) * 2;
+        *reinterpret_cast<uint4*>(to + ((c ^ (lane & 7)) * 16)) = make_uint4(hi[0].x, hi[0].y, hi[1].x, hi[1].y);
+        *reinterpret_cast<uint4*>(to + (((c + 1) ^ (lane & 7)) * 16)) = make_uint4(hi[2].x, hi[2].y, hi[3].x, hi[3].y);
+        *reinterpret_cast<uint4*>(to + 8192 + ((c ^ (lane & 7)) * 16)) = make_uint4(lo[0].x, lo[0].y, lo[1].x, lo[1].y);
+        *reinterpret_cast<uint4*>(to + 8192 + (((c + 1) ^ (lane & 7)) * 16)) = make_uint4(lo[2].x, lo[2].y, lo[3].x, lo[3].y);
+        if (wid == 0) inv_s[t * 32 + lane] = inv;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        bar_windows();
+        if (tid == 0) mbar_arrive(smem_u32(&bar_err[t]));
+      }
+      if (live) {
+        unsigned short* code_out = a.codesT + (long long)col0 * a.out + row;
+#pragma unroll
+        for (int i = 0; i < SUB; ++i) code_out[(long long)i * a.out] = (unsigned short)cd[i];
+        if (ga.store_errors) {
+          if (wid == 0) a.err_scale[(long long)t * a.lde + row] = inv;
+          __half* to = a.errp + (long long)(t * BLK + wid * SUB) * a.lde + row;
+#pragma unroll
+          for (int v = 0; v < 4; ++v) store_halves(to + 4 * v * a.lde, a.lde, a.err_plane, hi[v], lo[v]);
+        }
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (wid == 9) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem_base) : "memory");
+  }
+}
+
+// the groups of blocks that gptq_group_kernel takes: `blocks` full blocks from column i1 on
+bool group_fits(const ColArgs& a, int sm_count) {
+  return (a.gs == -1 || (a.mse_steps == 0 && a.gs % SUB == 0 && BLK % a.gs == 0)) &&
+         (long long)oc_div_up(a.out, 32) * a.batch <= sm_count;
+}
+
+int launch_group(const GroupArgs& a, const CUtensorMap& map_u, cudaStream_t stream) {
+  OC_OPT_IN_SMEM(gptq_group_kernel, GROUP_SMEM);
+  gptq_group_kernel<<<dim3(oc_div_up(a.c.out, 32), a.c.batch), 320, GROUP_SMEM, stream>>>(map_u, a);
+  OC_CHECK_LAUNCH();
+  return OC_OK;
+}
+
 // ---- preparation: fp16 -> fp32, act-order gather, dead columns, per-channel parameters ----
 // Wf[r][j] = dead[perm[j]] ? 0 : float(W[r][perm[j]]).  Per-channel scale / zero are fitted on
 // the whole original row before dead columns are zeroed (reference :690-695).
@@ -1128,6 +1403,7 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   }
   const bool two_level = (groupsize == -1) || ((SUPER * blocksize) % groupsize == 0);
   const int super_cols = (two_level ? SUPER : 1) * blocksize;
+  // Groups of full blocks in one launch each, where every SM has one set of rows at most.
   OcSplitOperand u_op{};
   u_op.planes = Up; u_op.plane = d * ldu_p; u_op.ld = ldu_p; u_op.mn_major = 1; u_op.terms = 2; u_op.stride1 = 2 * d * ldu_p;
   u_op.scale = u_table; u_op.scale_k = nb_u; u_op.scale_r = 1; u_op.scale1 = nTab;
@@ -1136,6 +1412,16 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
                    groupsize, maxq, sym, mse_steps, (float)q_grid, q_norm, nWf, sU, nErr, nCodes, nPar, 2 * nErrP,
                    SUPER * lde, batch};
   };
+  GroupArgs group_args{col_args(0, BLK, ErrT, (__half*)ErrT, err_scale), 0, u_table, nb_u, nTab, 0, nullptr};
+  const bool grouped = split && two_level && windows_fit(group_args.c) && group_fits(group_args.c, sm_count);
+  CUtensorMap map_u;
+  if (grouped) {
+    OcGemmDevice dev;
+    int rc = octc::make_split_map(&map_u, u_op, d, d, batch, 1, 0);
+    if (!rc) rc = oc_gemm_device(dev);
+    if (rc) return rc;
+    group_args.status = dev.status;
+  }
   // W[:, n0 .. n1) -= Err U[k0 .. k0 + k, n0 .. n1), Err the planes of the group that starts at column s0
   auto split_update = [&](int s0, int k0, int k, int n0, int n1) {
     OcSplitGemm g{};
@@ -1153,6 +1439,17 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
     const int s0 = (i1 / super_cols) * super_cols;          // first column of the group
     const int s1 = min(d, s0 + super_cols);                 // one past its last column
     int rc;
+    if (grouped && s1 - i1 >= BLK) {                        // (i1 == s0)
+      const int blocks = (s1 - s0) / BLK;
+      i2 = s0 + blocks * BLK;
+      group_args.c.i1 = i1; group_args.blocks = blocks; group_args.store_errors = i2 < d;
+      rc = launch_group(group_args, map_u, stream);
+      // a partial block behind the last group, block by block as in the other schedule
+      for (int j = 0; !rc && i2 < s1 && j < blocks; ++j) rc = split_update(s0, s0 + j * BLK, BLK, i2, s1);
+      if (!rc && i2 == s1 && i2 < d) rc = split_update(s0, s0, i2 - s0, i2, d);
+      if (rc) return rc;
+      continue;
+    }
     const int count = min(blocksize, d - i1);
     i2 = i1 + count;
     float* err_rows = ErrT + (long long)(i1 - s0) * lde;
