@@ -1296,6 +1296,23 @@ int launch_block(const ColArgs& a, cudaStream_t stream) {
   return aligned ? launch_block_t<WARPS, true>(a, stream) : launch_block_t<WARPS, false>(a, stream);
 }
 
+// The fewest sets of 32 rows per CTA for which all CTAs run at once; eight where even that takes several waves.
+int launch_blocks(const ColArgs& a, int sm_count, cudaStream_t stream) {
+  const int sets = oc_div_up(a.out, 32);
+  int per_cta = 1;
+  while (per_cta < 8 && (long long)oc_div_up(sets, per_cta) * a.batch > sm_count) ++per_cta;
+  switch (per_cta) {
+    case 1: return launch_block<1>(a, stream);
+    case 2: return launch_block<2>(a, stream);
+    case 3: return launch_block<3>(a, stream);
+    case 4: return launch_block<4>(a, stream);
+    case 5: return launch_block<5>(a, stream);
+    case 6: return launch_block<6>(a, stream);
+    case 7: return launch_block<7>(a, stream);
+    default: return launch_block<8>(a, stream);
+  }
+}
+
 long long round4(long long x) { return (x + 3) / 4 * 4; }
 long long round8(long long x) { return (x + 7) / 8 * 8; }
 long long u_blocks(int d) { return (d + OC_SPLIT_BLOCK - 1) / OC_SPLIT_BLOCK; }
@@ -1456,10 +1473,7 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
     const ColArgs a = col_args(i1, count, err_rows, split && i2 < d ? (__half*)ErrT + (long long)(i1 - s0) * lde : nullptr,
                                err_scale + (i1 - s0) / BLK * lde);
     if (per_sm <= 2 && windows_fit(a)) rc = launch_windows(a, stream);
-    else if (per_sm <= 1) rc = launch_block<1>(a, stream);
-    else if (per_sm <= 2) rc = launch_block<2>(a, stream);
-    else if (per_sm <= 4) rc = launch_block<4>(a, stream);
-    else rc = launch_block<8>(a, stream);
+    else rc = launch_blocks(a, sm_count, stream);
     if (rc) return rc;
     if (i2 >= d) break;
     // near: the rest of the group, behind this block; far: everything behind the group, at its end
