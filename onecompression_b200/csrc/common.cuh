@@ -43,6 +43,36 @@
 void oc_set_last_error(const char* msg);
 void oc_count_launches(int n);
 
+// Dependent launches.  The path is chains of kernels of a few to a few dozen microseconds, and between two of them lie
+// about 2 us of launch and start-up.  A kernel launched with OC_LAUNCH may start when every CTA of the one before it in
+// the stream has called oc_let_next (near its end: CTAs that wait hold room that other streams could use) or is
+// done; it calls oc_wait_before, in every CTA, before its first access to global memory, which returns when that
+// kernel is complete and its writes are visible.
+__device__ __forceinline__ void oc_wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void oc_let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t oc_launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+// (kernel)(grid, block, smem, stream, arguments...)
+#define OC_LAUNCH(kernel, ...)                                                        \
+  do {                                                                                \
+    oc_count_launches(1);                                                             \
+    cudaError_t e__ = oc_launch_dependent(kernel, __VA_ARGS__);                       \
+    if (e__ != cudaSuccess) {                                                         \
+      cudaGetLastError();                                                             \
+      oc_set_last_error(cudaGetErrorString(e__));                                     \
+      return OC_ERR_CUDA;                                                             \
+    }                                                                                 \
+  } while (0)
+
 // 16-bit element types of weights and activations (the `dtype` arguments of the C ABI)
 enum : int { OC_DTYPE_F16 = 0, OC_DTYPE_BF16 = 1 };
 

@@ -32,7 +32,10 @@ constexpr int BUILD_STAGED_N = 49152;   // widest row that the act-order gather 
 // equil[j] = 2^-e with (diagv[j] + shift) / 4^e in [1, 4)
 __global__ void diag_stats_kernel(const float* __restrict__ H, long long ld, int n, float percdamp, float rel_shift,
                                   float* __restrict__ diagv, unsigned char* __restrict__ dead,
-                                  float* __restrict__ damp_out, float* __restrict__ equil, long long sH, long long sW) {
+                                  float* __restrict__ damp_out, float* __restrict__ equil, int* __restrict__ status,
+                                  long long sH, long long sW) {
+  oc_wait_before();
+  if (threadIdx.x == 0) status[blockIdx.x] = 0;
   {
     const long long b = blockIdx.x;
     H += b * sH; diagv += b * sW; dead += b * n; damp_out += b * 2; equil += b * sW;
@@ -58,6 +61,7 @@ __global__ void diag_stats_kernel(const float* __restrict__ H, long long ld, int
     damp_out[1] = (float)(t / (double)n);
   }
   __syncthreads();
+  oc_let_next();
   const float shift = rel_shift * damp_s;
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
     const float v = diagv[j] + shift;
@@ -72,6 +76,8 @@ __global__ void diag_stats_kernel(const float* __restrict__ H, long long ld, int
 // which every later pass uses as an index, would keep what was in memory.
 __device__ __forceinline__ float rank_key(float v) { return v == v ? v : __int_as_float(0x7f800000); }
 __global__ void rank_sort_kernel(const float* __restrict__ key, int n, int* __restrict__ perm, long long sW) {
+  oc_wait_before();
+  oc_let_next();
   key += (long long)blockIdx.y * sW;
   perm += (long long)blockIdx.y * n;
   __shared__ float tile[1024];
@@ -92,12 +98,16 @@ __global__ void rank_sort_kernel(const float* __restrict__ key, int n, int* __re
   if (i < n) perm[rank] = i;
 }
 
-__global__ void iota_kernel(int* __restrict__ perm, int n) {
+__global__ void iota_kernel(int* __restrict__ perm, int* __restrict__ inv, int n) {
+  oc_wait_before();
+  oc_let_next();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) perm[(long long)blockIdx.y * n + i] = i;
+  if (i < n) { perm[(long long)blockIdx.y * n + i] = i; inv[(long long)blockIdx.y * n + i] = i; }
 }
 
 __global__ void invert_perm_kernel(const int* __restrict__ perm, int* __restrict__ inv, int n) {
+  oc_wait_before();
+  oc_let_next();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   perm += (long long)blockIdx.y * n;
   inv += (long long)blockIdx.y * n;
@@ -115,6 +125,8 @@ __global__ void __launch_bounds__(256) build_reversed_kernel(
     const float* __restrict__ diagv, const float* __restrict__ damp, float rel_shift, const float* __restrict__ equil,
     float* __restrict__ equil_p, float* __restrict__ A, long long lda, long long sH, long long sW, int vec, int staged) {
   extern __shared__ __align__(16) float row_s[];
+  oc_wait_before();
+  oc_let_next();
   const int i = blockIdx.x;
   {
     const long long b = blockIdx.y;
@@ -159,6 +171,8 @@ __global__ void __launch_bounds__(256) build_reversed_kernel(
 __global__ void __launch_bounds__(256) reverse_upper_kernel(const float* __restrict__ X, long long ldx, int n,
                                                             const float* __restrict__ equil_p, float* __restrict__ U,
                                                             long long ldu, long long sW, long long sU, int vec) {
+  oc_wait_before();
+  oc_let_next();
   const int i = blockIdx.x;
   const float* x = X + (long long)blockIdx.y * sW + (long long)(n - 1 - i) * ldx;
   float* u = U + (long long)blockIdx.y * sU + (long long)i * ldu;
@@ -241,6 +255,7 @@ __device__ __forceinline__ void solve_row8(float (&y)[8], const float (&l)[8][8]
 
 __global__ void __launch_bounds__(ROW_THREADS + 32, 1)
 potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb, int* __restrict__ status, long long sW) {
+  oc_wait_before();
   A += (long long)blockIdx.x * sW;
   status += blockIdx.x;
   __shared__ __align__(16) float Lp[8 * LP + 16];  // the micro-panel's columns, [8][row]
@@ -255,6 +270,7 @@ potrf_block_kernel(float* __restrict__ A, long long lda, int k0, int nb, int* __
     __syncthreads();                               // Nv (block 0), Qs[0], Pre[0] are there
 #pragma unroll 1
     for (int jb = 0; jb < NB / 8; ++jb) {
+      if (jb == NB / 8 - 2) oc_let_next();
       float l[8][8];
       load_block8(Nv, l);
       int bad = 8;                                 // first column with an unusable pivot
@@ -463,6 +479,7 @@ constexpr float L_SCALE = 8192.f;          // entries of L are below 2
 template <int TR, bool SPLIT>              // rows per CTA
 __global__ void __launch_bounds__(TRT, 2) trsm_panel_kernel(float* __restrict__ A, long long lda, int k0, int rest,
                                                          long long sW, __half* __restrict__ planes, long long plane) {
+  oc_wait_before();
   A += (long long)blockIdx.y * sW;
   if (SPLIT) planes += (long long)blockIdx.y * sW * 2;
   extern __shared__ __align__(16) float sm[];
@@ -544,6 +561,7 @@ __global__ void __launch_bounds__(TRT, 2) trsm_panel_kernel(float* __restrict__ 
     }
   }
   __syncthreads();
+  oc_let_next();
 #pragma unroll
   for (int it = 0; it < TR * NB / 4 / TRT; ++it) {
     const int e = it * TRT + tid, r = e / (NB / 4), c4 = e % (NB / 4);
@@ -567,9 +585,8 @@ template <int TR, bool SPLIT>
 int launch_trsm(float* A, long long ld, int k0, int rest, int batch, long long sW, __half* planes, long long plane,
                 cudaStream_t stream) {
   OC_OPT_IN_SMEM((trsm_panel_kernel<TR, SPLIT>), TRSM_SMEM<TR>);
-  trsm_panel_kernel<TR, SPLIT><<<dim3(oc_div_up(rest, TR), batch), TRT, TRSM_SMEM<TR>, stream>>>(A, ld, k0, rest, sW,
-                                                                                              planes, plane);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH((trsm_panel_kernel<TR, SPLIT>), dim3(oc_div_up(rest, TR), batch), TRT, TRSM_SMEM<TR>, stream, A, ld, k0, rest, sW,
+            planes, plane);
   return OC_OK;
 }
 
@@ -584,6 +601,7 @@ __global__ void __launch_bounds__(DINV_T) diag_inverse_kernel(const float* __res
                                                            float* __restrict__ X, long long ldx, int n,
                                                            long long sW, __half* __restrict__ planes, long long plane,
                                                            float* __restrict__ table, int ldt) {
+  oc_wait_before();
   A += (long long)blockIdx.y * sW;
   X += (long long)blockIdx.y * sW;
   extern __shared__ __align__(16) float sm[];
@@ -666,6 +684,7 @@ __global__ void __launch_bounds__(DINV_T) diag_inverse_kernel(const float* __res
     }
     __syncthreads();
   }
+  oc_let_next();
   if (nb == NB) {
 #pragma unroll 4
     for (int it = 0; it < NB * NB / 4 / DINV_T; ++it) {
@@ -823,25 +842,24 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
   float *diagv = ws.diagv(w0), *equil = ws.equil(w0), *equil_p = ws.equil_p(w0);
   const bool split = oc_split_engine_on() && n > NB;     // (and then the workspace is aligned)
 
-  OC_CUDA(cudaMemsetAsync(status, 0, sizeof(int) * batch, stream));
-  diag_stats_kernel<<<batch, 1024, 0, stream>>>(H, ldh, n, percdamp, rel_shift, diagv, dead, damp_out, equil, sH, sW);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(diag_stats_kernel, batch, 1024, 0, stream, H, ldh, n, percdamp, rel_shift, diagv, dead, damp_out, equil, status,
+            sH, sW);
   const int tb = 256, gb = oc_div_up(n, tb);
   if (!reuse_perm) {
-    if (actorder) rank_sort_kernel<<<dim3(gb, batch), tb, 0, stream>>>(diagv, n, perm, sW);
-    else iota_kernel<<<dim3(gb, batch), tb, 0, stream>>>(perm, n);
-    OC_CHECK_LAUNCH();
-    invert_perm_kernel<<<dim3(gb, batch), tb, 0, stream>>>(perm, invperm, n);
-    OC_CHECK_LAUNCH();
+    if (actorder) {
+      OC_LAUNCH(rank_sort_kernel, dim3(gb, batch), tb, 0, stream, diagv, n, perm, sW);
+      OC_LAUNCH(invert_perm_kernel, dim3(gb, batch), tb, 0, stream, perm, invperm, n);
+    } else {
+      OC_LAUNCH(iota_kernel, dim3(gb, batch), tb, 0, stream, perm, invperm, n);
+    }
   }
   const bool vec_h = n % 4 == 0 && ldh % 4 == 0 && sH % 4 == 0 && aligned(H) && aligned(A);
   // (with reuse_perm the caller's perm counts, whatever actorder says)
   const int permuted = actorder || reuse_perm;
   const bool staged = permuted && n <= BUILD_STAGED_N;
   if (staged) OC_OPT_IN_SMEM(build_reversed_kernel, BUILD_STAGED_N * 4);
-  build_reversed_kernel<<<dim3(n, batch), 256, staged ? n * 4 : 0, stream>>>(
-      H, ldh, n, perm, permuted, diagv, damp_out, rel_shift, equil, equil_p, A, ld, sH, sW, vec_h, staged);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(build_reversed_kernel, dim3(n, batch), 256, staged ? n * 4 : 0, stream,
+            H, ldh, n, perm, permuted, diagv, damp_out, rel_shift, equil, equil_p, A, ld, sH, sW, vec_h, staged);
 
   // ---- blocked right-looking Cholesky --------------------------------------------------
   OC_OPT_IN_SMEM(diag_inverse_kernel, DINV_SMEM);
@@ -874,8 +892,7 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     const int kend = min(n, K0 + OB);
     for (int k0 = K0; k0 < kend; k0 += NB) {
       const int nb = min(NB, n - k0);
-      potrf_block_kernel<<<batch, ROW_THREADS + 32, 0, stream>>>(A, ld, k0, nb, status, sW);
-      OC_CHECK_LAUNCH();
+      OC_LAUNCH(potrf_block_kernel, batch, ROW_THREADS + 32, 0, stream, A, ld, k0, nb, status, sW);
       const int rest = n - k0 - nb;
       if (rest <= 0) break;
       OC_REQUIRE(nb == NB, "hinv_factor: a panel with rows below it is a full panel");
@@ -901,9 +918,8 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     if (rc2) return rc2;
   }
   // inverses of the diagonal blocks, all at once: the seeds of the blocked inverse below
-  diag_inverse_kernel<<<dim3(oc_div_up(n, NB), batch), DINV_T, DINV_SMEM, stream>>>(
-      A, ld, X, ld, n, sW, split ? ws.planesX(w0) : nullptr, ws.mat, ws.tableX(w0), (int)ws.nblk);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(diag_inverse_kernel, dim3(oc_div_up(n, NB), batch), DINV_T, DINV_SMEM, stream,
+            A, ld, X, ld, n, sW, split ? ws.planesX(w0) : nullptr, ws.mat, ws.tableX(w0), (int)ws.nblk);
 
   // ---- recursive blocked inverse of L: X holds the inverted diagonal blocks -----------------
   // The uniform problems of a level form one batched product (of both batch dimensions: problems and
@@ -949,8 +965,7 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     }
   }
   const bool vec_u = n % 4 == 0 && ldu % 4 == 0 && sU % 4 == 0 && aligned(U) && aligned(X);
-  reverse_upper_kernel<<<dim3(n, batch), 256, 0, stream>>>(X, ld, n, equil_p, U, ldu, sW, sU, vec_u);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(reverse_upper_kernel, dim3(n, batch), 256, 0, stream, X, ld, n, equil_p, U, ldu, sW, sU, vec_u);
   return OC_OK;
 }
 

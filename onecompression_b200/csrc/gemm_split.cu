@@ -179,6 +179,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
+  oc_wait_before();
   Walker<BN> walk;
   Tile t;
 
@@ -201,6 +202,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      oc_let_next();
       if (!ok) {
         // let copies already issued land before the CTA's shared memory is released
         const unsigned long long t0 = globaltimer_ns();
@@ -345,8 +347,7 @@ int make_map_c(CUtensorMap* map, const OcSplitGemm& g) {
 template <bool A_MN, bool B_MN, class S>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const Params& p, int grid, cudaStream_t s) {
   OC_OPT_IN_SMEM((gemm_split_kernel<A_MN, B_MN, S>), S::SMEM_DYN);
-  gemm_split_kernel<A_MN, B_MN, S><<<grid, THREADS, S::SMEM_DYN, s>>>(ma, mb, mc, p);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH((gemm_split_kernel<A_MN, B_MN, S>), grid, THREADS, S::SMEM_DYN, s, ma, mb, mc, p);
   return OC_OK;
 }
 

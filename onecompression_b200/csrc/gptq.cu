@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
   float* Ws = sm + BLK * BLK;   // [NROWS][WS], block-entry values of the rows' columns
   float* rdiag = Ws + NROWS * WS;   // [BLK] reciprocals of U's diagonal
   float* Es = rdiag + BLK;          // [2][SUB][NROWS] errors of the last two windows (helpers only)
+  oc_wait_before();
   const int tid = threadIdx.x;
   const int row0 = blockIdx.x * NROWS;
   const int count = a.count, i1 = a.i1;
@@ -412,6 +413,7 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
       }
     }
   }
+  oc_let_next();
   if (a.errp && owner) {        // a full block
     float mx = 0.f;
 #pragma unroll 4
@@ -560,6 +562,7 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
   float* Es = pz + NWIN * 32;                    // [SUB][32] errors of the window whose turn it is
   const int tid = threadIdx.x, wid = tid >> 5, lane = tid & 31;
   const int i1 = a.i1, gs = a.gs;
+  oc_wait_before();
   {
     const long long b = blockIdx.y;      // problem of a batch
     a.Wf += b * a.sW; a.U += b * a.sU; a.ErrT += b * a.sE; a.codesT += b * a.sC;
@@ -636,6 +639,7 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
   }
   float er[SUB], cd[SUB];
   window_chain(wid, lane, w, Us, rdiag + wid * SUB, Es, scale, zero, (float)a.maxq, er, cd);
+  if (wid == NWIN - 1) oc_let_next();
   if (live) {
     unsigned short* code_out = a.codesT + (long long)col0 * a.out + row;
 #pragma unroll
@@ -668,8 +672,7 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
 int launch_windows(const ColArgs& a, cudaStream_t stream) {
   const int smem = (BLK * BLK + BLK + (4 * NWIN + SUB) * 32) * (int)sizeof(float);
   OC_OPT_IN_SMEM(gptq_window_kernel, smem);
-  gptq_window_kernel<<<dim3(oc_div_up(a.out, 32), a.batch), 256, smem, stream>>>(a);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(gptq_window_kernel, dim3(oc_div_up(a.out, 32), a.batch), 256, smem, stream, a);
   return OC_OK;
 }
 
@@ -745,6 +748,7 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
+  oc_wait_before();
   // accumulator of source block j and target block t
   auto acc_at = [&](int j, int t) { return tmem_base + (uint32_t)(t * (t - 1) / 2 + j) * 32u; };
 
@@ -896,6 +900,7 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
       mm_hi[wid * 32 + lane] = mxe;
       bar_windows();
       const bool more = t + 1 < ga.blocks;
+      if (!more) oc_let_next();
       if (more) request(i1 + BLK);       // (nobody reads this block of U any more)
 #pragma unroll
       for (int v = 0; v < NWIN; ++v) mxe = fmaxf(mxe, mm_hi[v * 32 + lane]);
@@ -948,8 +953,7 @@ bool group_fits(const ColArgs& a, int sm_count) {
 
 int launch_group(const GroupArgs& a, const CUtensorMap& map_u, cudaStream_t stream) {
   OC_OPT_IN_SMEM(gptq_group_kernel, GROUP_SMEM);
-  gptq_group_kernel<<<dim3(oc_div_up(a.c.out, 32), a.c.batch), 320, GROUP_SMEM, stream>>>(map_u, a);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(gptq_group_kernel, dim3(oc_div_up(a.c.out, 32), a.c.batch), 320, GROUP_SMEM, stream, map_u, a);
   return OC_OK;
 }
 
@@ -969,6 +973,8 @@ gptq_prepare_kernel(const void* __restrict__ W, int bf16, long long ldw_in, int 
                     float* __restrict__ scales, float* __restrict__ zeros,
                     long long s_win, long long s_wf, long long s_par, int vec, int staged) {
   extern __shared__ __align__(16) float row_s[];
+  oc_wait_before();
+  oc_let_next();
   const int row = blockIdx.x;
   {
     const long long b = blockIdx.y;      // problem of a batch
@@ -1083,41 +1089,42 @@ __device__ __forceinline__ void pack3(const unsigned (&v)[32], unsigned (&w)[3])
   }
 }
 
-// qzeros[g][w]: (zero - 1) & mask of rows w*f .. w*f+f-1 (3 bit: 32 rows -> 3 words)
-__global__ void pack_qzeros_kernel(const float* __restrict__ zeros, int out, int G, int bits,
-                                   int* __restrict__ qzeros, long long ldz) {
-  const int g = blockIdx.y;
+// Group g of problem b: scales as fp16 and fp32, raw zero points, and the packed ones, qzeros[g][w]: (zero - 1) & mask of
+// rows w*f .. w*f+f-1 (3 bit: 32 rows -> 3 words).  One thread per row; the first row of a word packs it.
+__global__ void params_kernel(const float* __restrict__ scales, const float* __restrict__ zeros, int out, int G,
+                              long long s_par, __half* __restrict__ scales16, float* __restrict__ scales32,
+                              int* __restrict__ zeros_i32, long long lds, long long s_out, int bits,
+                              int* __restrict__ qzeros, long long ldz, long long s_qz) {
+  oc_wait_before();
+  oc_let_next();
+  const int r = blockIdx.x * blockDim.x + threadIdx.x, g = blockIdx.y;
+  const long long b = blockIdx.z, at = b * s_out + g * lds + r;
+  if (r >= out) return;
+  const float* zr = zeros + b * s_par + (long long)g * out;
+  if (scales16 || scales32) {
+    const float s = scales[b * s_par + (long long)g * out + r];
+    if (scales16) scales16[at] = __float2half_rn(s);
+    if (scales32) scales32[at] = s;
+  }
+  if (zeros_i32) zeros_i32[at] = (int)zr[r];
+  if (!qzeros) return;
   const unsigned mask = (1u << bits) - 1u;
-  const float* zr = zeros + (long long)g * out;
+  int* q = qzeros + b * s_qz + g * ldz;
   if (bits == 3) {
-    const int blk = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blk * 32 >= out) return;
+    if (r % 32) return;
     unsigned v[32], w[3];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) v[k] = (unsigned)((int)zr[blk * 32 + k] - 1) & mask;
+    for (int k = 0; k < 32; ++k) v[k] = (unsigned)((int)zr[r + k] - 1) & mask;
     pack3(v, w);
 #pragma unroll
-    for (int t = 0; t < 3; ++t) qzeros[(long long)g * ldz + blk * 3 + t] = (int)w[t];
+    for (int t = 0; t < 3; ++t) q[r / 32 * 3 + t] = (int)w[t];
   } else {
     const int f = 32 / bits;
-    const int wi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (wi * f >= out) return;
+    if (r % f) return;
     unsigned word = 0u;
-    for (int k = 0; k < f; ++k) word |= ((unsigned)((int)zr[wi * f + k] - 1) & mask) << (k * bits);
-    qzeros[(long long)g * ldz + wi] = (int)word;
+    for (int k = 0; k < f; ++k) word |= ((unsigned)((int)zr[r + k] - 1) & mask) << (k * bits);
+    q[r / f] = (int)word;
   }
-}
-
-__global__ void cast_params_kernel(const float* __restrict__ scales, const float* __restrict__ zeros,
-                                   int out, int G, __half* __restrict__ scales16, long long lds,
-                                   float* __restrict__ scales32, int* __restrict__ zeros_i32) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  const int g = blockIdx.y;
-  if (r >= out) return;
-  const float s = scales[(long long)g * out + r];
-  if (scales16) scales16[(long long)g * lds + r] = __float2half_rn(s);
-  if (scales32) scales32[(long long)g * lds + r] = s;
-  if (zeros_i32) zeros_i32[(long long)g * lds + r] = (int)zeros[(long long)g * out + r];
 }
 
 // Original-order outputs in one pass over the codes: packed words, integer codes [out][d] and the
@@ -1143,6 +1150,7 @@ struct FinishArgs {
 template <int BITS>   // 0: nothing is packed
 __global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
   extern __shared__ unsigned fin_s[];        // one tile per row-major output
+  oc_wait_before();
   unsigned* tw = fin_s;
   unsigned* tq = fin_s + (a.what ? FIN_TILE : 0);
   {
@@ -1235,6 +1243,7 @@ __global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
       }
     }
   }
+  oc_let_next();
   if (!a.what && !a.codes) return;
   __syncthreads();
   const bool vec = ((a.ldwh | a.d) & 1) == 0 && (reinterpret_cast<uintptr_t>(a.what) & 3) == 0;
@@ -1267,14 +1276,9 @@ __global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
 int launch_finish(const FinishArgs& a, int bits, int batch, cudaStream_t stream) {
   const dim3 grid(oc_div_up(a.d, FIN_COLS), oc_div_up(a.out, FIN_ROWS), batch);
   const int smem = ((a.what ? 1 : 0) + (a.codes ? 1 : 0)) * FIN_TILE * 4;
-  switch (bits) {
-    case 2: finish_kernel<2><<<grid, 128, smem, stream>>>(a); break;
-    case 3: finish_kernel<3><<<grid, 128, smem, stream>>>(a); break;
-    case 4: finish_kernel<4><<<grid, 128, smem, stream>>>(a); break;
-    case 8: finish_kernel<8><<<grid, 128, smem, stream>>>(a); break;
-    default: finish_kernel<0><<<grid, 128, smem, stream>>>(a);
-  }
-  OC_CHECK_LAUNCH();
+  void (*kernel)(FinishArgs) = bits == 2 ? finish_kernel<2> : bits == 3 ? finish_kernel<3> : bits == 4 ? finish_kernel<4>
+                               : bits == 8 ? finish_kernel<8> : finish_kernel<0>;
+  OC_LAUNCH(kernel, grid, 128, smem, stream, a);
   return OC_OK;
 }
 
@@ -1283,8 +1287,7 @@ int launch_block_t(const ColArgs& a, cudaStream_t stream) {
   // tiles, plus the error windows the helper threads read (only CTAs with few rows have helpers)
   const int smem = (BLK * BLK + WARPS * 32 * WS + BLK + (WARPS <= 2 ? 2 * SUB * WARPS * 32 : 0)) * (int)sizeof(float);
   OC_OPT_IN_SMEM((gptq_block_kernel<WARPS, ALIGNED>), smem);
-  gptq_block_kernel<WARPS, ALIGNED><<<dim3(oc_div_up(a.out, WARPS * 32), a.batch), LOADERS, smem, stream>>>(a);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH((gptq_block_kernel<WARPS, ALIGNED>), dim3(oc_div_up(a.out, WARPS * 32), a.batch), LOADERS, smem, stream, a);
   return OC_OK;
 }
 
@@ -1392,10 +1395,9 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
                    (reinterpret_cast<uintptr_t>(dead) & 7) == 0;
   const bool staged = perm && d <= PREPARE_STAGED_D;
   if (staged) OC_OPT_IN_SMEM(gptq_prepare_kernel, PREPARE_STAGED_D * 4);
-  gptq_prepare_kernel<<<dim3(out, batch), 256, staged ? d * 4 : 0, stream>>>(
-      W, bf16, ldw_in, out, d, perm, dead, Wf, ldw, groupsize == -1 ? 1 : 0, maxq, sym, mse_steps,
-      (float)q_grid, q_norm, scales, zeros, sWin, nWf, nPar, vec, staged);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(gptq_prepare_kernel, dim3(out, batch), 256, staged ? d * 4 : 0, stream,
+            W, bf16, ldw_in, out, d, perm, dead, Wf, ldw, groupsize == -1 ? 1 : 0, maxq, sym, mse_steps,
+            (float)q_grid, q_norm, scales, zeros, sWin, nWf, nPar, vec, staged);
 
   if (sm_count <= 0) sm_count = 148;
   const int warps_total = oc_div_up(out, 32) * batch;
@@ -1506,21 +1508,10 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
     const int rc = launch_finish(f_args, qweight ? wbits : 0, batch, stream);
     if (rc) return rc;
   }
-  for (int b = 0; b < batch; ++b) {
-    const float* sc = scales + b * nPar;
-    const float* zr = zeros + b * nPar;
-    if (qzeros) {
-      pack_qzeros_kernel<<<dim3(oc_div_up(out / f, tb), G), tb, 0, stream>>>(zr, out, G, wbits,
-                                                                             qzeros + b * G * ldz, ldz);
-      OC_CHECK_LAUNCH();
-    }
-    if (scales16 || scales32 || zeros_i32) {
-      cast_params_kernel<<<dim3(oc_div_up(out, tb), G), tb, 0, stream>>>(
-          sc, zr, out, G, scales16 ? scales16 + b * G * ld_out : nullptr, ld_out,
-          scales32 ? scales32 + b * G * ld_out : nullptr, zeros_i32 ? zeros_i32 + b * G * ld_out : nullptr);
-      OC_CHECK_LAUNCH();
-    }
-  }
+  // scales, zero points (raw and packed), all problems in one launch
+  if (qzeros || scales16 || scales32 || zeros_i32)
+    OC_LAUNCH(params_kernel, dim3(oc_div_up(out, tb), G, batch), tb, 0, stream, scales, zeros, out, G, nPar, scales16, scales32,
+              zeros_i32, ld_out, (long long)G * ld_out, wbits, qzeros, ldz, (long long)G * ldz);
   return OC_OK;
 }
 

@@ -126,6 +126,8 @@ __global__ void delta_split_kernel(const uint4* __restrict__ xf, const uint4* __
 constexpr int MT = 64;
 __global__ void __launch_bounds__(256) mirror_upper_kernel(float* __restrict__ M, long long ld, int n, int vec) {
   __shared__ float t[MT][MT + 1];
+  oc_wait_before();
+  oc_let_next();
   const int bi = blockIdx.y, bj = blockIdx.x;
   if (bj < bi) return;  // only tiles on or above the diagonal are sources
   const int tid = threadIdx.x;
@@ -218,7 +220,6 @@ extern "C" int oc_mirror_upper(float* M, long long ld, int n, void* stream) {
   OC_REQUIRE(M && n > 0 && ld >= n, "mirror_upper: bad arguments");
   const int t = oc_div_up(n, MT);
   const bool vec = n % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(M) & 15) == 0;
-  mirror_upper_kernel<<<dim3(t, t), 256, 0, (cudaStream_t)stream>>>(M, ld, n, vec);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(mirror_upper_kernel, dim3(t, t), 256, 0, (cudaStream_t)stream, M, ld, n, vec);
   return OC_OK;
 }

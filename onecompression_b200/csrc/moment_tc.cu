@@ -141,6 +141,7 @@ moment_tc_kernel(const __grid_constant__ CUtensorMap map_xq, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
+  oc_wait_before();
 
   const int total_items = p.h_tiles + p.c_tiles;
   const int total_stages = (int)((p.n_tok + BK - 1) / BK);
@@ -177,6 +178,7 @@ moment_tc_kernel(const __grid_constant__ CUtensorMap map_xq, const __grid_consta
           }
         }
       }
+      oc_let_next();
       if (!ok) {
         // let copies already issued land before the CTA's shared memory is released
         const unsigned long long t0 = globaltimer_ns();
@@ -358,7 +360,6 @@ extern "C" int oc_moment_accum(const void* xq, const void* xf, void* delta_scrat
   OC_OPT_IN_SMEM(moment_tc_kernel, SMEM_DYN);
   if (sm_count <= 0) sm_count = 148;
   const int grid = min(sm_count, p.h_tiles + p.c_tiles);
-  moment_tc_kernel<<<grid, NUM_THREADS, SMEM_DYN, stream>>>(map_xq, map_delta, p);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(moment_tc_kernel, grid, NUM_THREADS, SMEM_DYN, stream, map_xq, map_delta, p);
   return OC_OK;
 }

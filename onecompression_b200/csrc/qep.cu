@@ -57,6 +57,8 @@ __global__ void qep_load_kernel(const void* __restrict__ W, long long ldw_in, in
 __global__ void __launch_bounds__(256) qep_plane_kernel(const void* __restrict__ W, long long ldw_in, int out, int d,
                                                         const unsigned char* __restrict__ dead, __half* __restrict__ plane,
                                                         long long ldp, float* __restrict__ table, int bf16, int vec) {
+  oc_wait_before();
+  oc_let_next();
   const int lane = threadIdx.x & 31, r = blockIdx.y * 8 + (threadIdx.x >> 5), c = blockIdx.x * 128 + lane * 4;
   if (r >= out) return;
   float v[4] = {0.f, 0.f, 0.f, 0.f};
@@ -99,6 +101,8 @@ __global__ void gather_cols_kernel(const float* __restrict__ src, long long lds,
 __global__ void qep_store_kernel(const unsigned char* __restrict__ dead, const float* __restrict__ T,
                                  long long ldt, int out, int d, const int* __restrict__ perm,
                                  float perccorr, void* __restrict__ W, long long ldw_out, int bf16, int vec) {
+  oc_wait_before();
+  oc_let_next();
   const int r = blockIdx.y;
   if (vec) {
     const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -155,8 +159,7 @@ int split_products(const void* W, long long ldw_io, int out, int d, const float*
   float* tabR = (float*)(workspace + ws.planes + ws.result + ws.right + ws.tab_rows);
   const long long nb = blocks(d);
   delta = R;
-  qep_plane_kernel<<<dim3((int)nb, oc_div_up(out, 8)), 256, 0, stream>>>(W, ldw_io, out, d, dead, Lp, ws.ld, tabL, bf16, vec);
-  OC_CHECK_LAUNCH();
+  OC_LAUNCH(qep_plane_kernel, dim3((int)nb, oc_div_up(out, 8)), 256, 0, stream, W, ldw_io, out, d, dead, Lp, ws.ld, tabL, bf16, vec);
   OcSplitArgs right{};
   right.rows = right.cols = d; right.planes = Rp; right.plane = d * ws.ld; right.ldp = ws.ld; right.table = tabR;
   right.ldt = nb; right.nb1 = right.nb2 = 1;
@@ -232,9 +235,8 @@ extern "C" int oc_qep_adjust(void* W_, long long ldw_io, int out, int d, const f
     const int rc = split_products(W, ldw_io, out, d, C, ldc, U, ldu, perm, dead, bf16, vec_w, (char*)workspace, delta, stream);
     if (rc) return rc;
     const bool vec_st = vec_w && !perm;
-    qep_store_kernel<<<vec_st ? grid4 : grid, tb, 0, stream>>>(dead, delta, QepWs(out, d).ld, out, d, perm, perccorr, W,
-                                                              ldw_io, bf16, vec_st);
-    OC_CHECK_LAUNCH();
+    OC_LAUNCH(qep_store_kernel, vec_st ? grid4 : grid, tb, 0, stream, dead, delta, QepWs(out, d).ld, out, d, perm, perccorr, W,
+              ldw_io, bf16, vec_st);
     return OC_OK;
   }
   qep_load_kernel<<<vec ? grid4 : grid, tb, 0, stream>>>(W, ldw_io, out, d, dead, Wf, ld, bf16, vec);

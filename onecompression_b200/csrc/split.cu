@@ -9,6 +9,7 @@ constexpr int ST = 256;
 
 template <bool VEC, bool PER_ROW>
 __global__ void __launch_bounds__(ST) split_kernel(OcSplitArgs a) {
+  oc_wait_before();
   const int rb = blockIdx.y, cb = blockIdx.x;
   if (a.region == OC_SPLIT_UPPER && cb < (rb & ~1)) return;
   if (a.region == OC_SPLIT_LOWER && cb > (rb | 1)) return;
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(ST) split_kernel(OcSplitArgs a) {
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
     for (int i = 0; i < (PER_ROW ? 16 : 1); ++i) mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], o));
+  oc_let_next();
   float inv, s = 1.f;
   if (!PER_ROW) {
     if (lane == 0) red[warp] = mx[0];
@@ -89,12 +91,9 @@ int oc_split_launch(const OcSplitArgs& a, cudaStream_t stream) {
   const bool vec = !a.perm && a.cols % 4 == 0 && a.ld % 4 == 0 && a.src1 % 4 == 0 && a.src2 % 4 == 0 &&
                    (reinterpret_cast<uintptr_t>(a.src) & 15) == 0;
   if (a.per_row) {
-    if (vec) split_kernel<true, true><<<grid, ST, 0, stream>>>(a);
-    else split_kernel<false, true><<<grid, ST, 0, stream>>>(a);
+    OC_LAUNCH((vec ? split_kernel<true, true> : split_kernel<false, true>), grid, ST, 0, stream, a);
   } else {
-    if (vec) split_kernel<true, false><<<grid, ST, 0, stream>>>(a);
-    else split_kernel<false, false><<<grid, ST, 0, stream>>>(a);
+    OC_LAUNCH((vec ? split_kernel<true, false> : split_kernel<false, false>), grid, ST, 0, stream, a);
   }
-  OC_CHECK_LAUNCH();
   return OC_OK;
 }
