@@ -44,7 +44,29 @@ struct ColArgs {
   long long sW, sU, sE, sC, sS;
   long long sEp, sEs;
   int batch;
+  float minus_one;               // for update4
 };
+
+// t -= e * u, product and difference rounded each for itself, two entries per instruction.  The difference is the FMA
+// t + p * -1, which rounds like t - p; -1 comes in as a kernel argument, because the assembler contracts a
+// packed product and sum that it can see into one FMA (other bits).  28672 rows, general kernel: 48.4 -> 44 us a block,
+// bound by issue slots (0.6 instructions a cycle and scheduler with two warps on it).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void update2(float& t0, float& t1, f32x2 e2, float u0, float u1, f32x2 m2) {
+  f32x2 t = pack2(t0, t1), p;
+  const f32x2 u = pack2(u0, u1);
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(e2), "l"(u));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t) : "l"(p), "l"(m2), "l"(t));
+  unpack2(t, t0, t1);
+}
 
 // columns c .. c + 3 of a row's errors to their planes
 __device__ __forceinline__ void store_halves(__half* to, long long lde, long long plane, uint2 hi, uint2 lo) {
@@ -140,14 +162,14 @@ __device__ __noinline__ void fit_group(const float* __restrict__ src, int n, int
 // on who applies them.
 constexpr int LOADERS = 256;
 
-__device__ __forceinline__ void apply_window(float4& t, const float* __restrict__ es, const float* __restrict__ us) {
+__device__ __forceinline__ void apply_window(float4& t, const float* __restrict__ es, const float* __restrict__ us, f32x2 m2) {
   // es: this row's SUB errors (stride = rows of the CTA is folded in by the caller); us: U rows of the window
 #pragma unroll
   for (int i = 0; i < SUB; ++i) {
-    const float e = es[i];
+    const f32x2 e2 = pack2(es[i], es[i]);
     const float4 u = *reinterpret_cast<const float4*>(us + i * BLK);
-    t.x = __fsub_rn(t.x, __fmul_rn(e, u.x)); t.y = __fsub_rn(t.y, __fmul_rn(e, u.y));
-    t.z = __fsub_rn(t.z, __fmul_rn(e, u.z)); t.w = __fsub_rn(t.w, __fmul_rn(e, u.w));
+    update2(t.x, t.y, e2, u.x, u.y, m2);
+    update2(t.z, t.w, e2, u.z, u.w, m2);
   }
 }
 
@@ -288,6 +310,7 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
   float* wrow = Ws + (owner ? tid : 0) * WS;
   const float* grow = a.Wf + (long long)(owner ? row : 0) * a.ldw;  // block-entry state of the whole row
   const float maxqf = (float)a.maxq;
+  const f32x2 m2 = pack2(a.minus_one, a.minus_one);
   const int gs = a.gs;
   unsigned short* code_out = a.codesT + (long long)i1 * a.out + row;   // + column * out
   float* err_out = a.ErrT + row;                                        // + column * lde
@@ -370,13 +393,13 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
           float4 t1 = *reinterpret_cast<const float4*>(wrow + jc + 4);
 #pragma unroll
           for (int i = 0; i < SUB; ++i) {
-            const float e = er[i];
+            const f32x2 e2 = pack2(er[i], er[i]);
             const float4 u0 = *reinterpret_cast<const float4*>(Us + (cb + i) * BLK + jc);
             const float4 u1 = *reinterpret_cast<const float4*>(Us + (cb + i) * BLK + jc + 4);
-            t0.x = __fsub_rn(t0.x, __fmul_rn(e, u0.x)); t0.y = __fsub_rn(t0.y, __fmul_rn(e, u0.y));
-            t0.z = __fsub_rn(t0.z, __fmul_rn(e, u0.z)); t0.w = __fsub_rn(t0.w, __fmul_rn(e, u0.w));
-            t1.x = __fsub_rn(t1.x, __fmul_rn(e, u1.x)); t1.y = __fsub_rn(t1.y, __fmul_rn(e, u1.y));
-            t1.z = __fsub_rn(t1.z, __fmul_rn(e, u1.z)); t1.w = __fsub_rn(t1.w, __fmul_rn(e, u1.w));
+            update2(t0.x, t0.y, e2, u0.x, u0.y, m2);
+            update2(t0.z, t0.w, e2, u0.z, u0.w, m2);
+            update2(t1.x, t1.y, e2, u1.x, u1.y, m2);
+            update2(t1.z, t1.w, e2, u1.z, u1.w, m2);
           }
           *reinterpret_cast<float4*>(wrow + jc) = t0;
           *reinterpret_cast<float4*>(wrow + jc + 4) = t1;
@@ -395,7 +418,7 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
           float er[SUB];
 #pragma unroll
           for (int i = 0; i < SUB; ++i) er[i] = es_buf[i * NROWS + hrow];
-          apply_window(t, er, Us + cb * BLK + 4 * g);
+          apply_window(t, er, Us + cb * BLK + 4 * g, m2);
           *reinterpret_cast<float4*>(Ws + hrow * WS + 4 * g) = t;
         }
       }
@@ -407,7 +430,7 @@ __global__ void __launch_bounds__(LOADERS) gptq_block_kernel(ColArgs a) {
         for (int g = g_urgent; g < g_end; ++g) {
           if (g % NSEL != gsel) continue;
           float4 t = *reinterpret_cast<const float4*>(Ws + hrow * WS + 4 * g);
-          apply_window(t, er, Us + cb * BLK + 4 * g);
+          apply_window(t, er, Us + cb * BLK + 4 * g, m2);
           *reinterpret_cast<float4*>(Ws + hrow * WS + 4 * g) = t;
         }
       }
@@ -498,7 +521,7 @@ __device__ __forceinline__ bool produce_chunk(float (&w)[SUB], const float* __re
 // of the earlier windows, then er and cd the errors and codes of the warp's own.
 __device__ __forceinline__ void window_chain(int wid, int lane, float (&w)[SUB], const float* __restrict__ Us,
                                              const float* __restrict__ rdiag, float* Es, float scale, float zero,
-                                             float maxqf, float (&er)[SUB], float (&cd)[SUB]) {
+                                             float maxqf, f32x2 m2, float (&er)[SUB], float (&cd)[SUB]) {
   const float rs = safe_reciprocal(scale);
   const float lo = __fsub_rn(0.f, zero), hi = __fsub_rn(maxqf, zero);
 
@@ -515,14 +538,12 @@ __device__ __forceinline__ void window_chain(int wid, int lane, float (&w)[SUB],
       const float* ur = Us + (pw * SUB + q * CHUNK) * BLK + wid * SUB;
 #pragma unroll
       for (int c = 0; c < CHUNK; ++c) {
-        const float e = es[c * 32];
+        const f32x2 e2 = pack2(es[c * 32], es[c * 32]);
 #pragma unroll
         for (int v = 0; v < SUB / 4; ++v) {
           const float4 u = *reinterpret_cast<const float4*>(ur + c * BLK + 4 * v);
-          w[4 * v] = __fsub_rn(w[4 * v], __fmul_rn(e, u.x));
-          w[4 * v + 1] = __fsub_rn(w[4 * v + 1], __fmul_rn(e, u.y));
-          w[4 * v + 2] = __fsub_rn(w[4 * v + 2], __fmul_rn(e, u.z));
-          w[4 * v + 3] = __fsub_rn(w[4 * v + 3], __fmul_rn(e, u.w));
+          update2(w[4 * v], w[4 * v + 1], e2, u.x, u.y, m2);
+          update2(w[4 * v + 2], w[4 * v + 3], e2, u.z, u.w, m2);
         }
       }
     }
@@ -638,7 +659,7 @@ __global__ void __launch_bounds__(256, 2) gptq_window_kernel(ColArgs a) {
     }
   }
   float er[SUB], cd[SUB];
-  window_chain(wid, lane, w, Us, rdiag + wid * SUB, Es, scale, zero, (float)a.maxq, er, cd);
+  window_chain(wid, lane, w, Us, rdiag + wid * SUB, Es, scale, zero, (float)a.maxq, pack2(a.minus_one, a.minus_one), er, cd);
   if (wid == NWIN - 1) oc_let_next();
   if (live) {
     unsigned short* code_out = a.codesT + (long long)col0 * a.out + row;
@@ -891,7 +912,7 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
         }
       }
       float er[SUB], cd[SUB];
-      window_chain(wid, lane, w, Us, rdiag + wid * SUB, Es, scale, zero, maxqf, er, cd);
+      window_chain(wid, lane, w, Us, rdiag + wid * SUB, Es, scale, zero, maxqf, pack2(a.minus_one, a.minus_one), er, cd);
       // ---- the errors of a row leave under one scale, which is known when the last window is done
       float mxe = 0.f;
 #pragma unroll
@@ -1429,7 +1450,7 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   auto col_args = [&](int i1, int count, float* err_rows, __half* err_planes, float* err_sc) {
     return ColArgs{Wf, ldw, out, d, i1, count, U, ldu, err_rows, lde, err_planes, nErrP, err_sc, codesT, scales, zeros,
                    groupsize, maxq, sym, mse_steps, (float)q_grid, q_norm, nWf, sU, nErr, nCodes, nPar, 2 * nErrP,
-                   SUPER * lde, batch};
+                   SUPER * lde, batch, -1.f};
   };
   GroupArgs group_args{col_args(0, BLK, ErrT, (__half*)ErrT, err_scale), 0, u_table, nb_u, nTab, 0, nullptr};
   const bool grouped = split && two_level && windows_fit(group_args.c) && group_fits(group_args.c, sm_count);
