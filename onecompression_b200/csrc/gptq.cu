@@ -1155,8 +1155,11 @@ __global__ void params_kernel(const float* __restrict__ scales, const float* __r
 // the original order, a warp 32 of the columns, a lane two neighbouring rows: a lane sees whole packed
 // words of its rows, reads the codes coalesced along the rows, and reads scale and zero point only
 // where the group changes.  The row-major outputs leave through shared memory, a row segment of 128
-// bytes a warp.  Packing and dequantising read the codes separately before: 28672 x 4096, 4 bits:
-// 151 + 387 us, 215 us now; 4096 x 4096, 3 bits: 11 + 55, 34 us.
+// bytes a warp.  The codes of the two rows of a lane stay together in one register from the load to the stores:
+// up to 8 bits, q | 0x6400 is fp16(1024 + q), scale * (q - zero) is exact in fp32, so one fp16 subtraction (exact) and one
+// product give its rounding, and the packed words grow 16 bits a row at a time.  With the rows taken apart and
+// the arithmetic in fp32 issue slots bound it: 28672 x 4096, 4 bits 215 -> 113 us;
+// 4096 x 4096, 3 bits 34 -> 17 us.
 constexpr int FIN_ROWS = 64, FIN_COLS = 128;
 // Two neighbouring columns of a row share a 4-byte word of the tile.  Writers of a warp hold every other
 // row: 65 words apart, shifted by one in the second half, all 32 fall into different banks.
@@ -1166,11 +1169,14 @@ struct FinishArgs {
   const unsigned short* codesT; int out, d; const int* invperm; int gs;
   const float* scales; const float* zeros;
   int* qweight; long long ldq; int* codes; long long ldc; void* what; long long ldwh; int bf16;
+  int narrow;                                      // codes of at most 8 bits
   long long s_codes, s_par, s_qw, s_out, s_what;   // strides between the problems of a batch
 };
-template <int BITS>   // 0: nothing is packed
+// BITS 0: nothing is packed.  LOOKUP: columns are permuted, a group may change inside 32 columns, or the last 32 are fewer.
+template <int BITS, bool LOOKUP>
 __global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
   extern __shared__ unsigned fin_s[];        // one tile per row-major output
+  __shared__ int2 look[FIN_COLS];            // source column and group
   oc_wait_before();
   unsigned* tw = fin_s;
   unsigned* tq = fin_s + (a.what ? FIN_TILE : 0);
@@ -1186,81 +1192,110 @@ __global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
   const int r0 = blockIdx.y * FIN_ROWS, cb = blockIdx.x * FIN_COLS, c0 = cb + warp * 32;
   const int r = r0 + 2 * lane;
   const bool pair = (a.out & 1) == 0;          // two rows in one 4-byte access
-  if (c0 < a.d) {               // (the same for all lanes: they shuffle)
-    const bool one = r < a.out, two = r + 1 < a.out;
-    constexpr unsigned MASK = BITS ? (1u << BITS) - 1u : 0u;
-    unsigned word0[BITS ? BITS : 1], word1[BITS ? BITS : 1];   // the 32 columns' packed words of both rows
+  const bool one = r < a.out, two = r + 1 < a.out;
+  if (LOOKUP) {
+    const int c = cb + tid, j = c < a.d ? (a.invperm ? a.invperm[c] : c) : 0;
+    look[tid] = make_int2(j, a.gs == -1 ? 0 : j / a.gs);
+    __syncthreads();
+  }
+  if (c0 < a.d && one) {
+    unsigned q2[32];                           // codes of both rows
+    {
+      const unsigned short* p = a.codesT + (long long)c0 * a.out + r;
 #pragma unroll
-    for (int t = 0; t < (BITS ? BITS : 1); ++t) word0[t] = word1[t] = 0u;
-    // source column and group of column c0 + lane, handed round below
-    const int cl = c0 + lane;
-    const int jl = cl < a.d ? (a.invperm ? a.invperm[cl] : cl) : -1;
-    const int gl = (a.gs == -1 || jl < 0) ? 0 : jl / a.gs;
-    int group = -1;
-    float2 sc = make_float2(0.f, 0.f), zr = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k8 = 0; k8 < 32; k8 += 8) {
-      unsigned q2[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int j = __shfl_sync(0xffffffffu, jl, k8 + i);
-        q2[i] = 0u;
-        if (j >= 0 && one) {
-          const unsigned short* p = a.codesT + (long long)j * a.out + r;
-          if (pair) q2[i] = *reinterpret_cast<const unsigned*>(p);
-          else q2[i] = (unsigned)p[0] | (two ? (unsigned)p[1] << 16 : 0u);
+      for (int k = 0; k < 32; ++k) {
+        if (LOOKUP) p = a.codesT + (long long)look[warp * 32 + k].x * a.out + r;
+        q2[k] = 0u;
+        if (!LOOKUP || c0 + k < a.d) {
+          if (pair) q2[k] = *reinterpret_cast<const unsigned*>(p);
+          else q2[k] = (unsigned)p[0] | (two ? (unsigned)p[1] << 16 : 0u);
         }
-      }
-      unsigned short ua[2], ub[2];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int k = k8 + i;
-        const unsigned qa = q2[i] & 0xffffu, qb = q2[i] >> 16;
-        if (BITS) {
-          const int bit = k * BITS, wi = bit >> 5, off = bit & 31;
-          word0[wi] |= (qa & MASK) << off;
-          word1[wi] |= (qb & MASK) << off;
-          if (off + BITS > 32) {
-            word0[wi + 1 < BITS ? wi + 1 : wi] |= (qa & MASK) >> (32 - off);
-            word1[wi + 1 < BITS ? wi + 1 : wi] |= (qb & MASK) >> (32 - off);
-          }
-        }
-        if (a.what) {
-          const int g = __shfl_sync(0xffffffffu, gl, k);
-          if (g != group) {
-            group = g;
-            const float* sp = a.scales + (long long)g * a.out + r;
-            const float* zp = a.zeros + (long long)g * a.out + r;
-            if (one) { sc.x = __half2float(__float2half_rn(sp[0])); zr.x = zp[0]; }
-            if (two) { sc.y = __half2float(__float2half_rn(sp[1])); zr.y = zp[1]; }
-          }
-          // the reference rounds to fp16 first and casts to the module's dtype afterwards
-          const __half ha = __float2half_rn(__fmul_rn(sc.x, __fsub_rn((float)qa, zr.x)));
-          const __half hb = __float2half_rn(__fmul_rn(sc.y, __fsub_rn((float)qb, zr.y)));
-          if (a.bf16) {
-            ua[k & 1] = __bfloat16_as_ushort(__float2bfloat16_rn(__half2float(ha)));
-            ub[k & 1] = __bfloat16_as_ushort(__float2bfloat16_rn(__half2float(hb)));
-          } else { ua[k & 1] = __half_as_ushort(ha); ub[k & 1] = __half_as_ushort(hb); }
-          if (k & 1) {
-            tw[fin_at(2 * lane, warp * 32 + k)] = (unsigned)ua[0] | ((unsigned)ua[1] << 16);
-            tw[fin_at(2 * lane + 1, warp * 32 + k)] = (unsigned)ub[0] | ((unsigned)ub[1] << 16);
-          }
-        }
-        if (a.codes && (k & 1)) {
-          tq[fin_at(2 * lane, warp * 32 + k)] = (q2[i - 1 >= 0 ? i - 1 : 0] & 0xffffu) | (qa << 16);
-          tq[fin_at(2 * lane + 1, warp * 32 + k)] = (q2[i - 1 >= 0 ? i - 1 : 0] >> 16) | (qb << 16);
-        }
+        p += a.out;
       }
     }
-    if (BITS && a.qweight && one) {
+    if (BITS && a.qweight) {
+      constexpr int PIECES = BITS ? 2 * BITS : 1;
+      constexpr unsigned MASK = BITS ? (1u << BITS) - 1u : 0u;
+      unsigned piece[PIECES];                  // 16 bits of both rows' packed words each
+#pragma unroll
+      for (int t = 0; t < PIECES; ++t) piece[t] = 0u;
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        const int bit = k * BITS, pi = bit >> 4, off = bit & 15, low = min(BITS, 16 - off);   // bits in the first piece
+        piece[pi] |= (q2[k] & (((1u << low) - 1u) * 0x10001u)) << off;
+        if (low < BITS) piece[pi + 1 < PIECES ? pi + 1 : pi] |= (q2[k] >> low) & ((MASK >> low) * 0x10001u);
+      }
       const long long w0 = (long long)c0 / 32 * BITS;
       const int words = min(BITS, (int)((long long)(a.d - c0) * BITS / 32));   // d is a multiple of the pack factor
+      const bool both = two && (a.ldq & 1) == 0 && (reinterpret_cast<uintptr_t>(a.qweight) & 7) == 0;
 #pragma unroll
       for (int t = 0; t < BITS; ++t) {
         if (t >= words) continue;
         int* p = a.qweight + (w0 + t) * a.ldq + r;
-        p[0] = (int)word0[t];
-        if (two) p[1] = (int)word1[t];
+        const int wa = (int)__byte_perm(piece[2 * t], piece[2 * t + 1 < PIECES ? 2 * t + 1 : 0], 0x5410);
+        const int wb = (int)__byte_perm(piece[2 * t], piece[2 * t + 1 < PIECES ? 2 * t + 1 : 0], 0x7632);
+        if (both) *reinterpret_cast<int2*>(p) = make_int2(wa, wb);
+        else {
+          p[0] = wa;
+          if (two) p[1] = wb;
+        }
+      }
+    }
+    if (a.codes) {
+#pragma unroll
+      for (int k = 0; k < 32; k += 2) {
+        tq[fin_at(2 * lane, warp * 32 + k)] = __byte_perm(q2[k], q2[k + 1], 0x5410);
+        tq[fin_at(2 * lane + 1, warp * 32 + k)] = __byte_perm(q2[k], q2[k + 1], 0x7632);
+      }
+    }
+    if (a.what) {
+      int group = -1;
+      float2 zr = make_float2(0.f, 0.f);
+      __half2 s2 = __floats2half2_rn(0.f, 0.f), z2 = s2;
+      auto load_group = [&](int g) {
+        const float* sp = a.scales + (long long)g * a.out + r;
+        const float* zp = a.zeros + (long long)g * a.out + r;
+        zr = make_float2(zp[0], two ? zp[1] : 0.f);
+        s2 = __floats2half2_rn(sp[0], two ? sp[1] : 0.f);
+        z2 = __floats2half2_rn(1024.f + zr.x, 1024.f + zr.y);
+      };
+      if (!LOOKUP) load_group(a.gs == -1 ? 0 : c0 / a.gs);
+      // the reference rounds to fp16 first and casts to the module's dtype afterwards
+      auto each = [&](auto narrow, auto bf16) {
+#pragma unroll
+        for (int k = 0; k < 32; k += 2) {
+          unsigned w[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            if (LOOKUP) {
+              const int g = look[warp * 32 + k + i].y;
+              if (g != group) { group = g; load_group(g); }
+            }
+            __half2 h;
+            if (decltype(narrow)::value) {
+              const unsigned v = q2[k + i] | 0x64006400u;
+              h = __hmul2(s2, __hsub2(*reinterpret_cast<const __half2*>(&v), z2));
+            } else {
+              const float2 s = __half22float2(s2);
+              h = __floats2half2_rn(__fmul_rn(s.x, __fsub_rn((float)(q2[k + i] & 0xffffu), zr.x)),
+                                    __fmul_rn(s.y, __fsub_rn((float)(q2[k + i] >> 16), zr.y)));
+            }
+            if (decltype(bf16)::value) {
+              const float2 f = __half22float2(h);
+              const __nv_bfloat162 bb = __floats2bfloat162_rn(f.x, f.y);
+              w[i] = *reinterpret_cast<const unsigned*>(&bb);
+            } else w[i] = *reinterpret_cast<const unsigned*>(&h);
+          }
+          tw[fin_at(2 * lane, warp * 32 + k)] = __byte_perm(w[0], w[1], 0x5410);
+          tw[fin_at(2 * lane + 1, warp * 32 + k)] = __byte_perm(w[0], w[1], 0x7632);
+        }
+      };
+      if (BITS || a.narrow) {
+        if (a.bf16) each(std::true_type{}, std::true_type{});
+        else each(std::true_type{}, std::false_type{});
+      } else {
+        if (a.bf16) each(std::false_type{}, std::true_type{});
+        else each(std::false_type{}, std::false_type{});
       }
     }
   }
@@ -1268,6 +1303,8 @@ __global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
   if (!a.what && !a.codes) return;
   __syncthreads();
   const bool vec = ((a.ldwh | a.d) & 1) == 0 && (reinterpret_cast<uintptr_t>(a.what) & 3) == 0;
+  const bool vec_q = ((a.ldc | a.d) & 1) == 0 && (reinterpret_cast<uintptr_t>(a.codes) & 7) == 0;
+#pragma unroll 4
   for (int row = warp; row < FIN_ROWS; row += 4) {
     const int rr = r0 + row;
     if (rr >= a.out) break;
@@ -1287,19 +1324,26 @@ __global__ void __launch_bounds__(128) finish_kernel(FinishArgs a) {
       if (a.codes) {
         int* p = a.codes + (long long)rr * a.ldc + c;
         const unsigned v = tq[fin_at(row, k)];
-        p[0] = (int)(v & 0xffffu);
-        if (c + 1 < a.d) p[1] = (int)(v >> 16);
+        if (vec_q) *reinterpret_cast<int2*>(p) = make_int2((int)(v & 0xffffu), (int)(v >> 16));
+        else {
+          p[0] = (int)(v & 0xffffu);
+          if (c + 1 < a.d) p[1] = (int)(v >> 16);
+        }
       }
     }
   }
 }
 
+template <bool LOOKUP>
+void (*finish_of(int bits))(FinishArgs) {
+  return bits == 2 ? finish_kernel<2, LOOKUP> : bits == 3 ? finish_kernel<3, LOOKUP> : bits == 4 ? finish_kernel<4, LOOKUP>
+         : bits == 8 ? finish_kernel<8, LOOKUP> : finish_kernel<0, LOOKUP>;
+}
 int launch_finish(const FinishArgs& a, int bits, int batch, cudaStream_t stream) {
   const dim3 grid(oc_div_up(a.d, FIN_COLS), oc_div_up(a.out, FIN_ROWS), batch);
   const int smem = ((a.what ? 1 : 0) + (a.codes ? 1 : 0)) * FIN_TILE * 4;
-  void (*kernel)(FinishArgs) = bits == 2 ? finish_kernel<2> : bits == 3 ? finish_kernel<3> : bits == 4 ? finish_kernel<4>
-                               : bits == 8 ? finish_kernel<8> : finish_kernel<0>;
-  OC_LAUNCH(kernel, grid, 128, smem, stream, a);
+  const bool lookup = a.invperm || (a.gs != -1 && a.gs % 32 != 0) || a.d % 32 != 0;
+  OC_LAUNCH((lookup ? finish_of<true>(bits) : finish_of<false>(bits)), grid, 128, smem, stream, a);
   return OC_OK;
 }
 
@@ -1525,7 +1569,7 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   const long long prow = (wbits == 3) ? d / 32 * 3 : d / f;     // rows of one problem's packed weight
   if (qweight || codes || what) {
     FinishArgs f_args{codesT, out, d, invperm, groupsize, scales, zeros, qweight, ld_out, codes, d, what, ldwh, bf16,
-                      nCodes, nPar, prow * ld_out, (long long)out * d, (long long)out * ldwh};
+                      maxq < 256, nCodes, nPar, prow * ld_out, (long long)out * d, (long long)out * ldwh};
     const int rc = launch_finish(f_args, qweight ? wbits : 0, batch, stream);
     if (rc) return rc;
   }
