@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(320, 1)
 gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga) {
   using namespace octc;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_full[GROUP_STAGES], bar_empty[GROUP_STAGES], bar_err[SUPER], bar_acc[SUPER * SUPER];
+  __shared__ __align__(8) uint64_t bar_full[GROUP_STAGES], bar_empty[GROUP_STAGES], bar_err[SUPER], bar_acc[SUPER * SUPER], bar_u;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag_s;
   volatile int* abort_flag = &abort_flag_s;
@@ -756,6 +756,7 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
   if (tid == 0) {
     for (int s = 0; s < GROUP_STAGES; ++s) { mbar_init(smem_u32(&bar_full[s]), 1); mbar_init(smem_u32(&bar_empty[s]), 1); }
     for (int j = 0; j < SUPER; ++j) mbar_init(smem_u32(&bar_err[j]), 1);
+    mbar_init(smem_u32(&bar_u), 1);
     for (int j = 0; j < SUPER * SUPER; ++j) mbar_init(smem_u32(&bar_acc[j]), 1);
     abort_flag_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -850,13 +851,16 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
     float scale = 1.f, zero = 0.f;
     if (gs == -1 && live) { scale = a.scales[row]; zero = a.zeros[row]; }
     float wv[16], udiag = 0.f;
-    auto request = [&](int i1) {                        // what block i1 needs from global memory
-#pragma unroll
-      for (int it = 0; it < BLK * BLK / 4 / 256; ++it) {
-        const int e = it * 256 + tid, i = e / (BLK / 4), j4 = e % (BLK / 4);
-        if (4 * j4 + 3 >= i)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
-                       ::"r"(smem_u32(Us + i * BLK + 4 * j4)), "l"(a.U + (long long)(i1 + i) * a.ldu + i1 + 4 * j4) : "memory");
+    // What block i1 needs from global memory.  U's block comes in bulk copies, a row from its diagonal on each (the
+    // start rounded down to 16 bytes): 16 copies of 16 bytes by every thread took 2500 cycles of the chain.
+    constexpr uint32_t U_BYTES = 4 * 4 * (BLK / 4) * (BLK / 4 + 1) / 2 * 4;
+    auto expect_u = [&]() { mbar_expect_tx(smem_u32(&bar_u), U_BYTES); };       // one thread, before any copy
+    auto request = [&](int i1) {
+      if (lane < SUB) {
+        const int i = wid * SUB + lane, j = i & ~3;
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(smem_u32(Us + i * BLK + j)), "l"(a.U + (long long)(i1 + i) * a.ldu + i1 + j), "r"((BLK - j) * 4),
+                       "r"(smem_u32(&bar_u)) : "memory");
       }
 #pragma unroll
       for (int r = 0; r < 16; ++r) {
@@ -865,6 +869,8 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
       }
       if (tid < BLK) udiag = a.U[(long long)(i1 + tid) * a.ldu + i1 + tid];
     };
+    if (tid == 0) expect_u();
+    bar_windows();
     request(a.i1);
 
 #pragma unroll 1
@@ -884,7 +890,7 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
 #pragma unroll
       for (int r = 0; r < 16; ++r) tile[(quarter * 32 + lane) * 33 + half * 16 + r] = wv[r];
       if (tid < BLK) rdiag[tid] = safe_reciprocal(udiag);
-      asm volatile("cp.async.wait_all;" ::: "memory");
+      mbar_wait(smem_u32(&bar_u), t & 1, abort_flag, ga.status, 316);
       bar_windows();
       float w[SUB], mn = 0.f, mx = 0.f;
 #pragma unroll
@@ -919,8 +925,9 @@ gptq_group_kernel(const __grid_constant__ CUtensorMap map_u, const GroupArgs ga)
       for (int i = 0; i < SUB; ++i) mxe = fmaxf(mxe, oc_finite_abs(er[i]));
       bar_windows();                     // (the ranges have been read by all)
       mm_hi[wid * 32 + lane] = mxe;
-      bar_windows();
       const bool more = t + 1 < ga.blocks;
+      if (more && tid == 0) expect_u();
+      bar_windows();
       if (!more) oc_let_next();
       if (more) request(i1 + BLK);       // (nobody reads this block of U any more)
 #pragma unroll
