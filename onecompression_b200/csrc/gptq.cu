@@ -511,9 +511,11 @@ __device__ __forceinline__ bool produce_chunk(float (&w)[SUB], const float* __re
       er[i] = e;
       cd[i] = __fadd_rn(level, zero);
     }
-    es[c * 32] = er[i];
     propagate(w, i, er[i], ublk + i * BLK);
   }
+  // (not column by column: the loads of U would have to stay behind the stores)
+#pragma unroll
+  for (int c = 0; c < CHUNK; ++c) es[c * 32] = er[Q * CHUNK + c];
   return !bad;
 }
 
