@@ -771,7 +771,7 @@ extern "C" long long oc_hinv_workspace_bytes(int n) { return factor_ws_floats(n)
 
 // `count` problems of one level of the blocked inverse, for `batch` matrices: T21 = L21 X11, X21 = -X22 T21 with
 // X11, X22 of s and `rows` rows, the first at row and column r0, `step` entries apart.  T and X21 (unless no level
-// follows) are split into planes for the products that read them.
+// follows) leave as planes for the products that read them.
 static int invert_level_split(const FactorWs& ws, float* w0, int s, long long r0, int rows, int count, long long step,
                               int batch, long long sW, bool more, cudaStream_t stream) {
   const long long ld = ws.ld, mid = r0 + s, at = mid * ld + r0;
@@ -791,29 +791,25 @@ static int invert_level_split(const FactorWs& ws, float* w0, int s, long long r0
     const long long t = o.scale_k; o.scale_k = o.scale_r; o.scale_r = t;
     return o;
   };
-  auto split_block = [&](const float* src, __half* planes, float* table) {
-    OcSplitArgs a{};
-    a.src = src + at; a.ld = ld; a.rows = rows; a.cols = s;
-    a.planes = planes + at; a.plane = ws.mat; a.ldp = ld; a.table = table + tab_at; a.ldt = nblk;
-    a.nb1 = count; a.nb2 = batch;
-    a.src1 = a.dst1 = step; a.src2 = sW; a.dst2 = 2 * sW; a.tab1 = tab_step; a.tab2 = sW;
-    return oc_split_launch(a, stream);
+  auto goes_on = [&](OcSplitGemm& g, __half* planes, float* table, int only) {
+    g.out.mode = OC_SPLIT_OUT_BLOCKS; g.out.only = only;
+    g.out.planes = planes + at; g.out.plane = ws.mat; g.out.ld = ld; g.out.table = table + tab_at; g.out.ldt = nblk;
+    g.out.stride1 = step; g.out.stride2 = 2 * sW; g.out.tab1 = tab_step; g.out.tab2 = sW;
   };
   OcSplitGemm g{};
   g.ldc = ld; g.strideC1 = step; g.strideC2 = sW; g.nb1 = count; g.nb2 = batch; g.M = rows; g.N = s;
   g.A = operand(ws.planesL(w0), mid, r0, nullptr);
   g.B = stored_by_k(operand(ws.planesX(w0), r0, r0, ws.tableX(w0)));
   g.C = ws.T(w0) + at; g.K = s; g.alpha = 1.f / L_SCALE; g.flags = OC_GEMM_KLO_FROM_N;
-  int rc = oc_gemm_split_launch(g, stream);
-  if (rc) return rc;
-  rc = split_block(ws.T(w0), ws.planesT(w0), ws.tableT(w0));
+  goes_on(g, ws.planesT(w0), ws.tableT(w0), 1);
+  const int rc = oc_gemm_split_launch(g, stream);
   if (rc) return rc;
   g.A = operand(ws.planesX(w0), mid, mid, ws.tableX(w0));
   g.B = stored_by_k(operand(ws.planesT(w0), mid, r0, ws.tableT(w0)));
   g.C = ws.X(w0) + at; g.K = rows; g.alpha = -1.f; g.flags = OC_GEMM_KHI_FROM_M;
-  rc = oc_gemm_split_launch(g, stream);
-  if (rc || !more) return rc;
-  return split_block(ws.X(w0), ws.planesX(w0), ws.tableX(w0));
+  if (more) goes_on(g, ws.planesX(w0), ws.tableX(w0), 0);
+  else g.out = OcSplitOut{};
+  return oc_gemm_split_launch(g, stream);
 }
 
 // Factorisation of `batch` matrices of equal size laid out one after another (H [batch, n, ldh],

@@ -12,7 +12,7 @@
 //   warps 4..11 drain: accumulators leave TMEM every 128 k-values, are scaled by the powers of two of the blocks
 //               that were multiplied and summed in registers (the tensor core truncates when it
 //               accumulates, so chains are short); at the end of a tile they leave through shared memory as TMA
-//               stores (beta 0) or TMA reductions in L2 (beta 1).
+//               stores (beta 0) or TMA reductions in L2 (beta 1), or split again for the next product.
 // Tiles are 128 x 256 (4 stages of 48 KB) or 128 x 128 (6 stages of 32 KB).  Both cut k into the same chains on
 // the same grid of 128, so a product gives the same bits with either.
 // Operands may be stored [rows, K] or [K, rows]; both are native layouts.
@@ -50,6 +50,9 @@ struct Params {
   const float *a_scale, *b_scale;
   long long a_sk, a_sr, a_s1, a_s2, b_sk, b_sr, b_s1, b_s2;
   int a_row;
+  int out_mode, store_c;         // planes of the result (wide tiles only)
+  float* o_table;
+  long long o_ldt, o_t1, o_t2;
   int* status;
 };
 
@@ -84,6 +87,12 @@ __device__ __forceinline__ void tma_store(const CUtensorMap* map, uint32_t src, 
   else
     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
                  ::"l"(map), "r"(x), "r"(y), "r"(z1), "r"(z2), "r"(src) : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ void tma_store_plane(const CUtensorMap* map, uint32_t src, int x, int y, int z1, int z2, int plane) {
+  asm volatile("cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4, %5}], [%6];"
+               ::"l"(map), "r"(x), "r"(y), "r"(z1), "r"(z2), "r"(plane), "r"(src) : "memory");
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
@@ -146,12 +155,13 @@ __device__ __forceinline__ bool upper_half_in_use(const Params& p, const Tile& t
 template <bool A_MN, bool B_MN, class S>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ CUtensorMap map_c, const Params p) {
+                  const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_o, const Params p) {
   constexpr int BN = S::BN, STAGES = S::STAGES, STAGE_BYTES = S::STAGE_BYTES, A_BYTES = S::A_BYTES, DW = S::DW;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full[2], bar_acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag_s;
+  __shared__ float block_max[2][2][4];           // [tile & 1][half][quarter]
   volatile int* abort_flag = &abort_flag_s;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -259,6 +269,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     uint8_t* stg_ptr = stage_ptr + STAGES * STAGE_BYTES + (warp - FIRST_DRAIN) * 4096;
     const uint32_t stg = smem_u32(stg_ptr);
     uint32_t cc = 0;
+    int tiles = 0;
     bool ok = true;
     while (walk.next(p, t)) {
       const int n_stages = max(0, (t.k_hi - t.k_lo + BK - 1) / BK);
@@ -301,22 +312,70 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       }
       if (!ok) break;
       if (!in_use) continue;
+      if (BN == 128 || p.store_c) {
 #pragma unroll
-      for (int c = 0; c < DW / 32; ++c) {
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        __syncwarp();
+        for (int c = 0; c < DW / 32; ++c) {
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float* v = acc + c * 32 + j * 4;
-          // (16-byte chunks in the order of the 128-byte swizzle: free of bank conflicts)
-          *reinterpret_cast<float4*>(stg_ptr + lane * 128 + ((j ^ (lane & 7)) * 16)) =
-              make_float4(p.alpha * v[0], p.alpha * v[1], p.alpha * v[2], p.alpha * v[3]);
+          for (int j = 0; j < 8; ++j) {
+            const float* v = acc + c * 32 + j * 4;
+            // (16-byte chunks in the order of the 128-byte swizzle: free of bank conflicts)
+            *reinterpret_cast<float4*>(stg_ptr + lane * 128 + ((j ^ (lane & 7)) * 16)) =
+                make_float4(p.alpha * v[0], p.alpha * v[1], p.alpha * v[2], p.alpha * v[3]);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0 && row0 < p.M && col0 + c * 32 < p.N)
+            tma_store(&map_c, stg, col0 + c * 32, row0, t.z1, t.z2, p.add);
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0 && row0 < p.M && col0 + c * 32 < p.N)
-          tma_store(&map_c, stg, col0 + c * 32, row0, t.z1, t.z2, p.add);
       }
+      if (BN == 256 && p.out_mode) {
+        // The result as the next product's operand.  A thread has one row of a block of 128 columns, the four warps of a
+        // half its 128 rows.  As a pass of its own this read and wrote 8 bytes an entry: correction of 4096 x 4096
+        // 858 -> 821 us.
+        float mx = 0.f, inv;
+#pragma unroll
+        for (int i = 0; i < DW; ++i) { acc[i] *= p.alpha; mx = fmaxf(mx, oc_finite_abs(acc[i])); }
+        if (p.out_mode == OC_SPLIT_OUT_BLOCKS) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+          float* red = block_max[tiles & 1][half];
+          if (lane == 0) red[quarter] = mx;
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+          mx = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
+        }
+        const float se = oc_split_scale(mx, inv);
+        float* tab = p.o_table + t.z1 * p.o_t1 + t.z2 * p.o_t2;
+        if (col0 < p.N) {
+          if (p.out_mode == OC_SPLIT_OUT_BLOCKS) {
+            if (lane == 0 && quarter == 0) tab[(long long)(t.m0 / 128) * p.o_ldt + col0 / 128] = inv;
+          } else if (row0 + lane < p.M) {
+            tab[(long long)(col0 / 128) * p.o_ldt + row0 + lane] = inv;
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+          for (int pl = 0; pl < 2; ++pl) {         // 32 rows x 64 columns of a plane
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const float* v = acc + (DW == 128 ? c * 64 + j * 8 : 0);
+              uint2 h0, l0, h1, l1;
+              oc_split4(make_float4(v[0] * se, v[1] * se, v[2] * se, v[3] * se), h0, l0);
+              oc_split4(make_float4(v[4] * se, v[5] * se, v[6] * se, v[7] * se), h1, l1);
+              *reinterpret_cast<uint4*>(stg_ptr + lane * 128 + ((j ^ (lane & 7)) * 16)) =
+                  pl ? make_uint4(l0.x, l0.y, l1.x, l1.y) : make_uint4(h0.x, h0.y, h1.x, h1.y);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0 && row0 < p.M && col0 + c * 64 < p.N)
+              tma_store_plane(&map_o, stg, col0 + c * 64, row0, t.z1, t.z2, pl);
+          }
+      }
+      ++tiles;
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     __syncwarp();
@@ -344,10 +403,24 @@ int make_map_c(CUtensorMap* map, const OcSplitGemm& g) {
   return OC_OK;
 }
 
+int make_map_out(CUtensorMap* map, const OcSplitGemm& g) {
+  EncodeTiledFn enc = get_encode_fn();
+  const OcSplitOut& o = g.out;
+  const cuuint64_t whole = (cuuint64_t)g.M * (cuuint64_t)o.ld * 2;
+  cuuint64_t dims[5] = {(cuuint64_t)g.N, (cuuint64_t)g.M, (cuuint64_t)g.nb1, (cuuint64_t)g.nb2, 2};
+  cuuint64_t strides[4] = {(cuuint64_t)o.ld * 2, g.nb1 > 1 ? (cuuint64_t)o.stride1 * 2 : whole,
+                           g.nb2 > 1 ? (cuuint64_t)o.stride2 * 2 : whole, (cuuint64_t)o.plane * 2};
+  cuuint32_t box[5] = {64, 32, 1, 1, 1}, estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 5, o.planes, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { oc_set_last_error("split gemm: cuTensorMapEncodeTiled failed"); return OC_ERR_CUDA; }
+  return OC_OK;
+}
+
 template <bool A_MN, bool B_MN, class S>
-int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const Params& p, int grid, cudaStream_t s) {
+int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mc, const CUtensorMap& mo, const Params& p, int grid, cudaStream_t s) {
   OC_OPT_IN_SMEM((gemm_split_kernel<A_MN, B_MN, S>), S::SMEM_DYN);
-  OC_LAUNCH((gemm_split_kernel<A_MN, B_MN, S>), grid, THREADS, S::SMEM_DYN, s, ma, mb, mc, p);
+  OC_LAUNCH((gemm_split_kernel<A_MN, B_MN, S>), grid, THREADS, S::SMEM_DYN, s, ma, mb, mc, mo, p);
   return OC_OK;
 }
 
@@ -362,13 +435,18 @@ long long tiles_of(const OcSplitGemm& g) {
 
 template <class S>
 int launch_shape(const OcSplitGemm& g, const OcGemmDevice& dev, cudaStream_t stream) {
-  CUtensorMap ma, mb, mc;
+  CUtensorMap ma, mb, mc, mo;
   int rc = make_split_map(&ma, g.A, g.M, g.K, g.nb1, g.nb2, BM);
   if (rc) return rc;
   rc = make_split_map(&mb, g.B, g.N, g.K, g.nb1, g.nb2, S::BN);
   if (rc) return rc;
   rc = make_map_c(&mc, g);
   if (rc) return rc;
+  mo = mc;
+  if (S::BN == 256 && g.out.mode) {
+    rc = make_map_out(&mo, g);
+    if (rc) return rc;
+  }
   Params p{};
   p.C = g.C; p.ldc = g.ldc; p.strideC1 = g.strideC1; p.strideC2 = g.strideC2;
   p.M = g.M; p.N = g.N; p.K = g.K; p.nb1 = g.nb1; p.nb2 = g.nb2;
@@ -378,14 +456,16 @@ int launch_shape(const OcSplitGemm& g, const OcGemmDevice& dev, cudaStream_t str
   p.a_scale = g.A.scale; p.a_sk = g.A.scale_k; p.a_sr = g.A.scale_r; p.a_s1 = g.A.scale1; p.a_s2 = g.A.scale2;
   p.a_row = g.A.scale_row;
   p.b_scale = g.B.scale; p.b_sk = g.B.scale_k; p.b_sr = g.B.scale_r; p.b_s1 = g.B.scale1; p.b_s2 = g.B.scale2;
+  p.out_mode = g.out.mode; p.store_c = !(g.out.mode && g.out.only);
+  p.o_table = g.out.table; p.o_ldt = g.out.ldt; p.o_t1 = g.out.tab1; p.o_t2 = g.out.tab2;
   p.status = dev.status;
   const long long per = tiles_of<S::BN>(g), items = per * g.nb1 * g.nb2;
   OC_REQUIRE(items < (1ll << 30), "split gemm: too many tiles");
   p.per_problem = (int)per;
   const int grid = (int)(items < dev.sms ? items : dev.sms);
   if (g.A.mn_major)
-    return g.B.mn_major ? launch<true, true, S>(ma, mb, mc, p, grid, stream) : launch<true, false, S>(ma, mb, mc, p, grid, stream);
-  return g.B.mn_major ? launch<false, true, S>(ma, mb, mc, p, grid, stream) : launch<false, false, S>(ma, mb, mc, p, grid, stream);
+    return g.B.mn_major ? launch<true, true, S>(ma, mb, mc, mo, p, grid, stream) : launch<true, false, S>(ma, mb, mc, mo, p, grid, stream);
+  return g.B.mn_major ? launch<false, true, S>(ma, mb, mc, mo, p, grid, stream) : launch<false, false, S>(ma, mb, mc, mo, p, grid, stream);
 }
 
 // Time of a wide tile against a narrow one.
@@ -401,8 +481,10 @@ int oc_gemm_split_launch(const OcSplitGemm& g, cudaStream_t stream) {
   };
   OC_REQUIRE(g.K > 0 && fits(g.A) && fits(g.B) && g.B.terms == 2 && (g.A.terms == 2 || !g.A.mn_major), "split gemm: bad operand");
   OC_REQUIRE(al(g.C) && g.ldc % 4 == 0 && g.strideC1 % 4 == 0 && g.strideC2 % 4 == 0, "split gemm: C is not 16-byte aligned");
+  OC_REQUIRE(!g.out.mode || (!g.add && !(g.flags & OC_GEMM_SKIP_UPPER_TILES) && al(g.out.planes) && g.out.ld % 8 == 0 &&
+                             g.out.plane % 8 == 0 && g.out.stride1 % 8 == 0 && g.out.stride2 % 8 == 0), "split gemm: bad output");
   OcGemmDevice dev;
-  const int rc = oc_gemm_device(dev);
+  int rc = oc_gemm_device(dev);
   if (rc) return rc;
   int shape = dev.tile_shape;
   if (shape == 0) {
@@ -411,7 +493,16 @@ int oc_gemm_split_launch(const OcSplitGemm& g, cudaStream_t stream) {
     const double wide = WIDE_TILE_COST * (double)((tiles_of<256>(g) * nb + sms - 1) / sms);
     shape = wide < narrow ? 2 : 1;
   }
-  return shape == 2 ? launch_shape<Wide>(g, dev, stream) : launch_shape<Narrow>(g, dev, stream);
+  if (shape == 2) return launch_shape<Wide>(g, dev, stream);
+  rc = launch_shape<Narrow>(g, dev, stream);
+  if (rc || !g.out.mode) return rc;
+  // (a drain thread of a narrow tile has half of a block's columns: a pass of its own)
+  OcSplitArgs s{};
+  s.src = g.C; s.ld = g.ldc; s.rows = g.M; s.cols = g.N; s.nb1 = g.nb1; s.nb2 = g.nb2;
+  s.planes = g.out.planes; s.plane = g.out.plane; s.ldp = g.out.ld; s.table = g.out.table; s.ldt = g.out.ldt;
+  s.per_row = g.out.mode == OC_SPLIT_OUT_ROWS;
+  s.src1 = g.strideC1; s.src2 = g.strideC2; s.dst1 = g.out.stride1; s.dst2 = g.out.stride2; s.tab1 = g.out.tab1; s.tab2 = g.out.tab2;
+  return oc_split_launch(s, stream);
 }
 
 // ---- C entry for the tests --------------------------------------------------------------------------

@@ -135,15 +135,15 @@ long long round4(long long x) { return (x + 3) / 4 * 4; }
 long long round8(long long x) { return (x + 7) / 8 * 8; }
 long long blocks(long long x) { return (x + OC_SPLIT_BLOCK - 1) / OC_SPLIT_BLOCK; }
 
-// Workspace with split operands: the left operand's planes, an fp32 result, the planes of C (later those of U), and
-// their tables.
+// Workspace with split operands: planes of the left operands, in turn (a product reads one and writes the other), an
+// fp32 result, the planes of C (later those of U), and their tables.
 struct QepWs {
-  long long ld, planes, result, right, tab_rows, tab, total;
+  long long ld, left, right, tab_rows, tab, total;
   QepWs(int out, int d) {
     ld = round8(d);
-    planes = 4 * (long long)out * ld; result = 4 * (long long)out * ld; right = 4 * (long long)d * ld;
+    left = 4 * (long long)out * ld; right = 4 * (long long)d * ld;
     tab_rows = round8(blocks(d) * out) * 4; tab = round8(blocks(d) * blocks(d)) * 4;
-    total = planes + result + right + tab_rows + tab;
+    total = 3 * left + right + 2 * tab_rows + tab;
   }
 };
 
@@ -152,48 +152,59 @@ int split_products(const void* W, long long ldw_io, int out, int d, const float*
                    long long ldu, const int* perm, const unsigned char* dead, int bf16, int vec, char* workspace,
                    float*& delta, cudaStream_t stream) {
   const QepWs ws(out, d);
-  __half* Lp = (__half*)workspace;
-  float* R = (float*)(workspace + ws.planes);
-  __half* Rp = (__half*)(workspace + ws.planes + ws.result);
-  float* tabL = (float*)(workspace + ws.planes + ws.result + ws.right);
-  float* tabR = (float*)(workspace + ws.planes + ws.result + ws.right + ws.tab_rows);
-  const long long nb = blocks(d);
+  __half* Lp[2] = {(__half*)workspace, (__half*)(workspace + ws.left)};
+  float* R = (float*)(workspace + 2 * ws.left);
+  __half* Rp = (__half*)(workspace + 3 * ws.left);
+  char* tabs = workspace + 3 * ws.left + ws.right;
+  float* tabL[2] = {(float*)tabs, (float*)(tabs + ws.tab_rows)};
+  float* tabR = (float*)(tabs + 2 * ws.tab_rows);
+  const long long nb = blocks(d), plane_l = out * ws.ld, plane_r = d * ws.ld;
   delta = R;
-  OC_LAUNCH(qep_plane_kernel, dim3((int)nb, oc_div_up(out, 8)), 256, 0, stream, W, ldw_io, out, d, dead, Lp, ws.ld, tabL, bf16, vec);
+  OC_LAUNCH(qep_plane_kernel, dim3((int)nb, oc_div_up(out, 8)), 256, 0, stream, W, ldw_io, out, d, dead, Lp[0], ws.ld, tabL[0], bf16, vec);
   OcSplitArgs right{};
-  right.rows = right.cols = d; right.planes = Rp; right.plane = d * ws.ld; right.ldp = ws.ld; right.table = tabR;
+  right.rows = right.cols = d; right.planes = Rp; right.plane = plane_r; right.ldp = ws.ld; right.table = tabR;
   right.ldt = nb; right.nb1 = right.nb2 = 1;
   right.src = C; right.ld = ldc;
   int rc = oc_split_launch(right, stream);
   if (rc) return rc;
-  OcSplitArgs left{};
-  left.src = R; left.ld = ws.ld; left.rows = out; left.cols = d; left.planes = Lp; left.plane = out * ws.ld;
-  left.ldp = ws.ld; left.table = tabL; left.ldt = out; left.per_row = 1; left.nb1 = left.nb2 = 1;
   OcSplitGemm g{};
   g.C = R; g.ldc = ws.ld; g.M = out; g.N = d; g.K = d; g.nb1 = g.nb2 = 1; g.alpha = 1.f;
-  g.A.planes = Lp; g.A.plane = left.plane; g.A.ld = ws.ld; g.A.scale_k = out; g.A.scale_r = OC_SPLIT_BLOCK; g.A.scale_row = 1;
-  g.B.planes = Rp; g.B.plane = right.plane; g.B.ld = ws.ld; g.B.terms = 2; g.B.scale = tabR;
+  g.A.plane = plane_l; g.A.ld = ws.ld; g.A.scale_k = out; g.A.scale_r = OC_SPLIT_BLOCK; g.A.scale_row = 1;
+  g.B.planes = Rp; g.B.plane = plane_r; g.B.ld = ws.ld; g.B.terms = 2; g.B.scale = tabR;
+  auto left = [&](int i) { g.A.planes = Lp[i]; g.A.scale = tabL[i]; };
+  auto goes_on = [&](int i) {      // the result is the next left operand
+    g.out.mode = OC_SPLIT_OUT_ROWS; g.out.only = 1; g.out.planes = Lp[i]; g.out.plane = plane_l; g.out.ld = ws.ld;
+    g.out.table = tabL[i]; g.out.ldt = out;
+  };
   // R = Wz C
-  g.A.terms = 1; g.A.scale = bf16 ? tabL : nullptr;
+  left(0);
+  g.A.terms = 1;
+  if (!bf16) g.A.scale = nullptr;
   g.B.mn_major = 1; g.B.scale_k = nb; g.B.scale_r = 1;
+  if (!perm) goes_on(1);
   rc = oc_gemm_split_launch(g, stream);
   if (rc) return rc;
+  if (perm) {
+    OcSplitArgs s{};
+    s.src = R; s.ld = ws.ld; s.perm = perm; s.rows = out; s.cols = d; s.planes = Lp[1]; s.plane = plane_l; s.ldp = ws.ld;
+    s.table = tabL[1]; s.ldt = out; s.per_row = 1; s.nb1 = s.nb2 = 1;
+    rc = oc_split_launch(s, stream);
+    if (rc) return rc;
+  }
   // T = R P^T U^T      (U upper: U[n][k] = 0 for k < n)
   right.src = U; right.ld = ldu; right.region = OC_SPLIT_UPPER;
   rc = oc_split_launch(right, stream);
   if (rc) return rc;
-  left.perm = perm;
-  rc = oc_split_launch(left, stream);
-  if (rc) return rc;
-  g.A.terms = 2; g.A.scale = tabL;
+  left(1);
+  g.A.terms = 2;
   g.B.mn_major = 0; g.B.scale_k = 1; g.B.scale_r = nb; g.flags = OC_GEMM_KLO_FROM_N;
+  goes_on(0);
   rc = oc_gemm_split_launch(g, stream);
   if (rc) return rc;
   // dW P^T = T U       (U[k][n] = 0 for k > n)
-  left.perm = nullptr;
-  rc = oc_split_launch(left, stream);
-  if (rc) return rc;
+  left(0);
   g.B.mn_major = 1; g.B.scale_k = nb; g.B.scale_r = 1; g.flags = OC_GEMM_KHI_FROM_N;
+  g.out = OcSplitOut{};
   return oc_gemm_split_launch(g, stream);
 }
 

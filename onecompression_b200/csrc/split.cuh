@@ -62,6 +62,16 @@ struct OcSplitOperand {
   long long stride1, stride2, scale1, scale2;    // between the problems of the two batch dimensions
 };
 
+// Where a result goes on as an operand: its planes and table as oc_split_launch writes them, beside C or instead of it.
+enum : int { OC_SPLIT_OUT_NONE = 0, OC_SPLIT_OUT_ROWS = 1, OC_SPLIT_OUT_BLOCKS = 2 };
+struct OcSplitOut {
+  int mode;                                      // none, every row of a block scaled for itself, blocks
+  int only;                                      // C is scratch: nobody reads it
+  __half* planes; long long plane, ld;
+  float* table; long long ldt;
+  long long stride1, stride2, tab1, tab2;
+};
+
 // C[M,N] = alpha * A * B^T, or C += alpha * A * B^T (add), A [M,K], B [N,K] (logical); flags as in OcGemm.
 // C is written by TMA in 16-byte pieces: up to three columns behind the last one of a row are overwritten.
 struct OcSplitGemm {
@@ -70,6 +80,7 @@ struct OcSplitGemm {
   int M, N, K, nb1, nb2;
   float alpha;
   int add, flags;
+  OcSplitOut out;              // (not with add or lower tiles only)
 };
 int oc_gemm_split_launch(const OcSplitGemm& g, cudaStream_t stream);
 

@@ -115,3 +115,25 @@ def test_column_loop(out, d, gs, act):
     alone = K.gptq_quantize(w[r:r + 1].contiguous(), f, 4, gs, False, pack=False, want_codes=True)
     assert torch.equal(alone["codes"][0], new["codes"][r])
     assert K.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("n", [257, 640, 1027, 1160])
+def test_tile_shapes_give_the_same_bits(n):
+    """Wide tiles write a result that goes on as an operand as planes themselves, narrow ones leave that to a pass of its
+    own: the same values, whatever the workspace held."""
+    h = moment(n, 11)
+    f = as_factor(factor64(h, 0.01, torch.arange(n, device="cuda")), h)
+    w = torch.randn(333, n, generator=gen(12), device="cuda") * 0.02
+    c = 0.02 * h + 0.01 * torch.randn(n, n, generator=gen(13), device="cuda") / n**0.5
+    got = {}
+    for shape in (1, 2):
+        old = K.set_gemm_tile_shape(shape)
+        try:
+            K._workspace(1 << 26, w.device).fill_(0xff)
+            got[shape] = [K.factor_hessian(h, 0.01, False).u, K.factor_hessians_batched(torch.stack([h, h * 3]), 0.01, True)["u"]]
+            got[shape] += [K.qep_adjust(w.to(t), c, f, 0.5) for t in (torch.float16, torch.bfloat16)]
+        finally:
+            K.set_gemm_tile_shape(old)
+    for a, b in zip(got[1], got[2]):
+        assert torch.equal(a, b) and a.isfinite().all()
+    assert K.gemm_tc_status() == 0
