@@ -116,7 +116,8 @@ int oc_mirror_upper(float* M, long long ld, int n, void* stream);
  * Outputs: U [n,n] (ldu), perm/invperm int32 [n], dead uint8 [n] (original column
  * order), damp_out float[2] = {percdamp*mean, mean}, status int = 0 or (index+1) of
  * the first non-positive pivot (then U is meaningless: add damping and call again,
- * as the reference's retry loop does; reuse_perm = 1 keeps perm/invperm).
+ * as the reference's retry loop does; reuse_perm = 1 keeps perm/invperm), or minus the code of oc_gemm_tc_status()
+ * when a bounded wait of a tensor-core product has expired on the device (U is invalid, more damping is no help).
  */
 long long oc_hinv_workspace_bytes(int n);
 int oc_hinv_factor(const float* H, long long ldh, int n, float percdamp, float rel_shift,

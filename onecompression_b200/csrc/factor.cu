@@ -170,10 +170,13 @@ __global__ void __launch_bounds__(256) build_reversed_kernel(
 // 619 us, 183 us now; 4096 50, 14 us.
 __global__ void __launch_bounds__(256) reverse_upper_kernel(const float* __restrict__ X, long long ldx, int n,
                                                             const float* __restrict__ equil_p, float* __restrict__ U,
-                                                            long long ldu, long long sW, long long sU, int vec) {
+                                                            long long ldu, long long sW, long long sU, int vec,
+                                                            const int* __restrict__ gemm_status, int* __restrict__ status) {
   oc_wait_before();
   oc_let_next();
   const int i = blockIdx.x;
+  // an expired wait in a product makes the factor as invalid as a bad pivot does
+  if (i == 0 && threadIdx.x == 0 && *gemm_status) atomicCAS(status + blockIdx.y, 0, -*gemm_status);
   const float* x = X + (long long)blockIdx.y * sW + (long long)(n - 1 - i) * ldx;
   float* u = U + (long long)blockIdx.y * sU + (long long)i * ldu;
   equil_p += (long long)blockIdx.y * sW;
@@ -961,7 +964,9 @@ static int hinv_factor_impl(int batch, const float* H, long long ldh, int n, flo
     }
   }
   const bool vec_u = n % 4 == 0 && ldu % 4 == 0 && sU % 4 == 0 && aligned(U) && aligned(X);
-  OC_LAUNCH(reverse_upper_kernel, dim3(n, batch), 256, 0, stream, X, ld, n, equil_p, U, ldu, sW, sU, vec_u);
+  OcGemmDevice dev;
+  if (const int rc = oc_gemm_device(dev)) return rc;
+  OC_LAUNCH(reverse_upper_kernel, dim3(n, batch), 256, 0, stream, X, ld, n, equil_p, U, ldu, sW, sU, vec_u, dev.status, status);
   return OC_OK;
 }
 

@@ -294,8 +294,10 @@ def factor_hessian(h: torch.Tensor, percdamp: float, actorder: bool, max_retries
                 1 if actorder else 0, 1 if attempt > 0 else 0, ptr(u), d, ptr(perm), ptr(invperm),
                 ptr(dead), ptr(damp), ptr(status), ptr(ws), ws.numel(), stream_handle(),
             )
-            if int(status.item()) == 0:
-                check_gemm_status()
+            code = int(status.item())
+            if code < 0:
+                _raise_gemm_status(-code)
+            if code == 0:
                 return HessianFactor(u, perm, invperm, dead, damp, bool(actorder), float(percdamp),
                                      rel, attempt + 1)
             mult *= 10.0
@@ -927,7 +929,11 @@ def check_gemm_status():
     where the host has synchronised anyway."""
     code = gemm_tc_status()
     if code != 0:
-        raise RuntimeError(f"fp32 tensor-core product: a bounded pipeline wait expired (code {code})")
+        _raise_gemm_status(code)
+
+
+def _raise_gemm_status(code):
+    raise RuntimeError(f"fp32 tensor-core product: a bounded pipeline wait expired (code {code})")
 
 
 def gemm_f32(a, b, c=None, alpha=1.0, beta=0.0, trans_a=False, trans_b=False, flags=0):

@@ -137,3 +137,28 @@ def test_tile_shapes_give_the_same_bits(n):
     for a, b in zip(got[1], got[2]):
         assert torch.equal(a, b) and a.isfinite().all()
     assert K.gemm_tc_status() == 0
+
+
+def test_an_expired_wait_is_not_retried(monkeypatch):
+    """A negative status is a product whose pipeline gave up, not a bad pivot: more damping is no help.  (The status is
+    planted behind the call; no kernel waits here.)"""
+    planted, calls = [], []
+    empty, call = torch.empty, K.call
+
+    def remembers(*args, **kw):
+        t = empty(*args, **kw)
+        if t.dtype == torch.int32 and t.numel() == 1:
+            planted.append(t)
+        return t
+
+    def plants(name, *args):
+        calls.append(name)
+        rc = call(name, *args)
+        planted[-1].fill_(-204)
+        return rc
+
+    monkeypatch.setattr(K.torch, "empty", remembers)
+    monkeypatch.setattr(K, "call", plants)
+    with pytest.raises(RuntimeError, match="bounded pipeline wait expired .code 204."):
+        K.factor_hessian(moment(256, 1), 0.01, False)
+    assert calls == ["oc_hinv_factor"]
