@@ -162,3 +162,46 @@ def test_an_expired_wait_is_not_retried(monkeypatch):
     with pytest.raises(RuntimeError, match="bounded pipeline wait expired .code 204."):
         K.factor_hessian(moment(256, 1), 0.01, False)
     assert calls == ["oc_hinv_factor"]
+
+
+def test_under_capture():
+    """The chains of dependent launches as a graph, behind a join of two streams and a copy: the bits of the plain calls."""
+    n, out = 640, 200
+    x = torch.randn(300, n, generator=gen(21), device="cuda").half()
+    w = (torch.randn(out, n, generator=gen(22), device="cuda") * 0.02).half()
+    c = torch.randn(n, n, generator=gen(23), device="cuda") / n
+    host = torch.randn(n, n, generator=torch.Generator().manual_seed(24)).pin_memory()
+    noise = torch.empty(n, n, device="cuda")
+    side, other = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def body():
+        here = torch.cuda.current_stream()
+        acc = K.MomentAccumulator(n, "cuda")
+        acc.add(x)
+        h = acc.finalize(check=False)[0]
+        other.wait_stream(here)
+        with torch.cuda.stream(other):
+            noise.copy_(host, non_blocking=True)
+            e = noise * 1e-3
+        here.wait_stream(other)
+        h = h + torch.diag(e.diagonal().abs())
+        p = K.factor_hessian_launch(h, 0.01, True)
+        f = K.HessianFactor(p["u"], p["perm"], p["invperm"], p["dead"], p["damp"], True, 0.01, 1.0, 1)
+        v = K.qep_adjust(w.clone(), c, f, 0.5)
+        q = K.gptq_quantize(v, f, 4, 128, False, want_codes=True)
+        return [h, f.u, f.perm, v, p["status"]] + [q[k] for k in sorted(q)]
+
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        want = [t.clone() for t in body()]
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            got = body()
+        for _ in range(3):
+            for t in got:
+                t.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert K.gemm_tc_status() == 0
