@@ -3,7 +3,7 @@
 // GPTQResult.compute_dequantized_weight, onecomp/quantizer/gptq/_gptq.py:84-168).
 // The column loop packs its own results; these entry points serve the callers
 // that hold integer codes or a packed result already.
-#include "common.cuh"
+#include "packed_field.cuh"
 
 namespace {
 
@@ -81,8 +81,10 @@ __global__ void unpack_axis_kernel(const int* __restrict__ in, long long in_stri
 // decodes 32 columns of one row (neighbouring lanes hold neighbouring rows, so the packed words,
 // scales and zero points load coalesced; each word is read once, and scale and zero only where the
 // group changes from one column to the next), and the tile leaves through shared memory in
-// 256-byte row segments.  14336 x 4096, 4 bits: 306 us with one word, scale and zero load per weight,
-// 56 us now (2.6 TB/s; the caller's launch and L2 flush included).
+// 256-byte row segments.  Eight columns of one group are decoded as pairs of fp16 (as in packed_linear.cu: q | 0x6400 is
+// 1024 + q, the subtraction is exact and the product rounds once, the same values): in fp32, one weight
+// after the other, issue slots bound it.  14336 x 4096, 4 bits: 54 -> 37 us
+// of kernel time, cold L2; 4096 x 14336, 3 bits: 54 -> 37 us (act-order, column by column: 106 -> 107 us).
 constexpr int DQ_ROWS = 64, DQ_COLS = 128, DQ_PITCH = DQ_COLS + 8;   // pitch: 16-byte accesses without conflicts
 template <int BITS>
 __global__ void __launch_bounds__(256) dequant_packed_kernel(const int* __restrict__ qweight,
@@ -102,34 +104,65 @@ __global__ void __launch_bounds__(256) dequant_packed_kernel(const int* __restri
     for (int j = 0; j < BITS; ++j) v[j] = j < words ? (unsigned)qweight[(w0 + j) * out + r] : 0u;
     int group = -1;
     float s = 0.f, z = 0.f;
+    auto load_group = [&](int g) {
+      if (g == group) return;
+      group = g;
+      s = __half2float(scales[(long long)g * out + r]);
+      unsigned zq;
+      if (BITS == 3) {
+        const int zb = 3 * (r & 31), zw = zb >> 5, zo = zb & 31;
+        const int* zr = qzeros + (long long)g * ldz + (r / 32) * 3;
+        zq = (unsigned)zr[zw] >> zo;
+        if (zo + 3 > 32) zq |= (unsigned)zr[zw + 1] << (32 - zo);
+      } else {
+        constexpr int F = 32 / (BITS == 3 ? 4 : BITS);
+        zq = (unsigned)qzeros[(long long)g * ldz + r / F] >> ((r % F) * BITS);
+      }
+      z = (float)(((zq & MASK) + 1u) & MASK);
+    };
+    const bool wide_idx = (reinterpret_cast<uintptr_t>(g_idx) & 15) == 0;
 #pragma unroll
     for (int k8 = 0; k8 < 4; ++k8) {
       __align__(16) __half h[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int k = k8 * 8 + i, c = c0 + k, bit = k * BITS, wi = bit >> 5, off = bit & 31;
-        if (c < d) {
-          const int g = g_idx ? g_idx[c] : 0;
-          if (g != group) {
-            group = g;
-            s = __half2float(scales[(long long)g * out + r]);
-            unsigned zq;
-            if (BITS == 3) {
-              const int zb = 3 * (r & 31), zw = zb >> 5, zo = zb & 31;
-              const int* zr = qzeros + (long long)g * ldz + (r / 32) * 3;
-              zq = (unsigned)zr[zw] >> zo;
-              if (zo + 3 > 32) zq |= (unsigned)zr[zw + 1] << (32 - zo);
-            } else {
-              constexpr int F = 32 / (BITS == 3 ? 4 : BITS);
-              zq = (unsigned)qzeros[(long long)g * ldz + r / F] >> ((r % F) * BITS);
-            }
-            z = (float)(((zq & MASK) + 1u) & MASK);
-          }
-          unsigned q = v[wi] >> off;
-          if (off + BITS > 32) q |= v[wi + 1 < BITS ? wi + 1 : wi] << (32 - off);
-          h[i] = __float2half_rn(s * ((float)(q & MASK) - z));
+      const int cu = c0 + k8 * 8;
+      int gi[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      bool uniform = cu + 8 <= d;
+      if (g_idx) {
+        if (uniform && wide_idx) {
+          const int4 ga = *reinterpret_cast<const int4*>(g_idx + cu), gb = *reinterpret_cast<const int4*>(g_idx + cu + 4);
+          gi[0] = ga.x; gi[1] = ga.y; gi[2] = ga.z; gi[3] = ga.w; gi[4] = gb.x; gi[5] = gb.y; gi[6] = gb.z; gi[7] = gb.w;
         } else {
-          h[i] = __ushort_as_half(0);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) gi[i] = cu + i < d ? g_idx[cu + i] : 0;
+        }
+#pragma unroll
+        for (int i = 1; i < 8; ++i) uniform = uniform && gi[i] == gi[0];
+      }
+      if (uniform) {
+        load_group(gi[0]);
+        const int first = Field<BITS>::first(k8);
+        const unsigned w2[2] = {v[first], Field<BITS>::WORDS > 1 ? v[first + 1 < BITS ? first + 1 : first] : 0u};
+        const __half2 s2 = __float2half2_rn(s), z2 = __float2half2_rn(1024.f + z);
+        unsigned p[4];                                 // columns (k, k + 4)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const __half2 x = __hmul2(s2, __hsub2(as_half2(Field<BITS>::pair(w2, k8, k) | 0x64006400u), z2));
+          p[k] = *reinterpret_cast<const unsigned*>(&x);
+        }
+        *reinterpret_cast<uint4*>(h) = make_uint4(__byte_perm(p[0], p[1], 0x5410), __byte_perm(p[2], p[3], 0x5410),
+                                                  __byte_perm(p[0], p[1], 0x7632), __byte_perm(p[2], p[3], 0x7632));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int k = k8 * 8 + i, c = c0 + k, bit = k * BITS, wi = bit >> 5, off = bit & 31;
+          if (c < d) {
+            load_group(gi[i]);
+            unsigned q = v[wi] >> off;
+            if (off + BITS > 32) q |= v[wi + 1 < BITS ? wi + 1 : wi] << (32 - off);
+            h[i] = __float2half_rn(s * ((float)(q & MASK) - z));
+          } else {
+            h[i] = __ushort_as_half(0);
+          }
         }
       }
       *reinterpret_cast<uint4*>(tile + lr * DQ_PITCH + lc + k8 * 8) = *reinterpret_cast<const uint4*>(h);
