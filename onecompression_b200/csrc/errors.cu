@@ -18,8 +18,7 @@ void oc_count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxe
 extern "C" long long oc_launch_count(void) { return g_launches.load(); }
 extern "C" long long oc_launch_count_reset(void) { return g_launches.exchange(0); }
 
-// Thin C entry over the fp32 GEMM engine (used by the host layer for the QEP
-// products and by the tests).
+// Thin C entry over the products of fp32 operands as they are (used by the tests).
 extern "C" int oc_gemm_f32(const float* A, long long lda, const float* B, long long ldb, float* C,
                            long long ldc, int M, int N, int K, float alpha, float beta, int transA,
                            int transB, int flags, void* stream) {

@@ -3,10 +3,9 @@
 // (gemm_tc.cu, 3xTF32) unless oc_set_gemm_engine(1) pins this one; this kernel takes every
 // other shape and is the reference the tensor-core engine is tested against.
 //
-// One engine serves every fp32 matrix product of the path: the lazy-batch
-// trailing update of the GPTQ column loop, the trailing update and panel solve
-// of the blocked Cholesky factorisation, the recursive triangular inverse and
-// the three products of the QEP weight correction.  128x128x16 tiles, 256
+// The products of the path - trailing updates of the column loop and of the Cholesky factorisation, the blocked
+// triangular inverse, the weight correction - run on split operands (gemm_split.cu) where workspaces are aligned and
+// blocks have 128 columns; otherwise, and with oc_set_gemm_engine(1), they come here.  128x128x16 tiles, 256
 // threads, 8x8 outputs per thread, register-prefetch double buffering.
 #include "common.cuh"
 

@@ -1,4 +1,5 @@
-// fp32-accurate GEMM on the tensor cores (3xTF32): C = beta*C + alpha*opA(A)*opB(B).
+// fp32-accurate GEMM on the tensor cores (3xTF32) for operands as they are: C = beta*C + alpha*opA(A)*opB(B).  Where the
+// operands can be split once, ahead of the products that read them, gemm_split.cu is twice as fast.
 //
 // Every fp32 operand value a is split into hi = tf32(a) (round to nearest, low 13 mantissa
 // bits zero) and lo = a - hi (exact in fp32); the product a*b is accumulated as
