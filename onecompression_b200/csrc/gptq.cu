@@ -17,8 +17,8 @@
 //                       in CTAs with few rows the other threads apply the updates behind the window
 // The lazy-batch trailing update W[:, i2:] -= Err * U[i1:i2, i2:] is a tensor-core product of operands in two fp16
 // planes each (split.cuh): U is split once per call, the column kernels leave the errors of a block of 128
-// columns split, transposed, every row under a scale of its own.  Other block sizes, unaligned workspaces and the FMA
-// engine take fp32 errors and oc_gemm_f32_launch.  Codes are kept
+// columns split, transposed, every row under a scale of its own.  2 and 3 bits, other block sizes, unaligned
+// workspaces and the FMA engine take fp32 errors and oc_gemm_f32_launch.  Codes are kept
 // transposed ([column][row], 16 bit) until a final pass packs them in original column order.
 #include "split_tc.cuh"
 #include <type_traits>
@@ -1483,8 +1483,12 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   // the same updates, grouped differently in the fp32 sum.
   // A group's parameters are fitted on columns that must carry every earlier update, so the
   // far update may only be postponed when no group reaches across the end of a block group.
-  // Full blocks of 128 columns with something behind them leave their errors split.
-  const bool split = oc_split_engine_on() && blocksize == BLK && d > BLK && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
+  // Full blocks of 128 columns with something behind them leave their errors split.  Not with 2 and 3 bits: sums in another
+  // order move a code where a weight lies next to the middle between two, and there one code is as much as the weight
+  // itself, so these keep the products they have had (tf32 terms, the same codes as before; 4096 x 4096, 3 bits: about
+  // 1.1 ms against 0.7).
+  const bool split = oc_split_engine_on() && wbits >= 4 && blocksize == BLK && d > BLK &&
+                     (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
   const long long nb_u = u_blocks(d), nTab = round4(nb_u * nb_u), nErrP = SUPER * BLK * lde;
   if (split) {
     OcSplitArgs us{};
