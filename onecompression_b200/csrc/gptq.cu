@@ -1485,8 +1485,8 @@ static int gptq_quantize_impl(int batch, const void* W, long long ldw_in, int ou
   // far update may only be postponed when no group reaches across the end of a block group.
   // Full blocks of 128 columns with something behind them leave their errors split.  Not with 2 and 3 bits: sums in another
   // order move a code where a weight lies next to the middle between two, and there one code is as much as the weight
-  // itself, so these keep the products they have had (tf32 terms, the same codes as before; 4096 x 4096, 3 bits: about
-  // 1.1 ms against 0.7).
+  // itself, so these keep the products they have had (tf32 terms, the same codes as before; 4096 x 4096, 3 bits: 1.17
+  // ms against 0.70; dependent launches of those products made it 1.25).
   const bool split = oc_split_engine_on() && wbits >= 4 && blocksize == BLK && d > BLK &&
                      (reinterpret_cast<uintptr_t>(workspace) & 15) == 0;
   const long long nb_u = u_blocks(d), nTab = round4(nb_u * nb_u), nErrP = SUPER * BLK * lde;
